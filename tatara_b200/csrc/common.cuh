@@ -130,6 +130,7 @@ int launch_cast_half(cudaStream_t s, const float* src, void* dst, int64_t n);
 // psv.cu
 int launch_psv_extract(cudaStream_t s, int feature_set, const void* d_psv, long long n, int* stm, int* nstm, int* nnz,
                        int* bucket, float* score, float* wdl);
+void psv_extract_trim();
 bool psv_feature_set_dims(int feature_set, int* ft_in, int* max_active);
 
 // dense_kernels.cu

@@ -3,6 +3,7 @@
 // copy stream).  Mirrors GpuTrainer (bins/nnue_train/src/trainer_layerstack.rs) and SimpleGpuTrainer
 // (bins/nnue_train/src/trainer_simple.rs) at the level of the TrainerBackend trait.
 #include "common.cuh"
+#include "host_mem.cuh"
 #include "peer_exchange.cuh"
 #include "../../include/tatara_b200.h"
 
@@ -846,7 +847,7 @@ void free_all(tb_trainer* t) {
     for (auto& e : t->ev_reduced) if (e) cudaEventDestroy(e);
     if (t->ev_opt_done) cudaEventDestroy(t->ev_opt_done);
     if (t->ev_comm_done) cudaEventDestroy(t->ev_comm_done);
-    if (t->copy_stream) cudaStreamDestroy(t->copy_stream);
+    if (t->copy_stream) { pinned_unwatch_stream(t->copy_stream); cudaStreamDestroy(t->copy_stream); }
     if (t->stream) cudaStreamDestroy(t->stream);
     delete t;
 }
@@ -873,6 +874,7 @@ int create_impl(tb_trainer* t) {
         CU(t, cudaStreamCreateWithPriority(&t->stream, cudaStreamNonBlocking, mid));
     }
     CU(t, cudaStreamCreateWithFlags(&t->copy_stream, cudaStreamNonBlocking));
+    pinned_watch_stream(t->copy_stream);
     const bool ls = c.arch == TB_ARCH_LAYERSTACK;
     const int64_t N = c.ft_in, F = c.ft_out, l1 = c.l1_out, l2 = c.l2_out, nb = c.num_buckets;
     t->p_tf32 = (c.precision & TB_PREC_TF32) != 0;
@@ -1046,6 +1048,13 @@ int create_impl(tb_trainer* t) {
     return TB_OK;
 }
 
+tb_trainer* new_trainer(const tb_config* cfg) {
+    tb_trainer* t = new tb_trainer();
+    t->cfg = *cfg;
+    for (int i = 0; i < PH_COUNT; ++i) { t->ph_start[i] = t->ph_stop[i] = nullptr; t->ph_used[i] = false; t->ph_ms[i] = 0.0; t->ph_launches[i] = 0; }
+    return t;
+}
+
 int validate_config(const tb_config* c) {
     if (!c) return fail(nullptr, TB_ERR_INVALID_ARGUMENT, "config is NULL");
     if (c->struct_size != (int32_t)sizeof(tb_config))
@@ -1103,10 +1112,16 @@ int tb_create(const tb_config* cfg, tb_trainer** out) {
     int n_dev = 0;
     if (cudaGetDeviceCount(&n_dev) != cudaSuccess || n_dev < 1) { cudaGetLastError(); return fail(nullptr, TB_ERR_NO_DEVICE, "no CUDA device is available"); }
     if (cfg->device < 0 || cfg->device >= n_dev) return fail(nullptr, TB_ERR_NO_DEVICE, "device %d out of range (%d devices)", cfg->device, n_dev);
-    tb_trainer* t = new tb_trainer();
-    t->cfg = *cfg;
-    for (int i = 0; i < PH_COUNT; ++i) { t->ph_start[i] = t->ph_stop[i] = nullptr; t->ph_used[i] = false; t->ph_ms[i] = 0.0; t->ph_launches[i] = 0; }
+    tb_trainer* t = new_trainer(cfg);
     rc = create_impl(t);
+    if (rc == TB_ERR_OUT_OF_MEMORY) {  // once more without the buffers that are only kept for later calls
+        free_all(t);
+        cudaGetLastError();
+        psv_extract_trim();
+        pinned_trim();
+        t = new_trainer(cfg);
+        rc = create_impl(t);
+    }
     if (rc != TB_OK) { g_create_error = t->err; free_all(t); return rc; }
     *out = t;
     return TB_OK;
@@ -1451,12 +1466,12 @@ int tb_nccl_unique_id(uint8_t out[128]) {
 
 int tb_host_alloc(void** out, size_t bytes) {
     if (!out) return TB_ERR_INVALID_ARGUMENT;
-    cudaError_t e = cudaHostAlloc(out, bytes ? bytes : 1, cudaHostAllocDefault);
-    if (e != cudaSuccess) { cudaGetLastError(); return fail(nullptr, TB_ERR_OUT_OF_MEMORY, "cudaHostAlloc(%zu): %s", bytes, cudaGetErrorString(e)); }
+    *out = pinned_alloc(bytes ? bytes : 1);
+    if (!*out) return fail(nullptr, TB_ERR_OUT_OF_MEMORY, "no %zu bytes of page-locked memory", bytes);
     return TB_OK;
 }
 int tb_host_free(void* p) {
-    if (p && cudaFreeHost(p) != cudaSuccess) { cudaGetLastError(); return TB_ERR_CUDA; }
+    if (p && !pinned_free(p)) return TB_ERR_CUDA;
     return TB_OK;
 }
 
