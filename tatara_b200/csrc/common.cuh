@@ -63,6 +63,12 @@ struct SmallGroups {
 
 static __device__ __forceinline__ float crelu01(float x) { return x < 0.0f ? 0.0f : (x > 1.0f ? 1.0f : x); }
 
+// SMs of the current device
+static inline int sm_count() {
+    int dev = 0, n = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n;
+}
 static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 static inline int64_t ceil_div64(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
@@ -110,18 +116,22 @@ size_t ft_backward_slice_slab_floats(int n_items, int A, int rows_per_slice, int
 const int* ft_slice_outside_flag(int* fwd_work, int n_items, int N, int rows_per_slice);
 int launch_inverse_slice(cudaStream_t s, const int* item_seg, int* fwd_work, int* bwd_work, int B, int A, int N,
                          int rows_per_slice, int n_persp);
-// the rows of slices [slice_begin, slice_begin + slice_count)
+// the rows of part `part` of `parts` equal ranges of slices: [slices * part / parts, slices * (part + 1) / parts), as planned
+// by launch_step_sorts with the same number of parts
 int launch_ft_backward_slice(cudaStream_t s, const void* dft_stm, const void* dft_nstm, int* fwd_work, int* bwd_work, int B,
-                             int A, int N, int F, int rows_per_slice, int n_persp, int slice_begin, int slice_count, float* grad,
+                             int A, int N, int F, int rows_per_slice, int n_persp, int part, int parts, float* grad,
                              float* slabs, int dft_half = 0);
 int sort_max_units(int max_tiles);
 // The two sorts of a step: positions by bucket -> order, bucket segments seg_start [nb + 2], tiles (room for max_tiles
 // tiles followed by the work units; n_tiles is {tile count, unit count}); items (position, perspective) of both
 // perspectives by the table slice of their features -> items, item_seg [slices + 2].  hist: scratch of
 // (nb + 1) * ceil(B / 1024) + (slices + 1) * ceil(n_persp * B / 1024) ints
+// fwd_work / bwd_work: also plan the slice-resident forward / weight gradient (the latter in bwd_parts launches over equal
+// ranges of slices)
 int launch_step_sorts(cudaStream_t s, const int* bucket /*may be NULL*/, int B, int nb, int* order, TileDesc* tiles, int* n_tiles,
                       int* seg_start, int max_tiles, const int* idx_stm, const int* idx_nstm, const int* nnz, int A, int N,
-                      int rows_per_slice, int n_persp, int* items, int* item_seg, int* hist);
+                      int rows_per_slice, int n_persp, int* items, int* item_seg, int* hist, int* fwd_work = nullptr,
+                      int* bwd_work = nullptr, int bwd_parts = 1);
 int launch_ft_reduce_virtual(cudaStream_t s, float* grad, int N, int pi, int F);
 int launch_ft_fold(cudaStream_t s, const float* w, void* comb, int N, int pi, int F, int half_comb = 0);
 // dst[i] = fp16(src[i]) (cast_f32_to_f16, native_kernels.cu:648), n a multiple of 4

@@ -180,64 +180,42 @@ int launch_ft_forward(cudaStream_t s, int mode, const void* table, const int* id
 // LayerStack strips hold columns [16s, 16s+16) and their pair partners [F/2 + 16s, F/2 + 16s + 16); the other
 // modes 32 adjacent columns.
 // ------------------------------------------------------------------------------------------------
-__global__ void k_fwd_plan(const int* __restrict__ item_seg, int n_keys, int ipc, FwdWork* __restrict__ work, int* __restrict__ n_work) {
-    // n_keys = slices + 1 (the last key collects items without a usable first index)
-    __shared__ int s_base[SORT_KEYS_MAX + 1], s_seg[SORT_KEYS_MAX + 2];
-    for (int k = threadIdx.x; k <= n_keys; k += blockDim.x) s_seg[k] = item_seg[k];  // one round trip, not n_keys
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int k = 0; k < n_keys; ++k) {
-            s_base[k] = run;
-            run += (s_seg[k + 1] - s_seg[k] + ipc - 1) / ipc;
-        }
-        s_base[n_keys] = run;
-        n_work[0] = run;
-        n_work[1] = 0;  // "some item has a row outside its slice", raised by k_fwd_codes
-    }
-    __syncthreads();
-    for (int k = 0; k < n_keys; ++k) {
-        const int b0 = s_seg[k], e0 = s_seg[k + 1];
-        const int n = s_base[k + 1] - s_base[k];
-        // equal runs, a multiple of the 128 items a block handles per round (<= ipc, itself such a multiple)
-        const int size = n > 0 ? ((e0 - b0 + n - 1) / n + 127) & ~127 : 0;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            FwdWork w;
-            w.slice = k;
-            w.begin = min(e0, b0 + i * size);
-            w.end = min(e0, w.begin + size);
-            w.pad = 0;
-            work[s_base[k] + i] = w;
-        }
-    }
-}
-
-// Row codes of the slice-resident forward, one thread per slot of the sorted item list: for every feature slot the
-// row number inside the item's slice (16 bits), SLICE_ZERO_ROW's stand-in rps for a slot without a feature (the strip
+// Row codes of the slice-resident forward, for every slot of the sorted item list: per feature slot the
+// row number inside the item's slice (16 bits), rps for a slot without a feature (the strip
 // keeps a row of zeros there), SLICE_OUTSIDE for a table row outside the slice (the kernel then reads the index list).
 // info[slot] = item | SLICE_SLOW_BIT when the item has an outside row.  Codes of consecutive slots are contiguous
 // (A_pad 16-bit codes each, A_pad a multiple of 8), so a warp copies its round of four items in 16-byte pieces.
+// A thread does eight cells (the lanes of a slot sit in one warp): the kernel is a chain of dependent loads, so what counts
+// is how many of them run side by side (a thread per slot: 8.4 us at 2048 items, 20 at 131 072).
 __global__ void __launch_bounds__(256) k_fwd_codes(const int* __restrict__ idx_stm, const int* __restrict__ idx_nstm,
                                                    const int* __restrict__ nnz, const int* __restrict__ items,
                                                    const int* __restrict__ item_seg, int n_keys, int n_items, int B, int N,
                                                    int A, int A_pad, int rps, uint4* __restrict__ codes,
                                                    int* __restrict__ info, int* __restrict__ outside_flag) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n_items) return;
-    int lo = 0, hi = n_keys - 1;  // the key whose segment holds slot s
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(item_seg + mid) <= s) lo = mid; else hi = mid - 1;
-    }
-    const int row0 = lo * rps;
-    const int rows = max(0, min(rps, N - row0));
-    const int it = __ldg(items + s);
-    const int p = it >= B, b = it - p * B;
-    int n = __ldg(nnz + b);
-    n = n < 0 ? 0 : (n > A ? A : n);
-    const int* ip = (p ? idx_nstm : idx_stm) + (size_t)b * A;
+    __shared__ int s_seg[SORT_KEYS_MAX + 2];
+    for (int k = threadIdx.x; k <= n_keys; k += blockDim.x) s_seg[k] = item_seg[k];
+    __syncthreads();
+    const int per = A_pad >> 3, slots_per_warp = 32 / per;
+    const int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int li = lane / per, part = lane - li * per;
+    const int s = warp * slots_per_warp + li;
+    const bool live = li < slots_per_warp && s < n_items;
     bool outside = false;
-    for (int q0 = 0; q0 < A_pad; q0 += 8) {
+    int it = 0;
+    if (live) {
+        it = __ldg(items + s);
+        int lo = 0, hi = n_keys - 1;  // the key whose segment holds slot s
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (s_seg[mid] <= s) lo = mid; else hi = mid - 1;
+        }
+        const int row0 = lo * rps;
+        const int rows = max(0, min(rps, N - row0));
+        const int p = it >= B, b = it - p * B;
+        int n = __ldg(nnz + b);
+        n = n < 0 ? 0 : (n > A ? A : n);
+        const int* ip = (p ? idx_nstm : idx_stm) + (size_t)b * A;
+        const int q0 = 8 * part;
         unsigned c[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
@@ -255,66 +233,80 @@ __global__ void __launch_bounds__(256) k_fwd_codes(const int* __restrict__ idx_s
         }
         codes[((size_t)s * A_pad + q0) >> 3] = make_uint4(c[0] | (c[1] << 16), c[2] | (c[3] << 16), c[4] | (c[5] << 16), c[6] | (c[7] << 16));
     }
-    info[s] = it | (outside ? SLICE_SLOW_BIT : 0);
-    if (outside) *outside_flag = 1;
+    const unsigned out = __ballot_sync(0xffffffffu, outside) >> (li * per) & ((1u << per) - 1u);
+    if (live && part == 0) {
+        info[s] = it | (out ? SLICE_SLOW_BIT : 0);
+        if (out) *outside_flag = 1;
+    }
 }
 
 // TH: the table holds fp16 rows (the strip is then 64 columns wide: a lane reads 16 bytes = eight columns of every row and
 // sums them in fp32, native_kernels.cu:743-801 sparse_ft_forward_fp16); OH: the pre-activations are stored as fp16 and the
 // activation is computed from the rounded value (sparse_ft_forward_fp16_out + ft_post_perspective_fwd_fp16, :837-863).
+// Persistent: one block per SM takes (run, strip) units from a counter, the runs largest first (k_step_plans).  (Prefetching
+// the next unit's strip into L2 meanwhile cost 1.5 %.)
 template <int MODE, bool TH, bool OH>
 __global__ void __launch_bounds__(1024, 1) k_ft_forward_slice(const void* __restrict__ table_v, const float* __restrict__ bias,
                                                                void* __restrict__ pre_stm_v, void* __restrict__ pre_nstm_v,
                                                                float* __restrict__ combined, const int* __restrict__ idx_stm,
                                                                const int* __restrict__ idx_nstm, const int* __restrict__ info,
                                                                const uint4* __restrict__ codes, const FwdWork* __restrict__ work,
-                                                               const int* __restrict__ n_work, int n_items, int B, int F, int N,
+                                                               int* __restrict__ n_work, int strips, int B, int F, int N,
                                                                int A, int A_pad, int rps, float scale) {
     constexpr int W = TH ? 8 : 4;          // columns per lane
     constexpr int TSZ = TH ? 2 : 4;        // bytes per table element
     constexpr int OSZ = OH ? 2 : 4;        // bytes per stored pre-activation
-    // strip [rps + 1][8 W] elements (128 bytes per row), then two buffers of [32 warps][4 items][A_pad] 16-bit row codes
+    // strip [rps + 1][8 W] elements (128 bytes per row), then two buffers of [warps][4 items][A_pad] 16-bit row codes
     extern __shared__ __align__(16) unsigned char s_raw[];
-    if ((int)blockIdx.x >= *n_work) return;
-    const FwdWork wk = work[blockIdx.x];
-    const int strip = blockIdx.y;
-    const int row0 = wk.slice * rps;
-    const int rows = max(0, min(rps, N - row0));
+    __shared__ int s_unit;
     const int half = F >> 1;
-    const int cA = MODE == 1 ? 4 * W * strip : 8 * W * strip;  // first column of the strip's first half (or of all its columns)
-    const int cB = MODE == 1 ? half + 4 * W * strip : cA + 4 * W;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 3, j = lane & 7;
-    const int mycol = j < 4 ? cA + W * j : cB + W * (j - 4);
     const unsigned char* __restrict__ table = static_cast<const unsigned char*>(table_v);
+    const int n_units = n_work[0] * strips;
+    // a round = four items per warp; their codes arrive by asynchronous copy one round ahead
+    const int code_bytes = 4 * A_pad * 2;  // per warp and buffer
+    const int buf_stride = (blockDim.x >> 5) * code_bytes;
+    unsigned char* s_codes = s_raw + ((size_t)rps + 1) * 128 + (size_t)warp * code_bytes;
+    const unsigned char* codes_b = reinterpret_cast<const unsigned char*>(codes);
+    const int chunk_item = (lane * 16) / (A_pad * 2);  // which of the four items this lane's 16-byte piece belongs to
+    const int per_round = 4 * (blockDim.x >> 5);
+    const unsigned char* s_lane = s_raw + 16 * j;
+    if (threadIdx.x < 32) reinterpret_cast<float*>(s_raw)[rps * 32 + threadIdx.x] = 0.f;  // the row of zeros
+    auto first_col = [&](int strip, int jj) {  // of the lanes with column index jj
+        return MODE == 1 ? (jj < 4 ? 4 * W * strip + W * jj : half + 4 * W * strip + W * (jj - 4)) : 8 * W * strip + W * jj;
+    };
+
+    // the first units go by block number (the counter starts behind them)
+    for (int unit = blockIdx.x; unit < n_units;) {
+    const FwdWork wk = work[unit / strips];
+    const int strip = unit % strips;
+    const int row0 = wk.slice * rps;
+    const int rows = max(0, min(rps, N - row0));
+    const int mycol = first_col(strip, j);
 
     // strip fill: thread e & 7 == j copies the 16 bytes it will later read, for rows e >> 3
     for (int e = threadIdx.x; e < rows * 8; e += blockDim.x)
         cp_async16(s_raw + (size_t)e * 16, table + ((size_t)(row0 + (e >> 3)) * F + mycol) * TSZ, 16);
-    if (threadIdx.x < 32) reinterpret_cast<float*>(s_raw)[rps * 32 + threadIdx.x] = 0.f;  // the row of zeros
+    cp_async_commit();
+    if (threadIdx.x == 0) s_unit = (int)gridDim.x + atomicAdd(n_work + 2, 1);
     for (int e = rows * 8 + threadIdx.x; e < rps * 8; e += blockDim.x)  // rows past the end of the table
         *reinterpret_cast<float4*>(s_raw + (size_t)e * 16) = make_float4(0.f, 0.f, 0.f, 0.f);
-
-    // a round = four items per warp; their codes arrive by asynchronous copy one round ahead
-    const int code_bytes = 4 * A_pad * 2;  // per warp and buffer
-    unsigned char* s_codes = s_raw + ((size_t)rps + 1) * 128 + (size_t)warp * code_bytes;
-    const int buf_stride = 32 * code_bytes;
-    const unsigned char* codes_b = reinterpret_cast<const unsigned char*>(codes);
-    const int chunk_item = (lane * 16) / (A_pad * 2);  // which of the four items this lane's 16-byte piece belongs to
-    auto fetch_codes = [&](int slot, int buf) {
+    auto fetch_codes = [&](int slot, int bf) {
         if (lane * 16 < code_bytes) {
-            // pieces of slots past the end of the run are filled with zeros (row 0): whatever lies there is never a
-            // valid offset into this block's strip
             const bool ok = slot + chunk_item < wk.end;
             const long long off = (long long)slot * A_pad * 2 + lane * 16;
-            cp_async16(s_codes + buf * buf_stride + lane * 16, codes_b + (ok ? off : 0), ok ? 16 : 0);
+            cp_async16(s_codes + bf * buf_stride + lane * 16, codes_b + (ok ? off : 0), ok ? 16 : 0);
         }
     };
-    const int per_round = 4 * (blockDim.x >> 5);
+    int buf = 0;
     fetch_codes(wk.begin + 4 * warp, 0);
     cp_async_commit();
+    auto fetch_info = [&](int slot) { return slot < wk.end ? __ldg(info + slot) : -1; };
+    int info_reg = fetch_info(wk.begin + 4 * warp + g);
     cp_async_wait<0>();
     __syncthreads();
+    const int next_unit = s_unit;
 
     // fp32 lanes keep the bias of their four columns and of the pair partner's in registers; fp16 lanes (eight columns)
     // read it in the epilogue instead (L1 hits), their registers are taken by the wider running sums
@@ -323,19 +315,18 @@ __global__ void __launch_bounds__(1024, 1) k_ft_forward_slice(const void* __rest
     float4 pbias = mybias;  // the pair partner's bias (LayerStack)
     pbias.x = __shfl_xor_sync(0xffffffffu, mybias.x, 4); pbias.y = __shfl_xor_sync(0xffffffffu, mybias.y, 4);
     pbias.z = __shfl_xor_sync(0xffffffffu, mybias.z, 4); pbias.w = __shfl_xor_sync(0xffffffffu, mybias.w, 4);
-    const unsigned char* s_lane = s_raw + 16 * j;
 
-    int buf = 0;
-    for (int base = wk.begin; base < wk.end; base += per_round, buf ^= 1) {
-        const int slot = base + 4 * warp + g;
-        const int inf = slot < wk.end ? __ldg(info + slot) : -1;
-        fetch_codes(base + per_round + 4 * warp, buf ^ 1);  // the other buffer was last read a round ago (warp barrier below)
+    for (int base = wk.begin; base < wk.end; base += per_round) {
+        const int inf = info_reg;
+        fetch_codes(base + per_round + 4 * warp, buf ^ 1);
         cp_async_commit();
         cp_async_wait<1>();
         __syncwarp();
+        info_reg = fetch_info(base + per_round + 4 * warp + g);
         const bool slow = __any_sync(0xffffffffu, inf >= 0 && (inf & SLICE_SLOW_BIT));
         const int it_c = inf < 0 ? -1 : (inf & ~SLICE_SLOW_BIT);
         const unsigned char* my_codes = s_codes + buf * buf_stride + g * A_pad * 2;
+        buf ^= 1;
 
         LaneAcc<TH> acc;
         acc.zero();
@@ -367,7 +358,7 @@ __global__ void __launch_bounds__(1024, 1) k_ft_forward_slice(const void* __rest
                 acc.add(v);
             }
         }
-        __syncwarp();  // all lanes are done with this round's codes before the next round overwrites the other buffer's twin
+        __syncwarp();  // all lanes are done with this round's codes before the next round's replace them
 
         // ---- epilogue: x[] = the lane's sums as the later kernels will read them (rounded to fp16 when stored so)
         float x[W];
@@ -439,7 +430,10 @@ __global__ void __launch_bounds__(1024, 1) k_ft_forward_slice(const void* __rest
             for (int i = 0; i < W; i += 4) __stcs(dst + i / 4, make_float4(a[i], a[i + 1], a[i + 2], a[i + 3]));
         }
     }
-    cp_async_wait<0>();  // nothing of this block is in flight when it leaves
+    cp_async_wait<0>();
+    __syncthreads();  // the strip has been read by all, s_unit too
+    unit = next_unit;
+    }
 }
 
 
@@ -448,11 +442,18 @@ size_t ft_forward_slice_work_ints(int n_items, int n_keys, int A) {
     return 4 * slice_max_work(n_items, n_keys) + 4 + ((size_t)n_items + 3) / 4 * 4 + ((size_t)n_items * slice_a_pad(A) + 1) / 2 + 4;
 }
 
-static inline size_t slice_smem_bytes(int rps, int A) { return ((size_t)rps + 1) * 128 + (size_t)2 * 32 * 4 * slice_a_pad(A) * 2; }
+// Warps of a block: 32, or what the shared memory beside the strip has room for (the sets of 1710 rows leave room for the
+// codes of 20: the shared-memory pipe, not the number of warps, sets the pace).  0: the strip does not fit.
+static inline int slice_warps(int rps, int A) {
+    const long long room = 227 * 1024 - 1024 - ((long long)rps + 1) * 128, per_warp = 2 * 4 * slice_a_pad(A) * 2;
+    const long long w = room / per_warp;
+    return w < 12 ? 0 : w > 32 ? 32 : (int)w;
+}
+static inline size_t slice_smem_bytes(int rps, int A) { return ((size_t)rps + 1) * 128 + (size_t)slice_warps(rps, A) * 2 * 4 * slice_a_pad(A) * 2; }
 
 bool ft_forward_slice_supported(int F, int N, int A, int rps) {
     int n_slices = ceil_div(N, rps);
-    return F % 128 == 0 && A <= 64 && rps < 0xFFFF && slice_smem_bytes(rps, A) <= 227 * 1024 && n_slices + 1 <= SORT_KEYS_MAX;
+    return F % 128 == 0 && A <= 64 && rps < 0xFFFF && slice_warps(rps, A) > 0 && n_slices + 1 <= SORT_KEYS_MAX;
 }
 
 int launch_ft_forward_slice(cudaStream_t s, int mode, const void* table, const int* idx_stm, const int* idx_nstm,
@@ -462,23 +463,22 @@ int launch_ft_forward_slice(cudaStream_t s, int mode, const void* table, const i
     if (B <= 0) return 0;
     const int n_items = n_persp * B;
     const int n_slices = ceil_div(N, rps), n_keys = n_slices + 1;
-    const int max_work = (int)slice_max_work(n_items, n_keys);
     const int A_pad = slice_a_pad(A);
     const SliceBuffers sb = slice_buffers(work, n_items, n_keys);
     FwdWork* wk = sb.work;
     int* n_work = sb.n_work;
     int* info = sb.info;
     uint4* codes = sb.codes;
-    k_fwd_plan<<<1, 128, 0, s>>>(item_seg, n_keys, SLICE_IPC, wk, n_work);
-    k_fwd_codes<<<ceil_div(n_items, 256), 256, 0, s>>>(idx_stm, idx_nstm, nnz, items, item_seg, n_keys, n_items, B, N, A, A_pad,
+    const int slots_per_block = 8 * (32 / (A_pad / 8));
+    k_fwd_codes<<<ceil_div(n_items, slots_per_block), 256, 0, s>>>(idx_stm, idx_nstm, nnz, items, item_seg, n_keys, n_items, B, N, A, A_pad,
                                                        rps, codes, info, sb.outside_flag);
     const size_t smem = slice_smem_bytes(rps, A);
-    dim3 grid(max_work, table_half ? F / 64 : F / 32);
+    const int strips = table_half ? F / 64 : F / 32, grid = sm_count(), threads = 32 * slice_warps(rps, A);
 #define FT_SLICE_LAUNCH(M, TH, OH)                                                                                       \
     do {                                                                                                                 \
         cudaFuncSetAttribute(k_ft_forward_slice<M, TH, OH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
-        k_ft_forward_slice<M, TH, OH><<<grid, 1024, smem, s>>>(table, bias, pre_stm, pre_nstm, combined, idx_stm, idx_nstm, \
-                                                               info, codes, wk, n_work, n_items, B, F, N, A, A_pad, rps, \
+        k_ft_forward_slice<M, TH, OH><<<grid, threads, smem, s>>>(table, bias, pre_stm, pre_nstm, combined, idx_stm, idx_nstm, \
+                                                               info, codes, wk, n_work, strips, B, F, N, A, A_pad, rps, \
                                                                scale);                                                   \
     } while (0)
     if (table_half) {  // fp16 table: the raw gather (mode 0) and the LayerStack activation, with fp32 or fp16 pre-activations
@@ -496,7 +496,7 @@ int launch_ft_forward_slice(cudaStream_t s, int mode, const void* table, const i
         }
     }
 #undef FT_SLICE_LAUNCH
-    return 3;
+    return 2;
 }
 
 // ------------------------------------------------------------------------------------------------

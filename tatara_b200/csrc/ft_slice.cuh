@@ -19,7 +19,7 @@ static inline size_t slice_max_work(int n_items, int n_keys) { return (size_t)n_
 // layout of the forward's work buffer (ft_forward_slice_work_ints): the weight-gradient kernels read info and codes
 struct SliceBuffers {
     FwdWork* work;
-    int* n_work;        // [0] number of records
+    int* n_work;        // [0] number of records, [2] units taken so far
     int* outside_flag;  // 1 when some item has a row outside its slice
     int* info;          // [n_items] item of every slot (| SLICE_SLOW_BIT)
     uint4* codes;       // [n_items][A_pad] 16-bit row codes
@@ -33,6 +33,75 @@ static inline SliceBuffers slice_buffers(int* work, int n_items, int n_keys) {
     b.info = b.n_work + 4;                                                             // 16-byte aligned
     b.codes = reinterpret_cast<uint4*>(b.info + ((size_t)n_items + 3) / 4 * 4);        // 16-byte aligned
     return b;
+}
+
+// ---- weight gradient: chunks, groups, inverse index -------------------------------------------------------------------
+#define INV_SORT_N 2048  // rows per slice limit (bitonic sort size)
+#define BWD_GROUP 4      // chunks per block: a slice of more chunks is shared by several blocks
+#define BWD_PARTS 8      // limit of the parts a launch may be cut into (data parallel)
+
+struct BwdLayout {
+    int CH;             // slots per chunk (multiple of 8)
+    int rps_pad;        // row records per chunk
+    int region;         // 16-bit list cells per chunk (every list is padded to a multiple of 8 cells: 16-byte code loads)
+    int max_chunks;
+    int max_groups, max_slabs;  // (slice, chunk group) work units; partial slabs of the groups behind a slice's first
+    size_t off_len, off_groups, off_sched, off_rowinfo, off_lists, total_ints;
+};
+
+static inline size_t bwd_region(int CH, int rps, int A_pad) { return (size_t)CH * A_pad + 8 * (size_t)rps; }
+
+static inline size_t bwd_smem_bytes(int CH, int rps, int A_pad) {
+    const int rps_pad = (rps + 3) / 4 * 4;
+    return ((size_t)CH + 1) * 128 + (size_t)rps_pad * 8 + bwd_region(CH, rps, A_pad) * 2;
+}
+
+static inline BwdLayout bwd_layout(int n_items, int A, int rps) {
+    BwdLayout L;
+    const int A_pad = slice_a_pad(A);
+    int CH = 0;
+    for (int c = 32; c <= 4096; c += 8) {
+        if (bwd_smem_bytes(c, rps, A_pad) + 2048 > 227 * 1024) break;  // 2 KB stay free for the kernels' static arrays
+        if (bwd_region(c, rps, A_pad) > 65535) break;
+        // k_inv_chunk: histograms, offsets and sort keys, the chunk's lists
+        if ((size_t)64 * ((rps + 1) & ~1) + (size_t)INV_SORT_N * 8 + bwd_region(c, rps, A_pad) * 2 + 2048 > 227 * 1024) break;
+        CH = c;
+    }
+    L.CH = CH;
+    L.rps_pad = (rps + 3) / 4 * 4;
+    L.region = (int)bwd_region(CH, rps, A_pad);
+    L.max_chunks = CH > 0 ? n_items / CH + SORT_KEYS_LIMIT + 2 : 0;
+    L.max_slabs = CH > 0 ? n_items / (CH * BWD_GROUP) + SORT_KEYS_LIMIT / BWD_GROUP + 2 : 0;
+    L.max_groups = SORT_KEYS_LIMIT + L.max_slabs;
+    size_t o = 4 * (size_t)L.max_chunks + 4;            // chunk records + their count
+    L.off_len = o; o += 4 * (size_t)L.max_chunks;  // per chunk {list cells, long-list records, non-empty records, 0}
+    // groups: [0] their count, [4 ..] first group of every slice (+ end), then {slice, first chunk, end chunk, slab or -1}
+    L.off_groups = o; o += 4 + (SORT_KEYS_LIMIT + 4) + 4 * (size_t)L.max_groups;
+    // schedule: [0 ..] units taken of every part, [BWD_PARTS ..] first position of every part (+ end), then the groups in the
+    // order the blocks take them
+    L.off_sched = o; o += 2 * BWD_PARTS + 4 + (size_t)(L.max_groups + 3) / 4 * 4;
+    L.off_rowinfo = o; o += 2 * (size_t)L.max_chunks * L.rps_pad;
+    L.off_lists = o; o += ((size_t)L.max_chunks * L.region + 1) / 2 + 4;
+    L.total_ints = o;
+    return L;
+}
+
+struct BwdPointers {
+    FwdWork* chunks;
+    int *n_chunks, *len, *groups, *sched;
+    unsigned long long* rowinfo;
+    unsigned short* lists;
+};
+static inline BwdPointers bwd_pointers(int* bwd_work, const BwdLayout& L) {
+    BwdPointers p;
+    p.chunks = reinterpret_cast<FwdWork*>(bwd_work);
+    p.n_chunks = bwd_work + 4 * (size_t)L.max_chunks;
+    p.len = bwd_work + L.off_len;
+    p.groups = bwd_work + L.off_groups;
+    p.sched = bwd_work + L.off_sched;
+    p.rowinfo = reinterpret_cast<unsigned long long*>(bwd_work + L.off_rowinfo);
+    p.lists = reinterpret_cast<unsigned short*>(bwd_work + L.off_lists);
+    return p;
 }
 
 #ifdef __CUDACC__
@@ -128,6 +197,7 @@ static __device__ __forceinline__ void cp_async16(void* dst_shared, const void* 
                  "r"(src_bytes)
                  : "memory");
 }
+static __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 static __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N_PENDING>
 static __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N_PENDING) : "memory"); }

@@ -25,54 +25,8 @@
 // kernels, gated the other way round, then do the work.
 #include "ft_slice.cuh"
 
-#define INV_SORT_N 2048  // rows per slice limit (bitonic sort size)
 #define BWD_HOT 256      // list length from which a list is summed as four quarters by the four groups of one warp
 #define BWD_DESC 64      // chunk descriptors a block stages in shared memory
-#define BWD_GROUP 4      // chunks per block: a slice of more chunks is shared by several blocks
-
-struct BwdLayout {
-    int CH;             // slots per chunk (multiple of 8)
-    int rps_pad;        // row records per chunk
-    int region;         // 16-bit list cells per chunk (every list is padded to a multiple of 8 cells: 16-byte code loads)
-    int max_chunks;
-    int max_groups, max_slabs;  // (slice, chunk group) work units; partial slabs of the groups behind a slice's first
-    size_t off_first, off_len, off_groups, off_rowinfo, off_lists, total_ints;
-};
-
-static inline size_t bwd_region(int CH, int rps, int A_pad) { return (size_t)CH * A_pad + 8 * (size_t)rps; }
-
-static inline size_t bwd_smem_bytes(int CH, int rps, int A_pad) {
-    const int rps_pad = (rps + 3) / 4 * 4;
-    return ((size_t)CH + 1) * 128 + (size_t)rps_pad * 8 + bwd_region(CH, rps, A_pad) * 2;
-}
-
-static inline BwdLayout bwd_layout(int n_items, int A, int rps) {
-    BwdLayout L;
-    const int A_pad = slice_a_pad(A);
-    int CH = 0;
-    for (int c = 32; c <= 4096; c += 8) {
-        if (bwd_smem_bytes(c, rps, A_pad) + 2048 > 227 * 1024) break;  // 2 KB stay free for the kernels' static arrays
-        if (bwd_region(c, rps, A_pad) > 65535) break;
-        // k_inv_chunk: histograms, offsets and sort keys, the chunk's lists
-        if ((size_t)64 * ((rps + 1) & ~1) + (size_t)INV_SORT_N * 8 + bwd_region(c, rps, A_pad) * 2 + 2048 > 227 * 1024) break;
-        CH = c;
-    }
-    L.CH = CH;
-    L.rps_pad = (rps + 3) / 4 * 4;
-    L.region = (int)bwd_region(CH, rps, A_pad);
-    L.max_chunks = CH > 0 ? n_items / CH + SORT_KEYS_LIMIT + 2 : 0;
-    L.max_slabs = CH > 0 ? n_items / (CH * BWD_GROUP) + SORT_KEYS_LIMIT / BWD_GROUP + 2 : 0;
-    L.max_groups = SORT_KEYS_LIMIT + L.max_slabs;
-    size_t o = 4 * (size_t)L.max_chunks + 4;            // chunk records + their count
-    L.off_first = o; o += SORT_KEYS_LIMIT + 4;          // first chunk of every slice (+ end)
-    L.off_len = o; o += 4 * (size_t)L.max_chunks;  // per chunk {list cells, long-list records, non-empty records, 0}
-    // groups: [0] their count, [4 ..] first group of every slice (+ end), then {slice, first chunk, end chunk, slab or -1}
-    L.off_groups = o; o += 4 + (SORT_KEYS_LIMIT + 4) + 4 * (size_t)L.max_groups;
-    L.off_rowinfo = o; o += 2 * (size_t)L.max_chunks * L.rps_pad;
-    L.off_lists = o; o += ((size_t)L.max_chunks * L.region + 1) / 2 + 4;
-    L.total_ints = o;
-    return L;
-}
 
 bool ft_backward_slice_supported(int F, int N, int A, int rps) {
     const int n_slices = ceil_div(N, rps);
@@ -85,50 +39,6 @@ size_t ft_backward_slice_slab_floats(int n_items, int A, int rps, int F) {
     return (size_t)bwd_layout(n_items, A, rps).max_slabs * (size_t)rps * (size_t)F;
 }
 
-// chunks of <= ipc consecutive slots of one slice; first[k] = index of slice k's first chunk, first[n_keys] = total
-__global__ void k_chunk_plan(const int* __restrict__ item_seg, int n_keys, int ipc, FwdWork* __restrict__ work,
-                             int* __restrict__ n_work, int* __restrict__ first, int* __restrict__ groups, int max_groups) {
-    __shared__ int s_base[SORT_KEYS_LIMIT + 1], s_seg[SORT_KEYS_LIMIT + 2];
-    for (int k = threadIdx.x; k <= n_keys; k += blockDim.x) s_seg[k] = item_seg[k];  // one round trip, not n_keys
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int k = 0; k < n_keys; ++k) {
-            s_base[k] = run;
-            run += (s_seg[k + 1] - s_seg[k] + ipc - 1) / ipc;
-        }
-        s_base[n_keys] = run;
-        *n_work = run;
-        // (slice, chunk group) work units of the real slices (the last key holds items without a slice: they have no rows)
-        int* group_first = groups + 4;
-        int4* rec = reinterpret_cast<int4*>(groups + 4 + SORT_KEYS_LIMIT + 4);
-        int gi = 0, slab = 0;
-        for (int k = 0; k < n_keys - 1; ++k) {
-            group_first[k] = gi;
-            const int c0 = s_base[k], nc = s_base[k + 1] - c0;
-            if (nc == 0 && gi < max_groups) rec[gi++] = make_int4(k, c0, c0, -1);  // an empty slice: its rows are zeroed
-            for (int c = 0; c < nc && gi < max_groups; c += BWD_GROUP) rec[gi++] = make_int4(k, c0 + c, c0 + min(nc, c + BWD_GROUP), c == 0 ? -1 : slab++);
-        }
-        group_first[n_keys - 1] = gi;
-        groups[0] = gi;
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k <= n_keys; k += blockDim.x) first[k] = s_base[k];
-    for (int k = 0; k < n_keys; ++k) {
-        const int b0 = s_seg[k], e0 = s_seg[k + 1];
-        const int n = s_base[k + 1] - s_base[k];
-        const int size = n > 0 ? ((e0 - b0 + n - 1) / n + 7) & ~7 : 0;  // equal chunks (<= ipc: ipc is a multiple of 8)
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            FwdWork w;
-            w.slice = k;
-            w.begin = min(e0, b0 + i * size);
-            w.end = min(e0, w.begin + size);
-            w.pad = 0;
-            work[s_base[k] + i] = w;
-        }
-    }
-}
-
 // Inverse index of one chunk.  Shared memory: hist [32 warps][rps_h] 16-bit cells, rowoff [rps] ints, sort keys
 // [INV_SORT_N] ints, the chunk's lists [region] 16-bit cells (copied out at the end in 16-byte pieces).  Warp w owns
 // a contiguous range of the chunk's slots and walks it slot by slot, so "warp, then slot" is ascending slot order.
@@ -139,8 +49,9 @@ __global__ void __launch_bounds__(1024) k_inv_chunk(const unsigned short* __rest
                                                     const int* __restrict__ n_work, const int* __restrict__ outside_flag,
                                                     int n_slices, int A_pad, int rps, int rps_pad, int CH, int region,
                                                     unsigned short* __restrict__ lists, unsigned long long* __restrict__ rowinfo,
-                                                    int* __restrict__ len) {
+                                                    int* __restrict__ len, int* __restrict__ sched) {
     extern __shared__ __align__(16) unsigned char s_raw[];
+    if (blockIdx.x == 0 && threadIdx.x < BWD_PARTS) sched[threadIdx.x] = 0;  // units taken by the gradient's blocks
     if ((int)blockIdx.x >= *n_work || *outside_flag) return;
     const FwdWork wk = work[blockIdx.x];
     if (wk.slice >= n_slices) return;  // items without a slice have no rows
@@ -303,11 +214,12 @@ __global__ void __launch_bounds__(1024) k_inv_chunk(const unsigned short* __rest
 template <bool DH>
 __global__ void __launch_bounds__(1024, 1) k_ft_backward_slice(const void* __restrict__ dft_stm, const void* __restrict__ dft_nstm,
                                                                 const int* __restrict__ info, const FwdWork* __restrict__ work,
-                                                                const int* __restrict__ groups, const int* __restrict__ len,
+                                                                const int* __restrict__ groups, int* __restrict__ sched,
+                                                                const int* __restrict__ len,
                                                                 const unsigned long long* __restrict__ rowinfo,
                                                                 const unsigned short* __restrict__ lists,
                                                                 const int* __restrict__ outside_flag, int B, int F, int N, int rps,
-                                                                int rps_pad, int CH, int region, int slice_begin, int slice_count,
+                                                                int rps_pad, int CH, int region, int part, int strips,
                                                                 float* __restrict__ grad, float* __restrict__ slabs) {
     constexpr int W = DH ? 8 : 4;    // columns per lane
     constexpr int DSZ = DH ? 2 : 4;  // bytes per dft element
@@ -318,19 +230,24 @@ __global__ void __launch_bounds__(1024, 1) k_ft_backward_slice(const void* __res
     __shared__ int s_ctl[4];
     __shared__ int s_desc[BWD_DESC][5];
     if (*outside_flag) return;
-    // the groups of this launch's slices; the grid has a block row per slice, so a block takes a second group only when
-    // some slice is shared (skewed data)
+    // Persistent: one block per SM takes (group, strip) units of this launch's part from a counter, the groups largest first
+    // (k_step_plans).
     // (the loop's state lives in shared memory: the body needs every register)
-    __shared__ int s_gid;
-    if (threadIdx.x == 0) s_gid = groups[4 + slice_begin] + (int)blockIdx.x;
+    __shared__ int s_unit, s_next;
+    if (threadIdx.x == 0) s_next = (int)blockIdx.x;  // the first units go by block number, the counter starts behind them
     for (;;) {
-    __syncthreads();  // s_gid written; the previous group's last reads of the shared buffers
-    const int gid = s_gid;
-    if (gid >= groups[4 + slice_begin + slice_count]) break;
-    __syncthreads();  // every thread has read s_gid
-    if (threadIdx.x == 0) s_gid = gid + (int)gridDim.x;
+    __syncthreads();  // s_next written; the previous group's last reads of the shared buffers
+    if (threadIdx.x == 0) s_unit = s_next;
+    __syncthreads();
+    const int unit = s_unit;
+    {
+        const int first = sched[BWD_PARTS + part], count = sched[BWD_PARTS + part + 1] - first;
+        if (unit >= count * strips) break;
+        if (threadIdx.x == 0) s_next = (int)gridDim.x + atomicAdd(sched + part, 1);
+    }
+    const int gid = sched[2 * BWD_PARTS + 4 + sched[BWD_PARTS + part] + unit / strips];
     const int4 gr = reinterpret_cast<const int4*>(groups + 4 + SORT_KEYS_LIMIT + 4)[gid];
-    const int k = gr.x, strip = blockIdx.y;
+    const int k = gr.x, strip = unit % strips;
     const int row0 = k * rps;
     const int rows = min(rps, N - row0);
     const int tid = threadIdx.x, lane = tid & 31;
@@ -536,24 +453,6 @@ __global__ void __launch_bounds__(256) k_bwd_combine(const int* __restrict__ gro
     }
 }
 
-struct BwdPointers {
-    FwdWork* chunks;
-    int *n_chunks, *first, *len, *groups;
-    unsigned long long* rowinfo;
-    unsigned short* lists;
-};
-static inline BwdPointers bwd_pointers(int* bwd_work, const BwdLayout& L) {
-    BwdPointers p;
-    p.chunks = reinterpret_cast<FwdWork*>(bwd_work);
-    p.n_chunks = bwd_work + 4 * (size_t)L.max_chunks;
-    p.first = bwd_work + L.off_first;
-    p.len = bwd_work + L.off_len;
-    p.groups = bwd_work + L.off_groups;
-    p.rowinfo = reinterpret_cast<unsigned long long*>(bwd_work + L.off_rowinfo);
-    p.lists = reinterpret_cast<unsigned short*>(bwd_work + L.off_lists);
-    return p;
-}
-
 const int* ft_slice_outside_flag(int* fwd_work, int n_items, int N, int rps) {
     return slice_buffers(fwd_work, n_items, ceil_div(N, rps) + 1).outside_flag;
 }
@@ -567,18 +466,17 @@ int launch_inverse_slice(cudaStream_t s, const int* item_seg, int* fwd_work, int
     const SliceBuffers sb = slice_buffers(fwd_work, n_items, n_keys);
     const BwdLayout L = bwd_layout(n_items, A, rps);
     const BwdPointers P = bwd_pointers(bwd_work, L);
-    k_chunk_plan<<<1, 128, 0, s>>>(item_seg, n_keys, L.CH, P.chunks, P.n_chunks, P.first, P.groups, L.max_groups);
     const int rps_h = (rps + 1) & ~1;
     const size_t inv_smem = (size_t)32 * rps_h * 2 + (size_t)INV_SORT_N * 4 * 2 + (size_t)L.region * 2;
     cudaFuncSetAttribute(k_inv_chunk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)inv_smem);
     k_inv_chunk<<<L.max_chunks, 1024, inv_smem, s>>>(reinterpret_cast<const unsigned short*>(sb.codes), P.chunks, P.n_chunks,
                                                      sb.outside_flag, n_slices, A_pad, rps, L.rps_pad, L.CH, L.region, P.lists,
-                                                     P.rowinfo, P.len);
-    return 2;
+                                                     P.rowinfo, P.len, P.sched);
+    return 1;
 }
 
 int launch_ft_backward_slice(cudaStream_t s, const void* dft_stm, const void* dft_nstm, int* fwd_work, int* bwd_work, int B,
-                             int A, int N, int F, int rps, int n_persp, int slice_begin, int slice_count, float* grad, float* slabs,
+                             int A, int N, int F, int rps, int n_persp, int part, int parts, float* grad, float* slabs,
                              int dft_half) {
     if (B <= 0) return 0;
     const int n_items = n_persp * B;
@@ -588,22 +486,18 @@ int launch_ft_backward_slice(cudaStream_t s, const void* dft_stm, const void* df
     const BwdLayout L = bwd_layout(n_items, A, rps);
     const BwdPointers P = bwd_pointers(bwd_work, L);
     const size_t smem = bwd_smem_bytes(L.CH, rps, A_pad);
-    if (slice_begin < 0 || slice_count <= 0 || slice_begin + slice_count > n_slices) return 0;
-    const int grid_x = slice_count;  // a block row per slice; rows take the extra groups of shared slices in turn
-    if (dft_half) {
-        cudaFuncSetAttribute(k_ft_backward_slice<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_ft_backward_slice<true><<<dim3(grid_x, F / 64), 1024, smem, s>>>(dft_stm, dft_nstm, sb.info, P.chunks, P.groups, P.len,
-                                                                                 P.rowinfo, P.lists, sb.outside_flag, B, F, N, rps,
-                                                                                 L.rps_pad, L.CH, L.region, slice_begin, slice_count, grad,
-                                                                                 slabs);
-    } else {
-        cudaFuncSetAttribute(k_ft_backward_slice<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_ft_backward_slice<false><<<dim3(grid_x, F / 32), 1024, smem, s>>>(dft_stm, dft_nstm, sb.info, P.chunks, P.groups, P.len,
-                                                                                  P.rowinfo, P.lists, sb.outside_flag, B, F, N, rps,
-                                                                                  L.rps_pad, L.CH, L.region, slice_begin, slice_count, grad,
-                                                                                  slabs);
-    }
-    k_bwd_combine<<<dim3(148, slice_count), 256, 0, s>>>(P.groups, sb.outside_flag, reinterpret_cast<const float4*>(slabs),
-                                                         reinterpret_cast<float4*>(grad), rps, F, N, slice_begin);
+    const int grid = sm_count();
+#define FT_BWD_LAUNCH(DH)                                                                                                      \
+    do {                                                                                                                       \
+        cudaFuncSetAttribute(k_ft_backward_slice<DH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                 \
+        k_ft_backward_slice<DH><<<grid, 1024, smem, s>>>(dft_stm, dft_nstm, sb.info, P.chunks, P.groups, P.sched, P.len,       \
+                                                         P.rowinfo, P.lists, sb.outside_flag, B, F, N, rps, L.rps_pad, L.CH,   \
+                                                         L.region, part, DH ? F / 64 : F / 32, grad, slabs);                   \
+    } while (0)
+    if (dft_half) FT_BWD_LAUNCH(true); else FT_BWD_LAUNCH(false);
+#undef FT_BWD_LAUNCH
+    const int k0 = (int)((int64_t)n_slices * part / parts), k1 = (int)((int64_t)n_slices * (part + 1) / parts);
+    k_bwd_combine<<<dim3(148, k1 - k0), 256, 0, s>>>(P.groups, sb.outside_flag, reinterpret_cast<const float4*>(slabs),
+                                                     reinterpret_cast<float4*>(grad), rps, F, N, k0);
     return 2;
 }

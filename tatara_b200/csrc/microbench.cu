@@ -119,7 +119,7 @@ extern "C" int tb_ft_microbench(int device, const int32_t* indices, const int32_
         k_fill_pattern<<<148 * 8, 256>>>(d_table, N * F, 0.05f, 1u);
         MB(tm.run(iters, [&] {
             launch_step_sorts(0, nullptr, batch, 0, d_order, d_tiles, d_ntiles, d_seg, max_tiles, d_idx, d_idx, d_nnz, max_active, ft_in, rps, 1,
-                              d_items, d_itemseg, d_hist);
+                              d_items, d_itemseg, d_hist, d_fwd_work, d_bwd_work);
             launch_ft_forward_slice(0, 0, d_table, d_idx, d_idx, d_nnz, nullptr, d_x, d_x, nullptr, d_items, d_itemseg, d_fwd_work, batch,
                                     ft_out, ft_in, max_active, rps, 1.f, 1);
         }));
@@ -130,7 +130,7 @@ extern "C" int tb_ft_microbench(int device, const int32_t* indices, const int32_
             k_fill_pattern<<<148 * 8, 256>>>(d_x, B * F, 1e-3f, 3u);
             MB(tm.run(iters, [&] {
                 launch_inverse_slice(0, d_itemseg, d_fwd_work, d_bwd_work, batch, max_active, ft_in, rps, 1);
-                launch_ft_backward_slice(0, d_x, d_x, d_fwd_work, d_bwd_work, batch, max_active, ft_in, ft_out, rps, 1, 0, ceil_div(ft_in, rps), d_grad, d_slabs);
+                launch_ft_backward_slice(0, d_x, d_x, d_fwd_work, d_bwd_work, batch, max_active, ft_in, ft_out, rps, 1, 0, 1, d_grad, d_slabs);
             }));
             out->bwd_slice_ms = (float)(tm.total / iters);
         }

@@ -3,79 +3,7 @@
 // (native_kernels.cu:1842; pointwise/ranger_step.rs:52-59), fused so that every parameter and moment
 // crosses HBM once per step.  The gradient is only read: every gradient buffer is fully rewritten by
 // the next backward pass, so the reference's grad = 0 store is not needed.
-#include "common.cuh"
-
-#include <cuda_fp16.h>
-
-static __device__ __forceinline__ unsigned ok_pack_h2(float lo, float hi) {
-    const __half2 h = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<const unsigned*>(&h);
-}
-static __device__ __forceinline__ float2 ok_unpack_h2(unsigned pair) { return __half22float2(*reinterpret_cast<const __half2*>(&pair)); }
-static __device__ __forceinline__ uint2 pack_h4(float4 v) { return make_uint2(ok_pack_h2(v.x, v.y), ok_pack_h2(v.z, v.w)); }
-
-// Four moments of one float4 of parameters.  fp32 state: as stored.  fp16 state (radam_step_f16state,
-// native_kernels.cu:1127-1181): stored = clamp(value * scale) rounded to fp16; read back as stored / scale.  The update
-// itself uses the unrounded new moments; the scales are powers of two, so scaling is exact.
-template <bool HS>
-static __device__ __forceinline__ float4 load_moment(const void* base, size_t i4, float inv_scale, bool streaming) {
-    if (HS) {
-        const uint2* p = static_cast<const uint2*>(base) + i4;
-        const uint2 u = streaming ? __ldcs(p) : *p;
-        const float2 a = ok_unpack_h2(u.x), b = ok_unpack_h2(u.y);
-        return make_float4(a.x * inv_scale, a.y * inv_scale, b.x * inv_scale, b.y * inv_scale);
-    }
-    const float4* p = static_cast<const float4*>(base) + i4;
-    return streaming ? __ldcs(p) : *p;
-}
-static __device__ __forceinline__ float clamp_h(float x, bool both) {
-    x = x > 65504.0f ? 65504.0f : x;  // comparisons keep a NaN, as the reference does
-    if (both) x = x < -65504.0f ? -65504.0f : x;
-    return x;
-}
-template <bool HS>
-static __device__ __forceinline__ void store_moment(void* base, size_t i4, float4 val, float scale, bool both, bool streaming) {
-    if (HS) {
-        const float4 q = make_float4(clamp_h(val.x * scale, both), clamp_h(val.y * scale, both), clamp_h(val.z * scale, both),
-                                     clamp_h(val.w * scale, both));
-        uint2* p = static_cast<uint2*>(base) + i4;
-        if (streaming) __stcs(p, pack_h4(q)); else *p = pack_h4(q);
-    } else {
-        float4* p = static_cast<float4*>(base) + i4;
-        if (streaming) __stcs(p, val); else *p = val;
-    }
-}
-static __device__ __forceinline__ float4 scale4(float4 g, float k) { return make_float4(g.x * k, g.y * k, g.z * k, g.w * k); }
-
-static __device__ __forceinline__ float radam_one(float p, float& m, float& v, float g, const OptScalars& sc, float rate,
-                                                   float decay_mul) {
-    p *= decay_mul;
-    const float mi = sc.beta1 * m + (1.0f - sc.beta1) * g;
-    const float vi = sc.beta2 * v + (1.0f - sc.beta2) * g * g;
-    m = mi;
-    v = vi;
-    float val = mi;
-    if (sc.denom != 0) val /= sqrtf(vi) + sc.eps;
-    p -= rate * val;
-    p = p < sc.min_w ? sc.min_w : p;
-    p = p > sc.max_w ? sc.max_w : p;
-    return p;
-}
-
-static __device__ __forceinline__ float4 radam_four(float4 p, float4& m, float4& v, float4 g, const OptScalars& sc,
-                                                     float rate, float decay_mul) {
-    float4 r;
-    r.x = radam_one(p.x, m.x, v.x, g.x, sc, rate, decay_mul);
-    r.y = radam_one(p.y, m.y, v.y, g.y, sc, rate, decay_mul);
-    r.z = radam_one(p.z, m.z, v.z, g.z, sc, rate, decay_mul);
-    r.w = radam_one(p.w, m.w, v.w, g.w, sc, rate, decay_mul);
-    return r;
-}
-
-static __device__ __forceinline__ float4 lerp_four(float4 w, float4 s, float alpha) {
-    const float oma = 1.0f - alpha;
-    return make_float4(alpha * w.x + oma * s.x, alpha * w.y + oma * s.y, alpha * w.z + oma * s.z, alpha * w.w + oma * s.w);
-}
+#include "radam.cuh"
 
 // plain streaming update of one large group (n multiple of 4); mirror: optional fp16 copy of the updated weights
 // (radam_step_fp16_mirror / radam_step_f16state_mirror + ranger_lookahead_lerp_fp16_mirror, native_kernels.cu:1183-1290)

@@ -5,8 +5,9 @@
 //    run at the same time gather from the same slice of the FT table and the slice stays in L2.
 // Both sorts share three launches (blockIdx.y / blockIdx.x selects the sort): per-block histogram, one-block scan of the
 // [key][block] matrix, stable scatter (rank inside a block = warp match + prefix over the block's warps); a fourth
-// launch cuts the bucket segments into tiles and work units.  Results do not depend on timing.
+// launch cuts the segments into what the later kernels work on.  Results do not depend on timing.
 #include "common.cuh"
+#include "ft_slice.cuh"
 
 #define SORT_BLOCK 1024
 #define SORT_MAX_KEYS 128
@@ -130,13 +131,15 @@ __global__ void __launch_bounds__(SORT_BLOCK) k_sort_scatter2(Fn0 f0, int n0, in
     else if ((int)blockIdx.x < G1) sort_scatter_body(f1, n1, K1, G1, b1, o1, s_cnt, blockIdx.x);
 }
 
+// ---- what the kernels behind the sorts work on, one block each -------------------------------------------------------
+// At most 128 keys; what depends on all of them is summed by a warp per key.  (One thread walking the keys took 14 us of
+// a step for the forward runs and 17 us for the chunks.)
+#define PLAN_THREADS 1024
+
 // tiles: runs of <= TB_TILE_M positions of one bucket; units: runs of <= TB_UNIT_TILES tiles of one bucket
-__global__ void __launch_bounds__(256) k_make_tiles(const int* __restrict__ seg_start, int K, TileDesc* __restrict__ tiles,
-                                                     int* __restrict__ n_tiles, TileDesc* __restrict__ units,
-                                                     int* __restrict__ n_units) {
-    __shared__ int s_tile_base[SORT_MAX_KEYS + 1], s_unit_base[SORT_MAX_KEYS + 1], s_seg[SORT_MAX_KEYS + 2];
-    for (int k = threadIdx.x; k <= K; k += blockDim.x) s_seg[k] = seg_start[k];  // one round trip, not K
-    __syncthreads();
+static __device__ void plan_tiles(const int* __restrict__ s_seg, int K, TileDesc* __restrict__ tiles, int* __restrict__ n_tiles,
+                                  TileDesc* __restrict__ units, int* __restrict__ n_units) {
+    __shared__ int s_tile_base[TB_MAX_BUCKETS + 3], s_unit_base[TB_MAX_BUCKETS + 3];
     if (threadIdx.x == 0) {
         int trun = 0, urun = 0;
         for (int k = 0; k < K; ++k) {
@@ -146,40 +149,182 @@ __global__ void __launch_bounds__(256) k_make_tiles(const int* __restrict__ seg_
             trun += nt;
             urun += (nt + TB_UNIT_TILES - 1) / TB_UNIT_TILES;
         }
+        s_tile_base[K] = trun;
+        s_unit_base[K] = urun;
         *n_tiles = trun;
         *n_units = urun;
     }
     __syncthreads();
-    for (int k = 0; k < K; ++k) {
-        const int s0 = s_seg[k], c = s_seg[k + 1] - s0;
-        const int nt = (c + TB_TILE_M - 1) / TB_TILE_M;
-        for (int t = threadIdx.x; t < nt; t += blockDim.x) {
-            TileDesc d;
-            d.start = s0 + t * TB_TILE_M;
-            d.count = min(TB_TILE_M, c - t * TB_TILE_M);
-            d.bucket = k;
-            d.pad = 0;
-            tiles[s_tile_base[k] + t] = d;
+    for (int t = threadIdx.x; t < s_tile_base[K]; t += PLAN_THREADS) {
+        int k = 0;
+        while (s_tile_base[k + 1] <= t) ++k;
+        const int i = t - s_tile_base[k];
+        TileDesc d;
+        d.start = s_seg[k] + i * TB_TILE_M;
+        d.count = min(TB_TILE_M, s_seg[k + 1] - d.start);
+        d.bucket = k;
+        d.pad = 0;
+        tiles[t] = d;
+    }
+    for (int u = threadIdx.x; u < s_unit_base[K]; u += PLAN_THREADS) {
+        int k = 0;
+        while (s_unit_base[k + 1] <= u) ++k;
+        TileDesc d;
+        d.start = s_tile_base[k] + (u - s_unit_base[k]) * TB_UNIT_TILES;
+        d.count = min(TB_UNIT_TILES, s_tile_base[k + 1] - d.start);
+        d.bucket = k;
+        d.pad = 0;
+        units[u] = d;
+    }
+}
+
+// Runs of the slice-resident forward: <= SLICE_IPC consecutive slots of one slice, the largest first.  The blocks take
+// (run, column strip) units in this order: king-bucket slices differ in size by two and more (a mirrored board has a centre
+// file), and with the units in slice order the busiest SM of a full batch worked 14 % longer than the average one.
+static __device__ void plan_forward(const int* __restrict__ s_seg, int n_keys, FwdWork* __restrict__ work, int* __restrict__ n_work) {
+    __shared__ int s_size[SORT_MAX_KEYS], s_n[SORT_MAX_KEYS];
+    const int k = threadIdx.x;
+    if (k < n_keys) {
+        const int len = s_seg[k + 1] - s_seg[k];
+        const int n = (len + SLICE_IPC - 1) / SLICE_IPC;
+        s_n[k] = n;
+        s_size[k] = n > 0 ? ((len + n - 1) / n + 127) & ~127 : 0;  // equal runs of whole rounds of 128 items
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int key = threadIdx.x >> 5; key < n_keys; key += PLAN_THREADS / 32) {
+        int base = 0;
+        for (int j = lane; j < n_keys; j += 32)
+            if (s_size[j] > s_size[key] || (s_size[j] == s_size[key] && j < key)) base += s_n[j];
+        base = __reduce_add_sync(0xffffffffu, base);
+        for (int i = lane; i < s_n[key]; i += 32) {
+            FwdWork w;
+            w.slice = key;
+            w.begin = min(s_seg[key + 1], s_seg[key] + i * s_size[key]);
+            w.end = min(s_seg[key + 1], w.begin + s_size[key]);
+            w.pad = 0;
+            work[base + i] = w;
         }
-        const int nu = (nt + TB_UNIT_TILES - 1) / TB_UNIT_TILES;
-        for (int u = threadIdx.x; u < nu; u += blockDim.x) {
-            TileDesc d;
-            d.start = s_tile_base[k] + u * TB_UNIT_TILES;
-            d.count = min(TB_UNIT_TILES, nt - u * TB_UNIT_TILES);
-            d.bucket = k;
-            d.pad = 0;
-            units[s_unit_base[k] + u] = d;
+    }
+    if (threadIdx.x < 32) {
+        int total = 0;
+        for (int j = lane; j < n_keys; j += 32) total += s_n[j];
+        total = __reduce_add_sync(0xffffffffu, total);
+        if (lane == 0) {
+            n_work[0] = total;
+            n_work[1] = 0;  // "some item has a row outside its slice", raised by k_fwd_codes
+            n_work[2] = 0;  // units taken by the forward's blocks
         }
     }
 }
 
+// Chunks of <= ch consecutive slots of one slice, in slice order; groups of <= BWD_GROUP chunks of one slice (an empty slice
+// has one group, its rows are zeroed); and per part (equal ranges of slices) the order in which the weight gradient's blocks
+// take the groups: the largest first.
+static __device__ void plan_backward(const int* __restrict__ s_seg, int n_keys, int ch, int parts, FwdWork* __restrict__ chunks,
+                                     int* __restrict__ n_chunks, int* __restrict__ groups, int* __restrict__ sched) {
+    __shared__ int s_nc[SORT_MAX_KEYS], s_size[SORT_MAX_KEYS], s_part[SORT_MAX_KEYS];
+    __shared__ int s_w[2 * SORT_MAX_KEYS], s_cnt[2 * SORT_MAX_KEYS];  // per slice: its full groups, its last smaller one
+    const int n_slices = n_keys - 1;  // the last key holds items without a slice: they have no rows
+    const int k = threadIdx.x;
+    if (k < n_keys) {
+        const int len = s_seg[k + 1] - s_seg[k];
+        const int n = (len + ch - 1) / ch;
+        s_nc[k] = n;
+        const int size = n > 0 ? ((len + n - 1) / n + 7) & ~7 : 0;  // equal chunks (<= ch: ch is a multiple of 8)
+        s_size[k] = size;
+        if (k < n_slices) {
+            const int full = n / BWD_GROUP, rest = n - full * BWD_GROUP;
+            s_w[2 * k] = BWD_GROUP * size;
+            s_cnt[2 * k] = full;
+            s_w[2 * k + 1] = rest * size;
+            s_cnt[2 * k + 1] = (rest > 0 || n == 0) ? 1 : 0;
+            int p = 0;
+            while (p + 1 < parts && k >= (int)((long long)n_slices * (p + 1) / parts)) ++p;
+            s_part[k] = p;
+        }
+    }
+    __syncthreads();
+    const unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int4* rec = reinterpret_cast<int4*>(groups + 4 + SORT_KEYS_LIMIT + 4);
+    int* order = sched + 2 * BWD_PARTS + 4;
+    for (int key = threadIdx.x >> 5; key < n_keys; key += PLAN_THREADS / 32) {
+        int c0 = 0, g0 = 0, slab = 0;
+        int base[2] = {0, 0};  // position of the slice's full groups and of its last smaller one among all groups
+        for (int j = lane; j < n_keys; j += 32) {
+            if (j < key) c0 += s_nc[j];
+            if (j >= n_slices) continue;
+            const int ng = s_cnt[2 * j] + s_cnt[2 * j + 1];
+            if (j < key) { g0 += ng; slab += ng - 1; }
+            if (key < n_slices) {
+                for (int h = 0; h < 4; ++h) {
+                    const int c = 2 * key + (h & 1), d = 2 * j + (h >> 1);
+                    const bool before = s_part[j] != s_part[key] ? s_part[j] < s_part[key] : (s_w[d] > s_w[c] || (s_w[d] == s_w[c] && d < c));
+                    if (before) base[h & 1] += s_cnt[d];
+                }
+            }
+        }
+        c0 = __reduce_add_sync(all, c0);
+        g0 = __reduce_add_sync(all, g0);
+        slab = __reduce_add_sync(all, slab);
+        base[0] = __reduce_add_sync(all, base[0]);
+        base[1] = __reduce_add_sync(all, base[1]);
+        const int nc = s_nc[key], size = s_size[key];
+        for (int i = lane; i < nc; i += 32) {
+            FwdWork w;
+            w.slice = key;
+            w.begin = min(s_seg[key + 1], s_seg[key] + i * size);
+            w.end = min(s_seg[key + 1], w.begin + size);
+            w.pad = 0;
+            chunks[c0 + i] = w;
+        }
+        if (lane == 0) {
+            groups[4 + key] = g0;  // first group of the slice; of the last key: the end
+            if (key == n_slices) {
+                *n_chunks = c0 + nc;
+                groups[0] = g0;
+            }
+        }
+        if (key < n_slices) {
+            const int full = s_cnt[2 * key], ng = full + s_cnt[2 * key + 1];
+            for (int i = lane; i < ng; i += 32) {
+                rec[g0 + i] = make_int4(key, c0 + min(i * BWD_GROUP, nc), c0 + min((i + 1) * BWD_GROUP, nc), i == 0 ? -1 : slab + i - 1);
+                order[i < full ? base[0] + i : base[1] + i - full] = g0 + i;
+            }
+        }
+    }
+    if ((int)threadIdx.x <= parts) {  // first position of every part, and the end
+        int first = 0;
+        for (int j = 0; j < n_slices; ++j)
+            if (s_part[j] < (int)threadIdx.x) first += s_cnt[2 * j] + s_cnt[2 * j + 1];
+        sched[BWD_PARTS + threadIdx.x] = first;
+    }
+}
+
+__global__ void __launch_bounds__(PLAN_THREADS) k_step_plans(const int* __restrict__ seg_start, int K0, TileDesc* __restrict__ tiles,
+                                                             int* __restrict__ n_tiles, TileDesc* __restrict__ units,
+                                                             const int* __restrict__ item_seg, int n_keys, FwdWork* __restrict__ work,
+                                                             int* __restrict__ n_work, int ch, int parts, FwdWork* __restrict__ chunks,
+                                                             int* __restrict__ n_chunks, int* __restrict__ groups, int* __restrict__ sched) {
+    __shared__ int s_seg[SORT_MAX_KEYS + 2];
+    const int* seg = blockIdx.x == 0 ? seg_start : item_seg;
+    const int n = blockIdx.x == 0 ? K0 : n_keys;
+    for (int k = threadIdx.x; k <= n; k += PLAN_THREADS) s_seg[k] = seg[k];
+    __syncthreads();
+    if (blockIdx.x == 0) plan_tiles(s_seg, K0, tiles, n_tiles, units, n_tiles + 1);
+    else if (blockIdx.x == 1) plan_forward(s_seg, n_keys, work, n_work);
+    else plan_backward(s_seg, n_keys, ch, parts, chunks, n_chunks, groups, sched);
+}
+
 int sort_max_units(int max_tiles) { return max_tiles / TB_UNIT_TILES + TB_MAX_BUCKETS + 2; }
 
-// Both sorts of a step in four launches: positions by bucket (order, tiles, units) and items by table slice.
+// Both sorts of a step in four launches: positions by bucket (order, tiles, units) and items by table slice, with the plans
+// of the slice-resident kernels where their work buffers are given.
 // hist: scratch of (nb + 1) * ceil(B / 1024) + (slices + 1) * ceil(n_persp * B / 1024) ints.
 int launch_step_sorts(cudaStream_t s, const int* bucket, int B, int nb, int* order, TileDesc* tiles, int* n_tiles, int* seg_start,
                       int max_tiles, const int* idx_stm, const int* idx_nstm, const int* nnz, int A, int N, int rows_per_slice,
-                      int n_persp, int* items, int* item_seg, int* hist) {
+                      int n_persp, int* items, int* item_seg, int* hist, int* fwd_work, int* bwd_work, int bwd_parts) {
     int n_slices = ceil_div(N, rows_per_slice);
     if (n_slices + 1 > SORT_MAX_KEYS) {
         rows_per_slice = ceil_div(N, SORT_MAX_KEYS - 1);
@@ -195,6 +340,17 @@ int launch_step_sorts(cudaStream_t s, const int* bucket, int B, int nb, int* ord
     k_sort_hist2<<<grid, SORT_BLOCK, 0, s>>>(f0, B, K0, G0, h0, f1, n1, K1, G1, h1);
     k_sort_scan2<<<2, 1024, 0, s>>>(h0, K0, G0, B, seg_start, h1, K1, G1, n1, item_seg);
     k_sort_scatter2<<<grid, SORT_BLOCK, 0, s>>>(f0, B, K0, G0, h0, order, f1, n1, K1, G1, h1, items);
-    k_make_tiles<<<1, 256, 0, s>>>(seg_start, K0, tiles, n_tiles, tiles + max_tiles, n_tiles + 1);
+    SliceBuffers sb = {};
+    BwdPointers bp = {};
+    int ch = 0;
+    if (fwd_work) sb = slice_buffers(fwd_work, n1, K1);
+    if (bwd_work) {
+        const BwdLayout L = bwd_layout(n1, A, rows_per_slice);
+        bp = bwd_pointers(bwd_work, L);
+        ch = L.CH;
+    }
+    k_step_plans<<<bwd_work ? 3 : fwd_work ? 2 : 1, PLAN_THREADS, 0, s>>>(seg_start, K0, tiles, n_tiles, tiles + max_tiles, item_seg, K1,
+                                                                          sb.work, sb.n_work, ch, bwd_parts, bp.chunks, bp.n_chunks,
+                                                                          bp.groups, bp.sched);
     return 4;
 }

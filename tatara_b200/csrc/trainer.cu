@@ -171,6 +171,7 @@ struct tb_trainer {
     int *feat_counts = nullptr, *feat_offsets = nullptr, *feat_cursor = nullptr, *feat_lists = nullptr;
     int *sort_hist = nullptr, *items = nullptr, *item_seg = nullptr, *bwd_plan = nullptr, *fwd_work = nullptr, *bwd_slice = nullptr;
     int dgrad_rows = 0;
+    int bwd_parts = 1;  // launches the FT weight gradient is cut into (data parallel)
     int n_sm = 148;
     cudaStream_t comm_stream = nullptr;  // data parallel: all-reduces behind the FT weight gradient
     cudaStream_t opt_stream = nullptr;   // data parallel: FT row updates behind their all-reduces
@@ -411,17 +412,18 @@ int run_forward(tb_trainer* t, const DevBatch& d, const tb_loss* loss, float lam
     void* pre0 = t->p_out16 ? t->pre_h[0] : (void*)t->pre[0];
     void* pre1 = t->p_out16 ? t->pre_h[1] : (void*)t->pre[1];
     t->last_n = B;
+    const int rps = c.piece_inputs > 0 ? c.piece_inputs : N;
+    t->slice_fwd = ft_forward_slice_supported(F, N, A, rps);
     if (backward) { t->opt_begun = false; t->ft_rows_updated = false; }
     { PhaseScope p(t, PH_SORT);
       // positions by bucket (order, tiles, units) and items of both perspectives by the king-bucket slice of the FT table
       int n = launch_step_sorts(t->stream, ls ? d.bucket : nullptr, B, ls ? c.num_buckets : 0, t->order, t->tiles, t->n_tiles,
-                                t->seg_start, t->max_tiles, d.stm, d.nstm, d.nnz, A, N, c.piece_inputs > 0 ? c.piece_inputs : N, 2,
-                                t->items, t->item_seg, t->sort_hist);
+                                t->seg_start, t->max_tiles, d.stm, d.nstm, d.nnz, A, N, rps, 2, t->items, t->item_seg,
+                                t->sort_hist, t->slice_fwd ? t->fwd_work : nullptr, t->slice_fwd && backward ? t->bwd_slice : nullptr,
+                                t->bwd_parts);
       p.done(n); }
     { PhaseScope p(t, PH_FT_FWD);
       const int mode = (ls || c.activation == TB_ACT_PAIRWISE) ? 1 : (c.activation == TB_ACT_CRELU ? 2 : 3);
-      const int rps = c.piece_inputs > 0 ? c.piece_inputs : N;
-      t->slice_fwd = ft_forward_slice_supported(F, N, A, rps);
       if (t->slice_fwd)
           p.done(launch_ft_forward_slice(t->stream, mode, table, d.stm, d.nstm, d.nnz, t->groups[1].w, pre0, pre1,
                                          t->combined, t->items, t->item_seg, t->fwd_work, B, F, N, A, rps, FT_POST_SCALE, 2,
@@ -523,8 +525,7 @@ int run_backward(tb_trainer* t, const DevBatch& d, float lr) {
           // first part, the loss with the last).  Whichever path wrote the rows (the gated generic kernels come first), they
           // are final when the part's event is recorded.
           const int n_slices = (N + rps - 1) / rps;
-          const int strips = t->p_out16 ? F / 64 : F / 32;
-          const int parts = c.world_size > 1 ? ar_parts_for(n_slices, strips, t->n_sm) : 1;
+          const int parts = t->bwd_parts;
           const bool pipeline = parts > 1;
           const int64_t ft_off = t->groups[0].grad - t->grad_arena;
           int rc = 0;
@@ -534,7 +535,7 @@ int run_backward(tb_trainer* t, const DevBatch& d, float lr) {
               // equal parts: shorter last parts (tapered sizes, or whole waves with a one-wave last part) were measured slower
               // on two and four GPUs, with NCCL and with the peer exchange
               const int k0 = (int)((int64_t)n_slices * part / parts), k1 = (int)((int64_t)n_slices * (part + 1) / parts);
-              n += launch_ft_backward_slice(t->stream, dft0, dft1, t->fwd_work, t->bwd_slice, B, A, N, F, rps, 2, k0, k1 - k0,
+              n += launch_ft_backward_slice(t->stream, dft0, dft1, t->fwd_work, t->bwd_slice, B, A, N, F, rps, 2, part, parts,
                                             t->groups[0].grad, t->bwd_slabs, t->p_out16);
               if (!pipeline) continue;
               CU(t, cudaEventRecord(t->ev_part[part], t->stream));
@@ -1011,6 +1012,7 @@ int create_impl(tb_trainer* t) {
         const int rps = c.piece_inputs > 0 ? c.piece_inputs : (int)N;
         if (ft_forward_slice_supported((int)F, (int)N, (int)A, rps) && ft_backward_slice_supported((int)F, (int)N, (int)A, rps))
         {
+            if (c.world_size > 1) t->bwd_parts = ar_parts_for((int)((N + rps - 1) / rps), (int)(t->p_out16 ? F / 64 : F / 32), t->n_sm);
             CU(t, dalloc(&t->bwd_slice, ft_backward_slice_ints((int)(2 * B), (int)A, rps)));
             CU(t, cudaMalloc((void**)&t->bwd_slabs, ft_backward_slice_slab_floats((int)(2 * B), (int)A, rps, (int)F) * sizeof(float)));
         }
