@@ -73,63 +73,95 @@ int launch_radam_small(cudaStream_t s, const SmallGroups& groups, int max_n, Opt
 }
 
 // ------------------------------------------------------------------------------------------------
-// Factorised FT table (N = KB * pi real rows + pi virtual rows).  One block per virtual row v, one
-// thread per float4 column:
-//   pass 1: update the KB real rows kb*pi + v and add up their gradients in kb order
-//           (ft_reduce_virtual_grad, sparse/ft_factorize.rs:109-121),
-//   then update the virtual row N + v with that sum (and store the sum as its gradient),
-//   pass 2: comb[kb*pi + v] = w[kb*pi + v] + w[N + v] (ft_fold_virtual, sparse/ft_factorize.rs:78-99);
-//           the real rows were written a moment ago by this block and are read back from L2.
+// Factorised FT table (N = KB * pi real rows + pi virtual rows).  A block owns 32 adjacent float4 columns of one virtual row
+// vr, its warps share that row's KB real rows kb*pi + vr, up to FACT_ROWS neighbours each:
+//   - every warp updates its rows and adds up their gradients in kb order;
+//   - the warps' sums, added in warp order, are the virtual row's gradient (ft_reduce_virtual_grad,
+//     sparse/ft_factorize.rs:109-121); the first warp updates the virtual row N + vr;
+//   - comb[kb*pi + v] = w[kb*pi + v] + w[N + v] (ft_fold_virtual, sparse/ft_factorize.rs:78-99), the real rows kept in
+//     shared memory.
 // Replaces radam_step on N_t*F elements + ft_reduce_virtual_grad + ranger_lookahead_lerp + ft_fold_virtual.
-// Two builds: rows of up to 384 float4 (F <= 1536) run three blocks per SM (56 registers), longer rows one or two.
+// HBM-bound.  With a thread per column walking all the rows twice, the second walk found them gone from L2 (122 MB of rows
+// in flight): 4.2 GB moved instead of the 3.8 needed.  Warps side by side also make enough loads in flight where the table
+// is narrow.  F = 1536 / 768 / 256, 45 king buckets, fp32: 730 / 373 / 140 us with the walks, 636 / 324 / 118 now (0.92 of
+// the measured HBM rate at 1536); fp16 moments and table at 1536: 566, now 490.  (Rows in registers: 667.  No folded table,
+// the forward adding the two rows as it loads a strip: 566 here, but 190 more there.)
 // ------------------------------------------------------------------------------------------------
+#define FACT_ROWS 9   // rows of a warp: 45 and 81 king buckets are 5 and 9 full warps
+#define FACT_BATCH 3  // of these, loaded together
 // HS: fp16 moments; HC: fp16 folded table.  The real rows' gradients are multiplied by sc.grad_scale on load; the virtual
 // row's gradient cell receives the sum of the scaled values (its true gradient).
-template <int MAX_THREADS, int MIN_BLOCKS, bool HS, bool HC>
-__global__ void __launch_bounds__(MAX_THREADS, MIN_BLOCKS) k_radam_factorized(float4* __restrict__ w, void* __restrict__ m, void* __restrict__ v,
+template <int MAX_WARPS, int MIN_BLOCKS, bool HS, bool HC>
+__global__ void __launch_bounds__(32 * MAX_WARPS, MIN_BLOCKS) k_radam_factorized(float4* __restrict__ w, void* __restrict__ m, void* __restrict__ v,
                                                             float4* __restrict__ g, float4* __restrict__ slow,
                                                             void* __restrict__ comb, int N, int pi, int row4, OptScalars sc) {
+    __shared__ float4 s_sum[MAX_WARPS][32], s_virt[32];
+    __shared__ float4 s_w[FACT_ROWS][32 * MAX_WARPS];  // the updated real rows
     const float inv_ms = 1.0f / TB_FT_OPT_M_SCALE, inv_vs = 1.0f / TB_FT_OPT_V_SCALE;
-    const int vr = blockIdx.x;
-    const int c = threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const size_t plane = (size_t)pi * row4;  // float4 of one king bucket
+    const size_t cell = (size_t)blockIdx.x * 32 + lane;  // a row is a multiple of 32 float4 long
+    const int KB = N / pi;
+    const int kb0 = warp * FACT_ROWS;
     const float rate = sc.lr * sc.step_size;
     const float decay_mul = 1.0f - sc.decay * rate;
-    const int KB = N / pi;
     float4 gsum = make_float4(0.f, 0.f, 0.f, 0.f);
-    // m, v and the gradient stream through once: evict-first loads / stores keep them from pushing the freshly
-    // written weights out of L2 before pass 2 reads them back
-#pragma unroll 4
-    for (int kb = 0; kb < KB; ++kb) {
-        const size_t i = (size_t)(kb * pi + vr) * row4 + c;
-        float4 gi = __ldcs(g + i);
-        if (HC) gi = scale4(gi, sc.grad_scale);  // loss-scaled sums exist only next to an fp16 table
-        float4 mi = load_moment<HS>(m, i, inv_ms, true), vi = load_moment<HS>(v, i, inv_vs, true);
-        float4 p = radam_four(w[i], mi, vi, gi, sc, rate, decay_mul);
-        store_moment<HS>(m, i, mi, TB_FT_OPT_M_SCALE, true, true);
-        store_moment<HS>(v, i, vi, TB_FT_OPT_V_SCALE, false, true);
-        if (sc.lerp) {
-            p = lerp_four(p, __ldcs(slow + i), sc.alpha);
-            __stcs(slow + i, p);
+    // everything streams through once: evict-first
+#pragma unroll 1
+    for (int b = 0; b < FACT_ROWS; b += FACT_BATCH) {
+        float4 p[FACT_BATCH], mi[FACT_BATCH], vi[FACT_BATCH], gi[FACT_BATCH];
+#pragma unroll
+        for (int u = 0; u < FACT_BATCH; ++u) {
+            const size_t i = (size_t)min(kb0 + b + u, KB - 1) * plane + cell;  // past the end: the last row, dropped below
+            p[u] = __ldcs(w + i);
+            mi[u] = load_moment<HS>(m, i, inv_ms, true);
+            vi[u] = load_moment<HS>(v, i, inv_vs, true);
+            gi[u] = __ldcs(g + i);
         }
-        w[i] = p;
-        gsum.x += gi.x; gsum.y += gi.y; gsum.z += gi.z; gsum.w += gi.w;
+#pragma unroll
+        for (int u = 0; u < FACT_BATCH; ++u) {
+            if (kb0 + b + u >= KB) break;
+            const size_t i = (size_t)(kb0 + b + u) * plane + cell;
+            if (HC) gi[u] = scale4(gi[u], sc.grad_scale);  // loss-scaled sums exist only next to an fp16 table
+            float4 q = radam_four(p[u], mi[u], vi[u], gi[u], sc, rate, decay_mul);
+            store_moment<HS>(m, i, mi[u], TB_FT_OPT_M_SCALE, true, true);
+            store_moment<HS>(v, i, vi[u], TB_FT_OPT_V_SCALE, false, true);
+            if (sc.lerp) {
+                q = lerp_four(q, __ldcs(slow + i), sc.alpha);
+                __stcs(slow + i, q);
+            }
+            __stcs(w + i, q);
+            s_w[b + u][threadIdx.x] = q;
+            gsum.x += gi[u].x; gsum.y += gi[u].y; gsum.z += gi[u].z; gsum.w += gi[u].w;
+        }
     }
-    const size_t iv = (size_t)(N + vr) * row4 + c;
-    g[iv] = gsum;
-    float4 mv = load_moment<HS>(m, iv, inv_ms, false), vv = load_moment<HS>(v, iv, inv_vs, false);
-    float4 pv = radam_four(w[iv], mv, vv, gsum, sc, rate, decay_mul);
-    store_moment<HS>(m, iv, mv, TB_FT_OPT_M_SCALE, true, false);
-    store_moment<HS>(v, iv, vv, TB_FT_OPT_V_SCALE, false, false);
-    if (sc.lerp) {
-        pv = lerp_four(pv, slow[iv], sc.alpha);
-        slow[iv] = pv;
+    s_sum[warp][lane] = gsum;
+    __syncthreads();
+    if (warp == 0) {
+        for (int q = 1; q < warps; ++q) {
+            const float4 x = s_sum[q][lane];
+            gsum.x += x.x; gsum.y += x.y; gsum.z += x.z; gsum.w += x.w;
+        }
+        const size_t iv = (size_t)KB * plane + cell;
+        g[iv] = gsum;
+        float4 mv = load_moment<HS>(m, iv, inv_ms, false), vv = load_moment<HS>(v, iv, inv_vs, false);
+        float4 pv = radam_four(w[iv], mv, vv, gsum, sc, rate, decay_mul);
+        store_moment<HS>(m, iv, mv, TB_FT_OPT_M_SCALE, true, false);
+        store_moment<HS>(v, iv, vv, TB_FT_OPT_V_SCALE, false, false);
+        if (sc.lerp) {
+            pv = lerp_four(pv, slow[iv], sc.alpha);
+            slow[iv] = pv;
+        }
+        w[iv] = pv;
+        s_virt[lane] = pv;
     }
-    w[iv] = pv;
-    // newest rows first: they are the ones most likely still in L2
-#pragma unroll 4
-    for (int kb = KB - 1; kb >= 0; --kb) {
-        const size_t i = (size_t)(kb * pi + vr) * row4 + c;
-        const float4 p = w[i];
+    __syncthreads();
+    const float4 pv = s_virt[lane];
+#pragma unroll
+    for (int u = 0; u < FACT_ROWS; ++u) {
+        if (kb0 + u >= KB) break;
+        const size_t i = (size_t)(kb0 + u) * plane + cell;
+        const float4 p = s_w[u][threadIdx.x];
         const float4 f = make_float4(p.x + pv.x, p.y + pv.y, p.z + pv.z, p.w + pv.w);
         if (HC) __stcs(static_cast<uint2*>(comb) + i, pack_h4(f));
         else __stcs(static_cast<float4*>(comb) + i, f);
@@ -224,14 +256,20 @@ int launch_radam_factorized_fold(cudaStream_t s, float* w, void* m, void* v, flo
 int launch_radam_factorized(cudaStream_t s, float* w, void* m, void* v, float* g, float* slow, void* comb, int N,
                             int pi, int F, OptScalars sc, int half_state, int half_comb) {
     float4 *w4 = reinterpret_cast<float4*>(w), *g4 = reinterpret_cast<float4*>(g), *s4 = reinterpret_cast<float4*>(slow);
-#define FUSED(T, MB, HS, HC) k_radam_factorized<T, MB, HS, HC><<<pi, F / 4, 0, s>>>(w4, m, v, g4, s4, comb, N, pi, F / 4, sc)
-    if (F / 4 <= 384) {
-        if (half_state) { if (half_comb) FUSED(384, 3, true, true); else FUSED(384, 3, true, false); }
-        else { if (half_comb) FUSED(384, 3, false, true); else FUSED(384, 3, false, false); }
-    } else {
-        if (half_state) { if (half_comb) FUSED(1024, 1, true, true); else FUSED(1024, 1, true, false); }
-        else { if (half_comb) FUSED(1024, 1, false, true); else FUSED(1024, 1, false, false); }
-    }
+    const int KB = N / pi, warps = ceil_div(KB, FACT_ROWS), blocks = (int)((long long)pi * (F / 4) / 32);
+#define FUSED(MW, MB, HS, HC) k_radam_factorized<MW, MB, HS, HC><<<blocks, 32 * warps, 0, s>>>(w4, m, v, g4, s4, comb, N, pi, F / 4, sc)
+#define FUSED_H(MW, MB, MBH)                                                                                                   \
+    do {                                                                                                                       \
+        if (half_state) { if (half_comb) FUSED(MW, MBH, true, true); else FUSED(MW, MBH, true, false); }                       \
+        else { if (half_comb) FUSED(MW, MB, false, true); else FUSED(MW, MB, false, false); }                                  \
+    } while (0)
+    // blocks per SM: more were slower again (F = 1536, fp32 / fp16 moments: 5 blocks 636 / 506 us, 6 641 / 490, 8 with one row at
+    // a time 800 / 568)
+    if (warps <= 5) FUSED_H(5, 5, 6);
+    else if (warps <= 9) FUSED_H(9, 3, 3);
+    else return launch_radam_factorized_rows(s, w, m, v, g, slow, N, pi, F, 0, KB, sc, half_state) +
+                launch_radam_factorized_fold(s, w, m, v, g, slow, comb, N, pi, F, sc, half_state, half_comb);
+#undef FUSED_H
 #undef FUSED
     return 1;
 }

@@ -5,7 +5,7 @@ import pytest
 
 import oracle_lib as O
 import tatara_b200 as tb
-from helpers import random_index_batch
+from helpers import assert_close, assert_close_scaled, random_index_batch
 from test_gpu_parity import _check_step, _oracle_for, _perturb, _sync_weights
 
 pytestmark = pytest.mark.gpu
@@ -40,3 +40,29 @@ def test_uneven_slices_step_matches_oracle(B, share):
     _sync_weights(tr, ot, init)
     batch = tb.BatchData(d["stm"], d["nstm"], d["nnz"], d["score"], d["wdl"], d["bucket"])
     _check_step(tr, ot, batch, tb.LossKind.sigmoid(), O.sigmoid_loss(), 1e-3, "layerstack", B, F, l1)
+
+
+@pytest.mark.parametrize("kb", [1, 8, 9, 10, 46, 81, 82])
+def test_factorized_optimizer_king_bucket_counts(kb):
+    """Nine king buckets a warp, nine warps a block, two launches above that: the step's weights, moments and folded table."""
+    fs = tb.FeatureSetSpec("test", 4, kb, 40, 8, True)
+    F, l1, l2, B = 256, 8, 16, 64
+    rng = np.random.default_rng(kb)
+    init = _perturb(tb.layerstack_default_init(fs, F, l1, l2, 9), rng, ["ft_w", "ft_b", "l1_b", "l1_shared_bias", "l2_b", "l3_b"])
+    d = random_index_batch(rng, B, fs.max_active, fs.piece_inputs, 1, fs.max_active)
+    for key in ("stm", "nstm"):
+        d[key] = np.where(d[key] >= 0, d[key] + rng.integers(0, kb, B)[:, None] * fs.piece_inputs, d[key]).astype(np.int32)
+    tr = tb.GpuTrainer(B, F, l1, l2, 9, fs, optimizer="ranger", init=init)
+    ot = _oracle_for(tr, "layerstack", fs, F, l1, l2, 9, "ranger", (0.01, 0.01, 0.01), B)
+    _sync_weights(tr, ot, init)
+    batch = tb.BatchData(d["stm"], d["nstm"], d["nnz"], d["score"], d["wdl"], d["bucket"])
+    for _ in range(7):
+        tr.train_step(batch, 1e-3, 0.0, tb.LossKind.sigmoid())
+        ot.step(d, 1e-3, 0.0, O.sigmoid_loss())
+    got = tr.download_group("ft_w", ("w", "m", "v", "slow"))
+    assert_close(got["w"], ot.group("ft_w"), 1e-5, "w")
+    assert_close(got["slow"], ot.group("ft_w", "slow"), 1e-5, "slow")
+    assert_close_scaled(got["m"], ot.group("ft_w", "m"), 1e-4, "m")
+    assert_close_scaled(got["v"], ot.group("ft_w", "v"), 1e-4, "v")
+    w = got["w"].reshape(kb + 1, -1)
+    assert np.array_equal(tr.read_buffer("comb", fs.ft_in * F), (w[:kb] + w[kb:]).reshape(-1))
