@@ -121,6 +121,9 @@ int launch_inverse_slice(cudaStream_t s, const int* item_seg, int* fwd_work, int
 int launch_ft_backward_slice(cudaStream_t s, const void* dft_stm, const void* dft_nstm, int* fwd_work, int* bwd_work, int B,
                              int A, int N, int F, int rows_per_slice, int n_persp, int part, int parts, float* grad,
                              float* slabs, int dft_half = 0);
+// *outside = 1 (memory the host sees) when a position of the batch has a row outside the slice of its first one
+int launch_slice_check(cudaStream_t s, const int* idx_stm, const int* idx_nstm, const int* nnz, int B, int A, int N,
+                       int rows_per_slice, int* outside);
 int sort_max_units(int max_tiles);
 // The two sorts of a step: positions by bucket -> order, bucket segments seg_start [nb + 2], tiles (room for max_tiles
 // tiles followed by the work units; n_tiles is {tile count, unit count}); items (position, perspective) of both
@@ -141,7 +144,7 @@ int launch_cast_half(cudaStream_t s, const float* src, void* dst, int64_t n);
 int launch_psv_extract(cudaStream_t s, int feature_set, const void* d_psv, long long n, int* stm, int* nstm, int* nnz,
                        int* bucket, float* score, float* wdl);
 void psv_extract_trim();
-bool psv_feature_set_dims(int feature_set, int* ft_in, int* max_active);
+bool psv_feature_set_dims(int feature_set, int* ft_in, int* max_active, int* piece_inputs);
 
 // dense_kernels.cu
 // tf32: run the contraction on the tensor cores with TF32 operands (l1_tc.cu) where the shape allows; error_flag: device

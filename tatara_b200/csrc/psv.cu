@@ -395,12 +395,13 @@ int launch_psv_extract(cudaStream_t s, int feature_set, const void* d_psv, long 
     return 1;
 }
 
-// dimensions of a feature set id: rows of the FT table and slots per perspective (feature_set.rs:1031-1038)
-bool psv_feature_set_dims(int feature_set, int* ft_in, int* max_active) {
+// dimensions of a feature set id: rows of the FT table, slots per perspective, rows per king bucket (feature_set.rs:1031-1038)
+bool psv_feature_set_dims(int feature_set, int* ft_in, int* max_active, int* piece_inputs) {
     FsSpec spec;
     if (!fs_spec(feature_set, &spec)) return false;
     *ft_in = (spec.mirror ? 45 : 81) * spec.piece_inputs;
     *max_active = spec.max_active;
+    *piece_inputs = spec.piece_inputs;
     return true;
 }
 

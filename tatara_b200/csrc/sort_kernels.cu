@@ -317,6 +317,36 @@ __global__ void __launch_bounds__(PLAN_THREADS) k_step_plans(const int* __restri
     else plan_backward(s_seg, n_keys, ch, parts, chunks, n_chunks, groups, sched);
 }
 
+// The question k_fwd_codes answers for the device, asked as soon as the batch is there, for the host: the slice of an item
+// is that of its first feature (ItemKey), slots beyond nnz and indices outside the table do not count.  A warp per position.
+__global__ void __launch_bounds__(256) k_slice_check(const int* __restrict__ idx_stm, const int* __restrict__ idx_nstm,
+                                                     const int* __restrict__ nnz, int B, int A, int N, int rps, int* outside) {
+    const int lane = threadIdx.x & 31;
+    bool out = false;
+    for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < B; b += (gridDim.x * blockDim.x) >> 5) {
+        const int n = min(max(nnz[b], 0), A);
+        for (int p = 0; p < 2; ++p) {
+            const int* ip = (p ? idx_nstm : idx_stm) + (size_t)b * A;
+            int slice = 0;
+            for (int q = lane; q < ((n + 31) & ~31); q += 32) {
+                const int f = q < n ? ip[q] : -1;
+                const int k = (unsigned)f < (unsigned)N ? f / rps : -1;
+                if (q < 32) slice = __shfl_sync(0xffffffffu, k, 0);
+                out = out || (k >= 0 && k != slice);
+            }
+        }
+    }
+    if (out) *outside = 1;
+}
+
+int launch_slice_check(cudaStream_t s, const int* idx_stm, const int* idx_nstm, const int* nnz, int B, int A, int N, int rows_per_slice,
+                       int* outside) {
+    if (B <= 0) return 0;
+    const int blocks = ceil_div(B, 8);
+    k_slice_check<<<blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, s>>>(idx_stm, idx_nstm, nnz, B, A, N, rows_per_slice, outside);
+    return 1;
+}
+
 int sort_max_units(int max_tiles) { return max_tiles / TB_UNIT_TILES + TB_MAX_BUCKETS + 2; }
 
 // Both sorts of a step in four launches: positions by bucket (order, tiles, units) and items by table slice, with the plans

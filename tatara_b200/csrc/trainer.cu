@@ -115,6 +115,11 @@ struct DevBatch {
     float *score = nullptr, *wdl = nullptr;
     int n_pos = 0;
     float norm = 0.f;
+    // Does some item have a row outside its king-bucket slice?  *outside (page-locked, written by the device) once `checked`
+    // has happened; a batch of extracted records has none.
+    int* outside = nullptr;
+    bool inside_known = false;
+    cudaEvent_t checked = nullptr;
 };
 
 struct HostStage {
@@ -360,6 +365,11 @@ int upload_batch(tb_trainer* t, const tb_batch* b, DevBatch* d, HostStage* st, c
     if (n * A * 4 > UPLOAD_PIECE) host_parallel((int)staged.size(), copy, send);
     else for (int i = 0; i < (int)staged.size(); ++i) { copy(i); send(i); }  // a small batch: waking a thread costs more than copying
     CU(t, e);
+    d->inside_known = false;
+    *d->outside = 0;
+    t->launches += launch_slice_check(cs, d->stm, d->nstm, d->nnz, b->n_pos, t->cfg.max_active, t->cfg.ft_in,
+                                      t->cfg.piece_inputs > 0 ? t->cfg.piece_inputs : t->cfg.ft_in, d->outside);
+    CU(t, cudaEventRecord(d->checked, cs));
     d->n_pos = b->n_pos;
     d->norm = b->per_pos_norm != 0.f ? b->per_pos_norm : 1.0f / ((float)b->n_pos * (float)t->cfg.world_size);
     return TB_OK;
@@ -510,14 +520,22 @@ int run_backward(tb_trainer* t, const DevBatch& d, float lr) {
     const void* dft1 = t->p_out16 ? t->dft_h[1] : (const void*)t->dft[1];
     const bool slice_bwd = t->slice_fwd && t->bwd_slice != nullptr;
     const int* gate = slice_bwd ? ft_slice_outside_flag(t->fwd_work, 2 * B, N, rps) : nullptr;
+    // The generic kernels are launched only for a batch that needs them.  The host knows by now: the check ran behind the
+    // upload, and what was launched above keeps the GPU busy (ten launches that found nothing to do were 28 us of every step).
+    bool generic = true;
+    if (slice_bwd) {
+        if (!d.inside_known) CU(t, cudaEventSynchronize(d.checked));
+        generic = !d.inside_known && *d.outside != 0;
+    }
     { PhaseScope p(t, PH_INV_INDEX);
       int n = 0;
       if (slice_bwd) n += launch_inverse_slice(t->stream, t->item_seg, t->fwd_work, t->bwd_slice, B, A, N, rps, 2);
-      n += launch_inverse_index(t->stream, gate, d.stm, d.nstm, d.nnz, B, A, N, 2, t->feat_counts, t->feat_offsets, t->feat_cursor,
+      if (generic) n += launch_inverse_index(t->stream, gate, d.stm, d.nstm, d.nnz, B, A, N, 2, t->feat_counts, t->feat_offsets, t->feat_cursor,
                                 t->feat_lists);
       p.done(n); }
     { PhaseScope p(t, PH_FT_BWD);
-      int n = launch_ft_backward_split(t->stream, gate, dft0, dft1, t->feat_offsets, t->feat_lists, B, A, N, F, 2,
+      int n = 0;
+      if (generic) n = launch_ft_backward_split(t->stream, gate, dft0, dft1, t->feat_offsets, t->feat_lists, B, A, N, F, 2,
                                        t->bwd_plan, t->bwd_partial, t->groups[0].grad, t->p_out16);
       if (slice_bwd) {
           // Data parallel: the slices are done in several launches (ar_parts_for) and the gradient rows of each part are all-reduced on a
@@ -816,6 +834,7 @@ int ring_upload_psv(tb_trainer* t, int feature_set, const uint8_t* psv, int n_po
     t->launches += n;
     d.n_pos = n_pos;
     d.norm = 1.0f / ((float)n_pos * (float)t->cfg.world_size);
+    d.inside_known = true;  // a position's rows lie in its king's bucket by construction
     CU(t, cudaEventRecord(t->ev_upload[s], t->copy_stream));
     t->upload_pending[s] = true;
     CU(t, cudaStreamWaitEvent(t->stream, t->ev_upload[s], 0));
@@ -838,7 +857,8 @@ void free_all(tb_trainer* t) {
     cudaFree(t->table_h); cudaFree(t->ft_m_h); cudaFree(t->ft_v_h); cudaFree(t->clamp_counter);
     cudaFree(t->tc_error); cudaFreeHost(t->tc_error_pinned);
     for (int i = 0; i < 2; ++i) { cudaFree(t->pre_h[i]); cudaFree(t->dft_h[i]); }
-    auto free_batch = [](DevBatch& d) { cudaFree(d.stm); cudaFree(d.nstm); cudaFree(d.nnz); cudaFree(d.bucket); cudaFree(d.score); cudaFree(d.wdl); };
+    auto free_batch = [](DevBatch& d) { cudaFree(d.stm); cudaFree(d.nstm); cudaFree(d.nnz); cudaFree(d.bucket); cudaFree(d.score); cudaFree(d.wdl);
+                                         cudaFreeHost(d.outside); if (d.checked) cudaEventDestroy(d.checked); };
     for (auto& d : t->ring) free_batch(d);
     for (auto& d : t->slots) free_batch(d);
     for (int i = 0; i < 2; ++i) { cudaFree(t->ring_psv[i]); cudaFreeHost(t->stage_psv[i]); }
@@ -878,6 +898,8 @@ int alloc_batch(tb_trainer* t, DevBatch* d) {
     const size_t B = (size_t)t->cfg.batch_capacity, A = (size_t)t->cfg.max_active;
     CU(t, dalloc(&d->stm, B * A)); CU(t, dalloc(&d->nstm, B * A)); CU(t, dalloc(&d->nnz, B)); CU(t, dalloc(&d->bucket, B));
     CU(t, dalloc(&d->score, B)); CU(t, dalloc(&d->wdl, B));
+    CU(t, cudaHostAlloc((void**)&d->outside, sizeof(int), cudaHostAllocDefault));
+    CU(t, cudaEventCreateWithFlags(&d->checked, cudaEventDisableTiming));
     return TB_OK;
 }
 
@@ -1273,8 +1295,8 @@ int tb_train_step_psv(tb_trainer* t, int feature_set, const uint8_t* psv, int n_
     if (n_pos > t->cfg.batch_capacity)
         return fail(t, TB_ERR_INVALID_ARGUMENT, "batch %d exceeds workspace capacity %d (the workspace is allocated once at creation)",
                     n_pos, t->cfg.batch_capacity);
-    int fs_in = 0, fs_active = 0;
-    if (!psv_feature_set_dims(feature_set, &fs_in, &fs_active)) return fail(t, TB_ERR_INVALID_ARGUMENT, "unknown feature set id %d", feature_set);
+    int fs_in = 0, fs_active = 0, fs_rows = 0;
+    if (!psv_feature_set_dims(feature_set, &fs_in, &fs_active, &fs_rows)) return fail(t, TB_ERR_INVALID_ARGUMENT, "unknown feature set id %d", feature_set);
     // the batch's feature set must be the trainer's (bins/nnue_train/src/trainer_common.rs:301-307)
     if (fs_in != t->cfg.ft_in || fs_active != t->cfg.max_active)
         return fail(t, TB_ERR_INVALID_ARGUMENT, "feature set %d has ft_in %d / max_active %d, the trainer was created with %d / %d",
@@ -1283,6 +1305,11 @@ int tb_train_step_psv(tb_trainer* t, int feature_set, const uint8_t* psv, int n_
     int s = 0;
     rc = ring_upload_psv(t, feature_set, psv, n_pos, &s);
     if (rc != TB_OK) return rc;
+    if (fs_rows != t->cfg.piece_inputs) {  // slices of the caller's own making: not known to hold a position's rows
+        t->ring[s].inside_known = false;
+        *t->ring[s].outside = 1;
+        CU(t, cudaEventRecord(t->ring[s].checked, t->copy_stream));
+    }
     rc = step_on(t, t->ring[s], lr, wdl_lambda, loss, loss_prev);
     if (rc != TB_OK) return rc;
     CU(t, cudaEventRecord(t->ev_consumed[s], t->stream));

@@ -66,3 +66,29 @@ def test_factorized_optimizer_king_bucket_counts(kb):
     assert_close_scaled(got["v"], ot.group("ft_w", "v"), 1e-4, "v")
     w = got["w"].reshape(kb + 1, -1)
     assert np.array_equal(tr.read_buffer("comb", fs.ft_in * F), (w[:kb] + w[kb:]).reshape(-1))
+
+
+def test_steps_alternate_between_inside_and_outside_batches():
+    """The generic gradient kernels are launched only for the batches that have a row outside its slice: training steps on
+    such a mix leave what gradient and optimizer run apart leave."""
+    F, l1, l2, B = 256, 8, 16, 256
+    fs = tb.FEATURE_SETS["halfka-hm-merged"]
+    rng = np.random.default_rng(5)
+    init = _perturb(tb.layerstack_default_init(fs, F, l1, l2, 9), rng, ["ft_b", "l1_b", "l1_shared_bias", "l2_b", "l3_b"])
+    init["ft_w"][:fs.ft_in * F] *= 30.0
+    a, b, c = (tb.GpuTrainer(B, F, l1, l2, 9, fs, optimizer="adamw", init=init) for _ in range(3))
+    loss = tb.LossKind.sigmoid()
+    for i in range(8):
+        batch = tb.synthetic_batch(tb.SYNTH_SEED + i, B, fs)
+        if i in (1, 2, 5):
+            batch.nstm_indices[i, 3] = (batch.nstm_indices[i, 4] + fs.piece_inputs) % fs.ft_in
+        a.train_step(batch, 1e-3, 0.25, loss)
+        b.forward_backward(batch, 0.25, loss)
+        b.apply_optimizer(1e-3)
+        c.stage_batch(i % 3, batch)
+        c.train_step_staged(i % 3, 1e-3, 0.25, loss)
+    for name in a.group_names:
+        x = a.download_group(name, ("w", "m", "v"))
+        for other in (b, c):
+            y = other.download_group(name, ("w", "m", "v"))
+            assert all(np.array_equal(x[k].view(np.uint32), y[k].view(np.uint32)) for k in x), name
