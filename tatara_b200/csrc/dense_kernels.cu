@@ -360,14 +360,21 @@ __global__ void __launch_bounds__(4 * L1) k_l1_forward_stream(const float* __res
     }
 }
 
+static inline bool l1_streams(int K, int l1) { return (l1 == 8 || l1 == 16 || l1 == 32) && K % LF_KC == 0; }
+
+int launch_l1_weff(cudaStream_t s, const float* wb, const float* bb, const float* ws, const float* bs, int K, int l1, int nb, float* weff) {
+    if (!l1_streams(K, l1)) return 0;
+    k_l1_weff<<<dim3(ceil_div(l1 * K, 256 * 4), nb + 1), 256, 0, s>>>(wb, bb, ws, bs, K, l1, wb ? nb : 0, weff, weff + (size_t)(nb + 1) * l1 * K);
+    return 1;
+}
+
 int launch_l1_forward(cudaStream_t s, const float* x, int K, const int* order, const TileDesc* tiles,
                       const int* n_tiles, int max_tiles, const float* wb, const float* bb, const float* ws,
-                      const float* bs, float* y, int l1, int nb, float* weff, int tf32, int* error_flag) {
-    if ((l1 == 8 || l1 == 16 || l1 == 32) && K % LF_KC == 0 && weff != nullptr) {
-        float* beff = weff + (size_t)(nb + 1) * l1 * K;
-        k_l1_weff<<<dim3(ceil_div(l1 * K, 256 * 4), nb + 1), 256, 0, s>>>(wb, bb, ws, bs, K, l1, wb ? nb : 0, weff, beff);
+                      const float* bs, float* y, int l1, int nb, const float* weff, int tf32, int* error_flag) {
+    if (l1_streams(K, l1)) {
+        const float* beff = weff + (size_t)(nb + 1) * l1 * K;
         if (tf32 && error_flag && l1_forward_tc_supported(K, l1))
-            return 1 + launch_l1_forward_tc(s, x, K, order, tiles, n_tiles, max_tiles, weff, beff, y, l1, wb ? nb : 0, error_flag);
+            return launch_l1_forward_tc(s, x, K, order, tiles, n_tiles, max_tiles, weff, beff, y, l1, wb ? nb : 0, error_flag);
         const int max_units = sort_max_units(max_tiles);
         const size_t smem = (size_t)LF_STAGES * (LF_POS + l1) * LF_LD * sizeof(float);
         const TileDesc* units = tiles + max_tiles;
@@ -375,7 +382,7 @@ int launch_l1_forward(cudaStream_t s, const float* x, int K, const int* order, c
         if (l1 == 8) k_l1_forward_stream<8><<<2 * max_units, 32, smem, s>>>(x, K, order, tiles, units, n_tiles + 1, weff, beff, y, nbe);
         else if (l1 == 16) k_l1_forward_stream<16><<<2 * max_units, 64, smem, s>>>(x, K, order, tiles, units, n_tiles + 1, weff, beff, y, nbe);
         else k_l1_forward_stream<32><<<2 * max_units, 128, smem, s>>>(x, K, order, tiles, units, n_tiles + 1, weff, beff, y, nbe);
-        return 2;
+        return 1;
     }
     const int nout = wb ? 2 * l1 : l1;
     if (l1 % 4 == 0 && nout <= 64) {

@@ -141,6 +141,13 @@ struct tb_trainer {
     tb_config cfg;
     std::string err;
     cudaStream_t stream = nullptr, copy_stream = nullptr;
+    // Work that the step's main chain does not wait for.  side[0]: the inverse index beside the dense layers, then the small
+    // layers' weight gradients; side[1]: the L1 weight gradient, then the update of all small groups beside the FT gradient
+    // and its update.  (With both weight gradients in one stream the second starved behind the FT gradient, whose blocks
+    // hold whole SMs: F = 1536, B = 65 536 4.34 ms against 4.21.)
+    cudaStream_t side[2] = {nullptr, nullptr};
+    cudaEvent_t ev_begin = nullptr, ev_weff = nullptr, ev_fwd = nullptr, ev_inv = nullptr, ev_tail = nullptr, ev_dense = nullptr, ev_wgrad = nullptr, ev_small = nullptr;
+    bool wgrad_forked = false;  // the side streams hold work of this step that the main stream has not joined
     std::vector<Group> groups;
     float* grad_arena = nullptr;
     int64_t arena_len = 0, arena_reduce_len = 0;
@@ -367,8 +374,9 @@ int upload_batch(tb_trainer* t, const tb_batch* b, DevBatch* d, HostStage* st, c
     CU(t, e);
     d->inside_known = false;
     *d->outside = 0;
-    t->launches += launch_slice_check(cs, d->stm, d->nstm, d->nnz, b->n_pos, t->cfg.max_active, t->cfg.ft_in,
-                                      t->cfg.piece_inputs > 0 ? t->cfg.piece_inputs : t->cfg.ft_in, d->outside);
+    // (not counted in `launches`: part of the upload, which a staged batch pays once)
+    launch_slice_check(cs, d->stm, d->nstm, d->nnz, b->n_pos, t->cfg.max_active, t->cfg.ft_in,
+                       t->cfg.piece_inputs > 0 ? t->cfg.piece_inputs : t->cfg.ft_in, d->outside);
     CU(t, cudaEventRecord(d->checked, cs));
     d->n_pos = b->n_pos;
     d->norm = b->per_pos_norm != 0.f ? b->per_pos_norm : 1.0f / ((float)b->n_pos * (float)t->cfg.world_size);
@@ -414,6 +422,26 @@ int check_loss(tb_trainer* t, const tb_loss* l) {
 }
 
 // ---- the step ------------------------------------------------------------------------------------------
+// `to` goes on when what is in `from` now is done
+int order_after(tb_trainer* t, cudaEvent_t ev, cudaStream_t from, cudaStream_t to) {
+    if (from == to) return TB_OK;
+    CU(t, cudaEventRecord(ev, from));
+    CU(t, cudaStreamWaitEvent(to, ev, 0));
+    return TB_OK;
+}
+#define AFTER(ev, from, to) do { const int arc_ = order_after(t, ev, from, to); if (arc_ != TB_OK) return arc_; } while (0)
+// per-phase timing brackets phases with events on the main stream: everything runs there then
+cudaStream_t side_stream(tb_trainer* t, int i) { return t->profile ? t->stream : t->side[i]; }
+
+// the main stream waits for the dense weight gradients (and their update)
+int join_wgrad(tb_trainer* t) {
+    if (!t->wgrad_forked) return TB_OK;
+    t->wgrad_forked = false;
+    AFTER(t->ev_wgrad, t->side[1], t->stream);
+    AFTER(t->ev_small, t->side[0], t->stream);
+    return TB_OK;
+}
+
 int run_forward(tb_trainer* t, const DevBatch& d, const tb_loss* loss, float lambda, int backward) {
     const tb_config& c = t->cfg;
     const int B = d.n_pos, F = c.ft_out, N = c.ft_in, A = c.max_active;
@@ -425,6 +453,15 @@ int run_forward(tb_trainer* t, const DevBatch& d, const tb_loss* loss, float lam
     const int rps = c.piece_inputs > 0 ? c.piece_inputs : N;
     t->slice_fwd = ft_forward_slice_supported(F, N, A, rps);
     if (backward) { t->opt_begun = false; t->ft_rows_updated = false; }
+    // the effective L1 weights depend on nothing of this batch
+    if (ls) {
+        AFTER(t->ev_begin, t->stream, side_stream(t, 1));
+        t->launches += launch_l1_weff(side_stream(t, 1), t->groups[2].w, t->groups[3].w, t->groups[4].w, t->groups[5].w, F, c.l1_out, c.num_buckets, t->l1_weff);
+    } else {
+        AFTER(t->ev_begin, t->stream, side_stream(t, 1));
+        t->launches += launch_l1_weff(side_stream(t, 1), nullptr, nullptr, t->groups[2].w, t->groups[3].w, t->K, c.l1_out, 0, t->l1_weff);
+    }
+    if (side_stream(t, 1) != t->stream) CU(t, cudaEventRecord(t->ev_weff, side_stream(t, 1)));
     { PhaseScope p(t, PH_SORT);
       // positions by bucket (order, tiles, units) and items of both perspectives by the king-bucket slice of the FT table
       int n = launch_step_sorts(t->stream, ls ? d.bucket : nullptr, B, ls ? c.num_buckets : 0, t->order, t->tiles, t->n_tiles,
@@ -441,6 +478,8 @@ int run_forward(tb_trainer* t, const DevBatch& d, const tb_loss* loss, float lam
       else
           p.done(launch_ft_forward(t->stream, mode, table, d.stm, d.nstm, d.nnz, t->groups[1].w, pre0, pre1, t->combined,
                                    t->items, B, F, N, A, FT_POST_SCALE, 2, t->p_ft16, t->p_out16)); }
+    if (backward && side_stream(t, 0) != t->stream) CU(t, cudaEventRecord(t->ev_fwd, t->stream));
+    if (side_stream(t, 1) != t->stream) CU(t, cudaStreamWaitEvent(t->stream, t->ev_weff, 0));
     LossParams lp = make_loss(loss, lambda, d.norm);
     if (lp.extended) {  // the weight sum of this batch first (trainer_simple.rs:1430-1478 launches wrm_weight_sum before loss_wrm)
         PhaseScope p(t, PH_TAIL);
@@ -478,14 +517,29 @@ int run_backward(tb_trainer* t, const DevBatch& d, float lr) {
     const tb_config& c = t->cfg;
     const int B = d.n_pos, F = c.ft_out, N = c.ft_in, A = c.max_active;
     const bool ls = c.arch == TB_ARCH_LAYERSTACK;
+    const int rps = c.piece_inputs > 0 ? c.piece_inputs : N;
+    const bool slice_bwd = t->slice_fwd && t->bwd_slice != nullptr;
+    const cudaStream_t si = side_stream(t, 0), sw = side_stream(t, 1);
+    // The inverse index needs the forward's row codes alone: it runs beside the dense layers, whose kernels leave most of the
+    // chip free (10 to 15 % of its warps).  In profile mode it is launched where its phase is.
+    auto inverse = [&]() { return slice_bwd ? launch_inverse_slice(si, t->item_seg, t->fwd_work, t->bwd_slice, B, A, N, rps, 2) : 0; };
+    if (si != t->stream) {
+        CU(t, cudaStreamWaitEvent(si, t->ev_fwd, 0));
+        t->launches += inverse();
+        CU(t, cudaEventRecord(t->ev_inv, si));
+    }
+    // the weight gradients of the dense layers wait for the tail alone, and nothing but their update waits for them
+    AFTER(t->ev_tail, t->stream, sw);
+    if (si != t->stream) CU(t, cudaStreamWaitEvent(si, t->ev_tail, 0));
+    t->wgrad_forked = sw != t->stream;
     if (ls) {
         { PhaseScope p(t, PH_SMALL_WGRAD);
-          p.done(launch_small_wgrad_layerstack(t->stream, t->order, t->seg_start, B, c.l1_out, c.l2_out, c.num_buckets, t->tail_a,
+          p.done(launch_small_wgrad_layerstack(si, t->order, t->seg_start, B, c.l1_out, c.l2_out, c.num_buckets, t->tail_a,
                                                t->tail_b, t->tail_c, t->dy, t->dl1, t->small_partials, t->groups[6].grad,
                                                t->groups[7].grad, t->groups[8].grad, t->groups[9].grad, t->groups[3].grad,
                                                t->groups[5].grad)); }
         { PhaseScope p(t, PH_L1_WGRAD);
-          p.done(launch_l1_wgrad(t->stream, t->combined, F, t->dl1, t->order, t->tiles, t->n_tiles, t->max_tiles, c.l1_out,
+          p.done(launch_l1_wgrad(sw, t->combined, F, t->dl1, t->order, t->tiles, t->n_tiles, t->max_tiles, c.l1_out,
                                  c.num_buckets, t->l1w_partials, t->groups[2].grad, t->groups[4].grad)); }
         { PhaseScope p(t, PH_L1_DGRAD);
           // fp16 dft rows carry gradient * 2^14 * batch (trainer_layerstack.rs:3617-3621); the FT weight gradient is summed
@@ -501,11 +555,11 @@ int run_backward(tb_trainer* t, const DevBatch& d, float lr) {
                                         t->dgrad_rows, t->p_out16, dft_scale, t->clamp_counter)); }
     } else {
         { PhaseScope p(t, PH_SMALL_WGRAD);
-          p.done(launch_small_wgrad_simple(t->stream, t->order, t->seg_start, B, c.l1_out, c.l2_out, t->tail_a, t->tail_b,
+          p.done(launch_small_wgrad_simple(si, t->order, t->seg_start, B, c.l1_out, c.l2_out, t->tail_a, t->tail_b,
                                            t->tail_c, t->dy, t->dl1, t->small_partials, t->groups[4].grad, t->groups[5].grad,
                                            t->groups[6].grad, t->groups[7].grad, t->groups[3].grad)); }
         { PhaseScope p(t, PH_L1_WGRAD);
-          p.done(launch_l1_wgrad(t->stream, t->combined, t->K, t->dl1, t->order, t->tiles, t->n_tiles, t->max_tiles, c.l1_out, 0,
+          p.done(launch_l1_wgrad(sw, t->combined, t->K, t->dl1, t->order, t->tiles, t->n_tiles, t->max_tiles, c.l1_out, 0,
                                  t->l1w_partials, nullptr, t->groups[2].grad)); }
         { PhaseScope p(t, PH_L1_DGRAD);
           p.done(launch_l1_dgrad_ftgrad(t->stream, c.activation == TB_ACT_PAIRWISE ? 1 : (c.activation == TB_ACT_CRELU ? 2 : 3), t->dl1, t->order, t->tiles, t->n_tiles,
@@ -515,10 +569,8 @@ int run_backward(tb_trainer* t, const DevBatch& d, float lr) {
     }
     // slice-resident path when this step's forward was; the generic kernels then run only for a batch with a row outside
     // its item's slice (device-side gate)
-    const int rps = c.piece_inputs > 0 ? c.piece_inputs : N;
     const void* dft0 = t->p_out16 ? t->dft_h[0] : (const void*)t->dft[0];
     const void* dft1 = t->p_out16 ? t->dft_h[1] : (const void*)t->dft[1];
-    const bool slice_bwd = t->slice_fwd && t->bwd_slice != nullptr;
     const int* gate = slice_bwd ? ft_slice_outside_flag(t->fwd_work, 2 * B, N, rps) : nullptr;
     // The generic kernels are launched only for a batch that needs them.  The host knows by now: the check ran behind the
     // upload, and what was launched above keeps the GPU busy (ten launches that found nothing to do were 28 us of every step).
@@ -529,10 +581,14 @@ int run_backward(tb_trainer* t, const DevBatch& d, float lr) {
     }
     { PhaseScope p(t, PH_INV_INDEX);
       int n = 0;
-      if (slice_bwd) n += launch_inverse_slice(t->stream, t->item_seg, t->fwd_work, t->bwd_slice, B, A, N, rps, 2);
+      if (si == t->stream) n += inverse();
+      else CU(t, cudaStreamWaitEvent(t->stream, t->ev_inv, 0));
       if (generic) n += launch_inverse_index(t->stream, gate, d.stm, d.nstm, d.nnz, B, A, N, 2, t->feat_counts, t->feat_offsets, t->feat_cursor,
                                 t->feat_lists);
       p.done(n); }
+    // the first exchanged part carries the small groups' gradients; a call for gradients alone returns with all of them
+    if (c.world_size > 1 || lr < 0.0f) { const int jrc = join_wgrad(t); if (jrc != TB_OK) return jrc; }
+    else if (t->wgrad_forked) CU(t, cudaEventRecord(t->ev_dense, t->stream));
     { PhaseScope p(t, PH_FT_BWD);
       int n = 0;
       if (generic) n = launch_ft_backward_split(t->stream, gate, dft0, dft1, t->feat_offsets, t->feat_lists, B, A, N, F, 2,
@@ -729,9 +785,15 @@ int run_optimizer(tb_trainer* t, float lr) {
             s.max_w = g.clamp;
             if (s.n > max_n) max_n = s.n;
         }
-        p.done(launch_radam_small(t->stream, sg, max_n, sc));
+        // beside the FT table's update, once the FT bias gradient is there and the L1 weights have been read
+        const cudaStream_t ss = t->wgrad_forked ? t->side[1] : t->stream;
+        if (t->wgrad_forked) {
+            CU(t, cudaStreamWaitEvent(ss, t->ev_dense, 0));
+            AFTER(t->ev_small, t->side[0], ss);
+        }
+        p.done(launch_radam_small(ss, sg, max_n, sc));
     }
-    return TB_OK;
+    return join_wgrad(t);
 }
 
 // Waits for a loss read-back.  With the peer exchange a lost peer shows as a stream that never finishes (its flags never
@@ -849,6 +911,8 @@ void free_all(tb_trainer* t) {
     if (!t) return;
     if (t->stream) cudaStreamSynchronize(t->stream);
     if (t->copy_stream) cudaStreamSynchronize(t->copy_stream);
+    for (cudaStream_t s : t->side) if (s) { cudaStreamSynchronize(s); cudaStreamDestroy(s); }
+    for (cudaEvent_t e : {t->ev_begin, t->ev_weff, t->ev_fwd, t->ev_inv, t->ev_tail, t->ev_dense, t->ev_wgrad, t->ev_small}) if (e) cudaEventDestroy(e);
     if (t->comm && g_nccl.CommDestroy) g_nccl.CommDestroy(t->comm);
     for (auto& g : t->groups) { cudaFree(g.w); cudaFree(g.m); cudaFree(g.v); cudaFree(g.slow); }
     px_destroy(t->px);
@@ -918,6 +982,9 @@ int create_impl(tb_trainer* t) {
         CU(t, cudaStreamCreateWithPriority(&t->stream, cudaStreamNonBlocking, mid));
     }
     CU(t, cudaStreamCreateWithFlags(&t->copy_stream, cudaStreamNonBlocking));
+    for (auto& s : t->side) CU(t, cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    for (cudaEvent_t* e : {&t->ev_begin, &t->ev_weff, &t->ev_fwd, &t->ev_inv, &t->ev_tail, &t->ev_dense, &t->ev_wgrad, &t->ev_small})
+        CU(t, cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     pinned_watch_stream(t->copy_stream);
     const bool ls = c.arch == TB_ARCH_LAYERSTACK;
     const int64_t N = c.ft_in, F = c.ft_out, l1 = c.l1_out, l2 = c.l2_out, nb = c.num_buckets;
