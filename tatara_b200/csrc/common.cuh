@@ -9,6 +9,8 @@
 #define TB_MAX_L2 64
 #define TB_TILE_M 32      // positions per dense tile; a tile never mixes LayerStack buckets
 #define TB_UNIT_TILES 8   // tiles per work unit (consecutive tiles of one bucket)
+// counts beside the tiles: {tiles, units, first unit of every bucket (and of the positions without one, and the end)}
+#define TB_TILE_COUNTS 16
 
 // One tile of positions for the bucket-grouped dense kernels: positions order[start .. start+count).
 // bucket == num_buckets marks positions whose bucket id is out of range (their per-bucket layers
@@ -126,7 +128,7 @@ int launch_slice_check(cudaStream_t s, const int* idx_stm, const int* idx_nstm, 
                        int rows_per_slice, int* outside);
 int sort_max_units(int max_tiles);
 // The two sorts of a step: positions by bucket -> order, bucket segments seg_start [nb + 2], tiles (room for max_tiles
-// tiles followed by the work units; n_tiles is {tile count, unit count}); items (position, perspective) of both
+// tiles followed by the work units; n_tiles: TB_TILE_COUNTS ints); items (position, perspective) of both
 // perspectives by the table slice of their features -> items, item_seg [slices + 2].  hist: scratch of
 // (nb + 1) * ceil(B / 1024) + (slices + 1) * ceil(n_persp * B / 1024) ints
 // fwd_work / bwd_work: also plan the slice-resident forward / weight gradient (the latter in bwd_parts launches over equal
@@ -172,6 +174,20 @@ int launch_tail_simple(cudaStream_t s, const float* l1_pre, const float* score, 
                        int act, int B, int l1, int l2, float* net_output, float* dy, float* dl1_pre,
                        float* l1_acted, float* dl2_pre, float* l2_acted, double* loss_partials,
                        double* loss_acc, int backward);
+// tail_kernels.cu: the same for l1 of 8, 16, 32 and l2 of 16, 32 (tail_tiled), with the blocks' sums of the small layers' weight
+// gradients; arch 0 LayerStack, 1 Simple CReLU, 2 Simple SCReLU.  partials: tail_partial_floats floats, loss_partials: one double
+// per block (tail_loss_blocks), summed by launch_reduce_double.
+bool tail_tiled(int l1, int l2);
+size_t tail_partial_floats(int arch, int l1, int l2, int max_tiles);
+int tail_loss_blocks(int max_tiles);
+int launch_tail(cudaStream_t s, int arch, const float* l1_rows, const int* order, const TileDesc* tiles, const int* n_tiles, int max_tiles,
+                const float* score, const float* wdl, const float* l2_w, const float* l2_b, const float* l3_w, const float* l3_b,
+                LossParams lp, int l1, int l2, int nb, float* net_output, float* dy, float* dl1, float* partials,
+                double* loss_partials, int backward);
+// the weight gradients from the blocks' sums; gb1_shared: LayerStack's shared L1 bias, else NULL
+int launch_tail_wgrad(cudaStream_t s, int arch, const float* partials, const int* n_tiles, int l1, int l2, int nb, float* gw2, float* gb2,
+                      float* gw3, float* gb3, float* gb1, float* gb1_shared);
+int launch_reduce_double(cudaStream_t s, const double* partials, int n, double* out);
 // per-bucket reductions of the small layers: out[g][cell] = sum over the positions of bucket g
 int launch_small_wgrad_layerstack(cudaStream_t s, const int* order, const int* seg_start, int B, int l1, int l2,
                                   int nb, const float* l2_input, const float* dl2_out, const float* l2_acted,

@@ -145,12 +145,14 @@ static __device__ void plan_tiles(const int* __restrict__ s_seg, int K, TileDesc
         for (int k = 0; k < K; ++k) {
             s_tile_base[k] = trun;
             s_unit_base[k] = urun;
+            n_tiles[2 + k] = urun;
             const int nt = (s_seg[k + 1] - s_seg[k] + TB_TILE_M - 1) / TB_TILE_M;
             trun += nt;
             urun += (nt + TB_UNIT_TILES - 1) / TB_UNIT_TILES;
         }
         s_tile_base[K] = trun;
         s_unit_base[K] = urun;
+        n_tiles[2 + K] = urun;
         *n_tiles = trun;
         *n_units = urun;
     }

@@ -442,6 +442,8 @@ int join_wgrad(tb_trainer* t) {
     return TB_OK;
 }
 
+int tail_arch(const tb_config& c) { return c.arch == TB_ARCH_LAYERSTACK ? 0 : c.activation == TB_ACT_SCRELU ? 2 : 1; }
+
 int run_forward(tb_trainer* t, const DevBatch& d, const tb_loss* loss, float lambda, int backward) {
     const tb_config& c = t->cfg;
     const int B = d.n_pos, F = c.ft_out, N = c.ft_in, A = c.max_active;
@@ -492,7 +494,7 @@ int run_forward(tb_trainer* t, const DevBatch& d, const tb_loss* loss, float lam
           p.done(launch_l1_forward(t->stream, t->combined, F, t->order, t->tiles, t->n_tiles, t->max_tiles, t->groups[2].w,
                                    t->groups[3].w, t->groups[4].w, t->groups[5].w, t->l1_out, c.l1_out, c.num_buckets, t->l1_weff,
                                    t->p_tf32, t->tc_error)); }
-        { PhaseScope p(t, PH_TAIL);
+        if (!tail_tiled(c.l1_out, c.l2_out)) { PhaseScope p(t, PH_TAIL);
           p.done(launch_tail_layerstack(t->stream, t->l1_out, d.bucket, d.score, d.wdl, t->groups[6].w, t->groups[7].w,
                                         t->groups[8].w, t->groups[9].w, lp, B, c.l1_out, c.l2_out, c.num_buckets,
                                         t->net_output, t->dy, t->dl1, t->tail_a, t->tail_b, t->tail_c, t->loss_partials,
@@ -501,10 +503,22 @@ int run_forward(tb_trainer* t, const DevBatch& d, const tb_loss* loss, float lam
         { PhaseScope p(t, PH_L1_FWD);
           p.done(launch_l1_forward(t->stream, t->combined, t->K, t->order, t->tiles, t->n_tiles, t->max_tiles, nullptr, nullptr,
                                    t->groups[2].w, t->groups[3].w, t->l1_out, c.l1_out, 0, t->l1_weff)); }
-        { PhaseScope p(t, PH_TAIL);
+        if (!tail_tiled(c.l1_out, c.l2_out)) { PhaseScope p(t, PH_TAIL);
           p.done(launch_tail_simple(t->stream, t->l1_out, d.score, d.wdl, t->groups[4].w, t->groups[5].w, t->groups[6].w,
                                     t->groups[7].w, lp, c.activation == TB_ACT_SCRELU ? 1 : 0, B, c.l1_out, c.l2_out, t->net_output, t->dy, t->dl1,
                                     t->tail_a, t->tail_b, t->tail_c, t->loss_partials, t->loss_acc, backward)); }
+    }
+    if (tail_tiled(c.l1_out, c.l2_out)) {
+        PhaseScope p(t, PH_TAIL);
+        const int g = ls ? 6 : 4;  // l2_w, l2_b, l3_w, l3_b
+        int n = launch_tail(t->stream, tail_arch(c), t->l1_out, t->order, t->tiles, t->n_tiles, t->max_tiles, d.score, d.wdl, t->groups[g].w,
+                            t->groups[g + 1].w, t->groups[g + 2].w, t->groups[g + 3].w, lp, c.l1_out, c.l2_out, ls ? c.num_buckets : 0,
+                            t->net_output, t->dy, t->dl1, t->small_partials, t->loss_partials, backward);
+        // in a training step nothing but the loss read-back waits for the sum
+        const cudaStream_t sl = backward ? side_stream(t, 1) : t->stream;
+        AFTER(t->ev_tail, t->stream, sl);
+        n += launch_reduce_double(sl, t->loss_partials, tail_loss_blocks(t->max_tiles), t->loss_acc);
+        p.done(n);
     }
     return TB_OK;
 }
@@ -532,8 +546,15 @@ int run_backward(tb_trainer* t, const DevBatch& d, float lr) {
     AFTER(t->ev_tail, t->stream, sw);
     if (si != t->stream) CU(t, cudaStreamWaitEvent(si, t->ev_tail, 0));
     t->wgrad_forked = sw != t->stream;
+    if (tail_tiled(c.l1_out, c.l2_out)) {
+        PhaseScope p(t, PH_SMALL_WGRAD);
+        const int g = ls ? 6 : 4;
+        p.done(launch_tail_wgrad(si, tail_arch(c), t->small_partials, t->n_tiles, c.l1_out, c.l2_out, ls ? c.num_buckets : 0, t->groups[g].grad,
+                                 t->groups[g + 1].grad, t->groups[g + 2].grad, t->groups[g + 3].grad, t->groups[3].grad,
+                                 ls ? t->groups[5].grad : nullptr));
+    }
     if (ls) {
-        { PhaseScope p(t, PH_SMALL_WGRAD);
+        if (!tail_tiled(c.l1_out, c.l2_out)) { PhaseScope p(t, PH_SMALL_WGRAD);
           p.done(launch_small_wgrad_layerstack(si, t->order, t->seg_start, B, c.l1_out, c.l2_out, c.num_buckets, t->tail_a,
                                                t->tail_b, t->tail_c, t->dy, t->dl1, t->small_partials, t->groups[6].grad,
                                                t->groups[7].grad, t->groups[8].grad, t->groups[9].grad, t->groups[3].grad,
@@ -554,7 +575,7 @@ int run_backward(tb_trainer* t, const DevBatch& d, float lr) {
                                         t->p_out16 ? t->dft_h[1] : (void*)t->dft[1], t->bias_partials, t->groups[1].grad,
                                         t->dgrad_rows, t->p_out16, dft_scale, t->clamp_counter)); }
     } else {
-        { PhaseScope p(t, PH_SMALL_WGRAD);
+        if (!tail_tiled(c.l1_out, c.l2_out)) { PhaseScope p(t, PH_SMALL_WGRAD);
           p.done(launch_small_wgrad_simple(si, t->order, t->seg_start, B, c.l1_out, c.l2_out, t->tail_a, t->tail_b,
                                            t->tail_c, t->dy, t->dl1, t->small_partials, t->groups[4].grad, t->groups[5].grad,
                                            t->groups[6].grad, t->groups[7].grad, t->groups[3].grad)); }
@@ -1084,10 +1105,12 @@ int create_impl(tb_trainer* t) {
     CU(t, dalloc(&t->wrm_weight_sum, 1));
     t->max_tiles = (int)(B / TB_TILE_M) + TB_MAX_BUCKETS + 2;
     t->max_units = sort_max_units(t->max_tiles);
-    CU(t, dalloc(&t->order, B)); CU(t, dalloc(&t->n_tiles, 2)); CU(t, dalloc(&t->seg_start, TB_MAX_BUCKETS + 3));
+    CU(t, dalloc(&t->order, B)); CU(t, dalloc(&t->n_tiles, TB_TILE_COUNTS)); CU(t, dalloc(&t->seg_start, TB_MAX_BUCKETS + 3));
     CU(t, dalloc(&t->tiles, (size_t)t->max_tiles + t->max_units));
     const size_t n_cells = ls ? (size_t)(l2 * t->l2in + 2 * l2 + 1 + l1) : (size_t)(l1 * l2 + 2 * l2 + 1 + l1);
-    CU(t, dalloc(&t->small_partials, (ls ? (size_t)(nb + 1) * 64 : (size_t)128) * n_cells));  // SW_SPLIT_LS partial rows per segment
+    size_t small = (ls ? (size_t)(nb + 1) * 64 : (size_t)128) * n_cells;  // SW_SPLIT_LS partial rows per segment
+    if (tail_tiled((int)l1, (int)l2)) small = tail_partial_floats(c.arch, (int)l1, (int)l2, t->max_tiles);
+    CU(t, dalloc(&t->small_partials, small));
     CU(t, dalloc(&t->l1w_partials, ((size_t)t->max_units + 1) * l1 * t->K));
     CU(t, dalloc(&t->l1_weff, (size_t)(nb + 1) * l1 * (t->K + 1)));  // effective L1 weights and biases per bucket
     t->dgrad_rows = DGRAD_CTAS > 2 * t->max_units ? DGRAD_CTAS : 2 * t->max_units;  // partial FT bias rows: one per block
