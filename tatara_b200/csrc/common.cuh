@@ -8,7 +8,11 @@
 #define TB_MAX_L1 32
 #define TB_MAX_L2 64
 #define TB_TILE_M 32      // positions per dense tile; a tile never mixes LayerStack buckets
-#define TB_UNIT_TILES 8   // tiles per work unit (consecutive tiles of one bucket)
+#define TB_UNIT_TILES 8   // most tiles of a work unit (consecutive tiles of one bucket)
+// Tiles per work unit for a batch: the dense kernels' blocks own half a unit and walk its positions one after the other, so a
+// batch that does not fill the chip with blocks of 128 positions gets smaller ones (B = 1024: the L1 input gradient took
+// 40 us on 16 of 148 SMs, 14 now).
+static inline int unit_tiles(int n_pos) { return n_pos >= 148 * 128 ? TB_UNIT_TILES : n_pos >= 148 * 64 ? 4 : 2; }
 // counts beside the tiles: {tiles, units, first unit of every bucket (and of the positions without one, and the end)}
 #define TB_TILE_COUNTS 16
 
@@ -127,6 +131,7 @@ int launch_ft_backward_slice(cudaStream_t s, const void* dft_stm, const void* df
 int launch_slice_check(cudaStream_t s, const int* idx_stm, const int* idx_nstm, const int* nnz, int B, int A, int N,
                        int rows_per_slice, int* outside);
 int sort_max_units(int max_tiles);
+int sort_units(int n_pos);  // the most work units a batch of n_pos positions has (sort_max_units: any batch of a trainer)
 // The two sorts of a step: positions by bucket -> order, bucket segments seg_start [nb + 2], tiles (room for max_tiles
 // tiles followed by the work units; n_tiles: TB_TILE_COUNTS ints); items (position, perspective) of both
 // perspectives by the table slice of their features -> items, item_seg [slices + 2].  hist: scratch of
@@ -154,13 +159,13 @@ bool psv_feature_set_dims(int feature_set, int* ft_in, int* max_active, int* pie
 int launch_l1_forward(cudaStream_t s, const float* x, int K, const int* order, const TileDesc* tiles,
                       const int* n_tiles, int max_tiles, const float* wb /*[nb][l1][K] or NULL*/,
                       const float* bb, const float* ws /*[K][l1]*/, const float* bs, float* y /*[B][l1]*/,
-                      int l1, int nb, const float* weff, int tf32 = 0, int* error_flag = nullptr);
+                      int l1, int nb, int n_pos, const float* weff, int tf32 = 0, int* error_flag = nullptr);
 // the effective weights and biases launch_l1_forward reads (l1 = 8, 16, 32; nothing otherwise): weff [(nb + 1) * l1 * (K + 1)]
 int launch_l1_weff(cudaStream_t s, const float* wb, const float* bb, const float* ws, const float* bs, int K, int l1, int nb, float* weff);
 // l1_tc.cu
 bool l1_forward_tc_supported(int K, int l1);
 int launch_l1_forward_tc(cudaStream_t s, const float* x, int K, const int* order, const TileDesc* tiles, const int* n_tiles,
-                         int max_tiles, const float* weff, const float* beff, float* y, int l1, int nb, int* error_flag);
+                         int max_tiles, int n_pos, const float* weff, const float* beff, float* y, int l1, int nb, int* error_flag);
 // sum over the batch of the extended WRM loss's per-position weights (wrm_weight_sum, native_kernels.cu:520-545), in a
 // fixed order; partials: scratch of ceil(B / 256) doubles
 int launch_wrm_weight_sum(cudaStream_t s, const float* score, int B, LossParams lp, double* partials, double* weight_sum);
@@ -179,8 +184,8 @@ int launch_tail_simple(cudaStream_t s, const float* l1_pre, const float* score, 
 // per block (tail_loss_blocks), summed by launch_reduce_double.
 bool tail_tiled(int l1, int l2);
 size_t tail_partial_floats(int arch, int l1, int l2, int max_tiles);
-int tail_loss_blocks(int max_tiles);
-int launch_tail(cudaStream_t s, int arch, const float* l1_rows, const int* order, const TileDesc* tiles, const int* n_tiles, int max_tiles,
+int tail_loss_blocks(int n_pos);
+int launch_tail(cudaStream_t s, int arch, int n_pos, const float* l1_rows, const int* order, const TileDesc* tiles, const int* n_tiles, int max_tiles,
                 const float* score, const float* wdl, const float* l2_w, const float* l2_b, const float* l3_w, const float* l3_b,
                 LossParams lp, int l1, int l2, int nb, float* net_output, float* dy, float* dl1, float* partials,
                 double* loss_partials, int backward);
@@ -200,7 +205,7 @@ int launch_small_wgrad_simple(cudaStream_t s, const int* order, const int* seg_s
                               float* l3_w_grad, float* l3_b_grad, float* l1_b_grad);
 // L1 weight gradient: LayerStack writes gw_bucket [nb][l1][K] and gw_shared [K][l1]; Simple only gw_shared.
 int launch_l1_wgrad(cudaStream_t s, const float* x, int K, const float* dl1, const int* order,
-                    const TileDesc* tiles, const int* n_tiles, int max_tiles, int l1, int nb, float* partials,
+                    const TileDesc* tiles, const int* n_tiles, int max_tiles, int n_pos, int l1, int nb, float* partials,
                     float* gw_bucket, float* gw_shared);
 // L1 input gradient fused with the FT activation gradient; writes dft of both perspectives and the
 // FT bias gradient.

@@ -247,10 +247,13 @@ __global__ void __launch_bounds__(64) k_l1_forward_tiled(const float* __restrict
 // ------------------------------------------------------------------------------------------------
 // L1 forward, streaming form for l1 = 8, 16 or 32.  The per-bucket and the shared layer see the same input and their
 // outputs are added, so they are one contraction with the effective weights weff[g] = wb[g] + ws^T (weff[nb] = ws^T for
-// positions without a bucket), built once per step by k_l1_weff.  A block owns 128 consecutive positions of the bucket
-// order (half a work unit); x rows and the weight rows arrive in K chunks of 16 through a three-stage ring of
-// asynchronous copies; a thread keeps a 4-position x 8-output tile of sums in registers and reads both operands as
-// 128-bit rows along k (row stride 20 floats: the rows a quarter warp touches fall into different banks).
+// positions without a bucket), built once per step by k_l1_weff.  A block owns up to 128 consecutive positions of the bucket
+// order, of one bucket; x rows and the weight rows arrive in K chunks of 64 through a three-stage ring of asynchronous
+// copies.  Every warp covers all of the block's positions and outputs for a quarter of each chunk's columns, so that a
+// thread's tile is large (RP positions x 8 outputs, two sums each for packed multiply-adds; RP = 8 has too few warps: 154 us) and an operand read from shared
+// memory is used often: the shared-memory pipe was what bound four-position tiles (128 us at K = 1536, l1 = 16, 65 536
+// positions; 113 now, the x rows at HBM rate take 62; K = 768, l1 = 8, 16 384 positions: 60 to 21 us).  Both operands are read as 128-bit rows along k; the row
+// stride spreads the rows a quarter warp touches over the banks.
 // ------------------------------------------------------------------------------------------------
 __global__ void k_l1_weff(const float* __restrict__ wb, const float* __restrict__ bb, const float* __restrict__ ws,
                           const float* __restrict__ bs, int K, int l1, int nb, float* __restrict__ weff, float* __restrict__ beff) {
@@ -270,93 +273,106 @@ __global__ void k_l1_weff(const float* __restrict__ wb, const float* __restrict_
     }
 }
 
-#define LF_POS 128
-#define LF_KC 16
-#define LF_LD 20
+#define LF_WARPS 4
+#define LF_KC 64       // columns per stage: 256 bytes of every row, a quarter of them for each warp
+#define LF_LD (LF_KC + 4)
 #define LF_STAGES 3
-static_assert(2 * LF_POS == TB_UNIT_TILES * TB_TILE_M, "a block of the streaming forward owns half a work unit");
-template <int L1>
-__global__ void __launch_bounds__(4 * L1) k_l1_forward_stream(const float* __restrict__ x, int K, const int* __restrict__ order,
+// x * w onto a pair of running sums (even and odd columns), one instruction for two multiply-adds
+static __device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long x, unsigned long long w) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(w));
+}
+template <int L1, int RP>
+struct L1Tile {
+    static constexpr int TX = L1 / 8, TY = 32 / TX, POS = TY * RP;  // a warp's threads over outputs and positions; positions of a block
+    static constexpr int STAGE_FLOATS = (POS + L1) * LF_LD;
+    static constexpr size_t SMEM = (size_t)LF_STAGES * STAGE_FLOATS * sizeof(float);
+    static_assert((size_t)LF_WARPS * POS * L1 <= (size_t)LF_STAGES * STAGE_FLOATS, "the warps' sums fit the ring");
+};
+template <int L1, int RP>
+__global__ void __launch_bounds__(32 * LF_WARPS) k_l1_forward_stream(const float* __restrict__ x, int K, const int* __restrict__ order,
                                                               const TileDesc* __restrict__ tiles, const TileDesc* __restrict__ units,
-                                                              const int* __restrict__ n_units, const float* __restrict__ weff,
+                                                              const int* __restrict__ n_units, int unit_blocks, const float* __restrict__ weff,
                                                               const float* __restrict__ beff, float* __restrict__ y, int nb) {
-    constexpr int TX = L1 / 8, TY = 32 / TX, NT = 32 * TX;
-    constexpr int STAGE_FLOATS = (LF_POS + L1) * LF_LD;
-    extern __shared__ __align__(16) float s_ring[];  // [LF_STAGES][LF_POS + L1][LF_LD]
-    __shared__ int s_pos[LF_POS];
-    const int u = blockIdx.x >> 1, h = blockIdx.x & 1;
+    typedef L1Tile<L1, RP> T;
+    constexpr int TX = T::TX, TY = T::TY, POS = T::POS, NT = 32 * LF_WARPS;
+    extern __shared__ __align__(16) float s_ring[];  // [LF_STAGES][POS + L1][LF_LD]
+    __shared__ int s_pos[POS];
+    const int u = blockIdx.x / unit_blocks, h = blockIdx.x - u * unit_blocks;
     if (u >= *n_units) return;
     const TileDesc ud = units[u];
-    const int per = LF_POS / TB_TILE_M;
+    constexpr int per = POS / TB_TILE_M;
     const int first = ud.start + h * per, last = min(ud.start + ud.count, first + per);
     if (first >= last) return;
     const int p_begin = tiles[first].start;
     const int n = tiles[last - 1].start + tiles[last - 1].count - p_begin;
     const int g = ud.bucket < nb ? ud.bucket : nb;
     const int tid = threadIdx.x;
-    for (int i = tid; i < LF_POS; i += NT) s_pos[i] = order[p_begin + (i < n ? i : 0)];  // rows past the end repeat the first
+    for (int i = tid; i < POS; i += NT) s_pos[i] = order[p_begin + (i < n ? i : 0)];  // rows past the end repeat the first
     __syncthreads();
     const float* __restrict__ wg = weff + (size_t)g * L1 * K;
     const int nk = K / LF_KC;
+    constexpr int PCS = LF_KC / 4;  // 16-byte pieces of a row's stage
     auto issue = [&](int it) {
         if (it < nk) {
-            float* st = s_ring + (size_t)(it % LF_STAGES) * STAGE_FLOATS;
+            float* st = s_ring + (size_t)(it % LF_STAGES) * T::STAGE_FLOATS;
             const int k0 = it * LF_KC;
-            for (int e = tid; e < LF_POS * 4; e += NT) {
-                const int r = e >> 2, pc = e & 3;
+#pragma unroll 8
+            for (int e = tid; e < POS * PCS; e += NT) {
+                const int r = e / PCS, pc = e % PCS;
                 dg_cp16(st + r * LF_LD + 4 * pc, x + (size_t)s_pos[r] * K + k0 + 4 * pc);
             }
-            for (int e = tid; e < L1 * 4; e += NT) {
-                const int o = e >> 2, pc = e & 3;
-                dg_cp16(st + (LF_POS + o) * LF_LD + 4 * pc, wg + (size_t)o * K + k0 + 4 * pc);
+            for (int e = tid; e < L1 * PCS; e += NT) {
+                const int o = e / PCS, pc = e % PCS;
+                dg_cp16(st + (POS + o) * LF_LD + 4 * pc, wg + (size_t)o * K + k0 + 4 * pc);
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     const int lane = tid & 31, warp = tid >> 5;
-    const int tx = lane % TX, ty = lane / TX;
-    const int row0 = warp * (4 * TY) + ty;  // the thread's positions: row0 + TY * i
-    float acc[4][8];
+    const int tx = lane % TX, ty = lane / TX;  // the thread's positions ty + TY * i, outputs tx + TX * j
+    unsigned long long acc[RP][8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < RP; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
 #pragma unroll
     for (int it = 0; it < LF_STAGES - 1; ++it) issue(it);
     for (int it = 0; it < nk; ++it) {
         asm volatile("cp.async.wait_group %0;" ::"n"(LF_STAGES - 2) : "memory");
         __syncthreads();  // chunk `it` has landed for every thread; chunk it - 1 has been consumed by every thread
         issue(it + LF_STAGES - 1);
-        const float* st = s_ring + (size_t)(it % LF_STAGES) * STAGE_FLOATS;
+        const float* st = s_ring + (size_t)(it % LF_STAGES) * T::STAGE_FLOATS + warp * (LF_KC / LF_WARPS);
 #pragma unroll
-        for (int kk = 0; kk < LF_KC; kk += 4) {
-            float4 xv[4], wv[8];
+        for (int kk = 0; kk < LF_KC / LF_WARPS; kk += 4) {
+            ulonglong2 wv[8];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) xv[i] = *reinterpret_cast<const float4*>(st + (row0 + TY * i) * LF_LD + kk);
+            for (int j = 0; j < 8; ++j) wv[j] = *reinterpret_cast<const ulonglong2*>(st + (POS + tx + TX * j) * LF_LD + kk);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) wv[j] = *reinterpret_cast<const float4*>(st + (LF_POS + tx + TX * j) * LF_LD + kk);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < RP; ++i) {
+                const ulonglong2 xv = *reinterpret_cast<const ulonglong2*>(st + (ty + TY * i) * LF_LD + kk);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    acc[i][j] += xv[i].x * wv[j].x;
-                    acc[i][j] += xv[i].y * wv[j].y;
-                    acc[i][j] += xv[i].z * wv[j].z;
-                    acc[i][j] += xv[i].w * wv[j].w;
+                    fma2(acc[i][j], xv.x, wv[j].x);
+                    fma2(acc[i][j], xv.y, wv[j].y);
                 }
+            }
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();  // the ring is free for the warps' sums [warp][POS][L1]
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = row0 + TY * i;
-        if (r >= n) continue;
-        float* yr = y + (size_t)s_pos[r] * L1;
+    for (int i = 0; i < RP; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int o = tx + TX * j;
-            yr[o] = acc[i][j] + beff[(size_t)g * L1 + o];
-        }
+        for (int j = 0; j < 8; ++j)
+            s_ring[(size_t)(warp * POS + ty + TY * i) * L1 + tx + TX * j] =
+                __uint_as_float((unsigned)acc[i][j]) + __uint_as_float((unsigned)(acc[i][j] >> 32));
+    __syncthreads();
+    for (int e = tid; e < n * L1; e += NT) {
+        const int r = e / L1, o = e % L1;
+        float sum = s_ring[e];
+#pragma unroll
+        for (int q = 1; q < LF_WARPS; ++q) sum += s_ring[(size_t)q * POS * L1 + e];
+        y[(size_t)s_pos[r] * L1 + o] = sum + beff[(size_t)g * L1 + o];
     }
 }
 
@@ -370,18 +386,26 @@ int launch_l1_weff(cudaStream_t s, const float* wb, const float* bb, const float
 
 int launch_l1_forward(cudaStream_t s, const float* x, int K, const int* order, const TileDesc* tiles,
                       const int* n_tiles, int max_tiles, const float* wb, const float* bb, const float* ws,
-                      const float* bs, float* y, int l1, int nb, const float* weff, int tf32, int* error_flag) {
+                      const float* bs, float* y, int l1, int nb, int n_pos, const float* weff, int tf32, int* error_flag) {
     if (l1_streams(K, l1)) {
         const float* beff = weff + (size_t)(nb + 1) * l1 * K;
         if (tf32 && error_flag && l1_forward_tc_supported(K, l1))
-            return launch_l1_forward_tc(s, x, K, order, tiles, n_tiles, max_tiles, weff, beff, y, l1, wb ? nb : 0, error_flag);
-        const int max_units = sort_max_units(max_tiles);
-        const size_t smem = (size_t)LF_STAGES * (LF_POS + l1) * LF_LD * sizeof(float);
+            return launch_l1_forward_tc(s, x, K, order, tiles, n_tiles, max_tiles, n_pos, weff, beff, y, l1, wb ? nb : 0, error_flag);
+        const int max_units = sort_units(n_pos);
         const TileDesc* units = tiles + max_tiles;
         const int nbe = wb ? nb : 0;
-        if (l1 == 8) k_l1_forward_stream<8><<<2 * max_units, 32, smem, s>>>(x, K, order, tiles, units, n_tiles + 1, weff, beff, y, nbe);
-        else if (l1 == 16) k_l1_forward_stream<16><<<2 * max_units, 64, smem, s>>>(x, K, order, tiles, units, n_tiles + 1, weff, beff, y, nbe);
-        else k_l1_forward_stream<32><<<2 * max_units, 128, smem, s>>>(x, K, order, tiles, units, n_tiles + 1, weff, beff, y, nbe);
+#define L1F(L, RP)                                                                                                          \
+    do {                                                                                                                    \
+        const int ub = unit_tiles(n_pos) * TB_TILE_M / L1Tile<L, RP>::POS;                                                  \
+        cudaFuncSetAttribute(k_l1_forward_stream<L, RP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L1Tile<L, RP>::SMEM); \
+        k_l1_forward_stream<L, RP><<<ub * max_units, 32 * LF_WARPS, L1Tile<L, RP>::SMEM, s>>>(x, K, order, tiles, units, n_tiles + 1, ub, \
+                                                                                            weff, beff, y, nbe);            \
+    } while (0)
+        // fewer positions per block where the batch has too few for every SM
+        if (l1 == 8) { if (n_pos >= 148 * 64) L1F(8, 2); else L1F(8, 1); }
+        else if (l1 == 16) { if (n_pos >= 148 * 64) L1F(16, 4); else L1F(16, 2); }
+        else L1F(32, 4);
+#undef L1F
         return 1;
     }
     const int nout = wb ? 2 * l1 : l1;
@@ -1154,11 +1178,11 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) k_l1_wgrad_stream(const f
 }
 
 int launch_l1_wgrad(cudaStream_t s, const float* x, int K, const float* dl1, const int* order,
-                    const TileDesc* tiles, const int* n_tiles, int max_tiles, int l1, int nb, float* partials,
+                    const TileDesc* tiles, const int* n_tiles, int max_tiles, int n_pos, int l1, int nb, float* partials,
                     float* gw_bucket, float* gw_shared) {
     const TileDesc* units = tiles + max_tiles;
     const int* n_units = n_tiles + 1;
-    const int max_units = sort_max_units(max_tiles);
+    const int max_units = sort_units(n_pos);
     if (l1 == 8 || l1 == 16 || l1 == 32) {
         const int threads = l1 == 32 ? 256 : 128;
         const size_t smem = (size_t)WG_POS * l1 * sizeof(float) + (size_t)WG_STAGES * 4 * threads * 16;
@@ -1316,14 +1340,14 @@ __global__ void __launch_bounds__(256) k_l1_dgrad_ftgrad(const float* __restrict
 // of four positions ahead of the arithmetic, which keeps the global loads in flight back to back.
 #define DG_POS 128     // positions per block
 #define DG_STAGES 3
-static_assert(2 * DG_POS == TB_UNIT_TILES * TB_TILE_M, "a block of the streaming kernel owns half a work unit");
+static_assert(2 * DG_POS == TB_UNIT_TILES * TB_TILE_M, "a block of the streaming kernel owns half a work unit at most");
 // HALF: pre-activations and dft rows are fp16 (ft_post_perspective_grad_fused_fp16, native_kernels.cu:2304-2353): the
 // gradient is multiplied by grad_scale, clamped to the fp16 range (clamps are counted) and rounded; the bias gradient
 // takes the unscaled fp32 value.
 template <int MODE, int L1, bool HALF>
 __global__ void __launch_bounds__(256) k_l1_dgrad_ftgrad_stream(const float* __restrict__ dl1, const int* __restrict__ order,
                                                                  const TileDesc* __restrict__ tiles, const TileDesc* __restrict__ units,
-                                                                 const int* __restrict__ n_units, const float* __restrict__ wb,
+                                                                 const int* __restrict__ n_units, int half_tiles, const float* __restrict__ wb,
                                                                  const float* __restrict__ ws, const void* __restrict__ pre_stm,
                                                                  const void* __restrict__ pre_nstm, const float* __restrict__ ft_bias,
                                                                  float scale, int F, int nb, int CW, void* __restrict__ dft_stm,
@@ -1352,8 +1376,7 @@ __global__ void __launch_bounds__(256) k_l1_dgrad_ftgrad_stream(const float* __r
     int p_begin = 0, n = 0, bucket = 0;
     if (u < *n_units) {
         const TileDesc ud = units[u];
-        const int per = DG_POS / TB_TILE_M;
-        const int first = ud.start + h * per, last = min(ud.start + ud.count, first + per);
+        const int first = ud.start + h * half_tiles, last = min(ud.start + ud.count, first + half_tiles);
         if (first < last) {
             p_begin = tiles[first].start;
             n = tiles[last - 1].start + tiles[last - 1].count - p_begin;
@@ -1534,10 +1557,8 @@ int launch_l1_dgrad_ftgrad(cudaStream_t s, int mode, const float* dl1, const int
                            const void* pre_stm, const void* pre_nstm, const float* ft_bias, float scale,
                            int B, int F, int l1, int nb, void* dft_stm, void* dft_nstm, float* bias_partials,
                            float* ft_b_grad, int n_ctas, int half_act, float grad_scale, unsigned long long* clamp_counter) {
-    (void)B;
-    (void)max_tiles;
     const int work_cols = mode == 1 ? F / 2 : F;
-    const int max_units = sort_max_units(max_tiles);
+    const int max_units = sort_units(B);
     int bias_rows = n_ctas;
     if ((l1 == 8 || l1 == 16 || l1 == 32) && n_ctas >= 2 * max_units) {
         int n_chunks = 1;
@@ -1549,7 +1570,7 @@ int launch_l1_dgrad_ftgrad(cudaStream_t s, int mode, const float* dl1, const int
 #define DGRAD_REG(M, L, H)                                                                                               \
     do {                                                                                                                 \
         cudaFuncSetAttribute(k_l1_dgrad_ftgrad_stream<M, L, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024); \
-        k_l1_dgrad_ftgrad_stream<M, L, H><<<grid, block, smem, s>>>(dl1, order, tiles, tiles + max_tiles, n_tiles + 1, wb, ws, pre_stm, \
+        k_l1_dgrad_ftgrad_stream<M, L, H><<<grid, block, smem, s>>>(dl1, order, tiles, tiles + max_tiles, n_tiles + 1, unit_tiles(B) / 2, wb, ws, pre_stm, \
                                                                     pre_nstm, ft_bias, scale, F, nb, CW, dft_stm, dft_nstm, \
                                                                     bias_partials, grad_scale, clamp_counter);           \
     } while (0)

@@ -4,7 +4,7 @@
 // bins/nnue_train/src/trainer_layerstack.rs:2388-2420, 2498-2506, bins/nnue_train/src/trainer_common.rs:691-727).
 //
 // Same contraction as k_l1_forward_stream: y[pos, :] = beff[g] + x[pos, :] . weff[g]^T with the effective weights
-// weff[g] = wb[g] + ws^T of the position's bucket g.  A block owns 128 consecutive positions of the bucket order (one
+// weff[g] = wb[g] + ws^T of the position's bucket g.  A block owns up to 128 consecutive positions of the bucket order (one
 // bucket), i.e. one 128 x l1 accumulator tile in tensor memory; x rows are reached through `order`, so the operands are
 // staged by 16-byte asynchronous copies straight into the tensor cores' canonical K-major layout without swizzle: core
 // matrices of 8 rows x 16 bytes, stored contiguously; the next 16 bytes along K lie 128 bytes further (leading byte
@@ -57,7 +57,7 @@ __device__ __forceinline__ unsigned long long umma_desc(unsigned addr, unsigned 
 template <int L1>
 __global__ void __launch_bounds__(128) k_l1_forward_tc(const float* __restrict__ x, int K, const int* __restrict__ order,
                                                         const TileDesc* __restrict__ tiles, const TileDesc* __restrict__ units,
-                                                        const int* __restrict__ n_units, const float* __restrict__ weff,
+                                                        const int* __restrict__ n_units, int half_tiles, const float* __restrict__ weff,
                                                         const float* __restrict__ beff, float* __restrict__ y, int nb,
                                                         int* __restrict__ error_flag) {
     constexpr int NB = L1 < 16 ? 16 : L1;             // N of the MMA (a multiple of 16 for M = 128)
@@ -76,8 +76,7 @@ __global__ void __launch_bounds__(128) k_l1_forward_tc(const float* __restrict__
     const int u = blockIdx.x >> 1, h = blockIdx.x & 1;
     if (u >= *n_units) return;
     const TileDesc ud = units[u];
-    const int per = TC_POS / TB_TILE_M;
-    const int first = ud.start + h * per, last = min(ud.start + ud.count, first + per);
+    const int first = ud.start + h * half_tiles, last = min(ud.start + ud.count, first + half_tiles);
     if (first >= last) return;
     const int p_begin = tiles[first].start;
     const int n = tiles[last - 1].start + tiles[last - 1].count - p_begin;
@@ -198,15 +197,15 @@ bool l1_forward_tc_supported(int K, int l1) { return (l1 == 8 || l1 == 16 || l1 
 
 // weff / beff: the effective weights and biases k_l1_weff has built for this step
 int launch_l1_forward_tc(cudaStream_t s, const float* x, int K, const int* order, const TileDesc* tiles, const int* n_tiles,
-                         int max_tiles, const float* weff, const float* beff, float* y, int l1, int nb, int* error_flag) {
-    const int max_units = sort_max_units(max_tiles);
+                         int max_tiles, int n_pos, const float* weff, const float* beff, float* y, int l1, int nb, int* error_flag) {
+    const int max_units = sort_units(n_pos);
     const TileDesc* units = tiles + max_tiles;
     const int NB = l1 < 16 ? 16 : l1;
     const size_t smem = (size_t)TC_STAGES * (TC_POS + NB) * TC_KC * 4 + 128;
 #define TC_LAUNCH(L)                                                                                                    \
     do {                                                                                                                \
         cudaFuncSetAttribute(k_l1_forward_tc<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);               \
-        k_l1_forward_tc<L><<<2 * max_units, 128, smem, s>>>(x, K, order, tiles, units, n_tiles + 1, weff, beff, y, nb, error_flag); \
+        k_l1_forward_tc<L><<<2 * max_units, 128, smem, s>>>(x, K, order, tiles, units, n_tiles + 1, unit_tiles(n_pos) / 2, weff, beff, y, nb, error_flag); \
     } while (0)
     if (l1 == 8) TC_LAUNCH(8); else if (l1 == 16) TC_LAUNCH(16); else TC_LAUNCH(32);
 #undef TC_LAUNCH

@@ -136,8 +136,8 @@ __global__ void __launch_bounds__(SORT_BLOCK) k_sort_scatter2(Fn0 f0, int n0, in
 // a step for the forward runs and 17 us for the chunks.)
 #define PLAN_THREADS 1024
 
-// tiles: runs of <= TB_TILE_M positions of one bucket; units: runs of <= TB_UNIT_TILES tiles of one bucket
-static __device__ void plan_tiles(const int* __restrict__ s_seg, int K, TileDesc* __restrict__ tiles, int* __restrict__ n_tiles,
+// tiles: runs of <= TB_TILE_M positions of one bucket; units: runs of <= ut tiles of one bucket
+static __device__ void plan_tiles(const int* __restrict__ s_seg, int K, int ut, TileDesc* __restrict__ tiles, int* __restrict__ n_tiles,
                                   TileDesc* __restrict__ units, int* __restrict__ n_units) {
     __shared__ int s_tile_base[TB_MAX_BUCKETS + 3], s_unit_base[TB_MAX_BUCKETS + 3];
     if (threadIdx.x == 0) {
@@ -148,7 +148,7 @@ static __device__ void plan_tiles(const int* __restrict__ s_seg, int K, TileDesc
             n_tiles[2 + k] = urun;
             const int nt = (s_seg[k + 1] - s_seg[k] + TB_TILE_M - 1) / TB_TILE_M;
             trun += nt;
-            urun += (nt + TB_UNIT_TILES - 1) / TB_UNIT_TILES;
+            urun += (nt + ut - 1) / ut;
         }
         s_tile_base[K] = trun;
         s_unit_base[K] = urun;
@@ -172,8 +172,8 @@ static __device__ void plan_tiles(const int* __restrict__ s_seg, int K, TileDesc
         int k = 0;
         while (s_unit_base[k + 1] <= u) ++k;
         TileDesc d;
-        d.start = s_tile_base[k] + (u - s_unit_base[k]) * TB_UNIT_TILES;
-        d.count = min(TB_UNIT_TILES, s_tile_base[k + 1] - d.start);
+        d.start = s_tile_base[k] + (u - s_unit_base[k]) * ut;
+        d.count = min(ut, s_tile_base[k + 1] - d.start);
         d.bucket = k;
         d.pad = 0;
         units[u] = d;
@@ -304,7 +304,7 @@ static __device__ void plan_backward(const int* __restrict__ s_seg, int n_keys, 
     }
 }
 
-__global__ void __launch_bounds__(PLAN_THREADS) k_step_plans(const int* __restrict__ seg_start, int K0, TileDesc* __restrict__ tiles,
+__global__ void __launch_bounds__(PLAN_THREADS) k_step_plans(const int* __restrict__ seg_start, int K0, int ut, TileDesc* __restrict__ tiles,
                                                              int* __restrict__ n_tiles, TileDesc* __restrict__ units,
                                                              const int* __restrict__ item_seg, int n_keys, FwdWork* __restrict__ work,
                                                              int* __restrict__ n_work, int ch, int parts, FwdWork* __restrict__ chunks,
@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) k_step_plans(const int* __restri
     const int n = blockIdx.x == 0 ? K0 : n_keys;
     for (int k = threadIdx.x; k <= n; k += PLAN_THREADS) s_seg[k] = seg[k];
     __syncthreads();
-    if (blockIdx.x == 0) plan_tiles(s_seg, K0, tiles, n_tiles, units, n_tiles + 1);
+    if (blockIdx.x == 0) plan_tiles(s_seg, K0, ut, tiles, n_tiles, units, n_tiles + 1);
     else if (blockIdx.x == 1) plan_forward(s_seg, n_keys, work, n_work);
     else plan_backward(s_seg, n_keys, ch, parts, chunks, n_chunks, groups, sched);
 }
@@ -349,7 +349,12 @@ int launch_slice_check(cudaStream_t s, const int* idx_stm, const int* idx_nstm, 
     return 1;
 }
 
-int sort_max_units(int max_tiles) { return max_tiles / TB_UNIT_TILES + TB_MAX_BUCKETS + 2; }
+int sort_units(int n_pos) { return n_pos / (unit_tiles(n_pos) * TB_TILE_M) + TB_MAX_BUCKETS + 2; }
+// at least the 148 units of the largest batches with smaller ones
+int sort_max_units(int max_tiles) {
+    const int n = max_tiles / TB_UNIT_TILES > 148 ? max_tiles / TB_UNIT_TILES : 148;
+    return n + TB_MAX_BUCKETS + 2;
+}
 
 // Both sorts of a step in four launches: positions by bucket (order, tiles, units) and items by table slice, with the plans
 // of the slice-resident kernels where their work buffers are given.
@@ -381,7 +386,7 @@ int launch_step_sorts(cudaStream_t s, const int* bucket, int B, int nb, int* ord
         bp = bwd_pointers(bwd_work, L);
         ch = L.CH;
     }
-    k_step_plans<<<bwd_work ? 3 : fwd_work ? 2 : 1, PLAN_THREADS, 0, s>>>(seg_start, K0, tiles, n_tiles, tiles + max_tiles, item_seg, K1,
+    k_step_plans<<<bwd_work ? 3 : fwd_work ? 2 : 1, PLAN_THREADS, 0, s>>>(seg_start, K0, unit_tiles(B), tiles, n_tiles, tiles + max_tiles, item_seg, K1,
                                                                           sb.work, sb.n_work, ch, bwd_parts, bp.chunks, bp.n_chunks,
                                                                           bp.groups, bp.sched);
     return 4;

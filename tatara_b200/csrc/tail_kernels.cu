@@ -3,7 +3,7 @@
 // trainer_simple.rs:1281-1508, :1560-1765; weight gradients dense_mm_bucket.rs:112-161).  For l1 = 8, 16, 32 and l2 = 16, 32;
 // dense_kernels.cu has the kernels for other sizes.
 //
-// A block owns 128 consecutive positions of the bucket order (one bucket), a thread one of them.  The bucket's weights sit in
+// A block owns up to 128 consecutive positions of the bucket order (one bucket), a thread one of them.  The bucket's weights sit in
 // shared memory and reach the threads as broadcasts, the position's vectors stay in registers; for the weight gradients the
 // threads put them side by side in shared memory and then own cells of the gradient instead.  What bounds it is the latency
 // of one block (a single wave covers 65 536 positions); the only large traffic is the L1 rows in and out.  A warp per position
@@ -13,7 +13,7 @@
 #include "loss.cuh"
 
 #define TT_POS 128
-static_assert(2 * TT_POS == TB_UNIT_TILES * TB_TILE_M, "a block owns half a work unit");
+static_assert(2 * TT_POS == TB_UNIT_TILES * TB_TILE_M, "a block owns half a work unit at most");
 
 namespace {
 
@@ -44,7 +44,7 @@ __device__ __forceinline__ float tail_act_grad(float a, float up) {
 template <int ARCH, int L1, int L2>
 __global__ void __launch_bounds__(TT_POS) k_tail(const float* __restrict__ l1_rows, const int* __restrict__ order,
                                                  const TileDesc* __restrict__ tiles, const TileDesc* __restrict__ units,
-                                                 const int* __restrict__ n_units, const float* __restrict__ score,
+                                                 const int* __restrict__ n_units, int half_tiles, const float* __restrict__ score,
                                                  const float* __restrict__ wdl, const float* __restrict__ l2_w,
                                                  const float* __restrict__ l2_b, const float* __restrict__ l3_w,
                                                  const float* __restrict__ l3_b, LossParams lp, int nb,
@@ -67,9 +67,8 @@ __global__ void __launch_bounds__(TT_POS) k_tail(const float* __restrict__ l1_ro
     int first = 0, last = 0, g = 0;
     if (u < *n_units) {
         const TileDesc ud = units[u];
-        const int per = TT_POS / TB_TILE_M;
-        first = ud.start + h * per;
-        last = min(ud.start + ud.count, first + per);
+        first = ud.start + h * half_tiles;
+        last = min(ud.start + ud.count, first + half_tiles);
         g = ud.bucket;
     }
     if (first >= last) {  // nothing here: the sums over the blocks read every row of the units there are
@@ -273,20 +272,20 @@ size_t tail_partial_floats(int arch, int l1, int l2, int max_tiles) {
     const int nin = arch == 0 ? 2 * (l1 - 1) : l1;
     return (size_t)2 * sort_max_units(max_tiles) * (nin * l2 + 2 * l2 + 1 + l1);
 }
-int tail_loss_blocks(int max_tiles) { return 2 * sort_max_units(max_tiles); }
+int tail_loss_blocks(int n_pos) { return 2 * sort_units(n_pos); }
 
-int launch_tail(cudaStream_t s, int arch, const float* l1_rows, const int* order, const TileDesc* tiles, const int* n_tiles, int max_tiles,
+int launch_tail(cudaStream_t s, int arch, int n_pos, const float* l1_rows, const int* order, const TileDesc* tiles, const int* n_tiles, int max_tiles,
                 const float* score, const float* wdl, const float* l2_w, const float* l2_b, const float* l3_w, const float* l3_b,
                 LossParams lp, int l1, int l2, int nb, float* net_output, float* dy, float* dl1, float* partials,
                 double* loss_partials, int backward) {
-    const int blocks = tail_loss_blocks(max_tiles);
+    const int blocks = tail_loss_blocks(n_pos);
     const TileDesc* units = tiles + max_tiles;
 #define TAIL_LAUNCH(A, L1, L2)                                                                                                    \
     do {                                                                                                                          \
         typedef TailShape<A, L1, L2> S;                                                                                           \
         const size_t smem = sizeof(float) * (S::W_FLOATS + (backward ? S::STAGE : 0));                                            \
         cudaFuncSetAttribute(k_tail<A, L1, L2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(float) * (S::W_FLOATS + S::STAGE))); \
-        k_tail<A, L1, L2><<<blocks, TT_POS, smem, s>>>(l1_rows, order, tiles, units, n_tiles + 1, score, wdl, l2_w, l2_b, l3_w,   \
+        k_tail<A, L1, L2><<<blocks, TT_POS, smem, s>>>(l1_rows, order, tiles, units, n_tiles + 1, unit_tiles(n_pos) / 2, score, wdl, l2_w, l2_b, l3_w,   \
                                                        l3_b, lp, nb, net_output, dy, dl1, partials, loss_partials, backward);     \
     } while (0)
 #define TAIL_L2(A, L1) do { if (l2 == 32) TAIL_LAUNCH(A, L1, 32); else TAIL_LAUNCH(A, L1, 16); } while (0)

@@ -492,7 +492,7 @@ int run_forward(tb_trainer* t, const DevBatch& d, const tb_loss* loss, float lam
     if (ls) {
         { PhaseScope p(t, PH_L1_FWD);
           p.done(launch_l1_forward(t->stream, t->combined, F, t->order, t->tiles, t->n_tiles, t->max_tiles, t->groups[2].w,
-                                   t->groups[3].w, t->groups[4].w, t->groups[5].w, t->l1_out, c.l1_out, c.num_buckets, t->l1_weff,
+                                   t->groups[3].w, t->groups[4].w, t->groups[5].w, t->l1_out, c.l1_out, c.num_buckets, B, t->l1_weff,
                                    t->p_tf32, t->tc_error)); }
         if (!tail_tiled(c.l1_out, c.l2_out)) { PhaseScope p(t, PH_TAIL);
           p.done(launch_tail_layerstack(t->stream, t->l1_out, d.bucket, d.score, d.wdl, t->groups[6].w, t->groups[7].w,
@@ -502,7 +502,7 @@ int run_forward(tb_trainer* t, const DevBatch& d, const tb_loss* loss, float lam
     } else {
         { PhaseScope p(t, PH_L1_FWD);
           p.done(launch_l1_forward(t->stream, t->combined, t->K, t->order, t->tiles, t->n_tiles, t->max_tiles, nullptr, nullptr,
-                                   t->groups[2].w, t->groups[3].w, t->l1_out, c.l1_out, 0, t->l1_weff)); }
+                                   t->groups[2].w, t->groups[3].w, t->l1_out, c.l1_out, 0, B, t->l1_weff)); }
         if (!tail_tiled(c.l1_out, c.l2_out)) { PhaseScope p(t, PH_TAIL);
           p.done(launch_tail_simple(t->stream, t->l1_out, d.score, d.wdl, t->groups[4].w, t->groups[5].w, t->groups[6].w,
                                     t->groups[7].w, lp, c.activation == TB_ACT_SCRELU ? 1 : 0, B, c.l1_out, c.l2_out, t->net_output, t->dy, t->dl1,
@@ -511,13 +511,13 @@ int run_forward(tb_trainer* t, const DevBatch& d, const tb_loss* loss, float lam
     if (tail_tiled(c.l1_out, c.l2_out)) {
         PhaseScope p(t, PH_TAIL);
         const int g = ls ? 6 : 4;  // l2_w, l2_b, l3_w, l3_b
-        int n = launch_tail(t->stream, tail_arch(c), t->l1_out, t->order, t->tiles, t->n_tiles, t->max_tiles, d.score, d.wdl, t->groups[g].w,
+        int n = launch_tail(t->stream, tail_arch(c), B, t->l1_out, t->order, t->tiles, t->n_tiles, t->max_tiles, d.score, d.wdl, t->groups[g].w,
                             t->groups[g + 1].w, t->groups[g + 2].w, t->groups[g + 3].w, lp, c.l1_out, c.l2_out, ls ? c.num_buckets : 0,
                             t->net_output, t->dy, t->dl1, t->small_partials, t->loss_partials, backward);
         // in a training step nothing but the loss read-back waits for the sum
         const cudaStream_t sl = backward ? side_stream(t, 1) : t->stream;
         AFTER(t->ev_tail, t->stream, sl);
-        n += launch_reduce_double(sl, t->loss_partials, tail_loss_blocks(t->max_tiles), t->loss_acc);
+        n += launch_reduce_double(sl, t->loss_partials, tail_loss_blocks(B), t->loss_acc);
         p.done(n);
     }
     return TB_OK;
@@ -560,7 +560,7 @@ int run_backward(tb_trainer* t, const DevBatch& d, float lr) {
                                                t->groups[7].grad, t->groups[8].grad, t->groups[9].grad, t->groups[3].grad,
                                                t->groups[5].grad)); }
         { PhaseScope p(t, PH_L1_WGRAD);
-          p.done(launch_l1_wgrad(sw, t->combined, F, t->dl1, t->order, t->tiles, t->n_tiles, t->max_tiles, c.l1_out,
+          p.done(launch_l1_wgrad(sw, t->combined, F, t->dl1, t->order, t->tiles, t->n_tiles, t->max_tiles, B, c.l1_out,
                                  c.num_buckets, t->l1w_partials, t->groups[2].grad, t->groups[4].grad)); }
         { PhaseScope p(t, PH_L1_DGRAD);
           // fp16 dft rows carry gradient * 2^14 * batch (trainer_layerstack.rs:3617-3621); the FT weight gradient is summed
@@ -580,7 +580,7 @@ int run_backward(tb_trainer* t, const DevBatch& d, float lr) {
                                            t->tail_c, t->dy, t->dl1, t->small_partials, t->groups[4].grad, t->groups[5].grad,
                                            t->groups[6].grad, t->groups[7].grad, t->groups[3].grad)); }
         { PhaseScope p(t, PH_L1_WGRAD);
-          p.done(launch_l1_wgrad(sw, t->combined, t->K, t->dl1, t->order, t->tiles, t->n_tiles, t->max_tiles, c.l1_out, 0,
+          p.done(launch_l1_wgrad(sw, t->combined, t->K, t->dl1, t->order, t->tiles, t->n_tiles, t->max_tiles, B, c.l1_out, 0,
                                  t->l1w_partials, nullptr, t->groups[2].grad)); }
         { PhaseScope p(t, PH_L1_DGRAD);
           p.done(launch_l1_dgrad_ftgrad(t->stream, c.activation == TB_ACT_PAIRWISE ? 1 : (c.activation == TB_ACT_CRELU ? 2 : 3), t->dl1, t->order, t->tiles, t->n_tiles,
