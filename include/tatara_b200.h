@@ -235,7 +235,7 @@ int tb_ft_microbench(int device, const int32_t* indices, const int32_t* nnz, int
  * For hosts that must not allocate device memory once they run — a framework whose allocator owns the
  * whole GPU, a process with a fixed memory plan — this variant of the FT backward keeps the working
  * memory of the inverse index and of the long-list partial sums in a static device array inside the
- * library (about 21.5 MB per GPU, held until exit) and calls no cudaMalloc / cudaFree.  ALL pointers are DEVICE memory owned by the caller;
+ * library (about 20.5 MB per GPU, held until exit) and calls no cudaMalloc / cudaFree.  ALL pointers are DEVICE memory owned by the caller;
  * the work is enqueued on `stream` (a cudaStream_t, NULL = default stream) and not synchronised.
  * Limits: ft_in <= TB_STATIC_SCRATCH_MAX_FT_IN and batch * max_active <= TB_STATIC_SCRATCH_MAX_PAIRS;
  * beyond them the call fails and writes the reason to err (may be NULL).  Calls share the one array:

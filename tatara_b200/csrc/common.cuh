@@ -11,7 +11,7 @@
 #define TB_UNIT_TILES 8   // most tiles of a work unit (consecutive tiles of one bucket)
 // Tiles per work unit for a batch: the dense kernels' blocks own half a unit and walk its positions one after the other, so a
 // batch that does not fill the chip with blocks of 128 positions gets smaller ones (B = 1024: the L1 input gradient took
-// 40 us on 16 of 148 SMs, 14 now).
+// 43 us on 16 of 148 SMs, 22 now).
 static inline int unit_tiles(int n_pos) { return n_pos >= 148 * 128 ? TB_UNIT_TILES : n_pos >= 148 * 64 ? 4 : 2; }
 // counts beside the tiles: {tiles, units, first unit of every bucket (and of the positions without one, and the end)}
 #define TB_TILE_COUNTS 16
@@ -98,23 +98,22 @@ int launch_ft_forward_slice(cudaStream_t s, int mode, const void* table, const i
                             const int* nnz, const float* bias, void* pre_stm, void* pre_nstm, float* combined,
                             const int* items, const int* item_seg, int* work, int B, int F, int N, int A,
                             int rows_per_slice, float scale, int n_persp, int table_half = 0, int out_half = 0);
-// scratch of the inverse index, in ints: histogram [2N], a counter, a queue of long lists [2N], scan block sums
-static inline size_t inverse_index_counts_len(int N) { return 4 * (size_t)N + 1 + 2 * ((size_t)N / 2048 + 2); }
-// counts: [inverse_index_counts_len(N)], offsets: [2][N+1], cursor: [2][N], lists: [4][B*A] (lists + sort scratch)
-// run_if (here and below): NULL, or a device flag; the launched kernels return at once while it is 0
-int launch_inverse_index(cudaStream_t s, const int* run_if, const int* idx_stm, const int* idx_nstm, const int* nnz, int B, int A,
-                         int N, int n_persp, int* counts, int* offsets, int* cursor, int* lists);
-// long lists are cut into parts summed by separate blocks; plan: [2 + 2 * max_work + 3 * N] ints,
-// partial: [max_work][F] floats with max_work = ft_backward_max_work(B, A, n_persp)
+// scratch of the inverse index, in ints: histogram [2N], counters, a queue of long lists [2N]
+static inline size_t inverse_index_counts_len(int N) { return 4 * (size_t)N + 8; }
+// counts: [inverse_index_counts_len(N)], offsets: [2N], lists: [4][B*A] (lists + ranks and sort scratch).  The gradient of
+// the same sizes follows with the same counts, offsets, lists and plan.
+// Very long lists are cut into parts summed separately; plan: [2 * max_work + 3 * N] ints, partial: [max_work][F] floats
+// with max_work = ft_backward_max_work(B, A, n_persp)
 int ft_backward_max_work(int B, int A, int n_persp);
+int launch_inverse_index(cudaStream_t s, const int* idx_stm, const int* idx_nstm, const int* nnz, int B, int A, int N, int n_persp,
+                         int* counts, int* offsets, int* lists, int* plan);
 // dft_half: the incoming gradient rows are fp16; the sums keep the rows' loss scale
-int launch_ft_backward_split(cudaStream_t s, const int* run_if, const void* dft_stm, const void* dft_nstm, const int* offsets,
+int launch_ft_backward_split(cudaStream_t s, const void* dft_stm, const void* dft_nstm, const int* counts, const int* offsets,
                              const int* lists, int B, int A, int N, int F, int n_persp, int* plan, float* partial,
                              float* grad, int dft_half = 0);
 // slice-resident weight gradient (ft_slice_bwd.cu).  Needs the slice-resident forward of the same step (its row codes
 // in fwd_work) and items / item_seg of the same rows_per_slice; bwd_work: ft_backward_slice_ints(...) ints.  The kernels
-// do nothing when the batch has a row outside its item's slice: *ft_slice_outside_flag(...) is then 1 and the generic
-// kernels, launched with it as run_if, do the work instead.
+// do nothing when the batch has a row outside its item's slice; the host launches the generic ones for such a batch.
 bool ft_backward_slice_supported(int F, int N, int A, int rows_per_slice);
 size_t ft_backward_slice_ints(int n_items, int A, int rows_per_slice);
 // floats of the partial slabs launch_ft_backward_slice needs (slices of many chunks are shared by several blocks)

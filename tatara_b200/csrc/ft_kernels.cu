@@ -501,35 +501,46 @@ int launch_ft_forward_slice(cudaStream_t s, int mode, const void* table, const i
 
 // ------------------------------------------------------------------------------------------------
 // inverse index: for every feature the list of positions that hold it (the counting sort of
-// native_kernels.cu:1630-1765: histogram, exclusive scan, ranked scatter).
+// native_kernels.cu:1630-1765: histogram, offsets, ranked scatter).
+//
+// The histogram's atomics hand out the ranks, so the scatter needs none.  The lists lie in the order in which the scan's
+// blocks take their room (an atomic per block of SCAN_CELLS rows): nothing needs them in row order, and one launch does
+// what a scan over all blocks took two for.  Its threads also plan the gradient: long lists are queued for sorting, very
+// long ones cut into parts.
 // ------------------------------------------------------------------------------------------------
-__global__ void k_feat_count(const int* __restrict__ idx_stm, const int* __restrict__ idx_nstm,
-                             const int* __restrict__ nnz, int B, int A, int N, int n_persp, int* __restrict__ counts, const int* __restrict__ run_if) {
-    if (run_if && *run_if == 0) return;  // gated: another path does this step's work
-    const long long total = (long long)n_persp * B * A;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const int p = (int)(i / ((long long)B * A));
-        const long long r = i - (long long)p * B * A;
-        const int b = (int)(r / A), a = (int)(r - (long long)b * A);
-        if (a >= nnz[b]) continue;
-        const int f = (p ? idx_nstm : idx_stm)[r];
-        if ((unsigned)f < (unsigned)N) atomicAdd(counts + (size_t)p * N + f, 1);
+// counters behind the histogram
+#define INV_ROOM 0   // [2] list cells taken so far, per perspective
+#define INV_QUEUED 2 // lists queued for k_lists_sort_long
+#define INV_PARTS 3  // parts of split rows
+#define INV_SPLIT 4  // split rows
+#define INV_COUNTERS 5
+
+// the unsigned 32-bit indices hold every list cell: batch * slots is an int everywhere else as well
+__global__ void __launch_bounds__(256) k_feat_count(const int* __restrict__ idx_stm, const int* __restrict__ idx_nstm,
+                                                    const int* __restrict__ nnz, unsigned cells, unsigned A, int N,
+                                                    int* __restrict__ counts, int* __restrict__ ranks) {
+    const int* idx = blockIdx.y ? idx_nstm : idx_stm;
+    int* cnt = counts + (size_t)blockIdx.y * N;
+    int* rank = ranks + (size_t)blockIdx.y * cells;
+    for (unsigned r = blockIdx.x * 256 + threadIdx.x; r < cells; r += gridDim.x * 256) {
+        const unsigned b = r / A, a = r - b * A;
+        const int f = idx[r];
+        if ((int)a < nnz[b] && (unsigned)f < (unsigned)N) rank[r] = atomicAdd(cnt + f, 1);
     }
 }
 
-// offsets[p][0..N] = exclusive prefix sum of counts[p][0..N), in two launches: block-local scans of 2048
-// cells with their sums, then every block adds the sums of the blocks before it.
 #define SCAN_CELLS 2048
-__global__ void __launch_bounds__(1024) k_feat_scan_local(const int* __restrict__ counts, int N, int* __restrict__ offsets,
-                                                           int* __restrict__ block_sums, const int* __restrict__ run_if) {
-    if (run_if && *run_if == 0) return;  // gated: another path does this step's work
-    __shared__ int warp_tot[32];
+#define BWD_PART 4096  // entries (both perspectives) from which a row is summed in parts
+__global__ void __launch_bounds__(1024) k_feat_scan(const int* __restrict__ counts, int N, int n_persp, int sort_limit,
+                                                    int* __restrict__ offsets, int* __restrict__ counters,
+                                                    int* __restrict__ long_queue, int2* __restrict__ work, int* __restrict__ split) {
+    __shared__ int s_warp[32], s_base;
     const int p = blockIdx.y;
     const int* c = counts + (size_t)p * N;
-    int* o = offsets + (size_t)p * (N + 1);
+    int* o = offsets + (size_t)p * N;
     const int i0 = blockIdx.x * SCAN_CELLS + 2 * threadIdx.x;
-    const int a = i0 < N ? c[i0] : 0, b = i0 + 1 < N ? c[i0 + 1] : 0;
-    const int sum = a + b;
+    const int n0 = i0 < N ? c[i0] : 0, n1 = i0 + 1 < N ? c[i0 + 1] : 0;
+    const int sum = n0 + n1;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     int incl = sum;
 #pragma unroll
@@ -537,134 +548,73 @@ __global__ void __launch_bounds__(1024) k_feat_scan_local(const int* __restrict_
         const int t = __shfl_up_sync(0xffffffffu, incl, d);
         if (lane >= d) incl += t;
     }
-    if (lane == 31) warp_tot[w] = incl;
+    if (lane == 31) s_warp[w] = incl;
     __syncthreads();
     if (w == 0) {
-        const int t = warp_tot[lane];
+        const int t = s_warp[lane];
         int ti = t;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const int u = __shfl_up_sync(0xffffffffu, ti, d);
             if (lane >= d) ti += u;
         }
-        warp_tot[lane] = ti - t;
-        if (lane == 31) block_sums[p * gridDim.x + blockIdx.x] = ti;
+        s_warp[lane] = ti - t;
+        if (lane == 31) s_base = atomicAdd(counters + INV_ROOM + p, ti);
     }
     __syncthreads();
-    const int excl = warp_tot[w] + incl - sum;
+    const int excl = s_base + s_warp[w] + incl - sum;
     if (i0 < N) o[i0] = excl;
-    if (i0 + 1 < N) o[i0 + 1] = excl + a;
-}
-
-__global__ void __launch_bounds__(1024) k_feat_scan_add(int N, int* __restrict__ offsets, int* __restrict__ cursor,
-                                                         const int* __restrict__ block_sums, const int* __restrict__ run_if) {
-    if (run_if && *run_if == 0) return;  // gated: another path does this step's work
-    __shared__ int s_off;
-    const int p = blockIdx.y;
-    int* o = offsets + (size_t)p * (N + 1);
-    int* cur = cursor + (size_t)p * N;
-    if (threadIdx.x < 32) {
-        int t = 0;
-        for (int j = threadIdx.x; j < (int)blockIdx.x; j += 32) t += block_sums[p * gridDim.x + j];
+    if (i0 + 1 < N) o[i0 + 1] = excl + n0;
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) t += __shfl_down_sync(0xffffffffu, t, d);
-        if (threadIdx.x == 0) s_off = t;
-    }
-    __syncthreads();
-    const int off = s_off;
-    const int i0 = blockIdx.x * SCAN_CELLS + 2 * threadIdx.x;
-    if (i0 < N) { const int v = o[i0] + off; o[i0] = v; cur[i0] = v; }
-    if (i0 + 1 < N) { const int v = o[i0 + 1] + off; o[i0 + 1] = v; cur[i0 + 1] = v; }
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) o[N] = off + block_sums[p * gridDim.x + blockIdx.x];
-}
-
-__global__ void k_feat_fill(const int* __restrict__ idx_stm, const int* __restrict__ idx_nstm,
-                            const int* __restrict__ nnz, int B, int A, int N, int n_persp, int* __restrict__ cursor,
-                            int* __restrict__ lists, const int* __restrict__ run_if) {
-    if (run_if && *run_if == 0) return;  // gated: another path does this step's work
-    const long long total = (long long)n_persp * B * A;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const int p = (int)(i / ((long long)B * A));
-        const long long r = i - (long long)p * B * A;
-        const int b = (int)(r / A), a = (int)(r - (long long)b * A);
-        if (a >= nnz[b]) continue;
-        const int f = (p ? idx_nstm : idx_stm)[r];
-        if ((unsigned)f < (unsigned)N) {
-            const int pos = atomicAdd(cursor + (size_t)p * N + f, 1);
-            lists[(size_t)p * B * A + pos] = b;
-        }
+    for (int k = 0; k < 2; ++k) {
+        const int f = i0 + k, n = k ? n1 : n0;
+        if (f >= N) continue;
+        const int other = n_persp > 1 ? counts[(size_t)(1 - p) * N + f] : 0;
+        if (n > 1 && max(n, other) > sort_limit) long_queue[atomicAdd(counters + INV_QUEUED, 1)] = p * N + f;
+        if (p > 0) continue;
+        const int len = n + other;
+        if (len <= BWD_PART) continue;
+        const int parts = (len + BWD_PART - 1) / BWD_PART;
+        const int base = atomicAdd(counters + INV_PARTS, parts), q = atomicAdd(counters + INV_SPLIT, 1);
+        split[3 * q + 0] = f;
+        split[3 * q + 1] = base;
+        split[3 * q + 2] = 0;  // (part, strip) sums done so far
+        for (int i = 0; i < parts; ++i) work[base + i] = make_int2(q, i);
     }
 }
 
-// The ranked scatter above leaves every list in arrival order.  The two kernels below sort each list
-// ascending, so that the backward sums always run in position order (deterministic results).
-// Short lists (<= 32 * SORT_WARP_VALUES = 256 entries): one warp ranks its entries against each other through shuffles.
-// Long lists: queued, then one block per list marks the positions in a shared-memory bitmap and reads
-// the set bits back in order; a list that names a position twice (only possible when the caller's
-// index row repeats a feature) falls back to ranking by counting.
-#define SORT_WARP_VALUES 8  // list entries a lane holds in the warp-level sort
-// one warp sorts L[0 .. len), len <= 32 V: lane l holds entries l, l + 32, ..; every entry is ranked against all entries of
-// the list (ties by index: the bitmap kernel's fallback treats repeated positions the same way)
-template <int V>
-static __device__ __forceinline__ void warp_rank_sort(int* __restrict__ L, int len, int lane) {
-    int v[V], r[V];
-#pragma unroll
-    for (int m = 0; m < V; ++m) {
-        v[m] = lane + 32 * m < len ? L[lane + 32 * m] : 0x7fffffff;
-        r[m] = 0;
-    }
-#pragma unroll
-    for (int k = 0; k < V; ++k) {
-        if (32 * k >= len) break;  // uniform over the warp
-        const int nj = min(32, len - 32 * k);
-        for (int l = 0; l < nj; ++l) {
-            const int u = __shfl_sync(0xffffffffu, v[k], l);
-            const int j = 32 * k + l;
-#pragma unroll
-            for (int m = 0; m < V; ++m) r[m] += (u < v[m]) || (u == v[m] && j < lane + 32 * m);
-        }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int m = 0; m < V; ++m)
-        if (lane + 32 * m < len) L[r[m]] = v[m];
-}
-
-__global__ void __launch_bounds__(256) k_lists_sort_short(const int* __restrict__ offsets, int N, int n_persp, int B, int A,
-                                                           int* __restrict__ lists, int* __restrict__ long_queue,
-                                                           int* __restrict__ long_count, const int* __restrict__ run_if) {
-    if (run_if && *run_if == 0) return;  // gated: another path does this step's work
-    const int lane = threadIdx.x & 31;
-    for (int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; warp < n_persp * N; warp += (gridDim.x * blockDim.x) >> 5) {
-    const int p = warp / N, f = warp - p * N;
-    const int beg = offsets[(size_t)p * (N + 1) + f], end = offsets[(size_t)p * (N + 1) + f + 1];
-    const int len = end - beg;
-    if (len < 2) continue;
-    if (len > 32 * SORT_WARP_VALUES) {
-        if (lane == 0) long_queue[atomicAdd(long_count, 1)] = warp;
-        continue;
-    }
-    int* L = lists + (size_t)p * B * A + beg;
-    if (len <= 64) warp_rank_sort<2>(L, len, lane);
-    else warp_rank_sort<SORT_WARP_VALUES>(L, len, lane);
+__global__ void __launch_bounds__(256) k_feat_fill(const int* __restrict__ idx_stm, const int* __restrict__ idx_nstm,
+                                                   const int* __restrict__ nnz, unsigned cells, unsigned A, int N,
+                                                   const int* __restrict__ offsets, const int* __restrict__ ranks,
+                                                   int* __restrict__ lists) {
+    const int* idx = blockIdx.y ? idx_nstm : idx_stm;
+    const int* off = offsets + (size_t)blockIdx.y * N;
+    const int* rank = ranks + (size_t)blockIdx.y * cells;
+    int* L = lists + (size_t)blockIdx.y * cells;
+    for (unsigned r = blockIdx.x * 256 + threadIdx.x; r < cells; r += gridDim.x * 256) {
+        const unsigned b = r / A, a = r - b * A;
+        const int f = idx[r];
+        if ((int)a < nnz[b] && (unsigned)f < (unsigned)N) L[off[f] + rank[r]] = (int)b;
     }
 }
 
-__global__ void __launch_bounds__(256) k_lists_sort_long(const int* __restrict__ offsets, int N, int B, int A,
-                                                          int* __restrict__ lists, int* __restrict__ scratch,
+// The ranked scatter leaves every list in arrival order; the backward sums run in position order (deterministic results).
+// Lists that fit the gradient kernel's shared memory are sorted there.  Longer ones are sorted here, one block per list: it
+// marks the positions in a shared-memory bitmap and reads the set bits back in order; a list that names a position twice
+// (only possible when the caller's index row repeats a feature) falls back to ranking by counting.
+__global__ void __launch_bounds__(256) k_lists_sort_long(const int* __restrict__ counts, const int* __restrict__ offsets, int N,
+                                                          size_t cells, int* __restrict__ lists, int* __restrict__ scratch,
                                                           const int* __restrict__ long_queue,
-                                                          const int* __restrict__ long_count, int bitmap_words, const int* __restrict__ run_if) {
-    if (run_if && *run_if == 0) return;  // gated: another path does this step's work
+                                                          const int* __restrict__ long_count, int bitmap_words) {
     extern __shared__ unsigned s_bits[];  // [bitmap_words]; 0 words: always use the counting fallback
     __shared__ int s_warp[8];
     __shared__ int s_total;
     const int n_long = *long_count;
     for (int q = blockIdx.x; q < n_long; q += gridDim.x) {
         const int id = long_queue[q];
-        const int p = id / N, f = id - p * N;
-        const int beg = offsets[(size_t)p * (N + 1) + f], end = offsets[(size_t)p * (N + 1) + f + 1];
-        const int len = end - beg;
-        int* L = lists + (size_t)p * B * A + beg;
+        const int p = id / N;
+        const int beg = offsets[id], len = counts[id];
+        int* L = lists + p * cells + beg;
         bool done = false;
         if (bitmap_words > 0) {
             for (int i = threadIdx.x; i < bitmap_words; i += blockDim.x) s_bits[i] = 0u;
@@ -709,7 +659,7 @@ __global__ void __launch_bounds__(256) k_lists_sort_long(const int* __restrict__
             __syncthreads();
         }
         if (!done) {
-            int* S = scratch + (size_t)p * B * A + beg;
+            int* S = scratch + p * cells + beg;
             for (int i = threadIdx.x; i < len; i += blockDim.x) S[i] = L[i];
             __syncthreads();
             for (int i = threadIdx.x; i < len; i += blockDim.x) {
@@ -726,176 +676,268 @@ __global__ void __launch_bounds__(256) k_lists_sort_long(const int* __restrict__
     }
 }
 
-int launch_inverse_index(cudaStream_t s, const int* run_if, const int* idx_stm, const int* idx_nstm, const int* nnz, int B, int A,
-                         int N, int n_persp, int* counts, int* offsets, int* cursor, int* lists) {
-    if (B <= 0) return 0;
-    // counts holds [2][N] histogram cells followed by one counter and a queue of [2*N] long-list ids
-    int* long_count = counts + (size_t)2 * N;
-    int* long_queue = long_count + 1;
-    cudaMemsetAsync(counts, 0, sizeof(int) * ((size_t)2 * N + 1), s);
-    const long long total = (long long)n_persp * B * A;
-    int blocks = (int)((total + 255) / 256);
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    k_feat_count<<<blocks, 256, 0, s>>>(idx_stm, idx_nstm, nnz, B, A, N, n_persp, counts, run_if);
-    {   // block sums live behind the long-list queue (which holds at most 2N ids)
-        int* block_sums = long_queue + (size_t)2 * N;
-        const dim3 sg(ceil_div(N, SCAN_CELLS), n_persp);
-        k_feat_scan_local<<<sg, 1024, 0, s>>>(counts, N, offsets, block_sums, run_if);
-        k_feat_scan_add<<<sg, 1024, 0, s>>>(N, offsets, cursor, block_sums, run_if);
-    }
-    k_feat_fill<<<blocks, 256, 0, s>>>(idx_stm, idx_nstm, nnz, B, A, N, n_persp, cursor, lists, run_if);
-    int* scratch = lists + (size_t)2 * B * A;  // the list buffer carries a second copy's worth of room
-    const long long warps = (long long)n_persp * N;
-    k_lists_sort_short<<<(int)(run_if && (warps * 32 + 255) / 256 > 148 * 32 ? 148 * 32 : (warps * 32 + 255) / 256), 256, 0, s>>>(offsets, N, n_persp, B, A, lists, long_queue, long_count, run_if);
-    int words = (B + 31) / 32;
-    if ((size_t)words * 4 > 160 * 1024) words = 0;
-    // per device and cheap: set before every launch (a process may drive several GPUs)
-    cudaFuncSetAttribute(k_lists_sort_long, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-    k_lists_sort_long<<<148 * 4, 256, (size_t)words * 4, s>>>(offsets, N, B, A, lists, scratch, long_queue, long_count, words, run_if);
-    return 6;
-}
-
 // ------------------------------------------------------------------------------------------------
-// backward: a block per feature row, a thread per float4 column.  The row of the gradient is written exactly once per
-// step (stm list first, then nstm list, each in ascending position order: the accumulation order of
-// sparse_ft_backward_cpu called for stm then nstm), with list splitting: a feature that is active in very many positions (the king square of a
-// king bucket, a pawn in hand) makes one block walk a list of thousands of rows; with real, skewed data such
-// lists reach tens of thousands of entries and would set the kernel's run time on their own.  Features whose
-// lists (stm + nstm) exceed BWD_PART entries are cut into parts of BWD_PART entries; every part is summed
-// by its own block into a scratch row, and a last kernel adds the parts of a feature in order.  Which
-// block gets which part depends on timing, the sums do not.
+// backward: groups of threads own a feature row each, a thread a float4 column of it.  The row of the gradient is written
+// exactly once per step (stm list first, then nstm list, each in ascending position order: the accumulation order of
+// sparse_ft_backward_cpu called for stm then nstm).
+//
+// Bound: the gradient rows of the positions are read once per list entry, from L2 (4.0 GB at 16 384 x 1536 with 40 slots: 290
+// us, 13.8 TB/s; 362 before).  What it took: strips of columns narrow enough that a strip of all rows stays in L2
+// (BWD_STRIP_BYTES), the rows of a group as one stream of entries with eight 16-byte loads in flight across the ends of rows
+// (lists of nine entries left half of the loads of their second round out), and two float4 columns per thread (the instructions
+// per byte were the bound then: 378 to 310 us).
+//
+// Every warp sorts the lists of its rows into shared memory first: they are short, a few entries in a large feature space, and
+// a separate pass over all rows took 27 to 30 us.
+//
+// Splitting: a feature that is active in very many positions (the king square of a king bucket, a pawn in hand) makes one
+// group walk a list of thousands of rows; with real, skewed data such lists reach tens of thousands of entries and would
+// set the kernel's run time on their own.  Rows whose lists (stm + nstm) exceed BWD_PART entries are cut into parts; every
+// part of a strip is summed by its own group, ahead of the short rows, and the last one to finish adds the parts of the row
+// in order.  Which group gets which part depends on timing, the sums do not.
 // ------------------------------------------------------------------------------------------------
-#define BWD_PART 4096
+#define BWD_SORT_CELLS 256            // list cells of a warp's rows in shared memory (per perspective)
+#define BWD_STRIP_BYTES (70ll << 20)
+#define BWD_CELL_LAST 0x80000000  // cell flags: the row's last entry; a position of the nstm list
+#define BWD_CELL_NSTM 0x40000000
+#define BWD_SPLIT_BLOCKS 296          // blocks in front of the short rows' that take the parts of split rows
 
-__global__ void k_bwd_plan(const int* __restrict__ offsets, int N, int n_persp, int* __restrict__ counters,
-                           int2* __restrict__ work, int* __restrict__ longf, const int* __restrict__ run_if) {
-    if (run_if && *run_if == 0) return;  // gated: another path does this step's work
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= N) return;
-    int len = 0;
-    for (int p = 0; p < n_persp; ++p) len += offsets[(size_t)p * (N + 1) + f + 1] - offsets[(size_t)p * (N + 1) + f];
-    if (len <= BWD_PART) return;
-    const int parts = (len + BWD_PART - 1) / BWD_PART;
-    const int base = atomicAdd(&counters[0], parts);
-    const int q = atomicAdd(&counters[1], 1);
-    longf[3 * q + 0] = f;
-    longf[3 * q + 1] = base;
-    longf[3 * q + 2] = parts;
-    for (int i = 0; i < parts; ++i) work[base + i] = make_int2(f, i);
-}
+// Rows of a warp: with lists of a few entries a block's start costs more than the sums of eight rows (1000 positions over
+// 125 388 rows of 256: 82 us with one row per warp, 66 with four).  Four rows share the sorting cells, so longer lists, which
+// would have to go through k_lists_sort_long, keep one.
+static inline int bwd_rows_per_warp(int B, int A, int N) { return (long long)B * A <= 16ll * N ? 4 : 1; }
 
 template <bool DH>
-static __device__ __forceinline__ float4 sum_rows(const void* __restrict__ d, const int* __restrict__ L, int beg, int end,
-                                                  int F, int c, float4 acc) {
-    for (int j = beg; j < end; j += 8) {
-        int bi[8];
+static __device__ __forceinline__ float4 sum_rows(const void* __restrict__ d, const int* L, int n, int F, int c, float4 acc) {
+    for (int j = 0; j < n; j += 8) {
         float4 v[8];
+        // all loads of a round are in flight together; the slots behind the end add nothing
 #pragma unroll
-        for (int u = 0; u < 8; ++u) bi[u] = __ldg(L + min(j + u, end - 1));
+        for (int u = 0; u < 8; ++u)
+            v[u] = j + u < n ? ld4<DH>(d, (size_t)L[j + u] * F + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = ld4<DH>(d, (size_t)bi[u] * F + 4 * c);
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            if (j + u < end) { acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w; }
-        }
+        for (int u = 0; u < 8; ++u) { acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w; }
     }
     return acc;
 }
 
 // DH: the incoming gradient rows are fp16 (summed in fp32, native_kernels.cu:1081-1140); the sums are then left in the
 // rows' loss scale, which the optimizer takes out again
-template <bool DH>
-__global__ void __launch_bounds__(512) k_ft_backward_short(const void* __restrict__ dft_stm, const void* __restrict__ dft_nstm,
-                                                             const int* __restrict__ offsets, const int* __restrict__ lists,
-                                                             int B, int A, int N, int F, int n_persp, float* __restrict__ grad, const int* __restrict__ run_if) {
-    if (run_if && *run_if == 0) return;  // gated: another path does this step's work
-    const int c = blockIdx.y * blockDim.x + threadIdx.x;
-    const int row4 = F >> 2;
-    for (int f = blockIdx.x; f < N; f += gridDim.x) {
-    int len = offsets[f + 1] - offsets[f];
-    if (n_persp > 1) len += offsets[(size_t)(N + 1) + f + 1] - offsets[(size_t)(N + 1) + f];
-    if (len > BWD_PART) continue;  // summed in parts by k_ft_backward_long
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int p = 0; p < n_persp; ++p) {
-        const int beg = offsets[(size_t)p * (N + 1) + f], end = offsets[(size_t)p * (N + 1) + f + 1];
-        // unconditional loads (a slot past the end re-reads the last row and is dropped), so that all eight row loads
-        // are in flight together
-        acc = sum_rows<DH>(p ? dft_nstm : dft_stm, lists + (size_t)p * B * A, beg, end, F, c, acc);
-    }
-    reinterpret_cast<float4*>(grad)[(size_t)f * row4 + c] = acc;
-    }
-}
+template <bool DH, int V>
+__global__ void __launch_bounds__(256) k_ft_backward(const void* __restrict__ dft_stm, const void* __restrict__ dft_nstm,
+                                                     const int* __restrict__ counts, const int* __restrict__ offsets,
+                                                     const int* __restrict__ lists, size_t cells, int N, int F, int n_persp,
+                                                     int strip4, int rpw, const int* __restrict__ counters,
+                                                     const int2* __restrict__ work, int* split, float* partial,
+                                                     float* __restrict__ grad) {
+    extern __shared__ int s_mem[];  // per warp: raw cells, then sorted cells of either perspective
+    __shared__ int s_off[2][32], s_len[2][32], s_beg[33], s_last[8];
+    const int ths = strip4 / V;  // threads of a group: thread ct owns the float4 columns ct, ct + ths, ..
+    const int groups = blockDim.x / ths, g = threadIdx.x / ths, ct = threadIdx.x - g * ths;
+    const int row4 = F >> 2, c = blockIdx.y * strip4 + ct;
 
-template <bool DH>
-__global__ void __launch_bounds__(512) k_ft_backward_long(const void* __restrict__ dft_stm, const void* __restrict__ dft_nstm,
-                                                            const int* __restrict__ offsets, const int* __restrict__ lists,
-                                                            int B, int A, int N, int F, int n_persp,
-                                                            const int* __restrict__ counters, const int2* __restrict__ work,
-                                                            float* __restrict__ partial, const int* __restrict__ run_if) {
-    if (run_if && *run_if == 0) return;  // gated: another path does this step's work
-    const int c = blockIdx.y * blockDim.x + threadIdx.x;
-    const int row4 = F >> 2;
-    const int n_work = counters[0];
-    for (int w = blockIdx.x; w < n_work; w += gridDim.x) {
-        const int2 wk = work[w];
-        const int f = wk.x;
-        int lo = wk.y * BWD_PART, hi = lo + BWD_PART;  // range in the concatenated (stm, nstm) list
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (blockIdx.x < BWD_SPLIT_BLOCKS) {
+        const int n_work = counters[INV_PARTS];
+        for (int w0 = blockIdx.x * groups; w0 < n_work; w0 += BWD_SPLIT_BLOCKS * groups) {
+            const int w = w0 + g;
+            int q = 0, f = 0, len0 = 0, len1 = 0;
+            if (w < n_work) {
+                const int2 wk = work[w];
+                q = wk.x;
+                f = split[3 * q];
+                len0 = counts[f];
+                len1 = n_persp > 1 ? counts[(size_t)N + f] : 0;
+                const int lo = wk.y * BWD_PART, hi = min(lo + BWD_PART, len0 + len1);  // range in the concatenated lists
+#pragma unroll
+                for (int i = 0; i < V; ++i) {
+                    const int ci = c + i * ths;
+                    if (ci >= row4) break;
+                    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (lo < len0) acc = sum_rows<DH>(dft_stm, lists + offsets[f] + lo, min(hi, len0) - lo, F, ci, acc);
+                    if (hi > len0) {
+                        const int a = max(lo - len0, 0);
+                        acc = sum_rows<DH>(dft_nstm, lists + cells + offsets[(size_t)N + f] + a, hi - len0 - a, F, ci, acc);
+                    }
+                    reinterpret_cast<float4*>(partial)[(size_t)w * row4 + ci] = acc;
+                }
+                __threadfence();
+            }
+            __syncthreads();
+            const int parts = (len0 + len1 + BWD_PART - 1) / BWD_PART;
+            if (ct == 0) s_last[g] = w < n_work && atomicAdd(split + 3 * q + 2, 1) == parts * (int)gridDim.y - 1;
+            __syncthreads();
+            if (s_last[g]) {  // every part of every strip is there
+                __threadfence();
+                const float4* p4 = reinterpret_cast<const float4*>(partial) + (size_t)split[3 * q + 1] * row4;
+                for (int k = ct; k < row4; k += ths) {
+                    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+                    for (int i = 0; i < parts; ++i) {
+                        const float4 v = __ldcg(p4 + (size_t)i * row4 + k);
+                        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+                    }
+                    reinterpret_cast<float4*>(grad)[(size_t)f * row4 + k] = acc;
+                }
+            }
+        }
+        return;
+    }
+
+    const int warps = blockDim.x >> 5, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int rows = warps * rpw, r0 = (blockIdx.x - BWD_SPLIT_BLOCKS) * rows;
+    const int limit = BWD_SORT_CELLS / rpw;
+    if (threadIdx.x < 32) {  // at most 32 rows
+        const int f = r0 + lane;
+        const bool in = lane < rows && f < N;
+        const int n0 = in ? counts[f] : 0, n1 = in && n_persp > 1 ? counts[(size_t)N + f] : 0;
+        s_off[0][lane] = in ? offsets[f] : 0;
+        s_off[1][lane] = in && n_persp > 1 ? offsets[(size_t)N + f] : 0;
+        s_len[0][lane] = n0;
+        s_len[1][lane] = n1;
+        const int n = max(n0, n1) <= limit ? n0 + n1 : 0;
+        int incl = n;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += t;
+        }
+        s_beg[lane + 1] = incl;
+        if (lane == 0) s_beg[0] = 0;
+    }
+    __syncthreads();
+    int* cells_s = s_mem + warps * BWD_SORT_CELLS;
+    {   // the warp's lists into shared memory, then every entry to its place: the number of smaller ones before it (equal
+        // ones, from a repeated feature, by index)
+        int* raw = s_mem + wid * BWD_SORT_CELLS;
         for (int p = 0; p < n_persp; ++p) {
-            const int beg = offsets[(size_t)p * (N + 1) + f], len = offsets[(size_t)p * (N + 1) + f + 1] - beg;
-            const int a = max(lo, 0), b = min(hi, len);
-            if (a < b)
-                acc = sum_rows<DH>(p ? dft_nstm : dft_stm, lists + (size_t)p * B * A, beg + a, beg + b, F, c, acc);
-            lo -= len;
-            hi -= len;
+            for (int j = 0; j < rpw; ++j) {
+                const int k = wid * rpw + j, n = s_len[p][k];
+                if (s_beg[k + 1] == s_beg[k]) continue;
+                const int* L = lists + p * cells + s_off[p][k];
+                for (int i = lane; i < n; i += 32) raw[j * limit + i] = L[i];
+            }
+            __syncwarp();
+            for (int j = 0; j < rpw; ++j) {
+                const int k = wid * rpw + j, n = s_len[p][k], end = s_beg[k + 1] - 1;
+                if (end < s_beg[k]) continue;
+                const int* L = raw + j * limit;
+                const int base = s_beg[k] + (p ? s_len[0][k] : 0);
+                for (int i = lane; i < n; i += 32) {
+                    const int v = L[i];
+                    int r = base;
+#pragma unroll 4
+                    for (int m = 0; m < n; ++m) {
+                        const int u = L[m];
+                        r += (u < v) || (u == v && m < i);
+                    }
+                    cells_s[r] = v | (p ? BWD_CELL_NSTM : 0) | (r == end ? BWD_CELL_LAST : 0);
+                }
+            }
+            __syncwarp();
         }
-        reinterpret_cast<float4*>(partial)[(size_t)w * row4 + c] = acc;
+    }
+    __syncthreads();
+    if (c >= row4) return;
+    float4* out = reinterpret_cast<float4*>(grad) + (size_t)r0 * row4 + c;
+    const int per = (rows + groups - 1) / groups, k0 = min(g * per, rows), k1 = min(min(k0 + per, rows), N - r0);
+    // rows without entries, and rows too long for shared memory
+    for (int k = k0; k < k1; ++k) {
+        if (s_beg[k + 1] > s_beg[k]) continue;
+        const int n0 = s_len[0][k], n1 = s_len[1][k];
+        if (n0 + n1 > BWD_PART) continue;  // summed in parts
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+            acc = sum_rows<DH>(dft_stm, lists + s_off[0][k], n0, F, c + i * ths, acc);
+            acc = sum_rows<DH>(dft_nstm, lists + cells + s_off[1][k], n1, F, c + i * ths, acc);
+            __stcs(out + (size_t)k * row4 + i * ths, acc);
+        }
+    }
+    // the other rows as one stream of entries, eight loads in flight across the ends of rows
+    constexpr int D = 8 / V;
+    const int e0 = s_beg[k0], e1 = k1 > k0 ? s_beg[k1] : e0;
+    float4 v[D][V], acc[V];
+    auto load = [&](int e, float4 (&x)[V]) {
+        const int cell = cells_s[e];
+        const void* d = cell & BWD_CELL_NSTM ? dft_nstm : dft_stm;
+        const size_t at = (size_t)(cell & (BWD_CELL_NSTM - 1)) * F + 4 * c;
+#pragma unroll
+        for (int i = 0; i < V; ++i) x[i] = ld4<DH>(d, at + 4 * i * ths);
+    };
+#pragma unroll
+    for (int u = 0; u < D; ++u)
+        if (e0 + u < e1) load(e0 + u, v[u]);
+#pragma unroll
+    for (int i = 0; i < V; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    int k = k0;
+    for (int e = e0; e < e1; e += D) {
+#pragma unroll
+        for (int u = 0; u < D; ++u) {
+            if (e + u >= e1) break;
+#pragma unroll
+            for (int i = 0; i < V; ++i) { acc[i].x += v[u][i].x; acc[i].y += v[u][i].y; acc[i].z += v[u][i].z; acc[i].w += v[u][i].w; }
+            if (e + u + D < e1) load(e + u + D, v[u]);
+            if (cells_s[e + u] < 0) {  // BWD_CELL_LAST
+                while (s_beg[k + 1] <= e + u) ++k;  // past rows without entries here
+#pragma unroll
+                for (int i = 0; i < V; ++i) {
+                    __stcs(out + (size_t)k * row4 + i * ths, acc[i]);  // not read again in this launch: L2 is the input's
+                    acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+            }
+        }
     }
 }
 
-__global__ void __launch_bounds__(512) k_ft_backward_long_final(const int* __restrict__ counters, const int* __restrict__ longf,
-                                                                  const float* __restrict__ partial, int F,
-                                                                  float* __restrict__ grad, const int* __restrict__ run_if) {
-    if (run_if && *run_if == 0) return;  // gated: another path does this step's work
-    const int c = blockIdx.y * blockDim.x + threadIdx.x;
-    const int row4 = F >> 2;
-    const int n_long = counters[1];
-    const float4* p4 = reinterpret_cast<const float4*>(partial);
-    for (int q = blockIdx.x; q < n_long; q += gridDim.x) {
-        const int f = longf[3 * q], base = longf[3 * q + 1], parts = longf[3 * q + 2];
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int i = 0; i < parts; ++i) {
-            const float4 v = p4[(size_t)(base + i) * row4 + c];
-            acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-        }
-        reinterpret_cast<float4*>(grad)[(size_t)f * row4 + c] = acc;
-    }
+int launch_inverse_index(cudaStream_t s, const int* idx_stm, const int* idx_nstm, const int* nnz, int B, int A, int N, int n_persp,
+                         int* counts, int* offsets, int* lists, int* plan) {
+    if (B <= 0) return 0;
+    const unsigned cells = (unsigned)B * (unsigned)A;
+    int* counters = counts + (size_t)2 * N;
+    int* long_queue = counters + INV_COUNTERS;
+    int* scratch = lists + (size_t)2 * cells;  // the ranks, then the long sort's copies
+    int2* work = reinterpret_cast<int2*>(plan);
+    int* split = plan + 2 * (size_t)ft_backward_max_work(B, A, n_persp);
+    cudaMemsetAsync(counts, 0, sizeof(int) * ((size_t)2 * N + INV_COUNTERS), s);
+    const dim3 grid((unsigned)min(ceil_div(cells, 256), 148 * 16), n_persp);
+    k_feat_count<<<grid, 256, 0, s>>>(idx_stm, idx_nstm, nnz, cells, A, N, counts, scratch);
+    k_feat_scan<<<dim3(ceil_div(N, SCAN_CELLS), n_persp), 1024, 0, s>>>(counts, N, n_persp, BWD_SORT_CELLS / bwd_rows_per_warp(B, A, N),
+                                                                        offsets, counters, long_queue, work, split);
+    k_feat_fill<<<grid, 256, 0, s>>>(idx_stm, idx_nstm, nnz, cells, A, N, offsets, scratch, lists);
+    int words = (B + 31) / 32;
+    if ((size_t)words * 4 > 160 * 1024) words = 0;
+    // per device and cheap: set before every launch (a process may drive several GPUs)
+    cudaFuncSetAttribute(k_lists_sort_long, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    k_lists_sort_long<<<148 * 4, 256, (size_t)words * 4, s>>>(counts, offsets, N, cells, lists, scratch, long_queue,
+                                                              counters + INV_QUEUED, words);
+    return 4;
 }
 
 int ft_backward_max_work(int B, int A, int n_persp) { return 2 * (int)(((long long)n_persp * B * A) / BWD_PART) + 2; }
 
-// plan: [2] counters, then [2 * max_work] work items, then [3 * N] long-feature records; partial: [max_work][F]
-int launch_ft_backward_split(cudaStream_t s, const int* run_if, const void* dft_stm, const void* dft_nstm, const int* offsets,
-                             const int* lists, int B, int A, int N, int F, int n_persp, int* plan, float* partial,
-                             float* grad, int dft_half) {
-    const int max_work = ft_backward_max_work(B, A, n_persp);
-    int* counters = plan;
-    int2* work = reinterpret_cast<int2*>(plan + 2);
-    int* longf = plan + 2 + 2 * max_work;
-    cudaMemsetAsync(counters, 0, 2 * sizeof(int), s);
-    k_bwd_plan<<<ceil_div(N, 256), 256, 0, s>>>(offsets, N, n_persp, counters, work, longf, run_if);
-    const int ny = ceil_div(F / 4, 512), bx = F / 4 / ny;  // at most 512 threads per block: room for 64 registers each
-    // a gated launch (run_if) normally returns at once: a small grid of row-striding blocks keeps that cheap
-    const dim3 gs(run_if && N > 148 * 32 ? 148 * 32 : N, ny), gl(148 * 4, ny);
-    if (dft_half) {
-        k_ft_backward_short<true><<<gs, bx, 0, s>>>(dft_stm, dft_nstm, offsets, lists, B, A, N, F, n_persp, grad, run_if);
-        k_ft_backward_long<true><<<gl, bx, 0, s>>>(dft_stm, dft_nstm, offsets, lists, B, A, N, F, n_persp, counters, work, partial, run_if);
-    } else {
-        k_ft_backward_short<false><<<gs, bx, 0, s>>>(dft_stm, dft_nstm, offsets, lists, B, A, N, F, n_persp, grad, run_if);
-        k_ft_backward_long<false><<<gl, bx, 0, s>>>(dft_stm, dft_nstm, offsets, lists, B, A, N, F, n_persp, counters, work, partial, run_if);
-    }
-    k_ft_backward_long_final<<<dim3(148 * 2, ny), bx, 0, s>>>(counters, longf, partial, F, grad, run_if);
-    return 4;
+int launch_ft_backward_split(cudaStream_t s, const void* dft_stm, const void* dft_nstm, const int* counts, const int* offsets,
+                             const int* lists, int B, int A, int N, int F, int n_persp, int* plan, float* partial, float* grad,
+                             int dft_half) {
+    const int2* work = reinterpret_cast<const int2*>(plan);
+    int* split = plan + 2 * (size_t)ft_backward_max_work(B, A, n_persp);
+    // The widest strips of whole 128-column pieces that keep the input in L2 and a group within a block; two pieces are not
+    // cut.  Two float4 columns per thread where the strips allow it: half the instructions per byte.
+    const int pieces = F / 128;
+    int ny = 0, per, v;
+    do {
+        per = ceil_div(pieces, ++ny);
+        v = per % 2 == 0 && pieces % per == 0 ? 2 : 1;
+    } while (per / v > 8 || (per > 2 && (long long)n_persp * B * per * (dft_half ? 256 : 512) > BWD_STRIP_BYTES));
+    ny = ceil_div(pieces, per);
+    const int strip4 = 32 * per, ths = strip4 / v, threads = ths * (ths < 256 ? 256 / ths : 1);
+    const int warps = threads / 32, rpw = bwd_rows_per_warp(B, A, N);
+    const dim3 grid(BWD_SPLIT_BLOCKS + ceil_div(N, warps * rpw), ny);
+    const size_t smem = sizeof(int) * BWD_SORT_CELLS * warps * (1 + n_persp);
+    const size_t cells = (size_t)B * A;
+    auto* kernel = dft_half ? (v == 2 ? k_ft_backward<true, 2> : k_ft_backward<true, 1>)
+                            : (v == 2 ? k_ft_backward<false, 2> : k_ft_backward<false, 1>);
+    kernel<<<grid, threads, smem, s>>>(dft_stm, dft_nstm, counts, offsets, lists, cells, N, F, n_persp, strip4, rpw,
+                                       counts + (size_t)2 * N, work, split, partial, grad);
+    return 1;
 }
 
 // ft_reduce_virtual_grad (sparse/ft_factorize.rs:109-121): grad[N + v] = sum over king buckets of grad[kb*pi + v]

@@ -58,7 +58,7 @@ extern "C" int tb_ft_microbench(int device, const int32_t* indices, const int32_
     const size_t B = batch, F = ft_out, N = ft_in, A = max_active;
     const int rps = rows_per_slice > 0 ? rows_per_slice : ft_in;
     float *d_table = nullptr, *d_x = nullptr, *d_grad = nullptr, *d_m = nullptr, *d_v = nullptr, *d_part = nullptr;
-    int *d_idx = nullptr, *d_nnz = nullptr, *d_cnt = nullptr, *d_off = nullptr, *d_cur = nullptr, *d_lists = nullptr, *d_plan = nullptr;
+    int *d_idx = nullptr, *d_nnz = nullptr, *d_cnt = nullptr, *d_off = nullptr, *d_lists = nullptr, *d_plan = nullptr;
     int *d_order = nullptr, *d_ntiles = nullptr, *d_seg = nullptr, *d_hist = nullptr, *d_items = nullptr, *d_itemseg = nullptr;
     int *d_fwd_work = nullptr, *d_bwd_work = nullptr;
     float* d_slabs = nullptr;
@@ -78,8 +78,8 @@ extern "C" int tb_ft_microbench(int device, const int32_t* indices, const int32_
     MB(cudaMalloc(&d_table, N * F * 4)); MB(cudaMalloc(&d_x, B * F * 4)); MB(cudaMalloc(&d_grad, N * F * 4));
     MB(cudaMalloc(&d_m, N * F * 4)); MB(cudaMalloc(&d_v, N * F * 4));
     MB(cudaMalloc(&d_idx, B * A * 4)); MB(cudaMalloc(&d_nnz, B * 4));
-    MB(cudaMalloc(&d_cnt, inverse_index_counts_len(ft_in) * 4)); MB(cudaMalloc(&d_off, 2 * (N + 1) * 4)); MB(cudaMalloc(&d_cur, 2 * N * 4));
-    MB(cudaMalloc(&d_lists, 4 * B * A * 4)); MB(cudaMalloc(&d_plan, (2 + 2 * max_work + 3 * N) * 4)); MB(cudaMalloc(&d_part, max_work * F * 4));
+    MB(cudaMalloc(&d_cnt, inverse_index_counts_len(ft_in) * 4)); MB(cudaMalloc(&d_off, 2 * N * 4));
+    MB(cudaMalloc(&d_lists, 4 * B * A * 4)); MB(cudaMalloc(&d_plan, (2 * max_work + 3 * N) * 4)); MB(cudaMalloc(&d_part, max_work * F * 4));
     MB(cudaMemcpy(d_idx, indices, B * A * 4, cudaMemcpyHostToDevice));
     MB(cudaMemcpy(d_nnz, nnz, B * 4, cudaMemcpyHostToDevice));
     k_fill_pattern<<<148 * 8, 256>>>(d_table, N * F, 0.05f, 1u);
@@ -98,8 +98,8 @@ extern "C" int tb_ft_microbench(int device, const int32_t* indices, const int32_
     out->fwd_ms = (float)(tm.total / iters);
     k_fill_pattern<<<148 * 8, 256>>>(d_x, B * F, 1e-3f, 3u);  // the incoming gradient rows
     MB(tm.run(iters, [&] {
-        launch_inverse_index(0, nullptr, d_idx, d_idx, d_nnz, batch, max_active, ft_in, 1, d_cnt, d_off, d_cur, d_lists);
-        launch_ft_backward_split(0, nullptr, d_x, d_x, d_off, d_lists, batch, max_active, ft_in, ft_out, 1, d_plan, d_part, d_grad);
+        launch_inverse_index(0, d_idx, d_idx, d_nnz, batch, max_active, ft_in, 1, d_cnt, d_off, d_lists, d_plan);
+        launch_ft_backward_split(0, d_x, d_x, d_cnt, d_off, d_lists, batch, max_active, ft_in, ft_out, 1, d_plan, d_part, d_grad);
     }));
     out->bwd_ms = (float)(tm.total / iters);
     MB(tm.run(iters, [&] { launch_radam(0, d_table, d_m, d_v, d_grad, nullptr, (int64_t)(N * F), sc); }));
@@ -137,7 +137,7 @@ extern "C" int tb_ft_microbench(int device, const int32_t* indices, const int32_
     }
 done:
     cudaFree(d_table); cudaFree(d_x); cudaFree(d_grad); cudaFree(d_m); cudaFree(d_v); cudaFree(d_part); cudaFree(d_idx); cudaFree(d_nnz);
-    cudaFree(d_cnt); cudaFree(d_off); cudaFree(d_cur); cudaFree(d_lists); cudaFree(d_plan); cudaFree(d_order); cudaFree(d_ntiles);
+    cudaFree(d_cnt); cudaFree(d_off); cudaFree(d_lists); cudaFree(d_plan); cudaFree(d_order); cudaFree(d_ntiles);
     cudaFree(d_seg); cudaFree(d_hist); cudaFree(d_items); cudaFree(d_itemseg); cudaFree(d_fwd_work); cudaFree(d_bwd_work); cudaFree(d_tiles); cudaFree(d_slabs);
     cudaFree(tm.flush);
     if (tm.e0) cudaEventDestroy(tm.e0);

@@ -5,11 +5,11 @@
 // latency-critical service and must not touch the driver's allocator on its hot path, or a harness that
 // forbids cudaMalloc after start-up so that fragmentation cannot surprise it hours into a run.  Such a
 // caller can hand over its own input and output buffers but has nowhere to get the working memory of the
-// inverse index (histogram, offsets, cursors, position lists) from.
+// inverse index (histogram, offsets, position lists) from.
 //
 // tb_ft_backward_static_scratch therefore keeps that working memory in a file-scope __device__ array of a
 // fixed size.  It calls no cudaMalloc / cudaFree and no allocating library routine.  The price:
-//   - every GPU on which this library's device code is used holds the array (about 21.5 MB) from that first
+//   - every GPU on which this library's device code is used holds the array (about 20.5 MB) from that first
 //     use until the process exits;
 //   - sizes are capped: ft_in <= TB_STATIC_SCRATCH_MAX_FT_IN rows, batch * max_active <=
 //     TB_STATIC_SCRATCH_MAX_PAIRS index slots; larger problems are refused with an error text;
@@ -28,13 +28,12 @@
 #define MAX_FT_IN TB_STATIC_SCRATCH_MAX_FT_IN
 #define MAX_PAIRS TB_STATIC_SCRATCH_MAX_PAIRS
 #define MAX_FT_OUT 4096
-// layout expected by launch_inverse_index: histogram + long-list queue + scan sums, offsets [2(N + 1)],
-// cursors [2N], lists + sort scratch [4P]; then what launch_ft_backward_split needs to cut long lists into parts:
-// its plan [2 + 2 * max_work + 3N] and the partial rows [max_work][F]
-#define COUNTS_INTS (4 * MAX_FT_IN + 1 + 2 * (MAX_FT_IN / 2048 + 2))
+// layout expected by launch_inverse_index: histogram + counters + long-list queue, offsets [2N], lists + sort scratch [4P]
+// and the plan for lists cut into parts [2 * max_work + 3N]; then launch_ft_backward_split's partial rows [max_work][F]
+#define COUNTS_INTS (4 * MAX_FT_IN + 8)
 #define MAX_WORK (2 * (MAX_PAIRS / 4096) + 2)   /* ft_backward_max_work at the slot limit */
-#define PLAN_INTS (2 + 2 * MAX_WORK + 3 * MAX_FT_IN)
-#define SCRATCH_INTS (COUNTS_INTS + 4 * MAX_FT_IN + 2 + 4 * MAX_PAIRS + PLAN_INTS + MAX_WORK * MAX_FT_OUT + 64)
+#define PLAN_INTS (2 * MAX_WORK + 3 * MAX_FT_IN)
+#define SCRATCH_INTS (COUNTS_INTS + 2 * MAX_FT_IN + 4 * MAX_PAIRS + PLAN_INTS + MAX_WORK * MAX_FT_OUT + 64)
 
 // In host code this name is only a handle for the runtime, not a device address: it must never be passed
 // to a kernel.  The address comes from cudaGetSymbolAddress below.
@@ -89,24 +88,22 @@ extern "C" int tb_ft_backward_static_scratch(const float* d_dft, const int32_t* 
     }
     const size_t N = (size_t)ft_in, P = (size_t)batch * max_active;
     int* counts = base;                                         // [inverse_index_counts_len(N)]
-    int* offsets = counts + inverse_index_counts_len(ft_in);    // [2(N + 1)]
-    int* cursor = offsets + 2 * (N + 1);      // [2N]
-    int* lists = cursor + 2 * N;              // [4P]
+    int* offsets = counts + inverse_index_counts_len(ft_in);    // [2N]
+    int* lists = offsets + 2 * N;                               // [4P]
     // The plan holds 8-byte records and the partial rows are moved as float4: both start on a 16-byte boundary of the
     // array itself (offsets from its 256-byte aligned base rounded up to a multiple of four ints).
     const size_t max_work = (size_t)ft_backward_max_work(batch, max_active, 1);  // <= MAX_WORK by the slot limit
     const size_t plan_off = ((size_t)(lists - base) + 4 * P + 3) / 4 * 4;
-    const size_t partial_off = (plan_off + 2 + 2 * max_work + 3 * N + 3) / 4 * 4;
-    int* plan = base + plan_off;              // [2 + 2 * max_work + 3N]
+    const size_t partial_off = (plan_off + 2 * max_work + 3 * N + 3) / 4 * 4;
+    int* plan = base + plan_off;              // [2 * max_work + 3N]
     float* partial = reinterpret_cast<float*>(base + partial_off);
     if (partial_off + max_work * (size_t)ft_out > (size_t)SCRATCH_INTS)   // cannot happen inside the limits checked above
         return report(err, err_len, TB_ERR_INVALID_ARGUMENT, "static scratch layout overflow");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // launch_inverse_index clears the histogram and the long-list counter itself, launch_ft_backward_split its two
-    // counters; offsets, cursors, lists, plan and partial rows are rewritten for the rows and slots this call uses
-    launch_inverse_index(s, nullptr, d_indices, d_indices, d_nnz, batch, max_active, ft_in, 1, counts, offsets, cursor, lists);
-    // the same launcher as tb_ft_backward_bench: lists of more than 4096 entries are summed in parts of 4096
-    launch_ft_backward_split(s, nullptr, d_dft, d_dft, offsets, lists, batch, max_active, ft_in, ft_out, 1, plan, partial, d_grad);
+    // launch_inverse_index clears the histogram and the counters itself; offsets, lists, plan and partial rows are rewritten
+    // for the rows and slots this call uses.  Lists of more than 4096 entries are summed in parts of 4096.
+    launch_inverse_index(s, d_indices, d_indices, d_nnz, batch, max_active, ft_in, 1, counts, offsets, lists, plan);
+    launch_ft_backward_split(s, d_dft, d_dft, counts, offsets, lists, batch, max_active, ft_in, ft_out, 1, plan, partial, d_grad);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
         if (err && err_len) snprintf(err, err_len, "kernel launch: %s", cudaGetErrorString(e));

@@ -180,7 +180,7 @@ struct tb_trainer {
     int *order = nullptr, *n_tiles = nullptr, *seg_start = nullptr;
     TileDesc* tiles = nullptr;
     float *small_partials = nullptr, *l1w_partials = nullptr, *bias_partials = nullptr, *l1_weff = nullptr;
-    int *feat_counts = nullptr, *feat_offsets = nullptr, *feat_cursor = nullptr, *feat_lists = nullptr;
+    int *feat_counts = nullptr, *feat_offsets = nullptr, *feat_lists = nullptr;
     int *sort_hist = nullptr, *items = nullptr, *item_seg = nullptr, *bwd_plan = nullptr, *fwd_work = nullptr, *bwd_slice = nullptr;
     int dgrad_rows = 0;
     int bwd_parts = 1;  // launches the FT weight gradient is cut into (data parallel)
@@ -588,11 +588,9 @@ int run_backward(tb_trainer* t, const DevBatch& d, float lr) {
                                         FT_POST_SCALE, B, F, c.l1_out, 0, t->dft[0], t->dft[1], t->bias_partials,
                                         t->groups[1].grad, t->dgrad_rows)); }
     }
-    // slice-resident path when this step's forward was; the generic kernels then run only for a batch with a row outside
-    // its item's slice (device-side gate)
+    // slice-resident path when this step's forward was, except for a batch with a row outside its item's slice
     const void* dft0 = t->p_out16 ? t->dft_h[0] : (const void*)t->dft[0];
     const void* dft1 = t->p_out16 ? t->dft_h[1] : (const void*)t->dft[1];
-    const int* gate = slice_bwd ? ft_slice_outside_flag(t->fwd_work, 2 * B, N, rps) : nullptr;
     // The generic kernels are launched only for a batch that needs them.  The host knows by now: the check ran behind the
     // upload, and what was launched above keeps the GPU busy (ten launches that found nothing to do were 28 us of every step).
     bool generic = true;
@@ -604,15 +602,15 @@ int run_backward(tb_trainer* t, const DevBatch& d, float lr) {
       int n = 0;
       if (si == t->stream) n += inverse();
       else CU(t, cudaStreamWaitEvent(t->stream, t->ev_inv, 0));
-      if (generic) n += launch_inverse_index(t->stream, gate, d.stm, d.nstm, d.nnz, B, A, N, 2, t->feat_counts, t->feat_offsets, t->feat_cursor,
-                                t->feat_lists);
+      if (generic) n += launch_inverse_index(t->stream, d.stm, d.nstm, d.nnz, B, A, N, 2, t->feat_counts, t->feat_offsets, t->feat_lists,
+                                             t->bwd_plan);
       p.done(n); }
     // the first exchanged part carries the small groups' gradients; a call for gradients alone returns with all of them
     if (c.world_size > 1 || lr < 0.0f) { const int jrc = join_wgrad(t); if (jrc != TB_OK) return jrc; }
     else if (t->wgrad_forked) CU(t, cudaEventRecord(t->ev_dense, t->stream));
     { PhaseScope p(t, PH_FT_BWD);
       int n = 0;
-      if (generic) n = launch_ft_backward_split(t->stream, gate, dft0, dft1, t->feat_offsets, t->feat_lists, B, A, N, F, 2,
+      if (generic) n = launch_ft_backward_split(t->stream, dft0, dft1, t->feat_counts, t->feat_offsets, t->feat_lists, B, A, N, F, 2,
                                        t->bwd_plan, t->bwd_partial, t->groups[0].grad, t->p_out16);
       if (slice_bwd) {
           // Data parallel: the slices are done in several launches (ar_parts_for) and the gradient rows of each part are all-reduced on a
@@ -960,7 +958,7 @@ void free_all(tb_trainer* t) {
     cudaFree(t->tail_a); cudaFree(t->tail_b); cudaFree(t->tail_c); cudaFree(t->loss_partials); cudaFree(t->loss_acc); cudaFree(t->wrm_weight_sum);
     cudaFree(t->order); cudaFree(t->n_tiles); cudaFree(t->seg_start); cudaFree(t->tiles);
     cudaFree(t->small_partials); cudaFree(t->l1w_partials); cudaFree(t->bias_partials); cudaFree(t->l1_weff);
-    cudaFree(t->feat_counts); cudaFree(t->feat_offsets); cudaFree(t->feat_cursor); cudaFree(t->feat_lists);
+    cudaFree(t->feat_counts); cudaFree(t->feat_offsets); cudaFree(t->feat_lists);
     cudaFree(t->fwd_work); cudaFree(t->bwd_slice); cudaFree(t->sort_hist); cudaFree(t->items); cudaFree(t->item_seg); cudaFree(t->bwd_plan); cudaFree(t->bwd_partial); cudaFree(t->bwd_slabs);
     if (t->ev_t0) cudaEventDestroy(t->ev_t0);
     if (t->ev_t1) cudaEventDestroy(t->ev_t1);
@@ -1115,7 +1113,7 @@ int create_impl(tb_trainer* t) {
     CU(t, dalloc(&t->l1_weff, (size_t)(nb + 1) * l1 * (t->K + 1)));  // effective L1 weights and biases per bucket
     t->dgrad_rows = DGRAD_CTAS > 2 * t->max_units ? DGRAD_CTAS : 2 * t->max_units;  // partial FT bias rows: one per block
     CU(t, dalloc(&t->bias_partials, (size_t)t->dgrad_rows * 2 * F));
-    CU(t, dalloc(&t->feat_counts, inverse_index_counts_len((int)N))); CU(t, dalloc(&t->feat_offsets, (size_t)2 * (N + 1)));
+    CU(t, dalloc(&t->feat_counts, inverse_index_counts_len((int)N))); CU(t, dalloc(&t->feat_offsets, (size_t)2 * N));
     // histograms of the item sort and of the bucket sort
     CU(t, dalloc(&t->sort_hist, (size_t)128 * (2 * B / 1024 + 2) + (size_t)(TB_MAX_BUCKETS + 1) * (B / 1024 + 2)));
     CU(t, dalloc(&t->items, 2 * B)); CU(t, dalloc(&t->item_seg, 130));
@@ -1131,10 +1129,10 @@ int create_impl(tb_trainer* t) {
     }
     {
         const size_t max_work = (size_t)ft_backward_max_work((int)B, (int)A, 2);
-        CU(t, dalloc(&t->bwd_plan, 2 + 2 * max_work + 3 * (size_t)N));
+        CU(t, dalloc(&t->bwd_plan, 2 * max_work + 3 * (size_t)N));
         CU(t, dalloc(&t->bwd_partial, max_work * (size_t)F));
     }
-    CU(t, dalloc(&t->feat_cursor, (size_t)2 * N)); CU(t, dalloc(&t->feat_lists, (size_t)4 * B * A));
+    CU(t, dalloc(&t->feat_lists, (size_t)4 * B * A));
     CU(t, cudaEventCreate(&t->ev_t0)); CU(t, cudaEventCreate(&t->ev_t1));
     for (int i = 0; i < PH_COUNT; ++i) {
         CU(t, cudaEventCreate(&t->ph_start[i])); CU(t, cudaEventCreate(&t->ph_stop[i]));
@@ -1663,31 +1661,31 @@ int tb_ft_backward_bench(int device, const float* dft, const int32_t* indices, c
     if (!dft || !indices || !nnz || batch < 1 || ft_out % 128 != 0 || iters < 1) return fail(nullptr, TB_ERR_INVALID_ARGUMENT, "bad argument");
     int rc = TB_OK;
     float *d_d = nullptr, *d_g = nullptr;
-    int *d_i = nullptr, *d_n = nullptr, *d_cnt = nullptr, *d_off = nullptr, *d_cur = nullptr, *d_lists = nullptr, *d_plan = nullptr;
+    int *d_i = nullptr, *d_n = nullptr, *d_cnt = nullptr, *d_off = nullptr, *d_lists = nullptr, *d_plan = nullptr;
     float* d_part = nullptr;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     const size_t B = batch, F = ft_out, N = ft_in, A = max_active;
     const size_t max_work = (size_t)ft_backward_max_work(batch, max_active, 1);
     CUX(cudaSetDevice(device));
     CUX(cudaMalloc(&d_d, B * F * 4)); CUX(cudaMalloc(&d_g, N * F * 4)); CUX(cudaMalloc(&d_i, B * A * 4)); CUX(cudaMalloc(&d_n, B * 4));
-    CUX(cudaMalloc(&d_cnt, inverse_index_counts_len(ft_in) * 4)); CUX(cudaMalloc(&d_off, 2 * (N + 1) * 4)); CUX(cudaMalloc(&d_cur, 2 * N * 4));
+    CUX(cudaMalloc(&d_cnt, inverse_index_counts_len(ft_in) * 4)); CUX(cudaMalloc(&d_off, 2 * N * 4));
     CUX(cudaMalloc(&d_lists, 4 * B * A * 4));
-    CUX(cudaMalloc(&d_plan, (2 + 2 * max_work + 3 * N) * 4)); CUX(cudaMalloc(&d_part, max_work * F * 4));
+    CUX(cudaMalloc(&d_plan, (2 * max_work + 3 * N) * 4)); CUX(cudaMalloc(&d_part, max_work * F * 4));
     CUX(cudaMemcpy(d_d, dft, B * F * 4, cudaMemcpyHostToDevice));
     CUX(cudaMemcpy(d_i, indices, B * A * 4, cudaMemcpyHostToDevice));
     CUX(cudaMemcpy(d_n, nnz, B * 4, cudaMemcpyHostToDevice));
     CUX(cudaEventCreate(&e0)); CUX(cudaEventCreate(&e1));
     for (int i = -1; i < iters; ++i) {
         if (i == 0) { CUX(cudaDeviceSynchronize()); CUX(cudaEventRecord(e0, 0)); }
-        launch_inverse_index(0, nullptr, d_i, d_i, d_n, batch, max_active, ft_in, 1, d_cnt, d_off, d_cur, d_lists);
-        launch_ft_backward_split(0, nullptr, d_d, d_d, d_off, d_lists, batch, max_active, ft_in, ft_out, 1, d_plan, d_part, d_g);
+        launch_inverse_index(0, d_i, d_i, d_n, batch, max_active, ft_in, 1, d_cnt, d_off, d_lists, d_plan);
+        launch_ft_backward_split(0, d_d, d_d, d_cnt, d_off, d_lists, batch, max_active, ft_in, ft_out, 1, d_plan, d_part, d_g);
     }
     CUX(cudaEventRecord(e1, 0));
     CUX(cudaEventSynchronize(e1));
     { float ms = 0.f; CUX(cudaEventElapsedTime(&ms, e0, e1)); if (ms_per_iter) *ms_per_iter = ms / iters; }
     if (grad) CUX(cudaMemcpy(grad, d_g, N * F * 4, cudaMemcpyDeviceToHost));
 done:
-    cudaFree(d_d); cudaFree(d_g); cudaFree(d_i); cudaFree(d_n); cudaFree(d_cnt); cudaFree(d_off); cudaFree(d_cur); cudaFree(d_lists);
+    cudaFree(d_d); cudaFree(d_g); cudaFree(d_i); cudaFree(d_n); cudaFree(d_cnt); cudaFree(d_off); cudaFree(d_lists);
     cudaFree(d_plan); cudaFree(d_part);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
