@@ -135,8 +135,9 @@ int sort_units(int n_pos);  // the most work units a batch of n_pos positions ha
 // tiles followed by the work units; n_tiles: TB_TILE_COUNTS ints); items (position, perspective) of both
 // perspectives by the table slice of their features -> items, item_seg [slices + 2].  hist: scratch of
 // (nb + 1) * ceil(B / 1024) + (slices + 1) * ceil(n_persp * B / 1024) ints
-// fwd_work / bwd_work: also plan the slice-resident forward / weight gradient (the latter in bwd_parts launches over equal
+// items NULL (B <= SORT_ONE_BLOCK): the positions alone, in one launch.  fwd_work / bwd_work: also plan the slice-resident forward / weight gradient (the latter in bwd_parts launches over equal
 // ranges of slices)
+#define SORT_ONE_BLOCK 8192  // most positions of launch_step_sorts without items
 int launch_step_sorts(cudaStream_t s, const int* bucket /*may be NULL*/, int B, int nb, int* order, TileDesc* tiles, int* n_tiles,
                       int* seg_start, int max_tiles, const int* idx_stm, const int* idx_nstm, const int* nnz, int A, int N,
                       int rows_per_slice, int n_persp, int* items, int* item_seg, int* hist, int* fwd_work = nullptr,

@@ -319,6 +319,57 @@ __global__ void __launch_bounds__(PLAN_THREADS) k_step_plans(const int* __restri
     else plan_backward(s_seg, n_keys, ch, parts, chunks, n_chunks, groups, sched);
 }
 
+// Positions by bucket and their tiles in one launch of one block, for batches of at most SORT_ONE_BLOCK positions whose items
+// need no order: every warp owns a run of positions, counts its keys, and places them behind those of the warps before it.
+// (The four launches cost 21 to 24 us however small the batch.)
+__global__ void __launch_bounds__(1024) k_sort_one_block(BucketKey fn, int n, int K, int ut, int* __restrict__ order, int* __restrict__ seg_start,
+                                                         TileDesc* __restrict__ tiles, int* __restrict__ n_tiles, TileDesc* __restrict__ units) {
+    __shared__ int s_cnt[TB_MAX_BUCKETS + 1][32], s_seg[TB_MAX_BUCKETS + 3];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (w < K) s_cnt[w][lane] = 0;
+    __syncthreads();
+    const int per = ((n + 31) / 32 + 31) & ~31, i0 = w * per, i1 = min(n, i0 + per);
+    // place = false: count; the counts are then turned into the first slots
+    auto walk = [&](bool place) {
+        for (int i = i0; i < i1; i += 32) {
+            const bool in = i + lane < i1;
+            const int k = in ? fn(i + lane) : K;
+            const unsigned same = __match_any_sync(0xffffffffu, k);
+            const int before = __popc(same & ((1u << lane) - 1));
+            int at = 0;
+            if (in) at = s_cnt[k][w] + before;
+            __syncwarp();
+            if (in && before == 0) s_cnt[k][w] += __popc(same);
+            if (in && place) order[at] = i + lane;
+            __syncwarp();
+        }
+    };
+    walk(false);
+    __syncthreads();
+    if (w < K) {
+        const int c = s_cnt[w][lane];
+        int incl = c;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += t;
+        }
+        s_cnt[w][lane] = incl - c;
+        if (lane == 31) s_seg[w + 1] = incl;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s_seg[0] = 0;
+        for (int k = 0; k < K; ++k) s_seg[k + 1] += s_seg[k];
+    }
+    __syncthreads();
+    if (w < K) s_cnt[w][lane] += s_seg[w];
+    if ((int)threadIdx.x <= K) seg_start[threadIdx.x] = s_seg[threadIdx.x];
+    __syncthreads();
+    walk(true);
+    plan_tiles(s_seg, K, ut, tiles, n_tiles, units, n_tiles + 1);
+}
+
 // The question k_fwd_codes answers for the device, asked as soon as the batch is there, for the host: the slice of an item
 // is that of its first feature (ItemKey), slots beyond nnz and indices outside the table do not count.  A warp per position.
 __global__ void __launch_bounds__(256) k_slice_check(const int* __restrict__ idx_stm, const int* __restrict__ idx_nstm,
@@ -357,7 +408,8 @@ int sort_max_units(int max_tiles) {
 }
 
 // Both sorts of a step in four launches: positions by bucket (order, tiles, units) and items by table slice, with the plans
-// of the slice-resident kernels where their work buffers are given.
+// of the slice-resident kernels where their work buffers are given; without `items` (B <= SORT_ONE_BLOCK) the positions alone,
+// in one launch.
 // hist: scratch of (nb + 1) * ceil(B / 1024) + (slices + 1) * ceil(n_persp * B / 1024) ints.
 int launch_step_sorts(cudaStream_t s, const int* bucket, int B, int nb, int* order, TileDesc* tiles, int* n_tiles, int* seg_start,
                       int max_tiles, const int* idx_stm, const int* idx_nstm, const int* nnz, int A, int N, int rows_per_slice,
@@ -368,6 +420,10 @@ int launch_step_sorts(cudaStream_t s, const int* bucket, int B, int nb, int* ord
         n_slices = ceil_div(N, rows_per_slice);
     }
     const int K0 = nb + 1, G0 = ceil_div(B, SORT_BLOCK);
+    if (!items) {
+        k_sort_one_block<<<1, 1024, 0, s>>>(BucketKey{bucket, nb}, B, K0, unit_tiles(B), order, seg_start, tiles, n_tiles, tiles + max_tiles);
+        return 1;
+    }
     const int n1 = n_persp * B, K1 = n_slices + 1, G1 = ceil_div(n1, SORT_BLOCK);
     int* h0 = hist;
     int* h1 = hist + (size_t)K0 * G0;

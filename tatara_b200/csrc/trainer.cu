@@ -110,9 +110,26 @@ struct Group {
     float *w = nullptr, *m = nullptr, *v = nullptr, *slow = nullptr, *grad = nullptr;
 };
 
+// The six arrays of a batch lie behind one another in one block, on the device and in the page-locked stage alike, packed for
+// the batch's own size: an upload is then one transfer where the caller's arrays have to be staged.
+struct BatchLayout {
+    size_t off[6], bytes;  // stm, nstm, nnz, bucket, score, wdl
+    BatchLayout(size_t n, size_t A) {
+        const size_t len[6] = {n * A * 4, n * A * 4, n * 4, n * 4, n * 4, n * 4};
+        size_t o = 0;
+        for (int i = 0; i < 6; ++i) { off[i] = o; o += (len[i] + 255) / 256 * 256; }
+        bytes = o;
+    }
+};
+
 struct DevBatch {
+    char* base = nullptr;
     int *stm = nullptr, *nstm = nullptr, *nnz = nullptr, *bucket = nullptr;
     float *score = nullptr, *wdl = nullptr;
+    void place(const BatchLayout& L) {
+        stm = (int*)(base + L.off[0]); nstm = (int*)(base + L.off[1]); nnz = (int*)(base + L.off[2]); bucket = (int*)(base + L.off[3]);
+        score = (float*)(base + L.off[4]); wdl = (float*)(base + L.off[5]);
+    }
     int n_pos = 0;
     float norm = 0.f;
     // Does some item have a row outside its king-bucket slice?  *outside (page-locked, written by the device) once `checked`
@@ -120,11 +137,6 @@ struct DevBatch {
     int* outside = nullptr;
     bool inside_known = false;
     cudaEvent_t checked = nullptr;
-};
-
-struct HostStage {
-    int *stm = nullptr, *nstm = nullptr, *nnz = nullptr, *bucket = nullptr;
-    float *score = nullptr, *wdl = nullptr;
 };
 
 enum Phase {
@@ -166,7 +178,7 @@ struct tb_trainer {
     uint64_t step_count = 0;
     // inputs
     DevBatch ring[2], slots[TB_NUM_SLOTS];
-    HostStage stage[2];
+    char* stage[2] = {nullptr, nullptr};  // page-locked, of the batch layout
     unsigned char* ring_psv[2] = {nullptr, nullptr};   // device: the 40-byte records of a batch fed as PackedSfenValue
     unsigned char* stage_psv[2] = {nullptr, nullptr};  // pinned staging for pageable record buffers
     cudaEvent_t ev_upload[2] = {nullptr, nullptr}, ev_consumed[2] = {nullptr, nullptr};
@@ -337,35 +349,53 @@ bool is_pinned(const void* p) {
 }
 
 #define UPLOAD_PIECE ((size_t)256 << 10)  // what a thread copies at a time
-#define UPLOAD_SEND 4                     // pieces per transfer: one transfer each leaves gaps (43 of 512 KB: 0.78 ms, 21 of 1 MB: 0.51)
+#define UPLOAD_SEND ((size_t)1 << 20)     // what a transfer carries at least: 43 of 512 KB leave gaps (0.78 ms), 21 of 1 MB do not (0.51)
+#define UPLOAD_DIRECT ((size_t)64 << 10)  // page-locked arrays below this are staged as well: a transfer costs more than the copy
+
+// Does a batch of n positions take the slice-resident FT kernels?  These read the whole table (and write the whole gradient)
+// in 128-byte pieces, whatever the batch holds; the gather reads rows of the lists alone, through L2, and is the faster one
+// until the lists hold a few entries per table row.  Forward of 1600 positions: 74 us against 162 at F = 1536, 21 against 60 at
+// F = 256, still 206 against 260 at 5500 and 7000 positions (6 and 4 entries per row).  Training step of 1008 positions: 0.92
+// against 1.13 ms and 0.35 against 0.42; equal at 4.5 and 4.2 entries per row.  Data parallel ranks stay with the slices: their
+// batches may differ in size, and the exchange of the gradient's parts may not.
+bool slice_path(const tb_trainer* t, int n, bool backward) {
+    const tb_config& c = t->cfg;
+    if (!ft_forward_slice_supported(c.ft_out, c.ft_in, c.max_active, c.piece_inputs > 0 ? c.piece_inputs : c.ft_in)) return false;
+    if (backward && c.world_size > 1) return true;
+    return 2ll * n * c.max_active > (backward ? 4ll : 5ll) * c.ft_in;
+}
 
 // Copies one host batch into a device batch on `cs`.  Page-locked caller memory is copied directly; pageable memory goes
-// through the library's page-locked staging buffers in pieces that are shared among the helper threads and sent off as they
+// through the library's page-locked staging buffer in pieces that are shared among the helper threads and sent off as they
 // are there.  (cudaMemcpyAsync on pageable memory does its staging on the calling thread alone: 1.5 ms for the 22 MB
 // of 65 536 positions.)
-int upload_batch(tb_trainer* t, const tb_batch* b, DevBatch* d, HostStage* st, cudaStream_t cs) {
+int upload_batch(tb_trainer* t, const tb_batch* b, DevBatch* d, char* stage, cudaStream_t cs, bool backward) {
     const size_t n = (size_t)b->n_pos, A = (size_t)t->cfg.max_active;
-    const bool ls = t->cfg.arch == TB_ARCH_LAYERSTACK;
-    struct Item { void* dst; const void* src; void* stage; size_t bytes; } items[6] = {
-        {d->stm, b->stm_indices, st->stm, n * A * 4}, {d->nstm, b->nstm_indices, st->nstm, n * A * 4}, {d->nnz, b->nnz, st->nnz, n * 4},
-        {d->bucket, b->bucket_idx, st->bucket, n * 4}, {d->score, b->score, st->score, n * 4}, {d->wdl, b->wdl, st->wdl, n * 4}};
-    struct Piece { const Item* item; size_t off, bytes; };
+    const BatchLayout L(n, A);
+    d->place(L);
+    const void* src[6] = {b->stm_indices, b->nstm_indices, b->nnz, t->cfg.arch == TB_ARCH_LAYERSTACK ? b->bucket_idx : nullptr, b->score, b->wdl};
+    struct Piece { const char* src; size_t off, bytes, end; };  // end: where the next array starts
     std::vector<Piece> staged;
     for (int i = 0; i < 6; ++i) {
-        if (i == 3 && !ls) continue;
-        const Item& it = items[i];
-        if (is_pinned(it.src)) CU(t, cudaMemcpyAsync(it.dst, it.src, it.bytes, cudaMemcpyHostToDevice, cs));
-        else for (size_t o = 0; o < it.bytes; o += UPLOAD_PIECE) staged.push_back({&it, o, it.bytes - o < UPLOAD_PIECE ? it.bytes - o : UPLOAD_PIECE});
+        if (!src[i]) continue;
+        const size_t bytes = i < 2 ? n * A * 4 : n * 4, next = i < 5 ? L.off[i + 1] : L.bytes;
+        if (bytes >= UPLOAD_DIRECT && is_pinned(src[i])) {
+            CU(t, cudaMemcpyAsync(d->base + L.off[i], src[i], bytes, cudaMemcpyHostToDevice, cs));
+            continue;
+        }
+        for (size_t o = 0; o < bytes; o += UPLOAD_PIECE) {
+            const size_t m = bytes - o < UPLOAD_PIECE ? bytes - o : UPLOAD_PIECE;
+            staged.push_back({(const char*)src[i] + o, L.off[i] + o, m, o + m < bytes ? L.off[i] + o + m : next});
+        }
     }
     cudaError_t e = cudaSuccess;
-    auto copy = [&](int i) { const Piece& p = staged[i]; host_copy_for_device((char*)p.item->stage + p.off, (const char*)p.item->src + p.off, p.bytes); };
+    auto copy = [&](int i) { host_copy_for_device(stage + staged[i].off, staged[i].src, staged[i].bytes); };
     int first = 0;  // pieces [first, i] are staged and not sent yet
     auto send = [&](int i) {
-        const Piece& p = staged[first];
-        const bool last = i + 1 == (int)staged.size() || staged[i + 1].item != p.item;
-        if (!last && i + 1 - first < UPLOAD_SEND) return;
-        const size_t bytes = staged[i].off + staged[i].bytes - p.off;
-        const cudaError_t x = cudaMemcpyAsync((char*)p.item->dst + p.off, (const char*)p.item->stage + p.off, bytes, cudaMemcpyHostToDevice, cs);
+        const size_t from = staged[first].off, to = staged[i].off + staged[i].bytes;
+        const bool last = i + 1 == (int)staged.size() || staged[i + 1].off != staged[i].end;
+        if (!last && to - from < UPLOAD_SEND) return;
+        const cudaError_t x = cudaMemcpyAsync(d->base + from, stage + from, to - from, cudaMemcpyHostToDevice, cs);
         if (e == cudaSuccess) e = x;
         first = i + 1;
     };
@@ -375,7 +405,7 @@ int upload_batch(tb_trainer* t, const tb_batch* b, DevBatch* d, HostStage* st, c
     d->inside_known = false;
     *d->outside = 0;
     // (not counted in `launches`: part of the upload, which a staged batch pays once)
-    launch_slice_check(cs, d->stm, d->nstm, d->nnz, b->n_pos, t->cfg.max_active, t->cfg.ft_in,
+    if (backward && slice_path(t, b->n_pos, true)) launch_slice_check(cs, d->stm, d->nstm, d->nnz, b->n_pos, t->cfg.max_active, t->cfg.ft_in,
                        t->cfg.piece_inputs > 0 ? t->cfg.piece_inputs : t->cfg.ft_in, d->outside);
     CU(t, cudaEventRecord(d->checked, cs));
     d->n_pos = b->n_pos;
@@ -453,7 +483,7 @@ int run_forward(tb_trainer* t, const DevBatch& d, const tb_loss* loss, float lam
     void* pre1 = t->p_out16 ? t->pre_h[1] : (void*)t->pre[1];
     t->last_n = B;
     const int rps = c.piece_inputs > 0 ? c.piece_inputs : N;
-    t->slice_fwd = ft_forward_slice_supported(F, N, A, rps);
+    t->slice_fwd = slice_path(t, B, backward != 0);
     if (backward) { t->opt_begun = false; t->ft_rows_updated = false; }
     // the effective L1 weights depend on nothing of this batch
     if (ls) {
@@ -464,10 +494,14 @@ int run_forward(tb_trainer* t, const DevBatch& d, const tb_loss* loss, float lam
         t->launches += launch_l1_weff(side_stream(t, 1), nullptr, nullptr, t->groups[2].w, t->groups[3].w, t->K, c.l1_out, 0, t->l1_weff);
     }
     if (side_stream(t, 1) != t->stream) CU(t, cudaEventRecord(t->ev_weff, side_stream(t, 1)));
+    // A gather of few row bytes goes without the order of the items (by slice, so that rows stay in L2): sorting them costs 12
+    // us more than the positions alone, and saves 7 us of the gather of 0.5 GB, 27 of 1.3 GB.
+    const bool few = 2ll * B * A * F * (t->p_ft16 ? 2 : 4) <= 640ll << 20;
+    int* items = t->slice_fwd || B > SORT_ONE_BLOCK || !few ? t->items : nullptr;
     { PhaseScope p(t, PH_SORT);
       // positions by bucket (order, tiles, units) and items of both perspectives by the king-bucket slice of the FT table
       int n = launch_step_sorts(t->stream, ls ? d.bucket : nullptr, B, ls ? c.num_buckets : 0, t->order, t->tiles, t->n_tiles,
-                                t->seg_start, t->max_tiles, d.stm, d.nstm, d.nnz, A, N, rps, 2, t->items, t->item_seg,
+                                t->seg_start, t->max_tiles, d.stm, d.nstm, d.nnz, A, N, rps, 2, items, t->item_seg,
                                 t->sort_hist, t->slice_fwd ? t->fwd_work : nullptr, t->slice_fwd && backward ? t->bwd_slice : nullptr,
                                 t->bwd_parts);
       p.done(n); }
@@ -479,7 +513,7 @@ int run_forward(tb_trainer* t, const DevBatch& d, const tb_loss* loss, float lam
                                          t->p_ft16, t->p_out16));
       else
           p.done(launch_ft_forward(t->stream, mode, table, d.stm, d.nstm, d.nnz, t->groups[1].w, pre0, pre1, t->combined,
-                                   t->items, B, F, N, A, FT_POST_SCALE, 2, t->p_ft16, t->p_out16)); }
+                                   items, B, F, N, A, FT_POST_SCALE, 2, t->p_ft16, t->p_out16)); }
     if (backward && side_stream(t, 0) != t->stream) CU(t, cudaEventRecord(t->ev_fwd, t->stream));
     if (side_stream(t, 1) != t->stream) CU(t, cudaStreamWaitEvent(t->stream, t->ev_weff, 0));
     LossParams lp = make_loss(loss, lambda, d.norm);
@@ -534,9 +568,12 @@ int run_backward(tb_trainer* t, const DevBatch& d, float lr) {
     const int rps = c.piece_inputs > 0 ? c.piece_inputs : N;
     const bool slice_bwd = t->slice_fwd && t->bwd_slice != nullptr;
     const cudaStream_t si = side_stream(t, 0), sw = side_stream(t, 1);
-    // The inverse index needs the forward's row codes alone: it runs beside the dense layers, whose kernels leave most of the
+    // The inverse index needs the forward's row codes, or the batch alone: it runs beside the dense layers, whose kernels leave most of the
     // chip free (10 to 15 % of its warps).  In profile mode it is launched where its phase is.
-    auto inverse = [&]() { return slice_bwd ? launch_inverse_slice(si, t->item_seg, t->fwd_work, t->bwd_slice, B, A, N, rps, 2) : 0; };
+    auto inverse = [&]() {
+        return slice_bwd ? launch_inverse_slice(si, t->item_seg, t->fwd_work, t->bwd_slice, B, A, N, rps, 2)
+                         : launch_inverse_index(si, d.stm, d.nstm, d.nnz, B, A, N, 2, t->feat_counts, t->feat_offsets, t->feat_lists, t->bwd_plan);
+    };
     if (si != t->stream) {
         CU(t, cudaStreamWaitEvent(si, t->ev_fwd, 0));
         t->launches += inverse();
@@ -602,8 +639,8 @@ int run_backward(tb_trainer* t, const DevBatch& d, float lr) {
       int n = 0;
       if (si == t->stream) n += inverse();
       else CU(t, cudaStreamWaitEvent(t->stream, t->ev_inv, 0));
-      if (generic) n += launch_inverse_index(t->stream, d.stm, d.nstm, d.nnz, B, A, N, 2, t->feat_counts, t->feat_offsets, t->feat_lists,
-                                             t->bwd_plan);
+      if (generic && slice_bwd) n += launch_inverse_index(t->stream, d.stm, d.nstm, d.nnz, B, A, N, 2, t->feat_counts, t->feat_offsets, t->feat_lists,
+                                                          t->bwd_plan);
       p.done(n); }
     // the first exchanged part carries the small groups' gradients; a call for gradients alone returns with all of them
     if (c.world_size > 1 || lr < 0.0f) { const int jrc = join_wgrad(t); if (jrc != TB_OK) return jrc; }
@@ -615,7 +652,7 @@ int run_backward(tb_trainer* t, const DevBatch& d, float lr) {
       if (slice_bwd) {
           // Data parallel: the slices are done in several launches (ar_parts_for) and the gradient rows of each part are all-reduced on a
           // second stream while the next part is computed (the small groups, ready since the dense backward, ride with the
-          // first part, the loss with the last).  Whichever path wrote the rows (the gated generic kernels come first), they
+          // first part, the loss with the last).  Whichever path wrote the rows (the generic kernels come first), they
           // are final when the part's event is recorded.
           const int n_slices = (N + rps - 1) / rps;
           const int parts = t->bwd_parts;
@@ -883,7 +920,7 @@ int ring_upload(tb_trainer* t, const tb_batch* b, int* slot_out) {
     if (t->upload_pending[s]) { CU(t, cudaEventSynchronize(t->ev_upload[s])); t->upload_pending[s] = false; }
     // the compute that read this device slot two steps ago must be done before it is overwritten
     if (t->consumed_pending[s]) { CU(t, cudaStreamWaitEvent(t->copy_stream, t->ev_consumed[s], 0)); }
-    int rc = upload_batch(t, b, &t->ring[s], &t->stage[s], t->copy_stream);
+    int rc = upload_batch(t, b, &t->ring[s], t->stage[s], t->copy_stream, true);
     if (rc != TB_OK) return rc;
     CU(t, cudaEventRecord(t->ev_upload[s], t->copy_stream));
     t->upload_pending[s] = true;
@@ -909,6 +946,7 @@ int ring_upload_psv(tb_trainer* t, int feature_set, const uint8_t* psv, int n_po
     if (!is_pinned(psv)) { host_stage(t->stage_psv[s], psv, bytes); src = t->stage_psv[s]; }
     CU(t, cudaMemcpyAsync(t->ring_psv[s], src, bytes, cudaMemcpyHostToDevice, t->copy_stream));
     DevBatch& d = t->ring[s];
+    d.place(BatchLayout((size_t)n_pos, (size_t)t->cfg.max_active));
     const int n = launch_psv_extract(t->copy_stream, feature_set, t->ring_psv[s], n_pos, d.stm, d.nstm, d.nnz,
                                      t->cfg.arch == TB_ARCH_LAYERSTACK ? d.bucket : nullptr, d.score, d.wdl);
     if (n < 0) return fail(t, TB_ERR_INVALID_ARGUMENT, "unknown feature set id %d", feature_set);
@@ -940,12 +978,12 @@ void free_all(tb_trainer* t) {
     cudaFree(t->table_h); cudaFree(t->ft_m_h); cudaFree(t->ft_v_h); cudaFree(t->clamp_counter);
     cudaFree(t->tc_error); cudaFreeHost(t->tc_error_pinned);
     for (int i = 0; i < 2; ++i) { cudaFree(t->pre_h[i]); cudaFree(t->dft_h[i]); }
-    auto free_batch = [](DevBatch& d) { cudaFree(d.stm); cudaFree(d.nstm); cudaFree(d.nnz); cudaFree(d.bucket); cudaFree(d.score); cudaFree(d.wdl);
+    auto free_batch = [](DevBatch& d) { cudaFree(d.base);
                                          cudaFreeHost(d.outside); if (d.checked) cudaEventDestroy(d.checked); };
     for (auto& d : t->ring) free_batch(d);
     for (auto& d : t->slots) free_batch(d);
     for (int i = 0; i < 2; ++i) { cudaFree(t->ring_psv[i]); cudaFreeHost(t->stage_psv[i]); }
-    for (auto& s : t->stage) { cudaFreeHost(s.stm); cudaFreeHost(s.nstm); cudaFreeHost(s.nnz); cudaFreeHost(s.bucket); cudaFreeHost(s.score); cudaFreeHost(s.wdl); }
+    for (char* s : t->stage) cudaFreeHost(s);
     for (int i = 0; i < 2; ++i) {
         cudaFree(t->pre[i]); cudaFree(t->dft[i]);
         if (t->ev_upload[i]) cudaEventDestroy(t->ev_upload[i]);
@@ -979,8 +1017,9 @@ void free_all(tb_trainer* t) {
 
 int alloc_batch(tb_trainer* t, DevBatch* d) {
     const size_t B = (size_t)t->cfg.batch_capacity, A = (size_t)t->cfg.max_active;
-    CU(t, dalloc(&d->stm, B * A)); CU(t, dalloc(&d->nstm, B * A)); CU(t, dalloc(&d->nnz, B)); CU(t, dalloc(&d->bucket, B));
-    CU(t, dalloc(&d->score, B)); CU(t, dalloc(&d->wdl, B));
+    const BatchLayout L(B, A);
+    CU(t, dalloc(&d->base, L.bytes));
+    d->place(L);
     CU(t, cudaHostAlloc((void**)&d->outside, sizeof(int), cudaHostAllocDefault));
     CU(t, cudaEventCreateWithFlags(&d->checked, cudaEventDisableTiming));
     return TB_OK;
@@ -1071,11 +1110,7 @@ int create_impl(tb_trainer* t) {
     const size_t B = (size_t)c.batch_capacity, A = (size_t)c.max_active;
     for (auto& d : t->ring) { int rc = alloc_batch(t, &d); if (rc) return rc; }
     for (auto& d : t->slots) { int rc = alloc_batch(t, &d); if (rc) return rc; }
-    for (auto& s : t->stage) {
-        CU(t, cudaHostAlloc((void**)&s.stm, B * A * 4, cudaHostAllocDefault)); CU(t, cudaHostAlloc((void**)&s.nstm, B * A * 4, cudaHostAllocDefault));
-        CU(t, cudaHostAlloc((void**)&s.nnz, B * 4, cudaHostAllocDefault)); CU(t, cudaHostAlloc((void**)&s.bucket, B * 4, cudaHostAllocDefault));
-        CU(t, cudaHostAlloc((void**)&s.score, B * 4, cudaHostAllocDefault)); CU(t, cudaHostAlloc((void**)&s.wdl, B * 4, cudaHostAllocDefault));
-    }
+    for (char*& s : t->stage) CU(t, cudaHostAlloc((void**)&s, BatchLayout(B, A).bytes, cudaHostAllocDefault));
     for (int i = 0; i < 2; ++i) {
         CU(t, dalloc(&t->ring_psv[i], B * 40));
         CU(t, cudaHostAlloc((void**)&t->stage_psv[i], B * 40, cudaHostAllocDefault));
@@ -1430,7 +1465,7 @@ int tb_validate_step(tb_trainer* t, const tb_batch* batch, float wdl_lambda, con
     DevBatch& d = t->slots[TB_NUM_SLOTS - 1];
     tb_batch b = *batch;
     if (b.per_pos_norm == 0.f) b.per_pos_norm = 1.0f / (float)b.n_pos;
-    rc = upload_batch(t, &b, &d, &t->stage[0], t->stream);
+    rc = upload_batch(t, &b, &d, t->stage[0], t->stream, false);
     if (rc != TB_OK) return rc;
     rc = run_forward(t, d, loss, wdl_lambda, 0);
     if (rc != TB_OK) return rc;
@@ -1467,7 +1502,7 @@ int tb_stage_batch(tb_trainer* t, int slot, const tb_batch* batch) {
     if (batch->n_pos == 0) return fail(t, TB_ERR_INVALID_ARGUMENT, "cannot stage an empty batch");
     CU(t, cudaSetDevice(t->cfg.device));
     CU(t, cudaStreamSynchronize(t->stream));
-    rc = upload_batch(t, batch, &t->slots[slot], &t->stage[0], t->stream);
+    rc = upload_batch(t, batch, &t->slots[slot], t->stage[0], t->stream, true);
     if (rc != TB_OK) return rc;
     CU(t, cudaStreamSynchronize(t->stream));
     return TB_OK;
@@ -1491,7 +1526,7 @@ int tb_forward_backward(tb_trainer* t, const tb_batch* batch, float wdl_lambda, 
     CU(t, cudaSetDevice(t->cfg.device));
     CU(t, cudaStreamSynchronize(t->stream));
     DevBatch& d = t->slots[TB_NUM_SLOTS - 1];
-    rc = upload_batch(t, batch, &d, &t->stage[0], t->stream);
+    rc = upload_batch(t, batch, &d, t->stage[0], t->stream, true);
     if (rc == TB_OK) rc = run_forward(t, d, loss, wdl_lambda, 1);
     if (rc == TB_OK) rc = run_backward(t, d, -1.0f);
     if (rc == TB_OK) rc = run_allreduce(t);
