@@ -36,6 +36,18 @@ static __device__ __forceinline__ float clamp_half_count(float v, unsigned& clam
     return v;
 }
 
+// x * w onto a pair of running sums, one instruction for two multiply-adds
+static __device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long x, unsigned long long w) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(w));
+}
+static __device__ __forceinline__ unsigned long long pair2(float lo, float hi) {
+    unsigned long long d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+static __device__ __forceinline__ float lo2(unsigned long long v) { return __uint_as_float((unsigned)v); }
+static __device__ __forceinline__ float hi2(unsigned long long v) { return __uint_as_float((unsigned)(v >> 32)); }
+
 #define FT_POST_SCALE (127.0f / 128.0f)  // bins/nnue_train/src/arch.rs:64-70
 
 // ------------------------------------------------------------------------------------------------
@@ -277,10 +289,6 @@ __global__ void k_l1_weff(const float* __restrict__ wb, const float* __restrict_
 #define LF_KC 64       // columns per stage: 256 bytes of every row, a quarter of them for each warp
 #define LF_LD (LF_KC + 4)
 #define LF_STAGES 3
-// x * w onto a pair of running sums (even and odd columns), one instruction for two multiply-adds
-static __device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long x, unsigned long long w) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(w));
-}
 template <int L1, int RP>
 struct L1Tile {
     static constexpr int TX = L1 / 8, TY = 32 / TX, POS = TY * RP;  // a warp's threads over outputs and positions; positions of a block
@@ -389,8 +397,10 @@ int launch_l1_forward(cudaStream_t s, const float* x, int K, const int* order, c
                       const float* bs, float* y, int l1, int nb, int n_pos, const float* weff, int tf32, int* error_flag) {
     if (l1_streams(K, l1)) {
         const float* beff = weff + (size_t)(nb + 1) * l1 * K;
+        // --tf32 allows the tensor cores' rounding and does not ask for it: below 32 outputs the fp32 kernel is the faster one (65 536
+        // x 1536, l1 = 16: 113 us against 161; 20 000 x 768, l1 = 8: 25 against 44; 40 000 x 1024, l1 = 32: 95 against 91)
         if (tf32 && error_flag && l1_forward_tc_supported(K, l1))
-            return launch_l1_forward_tc(s, x, K, order, tiles, n_tiles, max_tiles, n_pos, weff, beff, y, l1, wb ? nb : 0, error_flag);
+            return launch_l1_forward_tc(s, x, K, order, tiles, n_tiles, max_tiles, n_pos, weff, beff, y, wb ? nb : 0, error_flag);
         const int max_units = sort_units(n_pos);
         const TileDesc* units = tiles + max_tiles;
         const int nbe = wb ? nb : 0;
@@ -1049,57 +1059,56 @@ __global__ void __launch_bounds__(256) k_l1_wgrad(const float* __restrict__ x, i
     }
 }
 
-// Second stage: block column g adds the work units of bucket g in order (the units of a bucket are contiguous);
-// the last column (g == nb: positions with an out-of-range bucket id, or the whole batch for Simple) goes to a
-// scratch row.  Third stage: gw_shared[k][o] = sum over the columns.
-__global__ void __launch_bounds__(256) k_l1_wgrad_final(const float* __restrict__ partials, const TileDesc* __restrict__ units,
-                                                         const int* __restrict__ n_units, int K, int l1, int nb,
-                                                         float* __restrict__ gw_bucket, float* __restrict__ rest) {
-    __shared__ int s_range[2];
-    const int g = blockIdx.y;
-    const int nu = *n_units;
-    if (threadIdx.x == 0) { s_range[0] = nu; s_range[1] = nu; }
+// Second stage: the work units of bucket g, and of the positions with an out-of-range bucket id (the whole batch for
+// Simple), are added by `slices` warps each, in a fixed order; a block holds 128 elements and all buckets, so that the sum
+// over the buckets, gw_shared[k][o], comes from the same launch.  (One thread per element and bucket walking all units took
+// 104 us for the 266 units of a Simple batch, 8 now; 18 with the sum over the buckets for a LayerStack one, 8 now.)
+__global__ void __launch_bounds__(1024) k_l1_wgrad_final(const float* __restrict__ partials, const int* __restrict__ unit_base, int K, int l1,
+                                                         int nb, int slices, float* __restrict__ gw_bucket, float* __restrict__ gw_shared) {
+    __shared__ float4 s_sum[32][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = w / slices, sl = w - g * slices;
+    const int i4 = blockIdx.x * 32 + lane, n4 = l1 * K / 4;
+    const float4* __restrict__ p4 = reinterpret_cast<const float4*>(partials) + i4;
+    const int u1 = unit_base[g + 1];
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int u = unit_base[g] + sl; u < u1; u += 8 * slices) {
+        float4 v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            v[j] = u + j * slices < u1 ? p4[(size_t)(u + j * slices) * n4] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { sum.x += v[j].x; sum.y += v[j].y; sum.z += v[j].z; sum.w += v[j].w; }
+    }
+    s_sum[w][lane] = sum;
     __syncthreads();
-    for (int u = threadIdx.x; u < nu; u += blockDim.x) {  // first unit of bucket g, first unit of a later bucket
-        const int bk = units[u].bucket;
-        if (bk == g) atomicMin(&s_range[0], u);
-        if (bk > g) atomicMin(&s_range[1], u);
+    if (sl == 0) {
+        for (int j = 1; j < slices; ++j) {
+            const float4 v = s_sum[w + j][lane];
+            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+        }
+        s_sum[w][lane] = sum;
+        if (g < nb) reinterpret_cast<float4*>(gw_bucket)[(size_t)g * n4 + i4] = sum;
     }
     __syncthreads();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= l1 * K) return;
-    const int u0 = s_range[0], u1 = s_range[1];
-    float sum = 0.f;
-    int u = u0;
-    for (; u + 4 <= u1; u += 4) {  // four loads in flight, added in unit order
-        const float a = partials[(size_t)u * l1 * K + i], b = partials[(size_t)(u + 1) * l1 * K + i];
-        const float c = partials[(size_t)(u + 2) * l1 * K + i], d = partials[(size_t)(u + 3) * l1 * K + i];
-        sum += a; sum += b; sum += c; sum += d;
+    if (w != 0) return;
+    float4 total = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j <= nb; ++j) {
+        const float4 v = s_sum[j * slices][lane];
+        total.x += v.x; total.y += v.y; total.z += v.z; total.w += v.w;
     }
-    for (; u < u1; ++u) sum += partials[(size_t)u * l1 * K + i];
-    if (g < nb) gw_bucket[(size_t)g * l1 * K + i] = sum;
-    else rest[i] = sum;
-}
-
-__global__ void __launch_bounds__(256) k_l1_wgrad_shared(const float* __restrict__ gw_bucket, const float* __restrict__ rest,
-                                                          int K, int l1, int nb, float* __restrict__ gw_shared) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= l1 * K) return;
-    const int o = i / K, k = i - o * K;
-    float total = 0.f;
-    for (int g = 0; g < nb; ++g) total += gw_bucket[(size_t)g * l1 * K + i];
-    total += rest[i];
-    gw_shared[(size_t)k * l1 + o] = total;
+    const int o = 4 * i4 / K, k = 4 * i4 - o * K;
+    float* out = gw_shared + (size_t)k * l1 + o;
+    out[0] = total.x; out[l1] = total.y; out[2 * l1] = total.z; out[3 * l1] = total.w;
 }
 
 // Variant for l1 % 8 == 0: a thread owns four adjacent columns and OPT outputs (OPT = 8 or 16; two thread groups
 // split the outputs when l1 = 32), so that one 128-bit load of x feeds 4 * OPT multiply-adds and the dl1 values
-// come as broadcast 128-bit shared-memory loads.  The unit's positions (consecutive in the bucket order) and their dl1
+// come as broadcast 128-bit shared-memory loads; PACK: sums of two adjacent outputs share a packed multiply-add (which needs
+// the x values twice: at six blocks per SM the registers for 16 outputs do not allow it, 110 to 167 us).  The unit's positions (consecutive in the bucket order) and their dl1
 // rows are staged once, then the x rows arrive through a private ring of asynchronous copies (a thread copies the 16
 // bytes it reads itself), WG_STAGES rounds of four positions ahead of the arithmetic.
 #define WG_POS (TB_UNIT_TILES * TB_TILE_M)
-#define WG_STAGES 2
-template <int OPT, int THREADS, int MIN_BLOCKS>
+template <int OPT, int THREADS, int MIN_BLOCKS, int WG_STAGES, bool PACK>
 __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) k_l1_wgrad_stream(const float* __restrict__ x, int K, const float* __restrict__ dl1,
                                                           const int* __restrict__ order, const TileDesc* __restrict__ tiles,
                                                           const TileDesc* __restrict__ units, const int* __restrict__ n_units, int l1,
@@ -1121,9 +1130,10 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) k_l1_wgrad_stream(const f
     for (int i = threadIdx.x; i < WG_POS; i += blockDim.x) s_pos[i] = i < n ? order[p_begin + i] : -1;
     __syncthreads();
     const int l1q = l1 >> 2;
-    for (int e = threadIdx.x; e < n * l1q; e += blockDim.x) {
+    for (int e = threadIdx.x; e < ((n + 3) & ~3) * l1q; e += blockDim.x) {
         const int r = e / l1q, o4 = e - r * l1q;
-        reinterpret_cast<float4*>(sdl + (size_t)r * l1)[o4] = *reinterpret_cast<const float4*>(dl1 + (size_t)s_pos[r] * l1 + 4 * o4);
+        reinterpret_cast<float4*>(sdl + (size_t)r * l1)[o4] =
+            r < n ? *reinterpret_cast<const float4*>(dl1 + (size_t)s_pos[r] * l1 + 4 * o4) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     const int T = blockDim.x;
     const float4* __restrict__ x4 = reinterpret_cast<const float4*>(x);
@@ -1138,9 +1148,14 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) k_l1_wgrad_stream(const f
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    float4 acc[OPT];
+    float4 acc[PACK ? 1 : OPT];
+    unsigned long long acc2[PACK ? OPT / 2 : 1][4];  // (output 2 j, output 2 j + 1) of the thread's four columns
 #pragma unroll
-    for (int j = 0; j < OPT; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < (PACK ? 1 : OPT); ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < (PACK ? OPT / 2 : 1); ++j)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc2[j][c] = 0ull;
     const int n_rounds = (n + 3) >> 2;
 #pragma unroll
     for (int r = 0; r < WG_STAGES - 1; ++r) issue(r);
@@ -1152,28 +1167,46 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) k_l1_wgrad_stream(const f
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int r = 4 * round + q;
-            if (r >= n) break;
+            // PACK: no test, past the end the first position's row times zero: the four positions' loads then run ahead of the
+            // sums (l1 = 32: 91 to 70 us)
+            if (!PACK && r >= n) break;
             const float4 xv = ring[(size_t)(stage * 4 + q) * T + threadIdx.x];
 #pragma unroll
             for (int j4 = 0; j4 < OPT / 4; ++j4) {
-                const float4 g = *reinterpret_cast<const float4*>(sdl + (size_t)r * l1 + og * OPT + 4 * j4);
-                const float gv[4] = {g.x, g.y, g.z, g.w};
+                const float4* gp = reinterpret_cast<const float4*>(sdl + (size_t)r * l1 + og * OPT + 4 * j4);
+                if constexpr (PACK) {
+                    const unsigned long long xd[4] = {pair2(xv.x, xv.x), pair2(xv.y, xv.y), pair2(xv.z, xv.z), pair2(xv.w, xv.w)};
+                    const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(gp);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    acc[4 * j4 + j].x += gv[j] * xv.x;
-                    acc[4 * j4 + j].y += gv[j] * xv.y;
-                    acc[4 * j4 + j].z += gv[j] * xv.z;
-                    acc[4 * j4 + j].w += gv[j] * xv.w;
+                    for (int c = 0; c < 4; ++c) {
+                        fma2(acc2[2 * j4][c], g.x, xd[c]);
+                        fma2(acc2[2 * j4 + 1][c], g.y, xd[c]);
+                    }
+                } else {
+                    const float4 g = *gp;
+                    const float gv[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        acc[4 * j4 + j].x += gv[j] * xv.x;
+                        acc[4 * j4 + j].y += gv[j] * xv.y;
+                        acc[4 * j4 + j].z += gv[j] * xv.z;
+                        acc[4 * j4 + j].w += gv[j] * xv.w;
+                    }
                 }
             }
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     if (!active) return;
+    float4* out = reinterpret_cast<float4*>(partials + ((size_t)u * l1 + og * OPT) * K) + col4;
 #pragma unroll
     for (int j = 0; j < OPT; ++j) {
-        const int o = og * OPT + j;
-        reinterpret_cast<float4*>(partials + ((size_t)u * l1 + o) * K)[col4] = acc[j];
+        if constexpr (PACK) {
+            const unsigned long long* a = acc2[j / 2];
+            out[(size_t)j * K4] = j % 2 ? make_float4(hi2(a[0]), hi2(a[1]), hi2(a[2]), hi2(a[3])) : make_float4(lo2(a[0]), lo2(a[1]), lo2(a[2]), lo2(a[3]));
+        } else {
+            out[(size_t)j * K4] = acc[j];
+        }
     }
 }
 
@@ -1185,25 +1218,23 @@ int launch_l1_wgrad(cudaStream_t s, const float* x, int K, const float* dl1, con
     const int max_units = sort_units(n_pos);
     if (l1 == 8 || l1 == 16 || l1 == 32) {
         const int threads = l1 == 32 ? 256 : 128;
-        const size_t smem = (size_t)WG_POS * l1 * sizeof(float) + (size_t)WG_STAGES * 4 * threads * 16;
         const dim3 grid(ceil_div(K / 4, 128), max_units);
+#define WGRAD(OPT, T, MB, ST, P)                                                                                               \
+    do {                                                                                                                       \
+        const size_t smem = (size_t)WG_POS * l1 * sizeof(float) + (size_t)(ST) * 4 * threads * 16;                             \
+        cudaFuncSetAttribute(k_l1_wgrad_stream<OPT, T, MB, ST, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);   \
+        k_l1_wgrad_stream<OPT, T, MB, ST, P><<<grid, threads, smem, s>>>(x, K, dl1, order, tiles, units, n_units, l1, partials); \
+    } while (0)
         // 128-thread blocks at six per SM: with K = 1536 the 3 x 265 blocks of the benchmark then run as one wave
-        if (l1 == 8) {
-            cudaFuncSetAttribute(k_l1_wgrad_stream<8, 128, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-            k_l1_wgrad_stream<8, 128, 6><<<grid, threads, smem, s>>>(x, K, dl1, order, tiles, units, n_units, l1, partials);
-        } else if (l1 == 16) {
-            cudaFuncSetAttribute(k_l1_wgrad_stream<16, 128, 6>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-            k_l1_wgrad_stream<16, 128, 6><<<grid, threads, smem, s>>>(x, K, dl1, order, tiles, units, n_units, l1, partials);
-        } else {
-            cudaFuncSetAttribute(k_l1_wgrad_stream<16, 256, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-            k_l1_wgrad_stream<16, 256, 2><<<grid, threads, smem, s>>>(x, K, dl1, order, tiles, units, n_units, l1, partials);
-        }
+        if (l1 == 8) WGRAD(8, 128, 6, 2, true);
+        else if (l1 == 16) WGRAD(16, 128, 6, 2, false);
+        else WGRAD(16, 256, 2, 4, true);
+#undef WGRAD
     } else
         k_l1_wgrad<<<dim3(K / 128, max_units), 256, 0, s>>>(x, K, dl1, order, tiles, units, n_units, l1, partials);
-    float* rest = partials + (size_t)max_units * l1 * K;  // one more [l1][K] row behind the unit partials
-    k_l1_wgrad_final<<<dim3(ceil_div(l1 * K, 256), nb + 1), 256, 0, s>>>(partials, units, n_units, K, l1, nb, gw_bucket, rest);
-    k_l1_wgrad_shared<<<ceil_div(l1 * K, 256), 256, 0, s>>>(gw_bucket, rest, K, l1, nb, gw_shared);
-    return 3;
+    const int slices = 32 / (nb + 1) < 16 ? 32 / (nb + 1) : 16;
+    k_l1_wgrad_final<<<l1 * K / 128, 32 * slices * (nb + 1), 0, s>>>(partials, n_tiles + 2, K, l1, nb, slices, gw_bucket, gw_shared);
+    return 2;
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -1144,7 +1144,7 @@ int create_impl(tb_trainer* t) {
     size_t small = (ls ? (size_t)(nb + 1) * 64 : (size_t)128) * n_cells;  // SW_SPLIT_LS partial rows per segment
     if (tail_tiled((int)l1, (int)l2)) small = tail_partial_floats(c.arch, (int)l1, (int)l2, t->max_tiles);
     CU(t, dalloc(&t->small_partials, small));
-    CU(t, dalloc(&t->l1w_partials, ((size_t)t->max_units + 1) * l1 * t->K));
+    CU(t, dalloc(&t->l1w_partials, (size_t)t->max_units * l1 * t->K));
     CU(t, dalloc(&t->l1_weff, (size_t)(nb + 1) * l1 * (t->K + 1)));  // effective L1 weights and biases per bucket
     t->dgrad_rows = DGRAD_CTAS > 2 * t->max_units ? DGRAD_CTAS : 2 * t->max_units;  // partial FT bias rows: one per block
     CU(t, dalloc(&t->bias_partials, (size_t)t->dgrad_rows * 2 * F));
