@@ -165,7 +165,7 @@ int launch_l1_weff(cudaStream_t s, const float* wb, const float* bb, const float
 // l1_tc.cu
 bool l1_forward_tc_supported(int K, int l1);
 int launch_l1_forward_tc(cudaStream_t s, const float* x, int K, const int* order, const TileDesc* tiles, const int* n_tiles,
-                         int max_tiles, int n_pos, const float* weff, const float* beff, float* y, int nb, int* error_flag);
+                         int max_tiles, int n_pos, const float* weff, const float* beff, float* y, int l1, int nb, int* error_flag);
 // sum over the batch of the extended WRM loss's per-position weights (wrm_weight_sum, native_kernels.cu:520-545), in a
 // fixed order; partials: scratch of ceil(B / 256) doubles
 int launch_wrm_weight_sum(cudaStream_t s, const float* score, int B, LossParams lp, double* partials, double* weight_sum);

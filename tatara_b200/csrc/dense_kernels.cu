@@ -397,10 +397,8 @@ int launch_l1_forward(cudaStream_t s, const float* x, int K, const int* order, c
                       const float* bs, float* y, int l1, int nb, int n_pos, const float* weff, int tf32, int* error_flag) {
     if (l1_streams(K, l1)) {
         const float* beff = weff + (size_t)(nb + 1) * l1 * K;
-        // --tf32 allows the tensor cores' rounding and does not ask for it: below 32 outputs the fp32 kernel is the faster one (65 536
-        // x 1536, l1 = 16: 113 us against 161; 20 000 x 768, l1 = 8: 25 against 44; 40 000 x 1024, l1 = 32: 95 against 91)
         if (tf32 && error_flag && l1_forward_tc_supported(K, l1))
-            return launch_l1_forward_tc(s, x, K, order, tiles, n_tiles, max_tiles, n_pos, weff, beff, y, wb ? nb : 0, error_flag);
+            return launch_l1_forward_tc(s, x, K, order, tiles, n_tiles, max_tiles, n_pos, weff, beff, y, l1, wb ? nb : 0, error_flag);
         const int max_units = sort_units(n_pos);
         const TileDesc* units = tiles + max_tiles;
         const int nbe = wb ? nb : 0;

@@ -1,5 +1,5 @@
 // L1 forward on the 5th-generation tensor cores (tcgen05, TF32 operands, fp32 accumulators in tensor memory), used
-// for l1 = 32 when the trainer runs with --tf32 (bins/nnue_train/src/cli.rs:623-638; the reference then runs its L1 products as
+// when the trainer runs with --tf32 (bins/nnue_train/src/cli.rs:623-638; the reference then runs its L1 products as
 // cuBLAS Sgemm calls in TF32 tensor-op mode, one per bucket segment plus one for the shared layer:
 // bins/nnue_train/src/trainer_layerstack.rs:2388-2420, 2498-2506, bins/nnue_train/src/trainer_common.rs:691-727).
 //
@@ -9,7 +9,7 @@
 // staged by 16-byte asynchronous copies straight into the tensor cores' canonical K-major layout without swizzle: core
 // matrices of 8 rows x 16 bytes, stored contiguously; the next 16 bytes along K lie 128 bytes further (leading byte
 // offset), the next 8 rows TC_KC / 4 core matrices further (stride byte offset).  One thread issues the MMAs of a K chunk
-// (M = 128, N = l1 = 32, K = 8 each) and commits them to the stage's mbarrier, which frees the stage for the copies of
+// (M = 128, N = l1 or 16, K = 8 each) and commits them to the stage's mbarrier, which frees the stage for the copies of
 // a later chunk.  TF32 operands are the fp32 values as they are: the tensor cores read the upper 19 bits.
 // The contraction is read-bound (l1 <= 32 output columns): the tensor pipe is nearly idle by construction; what the
 // tensor cores buy is an instruction stream of copies only, so that the x rows stream at HBM speed.
@@ -54,20 +54,20 @@ __device__ __forceinline__ unsigned long long umma_desc(unsigned addr, unsigned 
 
 }  // namespace
 
-#define TC_L1 32  // outputs = N of the MMA
+template <int L1>
 __global__ void __launch_bounds__(128) k_l1_forward_tc(const float* __restrict__ x, int K, const int* __restrict__ order,
                                                         const TileDesc* __restrict__ tiles, const TileDesc* __restrict__ units,
                                                         const int* __restrict__ n_units, int half_tiles, const float* __restrict__ weff,
                                                         const float* __restrict__ beff, float* __restrict__ y, int nb,
                                                         int* __restrict__ error_flag) {
-    constexpr int L1 = TC_L1;
+    constexpr int NB = L1 < 16 ? 16 : L1;             // N of the MMA (a multiple of 16 for M = 128)
     constexpr int A_BYTES = TC_POS * TC_KC * 4;       // 32 KB
-    constexpr int B_BYTES = L1 * TC_KC * 4;
+    constexpr int B_BYTES = NB * TC_KC * 4;
     constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
     constexpr unsigned LBO = 128, SBO = (TC_KC / 4) * 128;
     // instruction descriptor: fp32 accumulator (bits 4-5 = 1), TF32 A and B (bits 7-9, 10-12 = 2), both K-major,
     // N >> 3 at bit 17, M >> 4 at bit 24
-    constexpr unsigned IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned)(L1 >> 3) << 17) | ((unsigned)(TC_POS >> 4) << 24);
+    constexpr unsigned IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned)(NB >> 3) << 17) | ((unsigned)(TC_POS >> 4) << 24);
     extern __shared__ __align__(16) unsigned char s_dyn[];
     __shared__ __align__(8) unsigned long long s_bar[TC_STAGES];
     __shared__ unsigned s_tmem;
@@ -90,9 +90,17 @@ __global__ void __launch_bounds__(128) k_l1_forward_tc(const float* __restrict__
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncwarp();
-    if (warp == 0) {  // tensor memory: 32 columns (the smallest allocation) hold the 128 x l1 fp32 tile
+    if (warp == 0) {  // tensor memory: 32 columns (the smallest allocation) hold the 128 x NB fp32 tile
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(32) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if constexpr (L1 < NB) {  // weight rows l1 .. 15 of every stage stay zero
+        constexpr int PAD = NB - L1;
+        for (int e = tid; e < TC_STAGES * PAD * (TC_KC / 4); e += 128) {
+            const int s = e / (PAD * (TC_KC / 4)), r = L1 + (e / (TC_KC / 4)) % PAD, kc = e % (TC_KC / 4);
+            unsigned char* p = s_dyn + (ring - smem_u32(s_dyn)) + (size_t)s * STAGE_BYTES + A_BYTES + (r >> 3) * SBO + kc * LBO + (r & 7) * 16;
+            *reinterpret_cast<float4*>(p) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -101,8 +109,8 @@ __global__ void __launch_bounds__(128) k_l1_forward_tc(const float* __restrict__
 
     // This thread's copies of one chunk: of x the 16-byte pieces kq and kq + 4 of row lane % 8 of the warp's four core-matrix
     // rows.  Eight neighbouring lanes write the eight rows of one core matrix, 128 consecutive bytes (eight pieces of one row
-    // each, which land 128 bytes apart, met in the same banks).  With 64 columns and two stages for 32 and three: 107 to 91 us at
-    // K = 1024, 40 000 positions.
+    // each, which land 128 bytes apart, met in the same banks).  With 64 columns and two stages for 32 and three: 176 to 161 us
+    // at K = 1536, l1 = 16, 65 536 positions, 107 to 91 at K = 1024, l1 = 32, 40 000.
     const int lane = tid & 31, rl = lane & 7, kq = lane >> 3;
     constexpr int PK = TC_KC / 16, TASKS = L1 / 8 * PK;  // (core-matrix row, 16 columns) copies of the weight rows, one warp each
     const float* __restrict__ wg = weff + (size_t)g * L1 * K;
@@ -177,8 +185,9 @@ __global__ void __launch_bounds__(128) k_l1_forward_tc(const float* __restrict__
         if (row < n) {
             float* yr = y + (size_t)s_pos[row] * L1 + c0;
             const float* bg = beff + (size_t)g * L1 + c0;
+            constexpr int NC = L1 - 0 < 16 ? L1 : 16;  // columns of this load that exist (l1 = 8: the first eight)
 #pragma unroll
-            for (int o = 0; o < 16; o += 4)
+            for (int o = 0; o < NC; o += 4)
                 *reinterpret_cast<float4*>(yr + o) = make_float4(__uint_as_float(v[o]) + bg[o], __uint_as_float(v[o + 1]) + bg[o + 1],
                                                                  __uint_as_float(v[o + 2]) + bg[o + 2], __uint_as_float(v[o + 3]) + bg[o + 3]);
         }
@@ -188,14 +197,21 @@ __global__ void __launch_bounds__(128) k_l1_forward_tc(const float* __restrict__
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(32) : "memory");
 }
 
-bool l1_forward_tc_supported(int K, int l1) { return l1 == TC_L1 && K % TC_KC == 0 && K / TC_KC >= TC_STAGES; }
+bool l1_forward_tc_supported(int K, int l1) { return (l1 == 8 || l1 == 16 || l1 == 32) && K % TC_KC == 0 && K / TC_KC >= TC_STAGES; }
 
 // weff / beff: the effective weights and biases k_l1_weff has built for this step
 int launch_l1_forward_tc(cudaStream_t s, const float* x, int K, const int* order, const TileDesc* tiles, const int* n_tiles,
-                         int max_tiles, int n_pos, const float* weff, const float* beff, float* y, int nb, int* error_flag) {
-    const size_t smem = (size_t)TC_STAGES * (TC_POS + TC_L1) * TC_KC * 4 + 128;
-    cudaFuncSetAttribute(k_l1_forward_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_l1_forward_tc<<<2 * sort_units(n_pos), 128, smem, s>>>(x, K, order, tiles, tiles + max_tiles, n_tiles + 1, unit_tiles(n_pos) / 2, weff, beff, y,
-                                                             nb, error_flag);
+                         int max_tiles, int n_pos, const float* weff, const float* beff, float* y, int l1, int nb, int* error_flag) {
+    const int max_units = sort_units(n_pos);
+    const TileDesc* units = tiles + max_tiles;
+    const int NB = l1 < 16 ? 16 : l1;
+    const size_t smem = (size_t)TC_STAGES * (TC_POS + NB) * TC_KC * 4 + 128;
+#define TC_LAUNCH(L)                                                                                                    \
+    do {                                                                                                                \
+        cudaFuncSetAttribute(k_l1_forward_tc<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);               \
+        k_l1_forward_tc<L><<<2 * max_units, 128, smem, s>>>(x, K, order, tiles, units, n_tiles + 1, unit_tiles(n_pos) / 2, weff, beff, y, nb, error_flag); \
+    } while (0)
+    if (l1 == 8) TC_LAUNCH(8); else if (l1 == 16) TC_LAUNCH(16); else TC_LAUNCH(32);
+#undef TC_LAUNCH
     return 1;
 }
