@@ -278,8 +278,8 @@ def run_microbench(tb, device, peak, iters=5):
             rows.append(row)
     return {"protocol": "one perspective, A=40 slots with 30..38 distinct indices, N=73305 rows, fp32; %d timed launches per cell, "
                         "each after a 256 MB L2 flush, CUDA events per launch; bwd includes the inverse index" % iters,
-            "kernels": {"uniform": "k_ft_forward (L2 gather), k_feat_* + k_lists_sort_* + k_ft_backward_short/long, k_radam",
-                        "sliced": "item sort + k_fwd_plan/k_fwd_codes + k_ft_forward_slice; k_chunk_plan + k_inv_chunk + k_ft_backward_slice"},
+            "kernels": {"uniform": "k_ft_forward (L2 gather), k_feat_* + k_lists_sort_long + k_ft_backward, k_radam",
+                        "sliced": "item sort + k_step_plans + k_fwd_codes + k_ft_forward_slice; k_inv_chunk + k_ft_backward_slice"},
             "bytes": "fwd U*F*4+B*F*4+B*A*4+B*4, bwd B*F*4+B*A*4+(N+1)*4+N*F*4, adam 28*N*F; GB/s of %.1f" % peak,
             "rows": rows}
 

@@ -21,8 +21,8 @@
 // own, and k_bwd_combine adds the slabs onto the rows in group order: one more fixed, non-sequential association, used
 // only by slices of more than BWD_GROUP chunks (about 3600 items).
 //
-// Both kernels return at once when the batch has a row outside its item's slice (outside_flag != 0); the generic
-// kernels, gated the other way round, then do the work.
+// Both kernels return at once when the batch has a row outside its item's slice (outside_flag != 0); the host launches the
+// kernels over global lists for such a batch.
 #include "ft_slice.cuh"
 
 #define BWD_HOT 256      // list length from which a list is summed as four quarters by the four groups of one warp
