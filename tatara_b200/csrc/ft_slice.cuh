@@ -197,7 +197,6 @@ static __device__ __forceinline__ void cp_async16(void* dst_shared, const void* 
                  "r"(src_bytes)
                  : "memory");
 }
-static __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 static __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N_PENDING>
 static __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N_PENDING) : "memory"); }
