@@ -211,11 +211,12 @@ int launch_l1_wgrad(cudaStream_t s, const float* x, int K, const float* dl1, con
 // FT bias gradient.
 // half_act: pre-activations and dft are fp16; dft is written as round(clamp(g * grad_scale)) and the clamped elements
 // are added to *clamp_counter.  Returns -1 for a combination that is not built.
+// ft_b_grad is summed on s_reduce, behind what it holds (ev_reduce: scratch event; unused when s_reduce is s)
 int launch_l1_dgrad_ftgrad(cudaStream_t s, int mode, const float* dl1, const int* order, const TileDesc* tiles,
                            const int* n_tiles, int max_tiles, const float* wb, const float* ws,
                            const void* pre_stm, const void* pre_nstm, const float* ft_bias, float scale,
                            int B, int F, int l1, int nb, void* dft_stm, void* dft_nstm, float* bias_partials,
-                           float* ft_b_grad, int n_ctas, int half_act = 0, float grad_scale = 1.0f,
+                           float* ft_b_grad, int n_ctas, cudaStream_t s_reduce, cudaEvent_t ev_reduce, int half_act = 0, float grad_scale = 1.0f,
                            unsigned long long* clamp_counter = nullptr);
 
 // opt_kernels.cu

@@ -1585,7 +1585,7 @@ int launch_l1_dgrad_ftgrad(cudaStream_t s, int mode, const float* dl1, const int
                            const int* n_tiles, int max_tiles, const float* wb, const float* ws,
                            const void* pre_stm, const void* pre_nstm, const float* ft_bias, float scale,
                            int B, int F, int l1, int nb, void* dft_stm, void* dft_nstm, float* bias_partials,
-                           float* ft_b_grad, int n_ctas, int half_act, float grad_scale, unsigned long long* clamp_counter) {
+                           float* ft_b_grad, int n_ctas, cudaStream_t s_reduce, cudaEvent_t ev_reduce, int half_act, float grad_scale, unsigned long long* clamp_counter) {
     const int work_cols = mode == 1 ? F / 2 : F;
     const int max_units = sort_units(B);
     int bias_rows = n_ctas;
@@ -1630,6 +1630,10 @@ int launch_l1_dgrad_ftgrad(cudaStream_t s, int mode, const float* dl1, const int
         else DGRAD_LAUNCH(3);
 #undef DGRAD_LAUNCH
     }
-    k_bias_partials_reduce<<<ceil_div(F, 8), 256, 0, s>>>(bias_partials, bias_rows, F, ft_b_grad);
+    if (s_reduce != s) {
+        cudaEventRecord(ev_reduce, s);
+        cudaStreamWaitEvent(s_reduce, ev_reduce, 0);
+    }
+    k_bias_partials_reduce<<<ceil_div(F, 8), 256, 0, s_reduce>>>(bias_partials, bias_rows, F, ft_b_grad);
     return 2;
 }
