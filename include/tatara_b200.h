@@ -272,7 +272,11 @@ int tb_init_sample(float* out, int64_t n, int64_t num_buckets, int64_t fan_in, i
                    float scale_value, int per_bucket_repeat, uint64_t seed);
 
 /* page-locked host memory for step inputs (pinned_host_alloc of the reference's runtime,
- * crates/cuda-native-runtime/src/runtime.rs:701-769) */
+ * crates/cuda-native-runtime/src/runtime.rs:701-769).  Any thread may call.  tb_host_free returns at once; a freed block is
+ * handed out again only after everything that any GPU of this process has been given to do by then, on the
+ * caller's streams as on the library's.  Freed blocks are kept for later calls: at most 256 MB of them, back to the system
+ * when 256 allocations have not matched them or when memory runs out.  Likewise tb_psv_extract keeps up to four sets of
+ * buffers per GPU, each of at most 96 MB of device memory and as much page-locked memory, until memory runs out. */
 int tb_host_alloc(void** out, size_t bytes);
 int tb_host_free(void* p);
 

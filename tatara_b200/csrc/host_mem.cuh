@@ -22,11 +22,7 @@ void host_copy_out(const HostCopy* items, int n);
 
 // page-locked memory from the pool; NULL when none can be had
 void* pinned_alloc(size_t bytes);
-// false: not a block of the pool
+// false: not a block of the pool.  The block is not handed out again before the work that any GPU has queued by then is done.
 bool pinned_free(void* p);
-// Streams that read page-locked caller memory without the caller waiting (a trainer's copy stream): a block that is given
-// back is not handed out again before the copies queued on them by then are done.
-void pinned_watch_stream(cudaStream_t s);
-void pinned_unwatch_stream(cudaStream_t s);
 // frees every cached block (called when memory runs out)
 void pinned_trim();

@@ -1011,7 +1011,7 @@ void free_all(tb_trainer* t) {
     for (auto& e : t->ev_reduced) if (e) cudaEventDestroy(e);
     if (t->ev_opt_done) cudaEventDestroy(t->ev_opt_done);
     if (t->ev_comm_done) cudaEventDestroy(t->ev_comm_done);
-    if (t->copy_stream) { pinned_unwatch_stream(t->copy_stream); cudaStreamDestroy(t->copy_stream); }
+    if (t->copy_stream) cudaStreamDestroy(t->copy_stream);
     if (t->stream) cudaStreamDestroy(t->stream);
     delete t;
 }
@@ -1044,7 +1044,6 @@ int create_impl(tb_trainer* t) {
     for (auto& s : t->side) CU(t, cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     for (cudaEvent_t* e : {&t->ev_begin, &t->ev_weff, &t->ev_fwd, &t->ev_inv, &t->ev_tail, &t->ev_dense, &t->ev_wgrad, &t->ev_small})
         CU(t, cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-    pinned_watch_stream(t->copy_stream);
     const bool ls = c.arch == TB_ARCH_LAYERSTACK;
     const int64_t N = c.ft_in, F = c.ft_out, l1 = c.l1_out, l2 = c.l2_out, nb = c.num_buckets;
     t->p_tf32 = (c.precision & TB_PREC_TF32) != 0;
