@@ -75,18 +75,26 @@ int launch_radam_small(cudaStream_t s, const SmallGroups& groups, int max_n, Opt
 // ------------------------------------------------------------------------------------------------
 // Factorised FT table (N = KB * pi real rows + pi virtual rows).  A block owns 32 adjacent float4 columns of one virtual row
 // vr, its warps share that row's KB real rows kb*pi + vr, up to FACT_ROWS neighbours each:
-//   - every warp updates its rows and adds up their gradients in kb order;
-//   - the warps' sums, added in warp order, are the virtual row's gradient (ft_reduce_virtual_grad,
-//     sparse/ft_factorize.rs:109-121); the first warp updates the virtual row N + vr;
-//   - comb[kb*pi + v] = w[kb*pi + v] + w[N + v] (ft_fold_virtual, sparse/ft_factorize.rs:78-99), the real rows kept in
-//     shared memory.
+//   - the rows' gradients go into shared memory, where 128 threads add them up in kb order, one chain per column: the virtual
+//     row's gradient (ft_reduce_virtual_grad, sparse/ft_factorize.rs:109-121);
+//   - every warp updates its rows, the first one also the virtual row N + vr;
+//   - comb[kb*pi + v] = w[kb*pi + v] + w[N + v] (ft_fold_virtual, sparse/ft_factorize.rs:78-99), the updated real rows kept in
+//     shared memory, where their gradients were.
 // Replaces radam_step on N_t*F elements + ft_reduce_virtual_grad + ranger_lookahead_lerp + ft_fold_virtual.
 // HBM-bound.  With a thread per column walking all the rows twice, the second walk found them gone from L2 (122 MB of rows
 // in flight): 4.2 GB moved instead of the 3.8 needed.  Warps side by side also make enough loads in flight where the table
-// is narrow.  F = 1536 / 768 / 256, 45 king buckets, fp32: 730 / 373 / 140 us with the walks, 636 / 324 / 118 now (0.92 of
-// the measured HBM rate at 1536); fp16 moments and table at 1536: 566, now 490.  (Rows in registers: 667.  No folded table,
-// the forward adding the two rows as it loads a strip: 566 here, but 190 more there.)
-// ------------------------------------------------------------------------------------------------
+// is narrow.  F = 1536 / 768 / 256, 45 king buckets, fp32: 730 / 373 / 140 us with the walks, 626 / 319 / 123 now (0.93 of
+// the measured HBM rate at 1536); fp16 moments and table at 1536: 566, now 499.  (Rows in registers: 667.  No folded table,
+// the forward adding the two rows as it loads a strip: 566 here, but 190 more there.  Every warp adding up its own rows and
+// the warps' sums after that: 637 / 325 / 122 and 492, another order.  The chain by a warp that reads the rows itself: 970.)
+// asynchronous copy of 8 or 16 bytes global -> shared (both aligned to that)
+template <int BYTES>
+static __device__ __forceinline__ void ok_cp(void* dst_shared, const void* src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst_shared);
+    if (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+}
+
 #define FACT_ROWS 9   // rows of a warp: 45 and 81 king buckets are 5 and 9 full warps
 #define FACT_BATCH 3  // of these, loaded together
 // HS: fp16 moments; HC: fp16 folded table.  The real rows' gradients are multiplied by sc.grad_scale on load; the virtual
@@ -95,8 +103,9 @@ template <int MAX_WARPS, int MIN_BLOCKS, bool HS, bool HC>
 __global__ void __launch_bounds__(32 * MAX_WARPS, MIN_BLOCKS) k_radam_factorized(float4* __restrict__ w, void* __restrict__ m, void* __restrict__ v,
                                                             float4* __restrict__ g, float4* __restrict__ slow,
                                                             void* __restrict__ comb, int N, int pi, int row4, OptScalars sc) {
-    __shared__ float4 s_sum[MAX_WARPS][32], s_virt[32];
-    __shared__ float4 s_w[FACT_ROWS][32 * MAX_WARPS];  // the updated real rows
+    __shared__ float4 s_virt[32];  // the virtual row: its gradient, then the updated weights
+    __shared__ float4 s_row[FACT_ROWS][32 * MAX_WARPS];  // the real rows: likewise
+    __shared__ float4 s_vw[32], s_vm[32], s_vv[32];  // weights and moments (as stored) of the virtual row
     const float inv_ms = 1.0f / TB_FT_OPT_M_SCALE, inv_vs = 1.0f / TB_FT_OPT_V_SCALE;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const size_t plane = (size_t)pi * row4;  // float4 of one king bucket
@@ -105,47 +114,50 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, MIN_BLOCKS) k_radam_factorized
     const int kb0 = warp * FACT_ROWS;
     const float rate = sc.lr * sc.step_size;
     const float decay_mul = 1.0f - sc.decay * rate;
-    float4 gsum = make_float4(0.f, 0.f, 0.f, 0.f);
-    // everything streams through once: evict-first
-#pragma unroll 1
-    for (int b = 0; b < FACT_ROWS; b += FACT_BATCH) {
-        float4 p[FACT_BATCH], mi[FACT_BATCH], vi[FACT_BATCH], gi[FACT_BATCH];
+#pragma unroll
+    for (int u = 0; u < FACT_ROWS; ++u)
+        if (kb0 + u < KB) ok_cp<16>(&s_row[u][threadIdx.x], g + (size_t)(kb0 + u) * plane + cell);
+    const size_t iv = (size_t)KB * plane + cell;
+    constexpr int MSZ = HS ? 8 : 16;  // bytes of four moments
+    if (warp == 0) {
+        ok_cp<16>(&s_vw[lane], w + iv);
+        ok_cp<MSZ>(reinterpret_cast<char*>(s_vm) + lane * MSZ, static_cast<const char*>(m) + iv * MSZ);
+        ok_cp<MSZ>(reinterpret_cast<char*>(s_vv) + lane * MSZ, static_cast<const char*>(v) + iv * MSZ);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    float4 p[FACT_BATCH], mi[FACT_BATCH], vi[FACT_BATCH];
+    auto load = [&](int b) {  // everything streams through once: evict-first
 #pragma unroll
         for (int u = 0; u < FACT_BATCH; ++u) {
             const size_t i = (size_t)min(kb0 + b + u, KB - 1) * plane + cell;  // past the end: the last row, dropped below
             p[u] = __ldcs(w + i);
             mi[u] = load_moment<HS>(m, i, inv_ms, true);
             vi[u] = load_moment<HS>(v, i, inv_vs, true);
-            gi[u] = __ldcs(g + i);
         }
+    };
+    load(0);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    for (int c = threadIdx.x; c < 128; c += blockDim.x) {
+        const float* col = reinterpret_cast<const float*>(s_row) + c;
+        float sum = 0.f;
+        int kb = 0;
+        for (int q = 0; q < warps; ++q)
 #pragma unroll
-        for (int u = 0; u < FACT_BATCH; ++u) {
-            if (kb0 + b + u >= KB) break;
-            const size_t i = (size_t)(kb0 + b + u) * plane + cell;
-            if (HC) gi[u] = scale4(gi[u], sc.grad_scale);  // loss-scaled sums exist only next to an fp16 table
-            float4 q = radam_four(p[u], mi[u], vi[u], gi[u], sc, rate, decay_mul);
-            store_moment<HS>(m, i, mi[u], TB_FT_OPT_M_SCALE, true, true);
-            store_moment<HS>(v, i, vi[u], TB_FT_OPT_V_SCALE, false, true);
-            if (sc.lerp) {
-                q = lerp_four(q, __ldcs(slow + i), sc.alpha);
-                __stcs(slow + i, q);
+            for (int u = 0; u < FACT_ROWS; ++u, ++kb) {
+                if (kb >= KB) break;
+                float x = col[(u * 32 * MAX_WARPS + 32 * q) * 4];
+                if (HC) x *= sc.grad_scale;  // loss-scaled sums exist only next to an fp16 table
+                sum += x;
             }
-            __stcs(w + i, q);
-            s_w[b + u][threadIdx.x] = q;
-            gsum.x += gi[u].x; gsum.y += gi[u].y; gsum.z += gi[u].z; gsum.w += gi[u].w;
-        }
+        reinterpret_cast<float*>(s_virt)[c] = sum;
     }
-    s_sum[warp][lane] = gsum;
     __syncthreads();
     if (warp == 0) {
-        for (int q = 1; q < warps; ++q) {
-            const float4 x = s_sum[q][lane];
-            gsum.x += x.x; gsum.y += x.y; gsum.z += x.z; gsum.w += x.w;
-        }
-        const size_t iv = (size_t)KB * plane + cell;
+        const float4 gsum = s_virt[lane];
         g[iv] = gsum;
-        float4 mv = load_moment<HS>(m, iv, inv_ms, false), vv = load_moment<HS>(v, iv, inv_vs, false);
-        float4 pv = radam_four(w[iv], mv, vv, gsum, sc, rate, decay_mul);
+        float4 mv = load_moment<HS>(s_vm, lane, inv_ms, false), vv = load_moment<HS>(s_vv, lane, inv_vs, false);
+        float4 pv = radam_four(s_vw[lane], mv, vv, gsum, sc, rate, decay_mul);
         store_moment<HS>(m, iv, mv, TB_FT_OPT_M_SCALE, true, false);
         store_moment<HS>(v, iv, vv, TB_FT_OPT_V_SCALE, false, false);
         if (sc.lerp) {
@@ -155,13 +167,33 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, MIN_BLOCKS) k_radam_factorized
         w[iv] = pv;
         s_virt[lane] = pv;
     }
+#pragma unroll 1
+    for (int b = 0; b < FACT_ROWS; b += FACT_BATCH) {
+#pragma unroll
+        for (int u = 0; u < FACT_BATCH; ++u) {
+            if (kb0 + b + u >= KB) break;
+            const size_t i = (size_t)(kb0 + b + u) * plane + cell;
+            float4 gi = s_row[b + u][threadIdx.x];
+            if (HC) gi = scale4(gi, sc.grad_scale);
+            float4 q = radam_four(p[u], mi[u], vi[u], gi, sc, rate, decay_mul);
+            store_moment<HS>(m, i, mi[u], TB_FT_OPT_M_SCALE, true, true);
+            store_moment<HS>(v, i, vi[u], TB_FT_OPT_V_SCALE, false, true);
+            if (sc.lerp) {
+                q = lerp_four(q, __ldcs(slow + i), sc.alpha);
+                __stcs(slow + i, q);
+            }
+            __stcs(w + i, q);
+            s_row[b + u][threadIdx.x] = q;
+        }
+        if (b + FACT_BATCH < FACT_ROWS) load(b + FACT_BATCH);
+    }
     __syncthreads();
     const float4 pv = s_virt[lane];
 #pragma unroll
     for (int u = 0; u < FACT_ROWS; ++u) {
         if (kb0 + u >= KB) break;
         const size_t i = (size_t)(kb0 + u) * plane + cell;
-        const float4 p = s_w[u][threadIdx.x];
+        const float4 p = s_row[u][threadIdx.x];
         const float4 f = make_float4(p.x + pv.x, p.y + pv.y, p.z + pv.z, p.w + pv.w);
         if (HC) __stcs(static_cast<uint2*>(comb) + i, pack_h4(f));
         else __stcs(static_cast<float4*>(comb) + i, f);
@@ -263,8 +295,8 @@ int launch_radam_factorized(cudaStream_t s, float* w, void* m, void* v, float* g
         if (half_state) { if (half_comb) FUSED(MW, MBH, true, true); else FUSED(MW, MBH, true, false); }                       \
         else { if (half_comb) FUSED(MW, MB, false, true); else FUSED(MW, MB, false, false); }                                  \
     } while (0)
-    // blocks per SM: more were slower again (F = 1536, fp32 / fp16 moments: 5 blocks 636 / 506 us, 6 641 / 490, 8 with one row at
-    // a time 800 / 568)
+    // blocks per SM, measured with the sums in registers (F = 1536, fp32 / fp16 moments): 5 blocks 636 / 506 us, 6 641 / 490, 8 with one row at
+    // a time 800 / 568
     if (warps <= 5) FUSED_H(5, 5, 6);
     else if (warps <= 9) FUSED_H(9, 3, 3);
     else return launch_radam_factorized_rows(s, w, m, v, g, slow, N, pi, F, 0, KB, sc, half_state) +
