@@ -179,19 +179,21 @@ int launch_tail_simple(cudaStream_t s, const float* l1_pre, const float* score, 
                        int act, int B, int l1, int l2, float* net_output, float* dy, float* dl1_pre,
                        float* l1_acted, float* dl2_pre, float* l2_acted, double* loss_partials,
                        double* loss_acc, int backward);
-// tail_kernels.cu: the same for l1 of 8, 16, 32 and l2 of 16, 32 (tail_tiled), with the blocks' sums of the small layers' weight
-// gradients; arch 0 LayerStack, 1 Simple CReLU, 2 Simple SCReLU.  partials: tail_partial_floats floats, loss_partials: one double
-// per block (tail_loss_blocks), summed by launch_reduce_double.
+// The order of the small layers' weight gradients: a bucket's positions in bucket order (Simple: all positions) are cut into this
+// many equal runs of one chain each; a warp's lane l adds the runs l, l + 32, .., then the lanes are added in halves.
+#define TB_RUNS_LS 64
+#define TB_RUNS_SIMPLE 128
+// tail_kernels.cu: the same for l1 of 8, 16, 32 and l2 of 16, 32 (tail_tiled), with the runs' sums of the small layers' weight
+// gradients; arch 0 LayerStack, 1 Simple CReLU, 2 Simple SCReLU.  A block per run: partials [tail_blocks][cells],
+// loss_partials [tail_blocks], summed by launch_reduce_double.
 bool tail_tiled(int l1, int l2);
-size_t tail_partial_floats(int arch, int l1, int l2, int max_tiles);
-int tail_loss_blocks(int n_pos);
-int launch_tail(cudaStream_t s, int arch, int n_pos, const float* l1_rows, const int* order, const TileDesc* tiles, const int* n_tiles, int max_tiles,
-                const float* score, const float* wdl, const float* l2_w, const float* l2_b, const float* l3_w, const float* l3_b,
-                LossParams lp, int l1, int l2, int nb, float* net_output, float* dy, float* dl1, float* partials,
-                double* loss_partials, int backward);
-// the weight gradients from the blocks' sums; gb1_shared: LayerStack's shared L1 bias, else NULL
-int launch_tail_wgrad(cudaStream_t s, int arch, const float* partials, const int* n_tiles, int l1, int l2, int nb, float* gw2, float* gb2,
-                      float* gw3, float* gb3, float* gb1, float* gb1_shared);
+int tail_blocks(int arch, int nb);
+int launch_tail(cudaStream_t s, int arch, int n_pos, const float* l1_rows, const int* order, const int* seg_start, const float* score,
+                const float* wdl, const float* l2_w, const float* l2_b, const float* l3_w, const float* l3_b, LossParams lp, int l1, int l2,
+                int nb, float* net_output, float* dy, float* dl1, float* partials, double* loss_partials, int backward);
+// the weight gradients from the runs' sums; gb1_shared: LayerStack's shared L1 bias, else NULL
+int launch_tail_wgrad(cudaStream_t s, int arch, const float* partials, int l1, int l2, int nb, float* gw2, float* gb2, float* gw3, float* gb3,
+                      float* gb1, float* gb1_shared);
 int launch_reduce_double(cudaStream_t s, const double* partials, int n, double* out);
 // per-bucket reductions of the small layers: out[g][cell] = sum over the positions of bucket g
 int launch_small_wgrad_layerstack(cudaStream_t s, const int* order, const int* seg_start, int B, int l1, int l2,

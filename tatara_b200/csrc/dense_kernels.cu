@@ -855,8 +855,6 @@ int launch_tail_simple(cudaStream_t s, const float* l1_pre, const float* score, 
 // (dense_mm_bucket.rs:112-161; native_kernels.cu:2591-2744 use register accumulators + atomics.)
 // ------------------------------------------------------------------------------------------------
 #define SW_CMAX 5
-#define SW_SPLIT_LS 64  // blocks per bucket segment (LayerStack; 59, two exact waves, measured slower); the Simple net splits
-                        // its one segment in 128
 __global__ void __launch_bounds__(1024) k_small_wgrad(const int* __restrict__ order, const int* __restrict__ seg_start,
                                                        const float* __restrict__ U, int dimU, const float* __restrict__ V,
                                                        int dimV, const float* __restrict__ Bsrc, const float* __restrict__ l2_acted,
@@ -985,7 +983,7 @@ int launch_small_wgrad_layerstack(cudaStream_t s, const int* order, const int* s
                                   float* l1s_b_grad) {
     (void)B;
     // L2 weight cell (o, i) = sum dl2_out[b][o] * l2_input[b][i]
-    return small_wgrad(s, order, seg_start, nb + 1, 1, SW_SPLIT_LS, dl2_out, l2, l2_input, 2 * (l1 - 1), dl2_out, l2_acted, l2, dy,
+    return small_wgrad(s, order, seg_start, nb + 1, 1, TB_RUNS_LS, dl2_out, l2, l2_input, 2 * (l1 - 1), dl2_out, l2_acted, l2, dy,
                        dl1_total, l1, partials, l2_w_grad, l2_b_grad, l3_w_grad, l3_b_grad, l1_b_grad, l1s_b_grad);
 }
 
@@ -995,7 +993,7 @@ int launch_small_wgrad_simple(cudaStream_t s, const int* order, const int* seg_s
                               float* l3_w_grad, float* l3_b_grad, float* l1_b_grad) {
     (void)B;
     // L2 weight cell (i, o) = sum l1_acted[b][i] * dl2_pre[b][o]; the whole batch is one segment
-    return small_wgrad(s, order, seg_start, 1, 0, 128, l1_acted, l1, dl2_pre, l2, dl2_pre, l2_acted, l2, dy, dl1_pre, l1,
+    return small_wgrad(s, order, seg_start, 1, 0, TB_RUNS_SIMPLE, l1_acted, l1, dl2_pre, l2, dl2_pre, l2_acted, l2, dy, dl1_pre, l1,
                        partials, l2_w_grad, l2_b_grad, l3_w_grad, l3_b_grad, l1_b_grad, nullptr);
 }
 

@@ -545,13 +545,13 @@ int run_forward(tb_trainer* t, const DevBatch& d, const tb_loss* loss, float lam
     if (tail_tiled(c.l1_out, c.l2_out)) {
         PhaseScope p(t, PH_TAIL);
         const int g = ls ? 6 : 4;  // l2_w, l2_b, l3_w, l3_b
-        int n = launch_tail(t->stream, tail_arch(c), B, t->l1_out, t->order, t->tiles, t->n_tiles, t->max_tiles, d.score, d.wdl, t->groups[g].w,
+        int n = launch_tail(t->stream, tail_arch(c), B, t->l1_out, t->order, t->seg_start, d.score, d.wdl, t->groups[g].w,
                             t->groups[g + 1].w, t->groups[g + 2].w, t->groups[g + 3].w, lp, c.l1_out, c.l2_out, ls ? c.num_buckets : 0,
                             t->net_output, t->dy, t->dl1, t->small_partials, t->loss_partials, backward);
         // in a training step nothing but the loss read-back waits for the sum
         const cudaStream_t sl = backward ? side_stream(t, 1) : t->stream;
         AFTER(t->ev_tail, t->stream, sl);
-        n += launch_reduce_double(sl, t->loss_partials, tail_loss_blocks(B), t->loss_acc);
+        n += launch_reduce_double(sl, t->loss_partials, tail_blocks(tail_arch(c), ls ? c.num_buckets : 0), t->loss_acc);
         p.done(n);
     }
     return TB_OK;
@@ -587,7 +587,7 @@ int run_backward(tb_trainer* t, const DevBatch& d, float lr) {
     if (tail_tiled(c.l1_out, c.l2_out)) {
         PhaseScope p(t, PH_SMALL_WGRAD);
         const int g = ls ? 6 : 4;
-        p.done(launch_tail_wgrad(si, tail_arch(c), t->small_partials, t->n_tiles, c.l1_out, c.l2_out, ls ? c.num_buckets : 0, t->groups[g].grad,
+        p.done(launch_tail_wgrad(si, tail_arch(c), t->small_partials, c.l1_out, c.l2_out, ls ? c.num_buckets : 0, t->groups[g].grad,
                                  t->groups[g + 1].grad, t->groups[g + 2].grad, t->groups[g + 3].grad, t->groups[3].grad,
                                  ls ? t->groups[5].grad : nullptr));
     }
@@ -1141,9 +1141,7 @@ int create_impl(tb_trainer* t) {
     CU(t, dalloc(&t->order, B)); CU(t, dalloc(&t->n_tiles, TB_TILE_COUNTS)); CU(t, dalloc(&t->seg_start, TB_MAX_BUCKETS + 3));
     CU(t, dalloc(&t->tiles, (size_t)t->max_tiles + t->max_units));
     const size_t n_cells = ls ? (size_t)(l2 * t->l2in + 2 * l2 + 1 + l1) : (size_t)(l1 * l2 + 2 * l2 + 1 + l1);
-    size_t small = (ls ? (size_t)(nb + 1) * 64 : (size_t)128) * n_cells;  // SW_SPLIT_LS partial rows per segment
-    if (tail_tiled((int)l1, (int)l2)) small = tail_partial_floats(c.arch, (int)l1, (int)l2, t->max_tiles);
-    CU(t, dalloc(&t->small_partials, small));
+    CU(t, dalloc(&t->small_partials, (ls ? (size_t)(nb + 1) * TB_RUNS_LS : (size_t)TB_RUNS_SIMPLE) * n_cells));  // one partial row per run
     CU(t, dalloc(&t->l1w_partials, (size_t)t->max_units * l1 * t->K));
     CU(t, dalloc(&t->l1_weff, (size_t)(nb + 1) * l1 * (t->K + 1)));  // effective L1 weights and biases per bucket
     t->dgrad_rows = DGRAD_CTAS > 2 * t->max_units ? DGRAD_CTAS : 2 * t->max_units;  // partial FT bias rows: one per block

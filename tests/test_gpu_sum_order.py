@@ -36,3 +36,127 @@ def test_virtual_row_gradient_is_one_chain_over_the_king_buckets(kb):
         want += g[k]
     assert np.count_nonzero(want) > want.size // 2
     _same_bits(g[kb], want, "virtual rows")
+
+
+# ---- fp32 arithmetic of the kernels: a product and its addition are rounded once (80-bit sums of exact products, rounded to
+# 24 bits: the same unless the 64-bit sum lies exactly between two floats, which random terms do not)
+def _fma(a, b, c):
+    return (np.asarray(a, np.longdouble) * np.asarray(b, np.longdouble) + np.asarray(c, np.longdouble)).astype(np.float32)
+
+
+def _chain(u, v, c=None):
+    """c + u[0] v[0] + u[1] v[1] + .., one after the other; the terms along the first axis."""
+    acc = np.zeros(np.broadcast_shapes(u.shape[1:], v.shape[1:]), np.float32) if c is None else np.broadcast_to(c, np.broadcast_shapes(u.shape[1:], v.shape[1:]))
+    for i in range(len(u)):
+        acc = _fma(u[i], v[i], acc)
+    return acc
+
+
+def _halves(t):
+    """Lane sums of a warp: lanes l and l + 16 first, then l and l + 8, .."""
+    while len(t) > 1:
+        t = t[: len(t) // 2] + t[len(t) // 2:]
+    return t[0]
+
+
+def _runs(u, v, order, seg, split):
+    """Sums of u[b] v[b] over the segments' positions: equal runs of one chain each, added by a warp's lanes."""
+    out = []
+    for beg, end in zip(seg[:-1], seg[1:]):
+        per = -(-(end - beg) // split)
+        run = np.zeros((split,) + np.broadcast_shapes(u.shape[1:], v.shape[1:]), np.float32)
+        for s in range(split):
+            at = order[beg + min(s * per, end - beg): beg + min((s + 1) * per, end - beg)]
+            if len(at):
+                run[s] = _chain(u[at], v[at])
+        lanes = np.zeros((32,) + run.shape[1:], np.float32)
+        for s in range(split):
+            lanes[s % 32] += run[s]
+        out.append(_halves(lanes))
+    return np.stack(out)
+
+
+def _crelu(x):
+    return np.clip(x, np.float32(0), np.float32(1))
+
+
+def _masked(x, up):
+    return np.where((x > 0) & (x < 1), up, np.float32(0)).astype(np.float32)
+
+
+def _trainer(arch, B, F, l1, l2, act, seed, fs=LS_FS.with_factorize(False)):
+    rng = np.random.default_rng(seed)
+    if arch == "layerstack":
+        init = _perturb(tb.layerstack_default_init(fs, F, l1, l2, 9), rng, ["ft_b", "l1_b", "l1_shared_bias", "l2_w", "l2_b", "l3_w", "l3_b"])
+        tr = tb.GpuTrainer(B, F, l1, l2, 9, fs, optimizer="adamw", init=dict(init, ft_w=init["ft_w"] * 30))
+    else:
+        init = _perturb(tb.simple_default_init(fs, F, l1, l2, pairwise=act == "pairwise"), rng, ["ft_b", "l1_b", "l2_w", "l2_b", "l3_w", "l3_b"])
+        tr = tb.SimpleGpuTrainer(B, F, l1, l2, fs, activation=act, optimizer="adamw", init=dict(init, ft_w=init["ft_w"] * 30))
+    batch = tb.synthetic_batch(tb.SYNTH_SEED + seed, B, fs, with_bucket=arch == "layerstack")
+    if arch == "layerstack":
+        batch.bucket_idx[:] = np.where(rng.random(B) < 0.4, 3, rng.choice([0, 1, 8, 9, -1], B)).astype(np.int32)  # some empty, some out of range
+    tr.forward_backward(batch, 0.25, tb.LossKind.sigmoid())
+    return tr, init, batch, rng
+
+
+def _segments(batch, B, nb):
+    key = np.zeros(B, np.int64) if nb == 0 else np.where((batch.bucket_idx >= 0) & (batch.bucket_idx < nb), batch.bucket_idx, nb)
+    return np.argsort(key, kind="stable"), np.concatenate([[0], np.cumsum(np.bincount(key, minlength=nb + 1))])
+
+
+@pytest.mark.parametrize("arch,l1,l2,B,act", [
+    # blocks of 64, 32 and 128 threads; l1 = 32 also 64 for longer runs
+    ("layerstack", 8, 16, 16, ""), ("layerstack", 16, 32, 1040, ""), ("layerstack", 16, 32, 8208, ""), ("layerstack", 16, 16, 21136, ""),
+    ("layerstack", 32, 32, 400, ""), ("layerstack", 32, 16, 8208, ""), ("layerstack", 32, 32, 41616, ""),
+    # blocks of 64, 32, 128 and 256 threads, the last one in one and in two rounds
+    ("simple", 8, 32, 16, "crelu"), ("simple", 32, 32, 4112, "crelu"), ("simple", 16, 16, 16400, "screlu"),
+    ("simple", 32, 32, 20000, "crelu"), ("simple", 32, 16, 33008, "pairwise")])
+def test_small_layers(arch, l1, l2, B, act):
+    F = 256
+    tr, w, batch, _ = _trainer(arch, B, F, l1, l2, act, B + l1)
+    ls = arch == "layerstack"
+    x = tr.read_buffer("l1_total", B * l1).reshape(B, l1)
+    dy, dl1 = tr.read_buffer("dy", B), tr.read_buffer("dl1_total", B * l1).reshape(B, l1)
+    order, seg = _segments(batch, B, 9 if ls else 0)
+    g = np.clip(batch.bucket_idx.astype(np.int64), 0, 8) if ls else np.zeros(B, np.int64)
+    live = (batch.bucket_idx >= 0) & (batch.bucket_idx < 9) if ls else np.ones(B, bool)
+    sqr = (lambda a: a * a) if act == "screlu" else (lambda a: a)
+    if ls:
+        m = x[:, : l1 - 1]
+        v = _crelu(np.concatenate([m * m * np.float32(127.0 / 128.0), m], 1))
+        w2, b2, w3 = w["l2_w"].reshape(9, l2, -1)[g], w["l2_b"].reshape(9, l2)[g], w["l3_w"].reshape(9, l2)[g]
+        b3, skip = w["l3_b"][g], x[:, l1 - 1]
+    else:
+        v = sqr(_crelu(x))
+        w2, b2, w3 = np.broadcast_to(w["l2_w"].reshape(l1, l2).T, (B, l2, l1)), w["l2_b"].reshape(1, l2), np.broadcast_to(w["l3_w"].reshape(1, l2), (B, l2))
+        b3, skip = w["l3_b"][g], None
+    a2 = _crelu(_chain(v.T[:, :, None], np.moveaxis(w2, 2, 0), b2))
+    act2 = sqr(a2)
+    if ls and l1 == 32:
+        out = _chain(act2.T, w3.T, b3)
+    else:
+        t = np.zeros((32, B), np.float32)
+        t[:l2] = (act2 * w3).T
+        out = b3 + _halves(t)
+    if ls:
+        out = np.where(live, out, np.float32(0)) + skip
+    _same_bits(tr.read_buffer("net_output", B), out, "net output")
+    up = dy[:, None] * w3
+    u = _masked(a2, up) if act != "screlu" else up * _masked(a2, 2 * a2)
+    u, act2 = np.where(live[:, None], u, np.float32(0)), np.where(live[:, None], act2, np.float32(0))
+    real = slice(0, 9 if ls else 1)
+    split = 64 if ls else 128
+    one = np.ones((B, 1), np.float32)
+    got = {k: tr.download_grad(k) for k in ("l2_w", "l2_b", "l3_w", "l3_b", "l1_b")}
+    w2g = _runs(u[:, :, None], v[:, None, :], order, seg, split)[real]
+    _same_bits(got["l2_w"], w2g if ls else np.moveaxis(w2g, 1, 2), "l2_w")
+    _same_bits(got["l2_b"], _runs(u, one, order, seg, split)[real], "l2_b")
+    _same_bits(got["l3_w"], _runs(act2, dy[:, None], order, seg, split)[real], "l3_w")
+    _same_bits(got["l3_b"], _runs(dy[:, None], one, order, seg, split)[real], "l3_b")
+    b1 = _runs(dl1, one, order, seg, split)
+    _same_bits(got["l1_b"], b1[real], "l1_b")
+    if ls:
+        total = np.zeros(l1, np.float32)
+        for q in b1:
+            total += q
+        _same_bits(tr.download_grad("l1_shared_bias"), total, "l1_shared_bias")
