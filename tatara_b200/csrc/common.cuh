@@ -160,8 +160,10 @@ int launch_l1_forward(cudaStream_t s, const float* x, int K, const int* order, c
                       const int* n_tiles, int max_tiles, const float* wb /*[nb][l1][K] or NULL*/,
                       const float* bb, const float* ws /*[K][l1]*/, const float* bs, float* y /*[B][l1]*/,
                       int l1, int nb, int n_pos, const float* weff, int tf32 = 0, int* error_flag = nullptr);
-// the effective weights and biases launch_l1_forward reads (l1 = 8, 16, 32; nothing otherwise): weff [(nb + 1) * l1 * (K + 1)]
-int launch_l1_weff(cudaStream_t s, const float* wb, const float* bb, const float* ws, const float* bs, int K, int l1, int nb, float* weff);
+// the effective weights and biases launch_l1_forward reads (l1 = 8, 16, 32; nothing otherwise), laid out for the kernel that the same
+// tf32 makes it take: weff [(nb + 1) * l1 * (K + 1)]
+int launch_l1_weff(cudaStream_t s, const float* wb, const float* bb, const float* ws, const float* bs, int K, int l1, int nb, float* weff,
+                   int tf32 = 0);
 // l1_tc.cu
 bool l1_forward_tc_supported(int K, int l1);
 int launch_l1_forward_tc(cudaStream_t s, const float* x, int K, const int* order, const TileDesc* tiles, const int* n_tiles,

@@ -259,16 +259,18 @@ __global__ void __launch_bounds__(64) k_l1_forward_tiled(const float* __restrict
 // ------------------------------------------------------------------------------------------------
 // L1 forward, streaming form for l1 = 8, 16 or 32.  The per-bucket and the shared layer see the same input and their
 // outputs are added, so they are one contraction with the effective weights weff[g] = wb[g] + ws^T (weff[nb] = ws^T for
-// positions without a bucket), built once per step by k_l1_weff.  A block owns up to 128 consecutive positions of the bucket
-// order, of one bucket; x rows and the weight rows arrive in K chunks of 64 through a three-stage ring of asynchronous
-// copies.  Every warp covers all of the block's positions and outputs for a quarter of each chunk's columns, so that a
-// thread's tile is large (RP positions x 8 outputs, two sums each for packed multiply-adds; RP = 8 has too few warps: 154 us) and an operand read from shared
-// memory is used often: the shared-memory pipe was what bound four-position tiles (128 us at K = 1536, l1 = 16, 65 536
-// positions; 113 now, the x rows at HBM rate take 62; K = 768, l1 = 8, 16 384 positions: 60 to 21 us).  Both operands are read as 128-bit rows along k; the row
-// stride spreads the rows a quarter warp touches over the banks.
+// positions without a bucket), built once per step by k_l1_weff.  An output is one chain of multiply-adds over k, then the bias:
+// that order is part of the results.  A packed multiply-add therefore holds two outputs of one position, and k_l1_weff stores the
+// weights by pairs of outputs; x enters it twice.  A block owns POS consecutive positions of the bucket order, of one bucket; x rows
+// and weights arrive in chunks of KC columns through a ring of asynchronous copies.  A thread keeps RP positions x 8 outputs and
+// reads both operands as 128-bit rows along k; the row stride spreads the rows a quarter warp touches over the banks.
+// What bounds it is the shared-memory pipe, and a block's latency where the batch is small.  65 536 positions, K = 1536, l1 = 16:
+// 114 us (the x rows at HBM rate take 62), 128 with scalar multiply-adds and four positions a thread; K = 512, l1 = 32: 72;
+// 16 384, K = 768, l1 = 8: 21, from 60; 10 000, K = 1024, l1 = 32: 46.  (The columns of a chunk shared by a block's warps and packed
+// pairs of columns, another order: 114, 83, 21, 38.)
 // ------------------------------------------------------------------------------------------------
 __global__ void k_l1_weff(const float* __restrict__ wb, const float* __restrict__ bb, const float* __restrict__ ws,
-                          const float* __restrict__ bs, int K, int l1, int nb, float* __restrict__ weff, float* __restrict__ beff) {
+                          const float* __restrict__ bs, int K, int l1, int nb, int pairs, float* __restrict__ weff, float* __restrict__ beff) {
     const int g = blockIdx.y;
     const size_t n = (size_t)l1 * K;
     const bool use_b = wb != nullptr && g < nb;
@@ -276,7 +278,8 @@ __global__ void k_l1_weff(const float* __restrict__ wb, const float* __restrict_
         const int o = (int)(i / K), k = (int)(i - (size_t)o * K);
         float v = ws[(size_t)k * l1 + o];
         if (use_b) v = wb[(size_t)g * n + i] + v;
-        weff[(size_t)g * n + i] = v;
+        // pairs: [l1 / 2][K][2], else [l1][K]
+        weff[(size_t)g * n + (pairs ? (size_t)(o >> 1) * 2 * K + 2 * k + (o & 1) : i)] = v;
     }
     if (blockIdx.x == 0 && (int)threadIdx.x < l1) {
         float b = bs ? bs[threadIdx.x] : 0.f;
@@ -285,25 +288,23 @@ __global__ void k_l1_weff(const float* __restrict__ wb, const float* __restrict_
     }
 }
 
-#define LF_WARPS 4
-#define LF_KC 64       // columns per stage: 256 bytes of every row, a quarter of them for each warp
-#define LF_LD (LF_KC + 4)
-#define LF_STAGES 3
-template <int L1, int RP>
+// RP, RO: positions and outputs of a thread; KC: columns per stage
+template <int L1, int RP, int RO, int WARPS, int KC, int STAGES>
 struct L1Tile {
-    static constexpr int TX = L1 / 8, TY = 32 / TX, POS = TY * RP;  // a warp's threads over outputs and positions; positions of a block
-    static constexpr int STAGE_FLOATS = (POS + L1) * LF_LD;
-    static constexpr size_t SMEM = (size_t)LF_STAGES * STAGE_FLOATS * sizeof(float);
-    static_assert((size_t)LF_WARPS * POS * L1 <= (size_t)LF_STAGES * STAGE_FLOATS, "the warps' sums fit the ring");
+    static constexpr int TX = L1 / RO, TY = 32 / TX, POS = WARPS * TY * RP;  // a warp's threads over outputs and positions; positions of a block
+    static constexpr int LDX = KC + 4, LDW = 2 * KC + 4;
+    static constexpr int STAGE_FLOATS = POS * LDX + L1 / 2 * LDW;
+    static constexpr size_t SMEM = (size_t)STAGES * STAGE_FLOATS * sizeof(float);
+    static_assert(POS % TB_TILE_M == 0 && POS <= 2 * TB_TILE_M, "whole tiles, within the smallest work unit");
 };
-template <int L1, int RP>
-__global__ void __launch_bounds__(32 * LF_WARPS) k_l1_forward_stream(const float* __restrict__ x, int K, const int* __restrict__ order,
+template <int L1, int RP, int RO, int WARPS, int KC, int STAGES>
+__global__ void __launch_bounds__(32 * WARPS) k_l1_forward_stream(const float* __restrict__ x, int K, const int* __restrict__ order,
                                                               const TileDesc* __restrict__ tiles, const TileDesc* __restrict__ units,
                                                               const int* __restrict__ n_units, int unit_blocks, const float* __restrict__ weff,
                                                               const float* __restrict__ beff, float* __restrict__ y, int nb) {
-    typedef L1Tile<L1, RP> T;
-    constexpr int TX = T::TX, TY = T::TY, POS = T::POS, NT = 32 * LF_WARPS;
-    extern __shared__ __align__(16) float s_ring[];  // [LF_STAGES][POS + L1][LF_LD]
+    typedef L1Tile<L1, RP, RO, WARPS, KC, STAGES> T;
+    constexpr int RQ = RO / 2, TX = T::TX, TY = T::TY, POS = T::POS, NT = 32 * WARPS, LDX = T::LDX, LDW = T::LDW;
+    extern __shared__ __align__(16) float s_ring[];  // [STAGES]{x [POS][LDX], weights [L1 / 2][LDW]}
     __shared__ int s_pos[POS];
     const int u = blockIdx.x / unit_blocks, h = blockIdx.x - u * unit_blocks;
     if (u >= *n_units) return;
@@ -318,77 +319,80 @@ __global__ void __launch_bounds__(32 * LF_WARPS) k_l1_forward_stream(const float
     for (int i = tid; i < POS; i += NT) s_pos[i] = order[p_begin + (i < n ? i : 0)];  // rows past the end repeat the first
     __syncthreads();
     const float* __restrict__ wg = weff + (size_t)g * L1 * K;
-    const int nk = K / LF_KC;
-    constexpr int PCS = LF_KC / 4;  // 16-byte pieces of a row's stage
+    const int nk = K / KC;
     auto issue = [&](int it) {
         if (it < nk) {
-            float* st = s_ring + (size_t)(it % LF_STAGES) * T::STAGE_FLOATS;
-            const int k0 = it * LF_KC;
+            float* st = s_ring + (size_t)(it % STAGES) * T::STAGE_FLOATS;
+            const int k0 = it * KC;
 #pragma unroll 8
-            for (int e = tid; e < POS * PCS; e += NT) {
-                const int r = e / PCS, pc = e % PCS;
-                dg_cp16(st + r * LF_LD + 4 * pc, x + (size_t)s_pos[r] * K + k0 + 4 * pc);
+            for (int e = tid; e < POS * (KC / 4); e += NT) {
+                const int r = e / (KC / 4), pc = e % (KC / 4);
+                dg_cp16(st + r * LDX + 4 * pc, x + (size_t)s_pos[r] * K + k0 + 4 * pc);
             }
-            for (int e = tid; e < L1 * PCS; e += NT) {
-                const int o = e / PCS, pc = e % PCS;
-                dg_cp16(st + (POS + o) * LF_LD + 4 * pc, wg + (size_t)o * K + k0 + 4 * pc);
+            for (int e = tid; e < L1 / 2 * (KC / 2); e += NT) {
+                const int o = e / (KC / 2), pc = e % (KC / 2);
+                dg_cp16(st + POS * LDX + o * LDW + 4 * pc, wg + ((size_t)o * K + k0) * 2 + 4 * pc);
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     const int lane = tid & 31, warp = tid >> 5;
-    const int tx = lane % TX, ty = lane / TX;  // the thread's positions ty + TY * i, outputs tx + TX * j
-    unsigned long long acc[RP][8];
+    const int tx = lane % TX, row0 = warp * (TY * RP) + lane / TX;  // the thread's positions row0 + TY * i, output pairs tx + TX * j
+    unsigned long long acc[RP][RQ];
 #pragma unroll
     for (int i = 0; i < RP; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
+        for (int j = 0; j < RQ; ++j) acc[i][j] = 0ull;
 #pragma unroll
-    for (int it = 0; it < LF_STAGES - 1; ++it) issue(it);
+    for (int it = 0; it < STAGES - 1; ++it) issue(it);
     for (int it = 0; it < nk; ++it) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(LF_STAGES - 2) : "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
         __syncthreads();  // chunk `it` has landed for every thread; chunk it - 1 has been consumed by every thread
-        issue(it + LF_STAGES - 1);
-        const float* st = s_ring + (size_t)(it % LF_STAGES) * T::STAGE_FLOATS + warp * (LF_KC / LF_WARPS);
+        issue(it + STAGES - 1);
+        const float* st = s_ring + (size_t)(it % STAGES) * T::STAGE_FLOATS;
 #pragma unroll
-        for (int kk = 0; kk < LF_KC / LF_WARPS; kk += 4) {
-            ulonglong2 wv[8];
+        for (int kk = 0; kk < KC; kk += 4) {
+            ulonglong2 wv[RQ][2];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) wv[j] = *reinterpret_cast<const ulonglong2*>(st + (POS + tx + TX * j) * LF_LD + kk);
+            for (int j = 0; j < RQ; ++j) {
+                const ulonglong2* w = reinterpret_cast<const ulonglong2*>(st + POS * LDX + (tx + TX * j) * LDW + 2 * kk);
+                wv[j][0] = w[0];
+                wv[j][1] = w[1];
+            }
 #pragma unroll
             for (int i = 0; i < RP; ++i) {
-                const ulonglong2 xv = *reinterpret_cast<const ulonglong2*>(st + (ty + TY * i) * LF_LD + kk);
+                const float4 xv = *reinterpret_cast<const float4*>(st + (row0 + TY * i) * LDX + kk);
+                const unsigned long long x0 = pair2(xv.x, xv.x), x1 = pair2(xv.y, xv.y), x2 = pair2(xv.z, xv.z), x3 = pair2(xv.w, xv.w);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    fma2(acc[i][j], xv.x, wv[j].x);
-                    fma2(acc[i][j], xv.y, wv[j].y);
-                }
+                for (int j = 0; j < RQ; ++j) fma2(acc[i][j], x0, wv[j][0].x);
+#pragma unroll
+                for (int j = 0; j < RQ; ++j) fma2(acc[i][j], x1, wv[j][0].y);
+#pragma unroll
+                for (int j = 0; j < RQ; ++j) fma2(acc[i][j], x2, wv[j][1].x);
+#pragma unroll
+                for (int j = 0; j < RQ; ++j) fma2(acc[i][j], x3, wv[j][1].y);
             }
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();  // the ring is free for the warps' sums [warp][POS][L1]
 #pragma unroll
-    for (int i = 0; i < RP; ++i)
+    for (int j = 0; j < RQ; ++j) {
+        const float2 b = *reinterpret_cast<const float2*>(beff + (size_t)g * L1 + 2 * (tx + TX * j));
 #pragma unroll
-        for (int j = 0; j < 8; ++j)
-            s_ring[(size_t)(warp * POS + ty + TY * i) * L1 + tx + TX * j] =
-                __uint_as_float((unsigned)acc[i][j]) + __uint_as_float((unsigned)(acc[i][j] >> 32));
-    __syncthreads();
-    for (int e = tid; e < n * L1; e += NT) {
-        const int r = e / L1, o = e % L1;
-        float sum = s_ring[e];
-#pragma unroll
-        for (int q = 1; q < LF_WARPS; ++q) sum += s_ring[(size_t)q * POS * L1 + e];
-        y[(size_t)s_pos[r] * L1 + o] = sum + beff[(size_t)g * L1 + o];
+        for (int i = 0; i < RP; ++i) {
+            const int r = row0 + TY * i;
+            if (r < n) *reinterpret_cast<float2*>(y + (size_t)s_pos[r] * L1 + 2 * (tx + TX * j)) = make_float2(lo2(acc[i][j]) + b.x, hi2(acc[i][j]) + b.y);
+        }
     }
 }
 
-static inline bool l1_streams(int K, int l1) { return (l1 == 8 || l1 == 16 || l1 == 32) && K % LF_KC == 0; }
+static inline bool l1_streams(int K, int l1) { return (l1 == 8 || l1 == 16 || l1 == 32) && K % 64 == 0; }
+static inline bool l1_on_tensor_cores(int K, int l1, int tf32) { return tf32 && l1_forward_tc_supported(K, l1); }
 
-int launch_l1_weff(cudaStream_t s, const float* wb, const float* bb, const float* ws, const float* bs, int K, int l1, int nb, float* weff) {
+int launch_l1_weff(cudaStream_t s, const float* wb, const float* bb, const float* ws, const float* bs, int K, int l1, int nb, float* weff, int tf32) {
     if (!l1_streams(K, l1)) return 0;
-    k_l1_weff<<<dim3(ceil_div(l1 * K, 256 * 4), nb + 1), 256, 0, s>>>(wb, bb, ws, bs, K, l1, wb ? nb : 0, weff, weff + (size_t)(nb + 1) * l1 * K);
+    k_l1_weff<<<dim3(ceil_div(l1 * K, 256 * 4), nb + 1), 256, 0, s>>>(wb, bb, ws, bs, K, l1, wb ? nb : 0, !l1_on_tensor_cores(K, l1, tf32), weff,
+                                                                      weff + (size_t)(nb + 1) * l1 * K);
     return 1;
 }
 
@@ -397,22 +401,27 @@ int launch_l1_forward(cudaStream_t s, const float* x, int K, const int* order, c
                       const float* bs, float* y, int l1, int nb, int n_pos, const float* weff, int tf32, int* error_flag) {
     if (l1_streams(K, l1)) {
         const float* beff = weff + (size_t)(nb + 1) * l1 * K;
-        if (tf32 && error_flag && l1_forward_tc_supported(K, l1))
+        if (l1_on_tensor_cores(K, l1, tf32))
             return launch_l1_forward_tc(s, x, K, order, tiles, n_tiles, max_tiles, n_pos, weff, beff, y, l1, wb ? nb : 0, error_flag);
         const int max_units = sort_units(n_pos);
         const TileDesc* units = tiles + max_tiles;
         const int nbe = wb ? nb : 0;
-#define L1F(L, RP)                                                                                                          \
+#define L1F(L, RP, RO, W, KC, ST)                                                                                           \
     do {                                                                                                                    \
-        const int ub = unit_tiles(n_pos) * TB_TILE_M / L1Tile<L, RP>::POS;                                                  \
-        cudaFuncSetAttribute(k_l1_forward_stream<L, RP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L1Tile<L, RP>::SMEM); \
-        k_l1_forward_stream<L, RP><<<ub * max_units, 32 * LF_WARPS, L1Tile<L, RP>::SMEM, s>>>(x, K, order, tiles, units, n_tiles + 1, ub, \
-                                                                                            weff, beff, y, nbe);            \
+        typedef L1Tile<L, RP, RO, W, KC, ST> T;                                                                             \
+        const int ub = unit_tiles(n_pos) * TB_TILE_M / T::POS;                                                              \
+        cudaFuncSetAttribute(k_l1_forward_stream<L, RP, RO, W, KC, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::SMEM); \
+        k_l1_forward_stream<L, RP, RO, W, KC, ST><<<ub * max_units, 32 * W, T::SMEM, s>>>(x, K, order, tiles, units, n_tiles + 1, ub, weff, beff, \
+                                                                                          y, nbe);                          \
     } while (0)
-        // fewer positions per block where the batch has too few for every SM
-        if (l1 == 8) { if (n_pos >= 148 * 64) L1F(8, 2); else L1F(8, 1); }
-        else if (l1 == 16) { if (n_pos >= 148 * 64) L1F(16, 4); else L1F(16, 2); }
-        else L1F(32, 4);
+        // Full batches: many outputs per thread, short chunks, many blocks (K = 1536, l1 = 16: 114 us, the small batches' shape 162;
+        // l1 = 32, K = 512: 70 against 97).  Batches that do not fill the chip: a chain's latency is what counts, so fewer
+        // outputs per thread and longer chunks (1024 positions, l1 = 16, K = 256: 10.5 us, the large batches' shape 14.4; 10 000, l1 = 32,
+        // K = 1024: 46 for either).
+        const int ut = unit_tiles(n_pos);
+        if (l1 == 8) { if (ut == TB_UNIT_TILES) L1F(8, 1, 8, 2, 16, 3); else L1F(8, 1, 4, 4, 64, 3); }
+        else if (l1 == 16) { if (ut == TB_UNIT_TILES) L1F(16, 2, 8, 2, 16, 3); else L1F(16, 2, 2, 4, 32, 3); }
+        else { if (ut > 2) L1F(32, 4, 8, 2, 32, 3); else L1F(32, 2, 4, 4, 32, 3); }
 #undef L1F
         return 1;
     }

@@ -488,7 +488,7 @@ int run_forward(tb_trainer* t, const DevBatch& d, const tb_loss* loss, float lam
     // the effective L1 weights depend on nothing of this batch
     if (ls) {
         AFTER(t->ev_begin, t->stream, side_stream(t, 1));
-        t->launches += launch_l1_weff(side_stream(t, 1), t->groups[2].w, t->groups[3].w, t->groups[4].w, t->groups[5].w, F, c.l1_out, c.num_buckets, t->l1_weff);
+        t->launches += launch_l1_weff(side_stream(t, 1), t->groups[2].w, t->groups[3].w, t->groups[4].w, t->groups[5].w, F, c.l1_out, c.num_buckets, t->l1_weff, t->p_tf32);
     } else {
         AFTER(t->ev_begin, t->stream, side_stream(t, 1));
         t->launches += launch_l1_weff(side_stream(t, 1), nullptr, nullptr, t->groups[2].w, t->groups[3].w, t->K, c.l1_out, 0, t->l1_weff);

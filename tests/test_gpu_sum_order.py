@@ -160,3 +160,27 @@ def test_small_layers(arch, l1, l2, B, act):
         for q in b1:
             total += q
         _same_bits(tr.download_grad("l1_shared_bias"), total, "l1_shared_bias")
+
+
+@pytest.mark.parametrize("arch,F,l1,B", [
+    # by batch size: units of 64, 128 and 256 positions; ragged tiles, short buckets, positions without a bucket
+    ("layerstack", 256, 8, 16), ("layerstack", 640, 8, 9488), ("layerstack", 256, 8, 18960),
+    ("layerstack", 256, 16, 272), ("layerstack", 384, 16, 9488), ("layerstack", 256, 16, 18960),
+    ("layerstack", 256, 32, 272), ("layerstack", 256, 32, 9488), ("simple", 256, 32, 1040), ("simple", 128, 16, 18960)])
+def test_l1_forward_is_one_chain_over_the_inputs(arch, F, l1, B):
+    tr, w, batch, _ = _trainer(arch, B, F, l1, 16, "crelu", B + l1)
+    ls = arch == "layerstack"
+    K = F if ls else 2 * F
+    x = tr.read_buffer("combined", B * K).reshape(B, K)
+    ws = w["l1_shared_weight" if ls else "l1_w"].reshape(K, l1)
+    bs = w["l1_shared_bias" if ls else "l1_b"]
+    weff, beff = np.broadcast_to(ws, (10, K, l1)).copy(), np.broadcast_to(bs, (10, l1)).copy()
+    if ls:
+        weff[:9] = np.moveaxis(w["l1_w"].reshape(9, l1, K), 1, 2) + ws
+        beff[:9] = w["l1_b"].reshape(9, l1) + bs
+    order, seg = _segments(batch, B, 9 if ls else 0)
+    want = np.empty((B, l1), np.float32)
+    for g, (beg, end) in enumerate(zip(seg[:-1], seg[1:])):
+        at = order[beg:end][:: max(1, (end - beg) // 300)]  # some of every bucket
+        want[at] = _chain(x[at].T[:, :, None], weff[g][:, None, :]) + beff[g]
+        _same_bits(tr.read_buffer("l1_total", B * l1).reshape(B, l1)[at], want[at], "bucket %d" % g)
