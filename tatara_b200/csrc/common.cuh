@@ -13,7 +13,10 @@
 // batch that does not fill the chip with blocks of 128 positions gets smaller ones (B = 1024: the L1 input gradient took
 // 43 us on 16 of 148 SMs, 22 now).
 static inline int unit_tiles(int n_pos) { return n_pos >= 148 * 128 ? TB_UNIT_TILES : n_pos >= 148 * 64 ? 4 : 2; }
-// counts beside the tiles: {tiles, units, first unit of every bucket (and of the positions without one, and the end)}
+// The L1 weight gradient's work units have TB_UNIT_TILES tiles whatever the batch: a unit is one chain of its fp32 sums, whose order
+// is part of a step's results.
+// counts beside the tiles: {tiles, units, weight units, first weight unit of every bucket (and of the positions without one, and
+// the end)}
 #define TB_TILE_COUNTS 16
 
 // One tile of positions for the bucket-grouped dense kernels: positions order[start .. start+count).
@@ -130,9 +133,12 @@ int launch_ft_backward_slice(cudaStream_t s, const void* dft_stm, const void* df
 int launch_slice_check(cudaStream_t s, const int* idx_stm, const int* idx_nstm, const int* nnz, int B, int A, int N,
                        int rows_per_slice, int* outside);
 int sort_max_units(int max_tiles);
+int sort_weight_units(int n_pos);  // the most weight units a batch of n_pos positions has
+const TileDesc* weight_units(const TileDesc* tiles, int max_tiles);  // where they lie behind the tiles and units
+size_t sort_tiles_len(int max_tiles);  // TileDescs of all three
 int sort_units(int n_pos);  // the most work units a batch of n_pos positions has (sort_max_units: any batch of a trainer)
 // The two sorts of a step: positions by bucket -> order, bucket segments seg_start [nb + 2], tiles (room for max_tiles
-// tiles followed by the work units; n_tiles: TB_TILE_COUNTS ints); items (position, perspective) of both
+// tiles followed by the work units and the weight units; n_tiles: TB_TILE_COUNTS ints); items (position, perspective) of both
 // perspectives by the table slice of their features -> items, item_seg [slices + 2].  hist: scratch of
 // (nb + 1) * ceil(B / 1024) + (slices + 1) * ceil(n_persp * B / 1024) ints
 // items NULL (B <= SORT_ONE_BLOCK): the positions alone, in one launch.  fwd_work / bwd_work: also plan the slice-resident forward / weight gradient (the latter in bwd_parts launches over equal

@@ -1064,46 +1064,64 @@ __global__ void __launch_bounds__(256) k_l1_wgrad(const float* __restrict__ x, i
     }
 }
 
-// Second stage: the work units of bucket g, and of the positions with an out-of-range bucket id (the whole batch for
-// Simple), are added by `slices` warps each, in a fixed order; a block holds 128 elements and all buckets, so that the sum
-// over the buckets, gw_shared[k][o], comes from the same launch.  (One thread per element and bucket walking all units took
-// 104 us for the 266 units of a Simple batch, 8 now; 18 with the sum over the buckets for a LayerStack one, 8 now.)
-__global__ void __launch_bounds__(1024) k_l1_wgrad_final(const float* __restrict__ partials, const int* __restrict__ unit_base, int K, int l1,
-                                                         int nb, int slices, float* __restrict__ gw_bucket, float* __restrict__ gw_shared) {
-    __shared__ float4 s_sum[32][32];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, g = w / slices, sl = w - g * slices;
-    const int i4 = blockIdx.x * 32 + lane, n4 = l1 * K / 4;
-    const float4* __restrict__ p4 = reinterpret_cast<const float4*>(partials) + i4;
-    const int u1 = unit_base[g + 1];
-    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int u = unit_base[g] + sl; u < u1; u += 8 * slices) {
-        float4 v[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            v[j] = u + j * slices < u1 ? p4[(size_t)(u + j * slices) * n4] : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) { sum.x += v[j].x; sum.y += v[j].y; sum.z += v[j].z; sum.w += v[j].w; }
-    }
-    s_sum[w][lane] = sum;
+// Second stage: the units of bucket g, and of the positions with an out-of-range bucket id (the whole batch for Simple), are
+// added in order, one chain per element, and the buckets' sums, in order too, are gw_shared[k][o].  A block owns 128 elements:
+// every warp brings rows of the units into shared memory, a group of WF_UNITS ahead of the 128 threads that add them up (as many
+// loads in flight as there are, where a thread that reads and adds its own element waits for memory every few units: 104 us for
+// the 266 units of a Simple batch).  With the gradient kernel, 65 536 positions: K = 1536, l1 = 16 123 us, Simple K = 512, l1 = 32 79;
+// the units in slices side by side, another order: 116, 78.
+#define WF_UNITS 64   // units of a stage
+#define WF_STAGES 2
+__global__ void __launch_bounds__(512) k_l1_wgrad_final(const float* __restrict__ partials, const int* __restrict__ unit_base, int K, int l1,
+                                                        int nb, float* __restrict__ gw_bucket, float* __restrict__ gw_shared) {
+    extern __shared__ __align__(16) float s_part[];  // [WF_STAGES][WF_UNITS][128]
+    __shared__ int s_base[TB_MAX_BUCKETS + 2];
+    if ((int)threadIdx.x <= nb + 1) s_base[threadIdx.x] = unit_base[threadIdx.x];
     __syncthreads();
-    if (sl == 0) {
-        for (int j = 1; j < slices; ++j) {
-            const float4 v = s_sum[w + j][lane];
-            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int n_units = s_base[nb + 1], n_stages = (n_units + WF_UNITS - 1) / WF_UNITS;
+    const size_t n = (size_t)l1 * K;
+    const float* __restrict__ src = partials + (size_t)blockIdx.x * 128 + 4 * lane;
+    auto issue = [&](int st) {
+        if (st < n_stages) {
+            float* dst = s_part + (size_t)(st % WF_STAGES) * WF_UNITS * 128 + 4 * lane;
+            for (int i = w; i < WF_UNITS && st * WF_UNITS + i < n_units; i += warps)
+                dg_cp16(dst + i * 128, src + (size_t)(st * WF_UNITS + i) * n);
         }
-        s_sum[w][lane] = sum;
-        if (g < nb) reinterpret_cast<float4*>(gw_bucket)[(size_t)g * n4 + i4] = sum;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const size_t i = (size_t)blockIdx.x * 128 + threadIdx.x;  // the element of a thread below 128
+    float sum = 0.f, total = 0.f;
+    int g = 0;
+    auto close = [&](int u) {  // the buckets that end before unit u
+        while (g <= nb && s_base[g + 1] <= u) {
+            if (g < nb) gw_bucket[(size_t)g * n + i] = sum;
+            total += sum;
+            sum = 0.f;
+            ++g;
+        }
+    };
+#pragma unroll
+    for (int st = 0; st < WF_STAGES - 1; ++st) issue(st);
+    for (int st = 0; st < n_stages; ++st) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(WF_STAGES - 2) : "memory");
+        __syncthreads();  // stage `st` has landed for every thread; stage st - 1 has been added
+        issue(st + WF_STAGES - 1);
+        if (threadIdx.x < 128) {
+            const float* p = s_part + (size_t)(st % WF_STAGES) * WF_UNITS * 128 + threadIdx.x;
+            for (int u = st * WF_UNITS; u < min((st + 1) * WF_UNITS, n_units);) {
+                close(u);
+                const int u1 = min(s_base[g + 1], min((st + 1) * WF_UNITS, n_units));
+#pragma unroll 8
+                for (; u < u1; ++u, p += 128) sum += *p;
+            }
+        }
     }
-    __syncthreads();
-    if (w != 0) return;
-    float4 total = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int j = 0; j <= nb; ++j) {
-        const float4 v = s_sum[j * slices][lane];
-        total.x += v.x; total.y += v.y; total.z += v.z; total.w += v.w;
-    }
-    const int o = 4 * i4 / K, k = 4 * i4 - o * K;
-    float* out = gw_shared + (size_t)k * l1 + o;
-    out[0] = total.x; out[l1] = total.y; out[2 * l1] = total.z; out[3 * l1] = total.w;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (threadIdx.x >= 128) return;
+    close(n_units);
+    const int o = (int)(i / K), k = (int)(i - (size_t)o * K);
+    gw_shared[(size_t)k * l1 + o] = total;
 }
 
 // Variant for l1 % 8 == 0: a thread owns four adjacent columns and OPT outputs (OPT = 8 or 16; two thread groups
@@ -1218,9 +1236,9 @@ __global__ void __launch_bounds__(THREADS, MIN_BLOCKS) k_l1_wgrad_stream(const f
 int launch_l1_wgrad(cudaStream_t s, const float* x, int K, const float* dl1, const int* order,
                     const TileDesc* tiles, const int* n_tiles, int max_tiles, int n_pos, int l1, int nb, float* partials,
                     float* gw_bucket, float* gw_shared) {
-    const TileDesc* units = tiles + max_tiles;
-    const int* n_units = n_tiles + 1;
-    const int max_units = sort_units(n_pos);
+    const TileDesc* units = weight_units(tiles, max_tiles);
+    const int* n_units = n_tiles + 2;
+    const int max_units = sort_weight_units(n_pos);
     if (l1 == 8 || l1 == 16 || l1 == 32) {
         const int threads = l1 == 32 ? 256 : 128;
         const dim3 grid(ceil_div(K / 4, 128), max_units);
@@ -1231,14 +1249,17 @@ int launch_l1_wgrad(cudaStream_t s, const float* x, int K, const float* dl1, con
         k_l1_wgrad_stream<OPT, T, MB, ST, P><<<grid, threads, smem, s>>>(x, K, dl1, order, tiles, units, n_units, l1, partials); \
     } while (0)
         // 128-thread blocks at six per SM: with K = 1536 the 3 x 265 blocks of the benchmark then run as one wave
-        if (l1 == 8) WGRAD(8, 128, 6, 2, true);
-        else if (l1 == 16) WGRAD(16, 128, 6, 2, false);
+        // fewer units than SMs: more rounds in flight (1024 positions, K = 256, l1 = 16: 36 to 27 us; 16 384, K = 768, l1 = 8: 37 to 35)
+        const bool few = n_pos < WG_POS * 148;
+        if (l1 == 8) { if (few) WGRAD(8, 128, 4, 6, true); else WGRAD(8, 128, 6, 2, true); }
+        else if (l1 == 16) { if (few) WGRAD(16, 128, 3, 6, true); else WGRAD(16, 128, 6, 2, false); }
         else WGRAD(16, 256, 2, 4, true);
 #undef WGRAD
     } else
         k_l1_wgrad<<<dim3(K / 128, max_units), 256, 0, s>>>(x, K, dl1, order, tiles, units, n_units, l1, partials);
-    const int slices = 32 / (nb + 1) < 16 ? 32 / (nb + 1) : 16;
-    k_l1_wgrad_final<<<l1 * K / 128, 32 * slices * (nb + 1), 0, s>>>(partials, n_tiles + 2, K, l1, nb, slices, gw_bucket, gw_shared);
+    const size_t smem = (size_t)WF_STAGES * WF_UNITS * 128 * sizeof(float);
+    cudaFuncSetAttribute(k_l1_wgrad_final, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_l1_wgrad_final<<<l1 * K / 128, 512, smem, s>>>(partials, n_tiles + 3, K, l1, nb, gw_bucket, gw_shared);
     return 2;
 }
 
@@ -1420,6 +1441,7 @@ __global__ void __launch_bounds__(256) k_l1_dgrad_ftgrad_stream(const float* __r
         }
     }
     if (n == 0) {  // the bias reduction reads every row
+        if (bias_partials == nullptr) return;
         *reinterpret_cast<float4*>(bp + wcol) = bacc0;
         if (MODE == 1) *reinterpret_cast<float4*>(bp + half + wcol) = bacc1;
         return;
@@ -1562,27 +1584,55 @@ __global__ void __launch_bounds__(256) k_l1_dgrad_ftgrad_stream(const float* __r
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    *reinterpret_cast<float4*>(bp + wcol) = bacc0;
-    if (MODE == 1) *reinterpret_cast<float4*>(bp + half + wcol) = bacc1;
+    if (bias_partials != nullptr) {
+        *reinterpret_cast<float4*>(bp + wcol) = bacc0;
+        if (MODE == 1) *reinterpret_cast<float4*>(bp + half + wcol) = bacc1;
+    }
     if (HALF) {
         clamps = __reduce_add_sync(0xffffffffu, clamps);
         if ((threadIdx.x & 31) == 0 && clamps) atomicAdd(clamp_counter, (unsigned long long)clamps);
     }
 }
 
+// The partial rows of the FT bias gradient where the streaming kernel's blocks are shorter than DG_POS positions: a row is one chain
+// over DG_POS positions, half a weight unit, whatever the batch size.  A thread per column reads the finished dft rows, from L2.
+// grid (rows, 2 perspectives, column blocks).
+__global__ void __launch_bounds__(128) k_bias_partial_rows(const int* __restrict__ order, const TileDesc* __restrict__ tiles,
+                                                           const TileDesc* __restrict__ wunits, const int* __restrict__ n_wunits,
+                                                           const float* __restrict__ dft_stm, const float* __restrict__ dft_nstm, int F,
+                                                           float* __restrict__ partials) {
+    __shared__ int s_pos[DG_POS];
+    const int u = blockIdx.x >> 1, h = blockIdx.x & 1, persp = blockIdx.y, c = blockIdx.z * 128 + threadIdx.x;
+    int n = 0;
+    if (u < *n_wunits) {
+        const TileDesc ud = wunits[u];
+        const int first = ud.start + h * (DG_POS / TB_TILE_M), last = min(ud.start + ud.count, first + DG_POS / TB_TILE_M);
+        if (first < last) {
+            const int p_begin = tiles[first].start;
+            n = tiles[last - 1].start + tiles[last - 1].count - p_begin;
+            if ((int)threadIdx.x < n) s_pos[threadIdx.x] = order[p_begin + threadIdx.x];
+        }
+    }
+    __syncthreads();
+    const float* __restrict__ dft = (persp ? dft_nstm : dft_stm) + c;
+    float sum = 0.f;
+#pragma unroll 16
+    for (int r = 0; r < n; ++r) sum += dft[(size_t)s_pos[r] * F];
+    partials[((size_t)blockIdx.x * 2 + persp) * F + c] = sum;
+}
+
 // out[c] = sum over the perspectives (stm first) and the blocks' partial rows; 32 lanes share a column's rows and
-// their partial sums are combined in lane order, a fixed order
-__global__ void __launch_bounds__(256) k_bias_partials_reduce(const float* __restrict__ partials, int n_rows, int F,
+// their partial sums are combined in lane order.  Row r of perspective p goes to lane (p * lane_rows + r) mod 32; lane_rows is the
+// row count of the largest batch, so that the order does not depend on the batch.
+__global__ void __launch_bounds__(256) k_bias_partials_reduce(const float* __restrict__ partials, int n_rows, int lane_rows, int F,
                                                               float* __restrict__ out) {
     const int lane = threadIdx.x & 31;
     const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);  // a warp per column
     if (c >= F) return;
     float sum = 0.f;
-    const int total = 2 * n_rows;  // index i = p * n_rows + r
-    for (int i = lane; i < total; i += 32) {
-        const int p = i / n_rows, r = i - p * n_rows;
-        sum += partials[((size_t)r * 2 + p) * F + c];
-    }
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+        for (int r = (lane - p * lane_rows) & 31; r < n_rows; r += 32) sum += partials[((size_t)r * 2 + p) * F + c];
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, d);
     if (lane == 0) out[c] = sum;
@@ -1595,20 +1645,24 @@ int launch_l1_dgrad_ftgrad(cudaStream_t s, int mode, const float* dl1, const int
                            float* ft_b_grad, int n_ctas, cudaStream_t s_reduce, cudaEvent_t ev_reduce, int half_act, float grad_scale, unsigned long long* clamp_counter) {
     const int work_cols = mode == 1 ? F / 2 : F;
     const int max_units = sort_units(B);
-    int bias_rows = n_ctas;
-    if ((l1 == 8 || l1 == 16 || l1 == 32) && n_ctas >= 2 * max_units) {
+    int bias_rows = n_ctas, lane_rows = n_ctas;
+    // the blocks' own rows are the chains that are wanted; fp16 rows are rounded, so that smaller blocks keep theirs there
+    bool own_rows = true;
+    if (l1 == 8 || l1 == 16 || l1 == 32) {
         int n_chunks = 1;
         while (work_cols / n_chunks > 1024 || (work_cols / n_chunks) % 128 != 0 && (work_cols / n_chunks) > 256) n_chunks *= 2;
         const int CW = work_cols / n_chunks;
-        bias_rows = 2 * max_units;
-        dim3 grid(bias_rows, 2, n_chunks), block(CW / 4);
+        own_rows = half_act || unit_tiles(B) == TB_UNIT_TILES;
+        bias_rows = 2 * (own_rows ? max_units : sort_weight_units(B));
+        lane_rows = 2 * (max_tiles / TB_UNIT_TILES + TB_MAX_BUCKETS + 2);
+        dim3 grid(2 * max_units, 2, n_chunks), block(CW / 4);
         const size_t smem = (size_t)DG_STAGES * 4 * (mode == 1 ? 2 : 1) * (CW / 4) * (half_act ? 8 : 16);
 #define DGRAD_REG(M, L, H)                                                                                               \
     do {                                                                                                                 \
         cudaFuncSetAttribute(k_l1_dgrad_ftgrad_stream<M, L, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024); \
         k_l1_dgrad_ftgrad_stream<M, L, H><<<grid, block, smem, s>>>(dl1, order, tiles, tiles + max_tiles, n_tiles + 1, unit_tiles(B) / 2, wb, ws, pre_stm, \
                                                                     pre_nstm, ft_bias, scale, F, nb, CW, dft_stm, dft_nstm, \
-                                                                    bias_partials, grad_scale, clamp_counter);           \
+                                                                    own_rows ? bias_partials : nullptr, grad_scale, clamp_counter); \
     } while (0)
         if (half_act) {  // fp16 activations: LayerStack only
             if (mode != 1) return -1;
@@ -1641,6 +1695,10 @@ int launch_l1_dgrad_ftgrad(cudaStream_t s, int mode, const float* dl1, const int
         cudaEventRecord(ev_reduce, s);
         cudaStreamWaitEvent(s_reduce, ev_reduce, 0);
     }
-    k_bias_partials_reduce<<<ceil_div(F, 8), 256, 0, s_reduce>>>(bias_partials, bias_rows, F, ft_b_grad);
-    return 2;
+    if (!own_rows)
+        k_bias_partial_rows<<<dim3(bias_rows, 2, F / 128), 128, 0, s_reduce>>>(order, tiles, weight_units(tiles, max_tiles), n_tiles + 2,
+                                                                               static_cast<const float*>(dft_stm), static_cast<const float*>(dft_nstm), F,
+                                                                               bias_partials);
+    k_bias_partials_reduce<<<ceil_div(F, 8), 256, 0, s_reduce>>>(bias_partials, bias_rows, lane_rows, F, ft_b_grad);
+    return own_rows ? 2 : 3;
 }

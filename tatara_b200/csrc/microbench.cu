@@ -110,7 +110,7 @@ extern "C" int tb_ft_microbench(int device, const int32_t* indices, const int32_
         // raw lists (item sort, run plan, row codes; chunk inverse index for the backward)
         const int n_keys = ceil_div(ft_in, rps) + 1;
         MB(cudaMalloc(&d_order, B * 4)); MB(cudaMalloc(&d_ntiles, TB_TILE_COUNTS * 4)); MB(cudaMalloc(&d_seg, (TB_MAX_BUCKETS + 3) * 4));
-        MB(cudaMalloc(&d_tiles, ((size_t)max_tiles + sort_max_units(max_tiles)) * sizeof(TileDesc)));
+        MB(cudaMalloc(&d_tiles, sort_tiles_len(max_tiles) * sizeof(TileDesc)));
         MB(cudaMalloc(&d_hist, ((size_t)128 * (B / 1024 + 2) + (size_t)(TB_MAX_BUCKETS + 1) * (B / 1024 + 2)) * 4));
         MB(cudaMalloc(&d_items, B * 4)); MB(cudaMalloc(&d_itemseg, 130 * 4));
         MB(cudaMalloc(&d_fwd_work, ft_forward_slice_work_ints(batch, n_keys, max_active) * 4));

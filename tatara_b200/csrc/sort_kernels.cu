@@ -136,25 +136,25 @@ __global__ void __launch_bounds__(SORT_BLOCK) k_sort_scatter2(Fn0 f0, int n0, in
 // a step for the forward runs and 17 us for the chunks.)
 #define PLAN_THREADS 1024
 
-// tiles: runs of <= TB_TILE_M positions of one bucket; units: runs of <= ut tiles of one bucket
+// tiles: runs of <= TB_TILE_M positions of one bucket; units: runs of <= ut tiles of one bucket; weight units: of <= TB_UNIT_TILES
 static __device__ void plan_tiles(const int* __restrict__ s_seg, int K, int ut, TileDesc* __restrict__ tiles, int* __restrict__ n_tiles,
-                                  TileDesc* __restrict__ units, int* __restrict__ n_units) {
-    __shared__ int s_tile_base[TB_MAX_BUCKETS + 3], s_unit_base[TB_MAX_BUCKETS + 3];
+                                  TileDesc* __restrict__ units, TileDesc* __restrict__ wunits) {
+    __shared__ int s_tile_base[TB_MAX_BUCKETS + 3], s_unit_base[TB_MAX_BUCKETS + 3], s_wunit_base[TB_MAX_BUCKETS + 3];
     if (threadIdx.x == 0) {
-        int trun = 0, urun = 0;
-        for (int k = 0; k < K; ++k) {
+        int trun = 0, urun = 0, wrun = 0;
+        for (int k = 0; k <= K; ++k) {
             s_tile_base[k] = trun;
             s_unit_base[k] = urun;
-            n_tiles[2 + k] = urun;
+            s_wunit_base[k] = n_tiles[3 + k] = wrun;
+            if (k == K) break;
             const int nt = (s_seg[k + 1] - s_seg[k] + TB_TILE_M - 1) / TB_TILE_M;
             trun += nt;
             urun += (nt + ut - 1) / ut;
+            wrun += (nt + TB_UNIT_TILES - 1) / TB_UNIT_TILES;
         }
-        s_tile_base[K] = trun;
-        s_unit_base[K] = urun;
-        n_tiles[2 + K] = urun;
-        *n_tiles = trun;
-        *n_units = urun;
+        n_tiles[0] = trun;
+        n_tiles[1] = urun;
+        n_tiles[2] = wrun;
     }
     __syncthreads();
     for (int t = threadIdx.x; t < s_tile_base[K]; t += PLAN_THREADS) {
@@ -168,16 +168,20 @@ static __device__ void plan_tiles(const int* __restrict__ s_seg, int K, int ut, 
         d.pad = 0;
         tiles[t] = d;
     }
-    for (int u = threadIdx.x; u < s_unit_base[K]; u += PLAN_THREADS) {
-        int k = 0;
-        while (s_unit_base[k + 1] <= u) ++k;
-        TileDesc d;
-        d.start = s_tile_base[k] + (u - s_unit_base[k]) * ut;
-        d.count = min(ut, s_tile_base[k + 1] - d.start);
-        d.bucket = k;
-        d.pad = 0;
-        units[u] = d;
-    }
+    auto cut = [&](const int* base, int size, TileDesc* out) {
+        for (int u = threadIdx.x; u < base[K]; u += PLAN_THREADS) {
+            int k = 0;
+            while (base[k + 1] <= u) ++k;
+            TileDesc d;
+            d.start = s_tile_base[k] + (u - base[k]) * size;
+            d.count = min(size, s_tile_base[k + 1] - d.start);
+            d.bucket = k;
+            d.pad = 0;
+            out[u] = d;
+        }
+    };
+    cut(s_unit_base, ut, units);
+    cut(s_wunit_base, TB_UNIT_TILES, wunits);
 }
 
 // Runs of the slice-resident forward: <= SLICE_IPC consecutive slots of one slice, the largest first.  The blocks take
@@ -305,7 +309,7 @@ static __device__ void plan_backward(const int* __restrict__ s_seg, int n_keys, 
 }
 
 __global__ void __launch_bounds__(PLAN_THREADS) k_step_plans(const int* __restrict__ seg_start, int K0, int ut, TileDesc* __restrict__ tiles,
-                                                             int* __restrict__ n_tiles, TileDesc* __restrict__ units,
+                                                             int* __restrict__ n_tiles, TileDesc* __restrict__ units, TileDesc* __restrict__ wunits,
                                                              const int* __restrict__ item_seg, int n_keys, FwdWork* __restrict__ work,
                                                              int* __restrict__ n_work, int ch, int parts, FwdWork* __restrict__ chunks,
                                                              int* __restrict__ n_chunks, int* __restrict__ groups, int* __restrict__ sched) {
@@ -314,7 +318,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) k_step_plans(const int* __restri
     const int n = blockIdx.x == 0 ? K0 : n_keys;
     for (int k = threadIdx.x; k <= n; k += PLAN_THREADS) s_seg[k] = seg[k];
     __syncthreads();
-    if (blockIdx.x == 0) plan_tiles(s_seg, K0, ut, tiles, n_tiles, units, n_tiles + 1);
+    if (blockIdx.x == 0) plan_tiles(s_seg, K0, ut, tiles, n_tiles, units, wunits);
     else if (blockIdx.x == 1) plan_forward(s_seg, n_keys, work, n_work);
     else plan_backward(s_seg, n_keys, ch, parts, chunks, n_chunks, groups, sched);
 }
@@ -323,7 +327,8 @@ __global__ void __launch_bounds__(PLAN_THREADS) k_step_plans(const int* __restri
 // need no order: every warp owns a run of positions, counts its keys, and places them behind those of the warps before it.
 // (The four launches cost 21 to 24 us however small the batch.)
 __global__ void __launch_bounds__(1024) k_sort_one_block(BucketKey fn, int n, int K, int ut, int* __restrict__ order, int* __restrict__ seg_start,
-                                                         TileDesc* __restrict__ tiles, int* __restrict__ n_tiles, TileDesc* __restrict__ units) {
+                                                         TileDesc* __restrict__ tiles, int* __restrict__ n_tiles, TileDesc* __restrict__ units,
+                                                         TileDesc* __restrict__ wunits) {
     __shared__ int s_cnt[TB_MAX_BUCKETS + 1][32], s_seg[TB_MAX_BUCKETS + 3];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (w < K) s_cnt[w][lane] = 0;
@@ -367,7 +372,7 @@ __global__ void __launch_bounds__(1024) k_sort_one_block(BucketKey fn, int n, in
     if ((int)threadIdx.x <= K) seg_start[threadIdx.x] = s_seg[threadIdx.x];
     __syncthreads();
     walk(true);
-    plan_tiles(s_seg, K, ut, tiles, n_tiles, units, n_tiles + 1);
+    plan_tiles(s_seg, K, ut, tiles, n_tiles, units, wunits);
 }
 
 // The question k_fwd_codes answers for the device, asked as soon as the batch is there, for the host: the slice of an item
@@ -400,12 +405,16 @@ int launch_slice_check(cudaStream_t s, const int* idx_stm, const int* idx_nstm, 
     return 1;
 }
 
+int sort_weight_units(int n_pos) { return n_pos / (TB_UNIT_TILES * TB_TILE_M) + TB_MAX_BUCKETS + 2; }
 int sort_units(int n_pos) { return n_pos / (unit_tiles(n_pos) * TB_TILE_M) + TB_MAX_BUCKETS + 2; }
 // at least the 148 units of the largest batches with smaller ones
 int sort_max_units(int max_tiles) {
     const int n = max_tiles / TB_UNIT_TILES > 148 ? max_tiles / TB_UNIT_TILES : 148;
     return n + TB_MAX_BUCKETS + 2;
 }
+
+const TileDesc* weight_units(const TileDesc* tiles, int max_tiles) { return tiles + max_tiles + sort_max_units(max_tiles); }
+size_t sort_tiles_len(int max_tiles) { return (size_t)max_tiles + sort_max_units(max_tiles) + max_tiles / TB_UNIT_TILES + TB_MAX_BUCKETS + 2; }
 
 // Both sorts of a step in four launches: positions by bucket (order, tiles, units) and items by table slice, with the plans
 // of the slice-resident kernels where their work buffers are given; without `items` (B <= SORT_ONE_BLOCK) the positions alone,
@@ -421,7 +430,8 @@ int launch_step_sorts(cudaStream_t s, const int* bucket, int B, int nb, int* ord
     }
     const int K0 = nb + 1, G0 = ceil_div(B, SORT_BLOCK);
     if (!items) {
-        k_sort_one_block<<<1, 1024, 0, s>>>(BucketKey{bucket, nb}, B, K0, unit_tiles(B), order, seg_start, tiles, n_tiles, tiles + max_tiles);
+        k_sort_one_block<<<1, 1024, 0, s>>>(BucketKey{bucket, nb}, B, K0, unit_tiles(B), order, seg_start, tiles, n_tiles, tiles + max_tiles,
+                                             const_cast<TileDesc*>(weight_units(tiles, max_tiles)));
         return 1;
     }
     const int n1 = n_persp * B, K1 = n_slices + 1, G1 = ceil_div(n1, SORT_BLOCK);
@@ -442,7 +452,8 @@ int launch_step_sorts(cudaStream_t s, const int* bucket, int B, int nb, int* ord
         bp = bwd_pointers(bwd_work, L);
         ch = L.CH;
     }
-    k_step_plans<<<bwd_work ? 3 : fwd_work ? 2 : 1, PLAN_THREADS, 0, s>>>(seg_start, K0, unit_tiles(B), tiles, n_tiles, tiles + max_tiles, item_seg, K1,
+    k_step_plans<<<bwd_work ? 3 : fwd_work ? 2 : 1, PLAN_THREADS, 0, s>>>(seg_start, K0, unit_tiles(B), tiles, n_tiles, tiles + max_tiles,
+                                                                          const_cast<TileDesc*>(weight_units(tiles, max_tiles)), item_seg, K1,
                                                                           sb.work, sb.n_work, ch, bwd_parts, bp.chunks, bp.n_chunks,
                                                                           bp.groups, bp.sched);
     return 4;

@@ -1139,13 +1139,15 @@ int create_impl(tb_trainer* t) {
     t->max_tiles = (int)(B / TB_TILE_M) + TB_MAX_BUCKETS + 2;
     t->max_units = sort_max_units(t->max_tiles);
     CU(t, dalloc(&t->order, B)); CU(t, dalloc(&t->n_tiles, TB_TILE_COUNTS)); CU(t, dalloc(&t->seg_start, TB_MAX_BUCKETS + 3));
-    CU(t, dalloc(&t->tiles, (size_t)t->max_tiles + t->max_units));
+    CU(t, dalloc(&t->tiles, sort_tiles_len(t->max_tiles)));
     const size_t n_cells = ls ? (size_t)(l2 * t->l2in + 2 * l2 + 1 + l1) : (size_t)(l1 * l2 + 2 * l2 + 1 + l1);
     CU(t, dalloc(&t->small_partials, (ls ? (size_t)(nb + 1) * TB_RUNS_LS : (size_t)TB_RUNS_SIMPLE) * n_cells));  // one partial row per run
-    CU(t, dalloc(&t->l1w_partials, (size_t)t->max_units * l1 * t->K));
+    CU(t, dalloc(&t->l1w_partials, (size_t)sort_weight_units((int)B) * l1 * t->K));
     CU(t, dalloc(&t->l1_weff, (size_t)(nb + 1) * l1 * (t->K + 1)));  // effective L1 weights and biases per bucket
-    t->dgrad_rows = DGRAD_CTAS > 2 * t->max_units ? DGRAD_CTAS : 2 * t->max_units;  // partial FT bias rows: one per block
-    CU(t, dalloc(&t->bias_partials, (size_t)t->dgrad_rows * 2 * F));
+    // partial FT bias rows: one per block of the streaming kernel, or per block of the general one, whose number decides the order of its sums
+    const int order_rows = 2 * (t->max_tiles / TB_UNIT_TILES + TB_MAX_BUCKETS + 2);
+    t->dgrad_rows = DGRAD_CTAS > order_rows ? DGRAD_CTAS : order_rows;
+    CU(t, dalloc(&t->bias_partials, (size_t)(t->dgrad_rows > 2 * t->max_units ? t->dgrad_rows : 2 * t->max_units) * 2 * F));
     CU(t, dalloc(&t->feat_counts, inverse_index_counts_len((int)N))); CU(t, dalloc(&t->feat_offsets, (size_t)2 * N));
     // histograms of the item sort and of the bucket sort
     CU(t, dalloc(&t->sort_hist, (size_t)128 * (2 * B / 1024 + 2) + (size_t)(TB_MAX_BUCKETS + 1) * (B / 1024 + 2)));

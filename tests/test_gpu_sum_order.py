@@ -84,14 +84,15 @@ def _masked(x, up):
     return np.where((x > 0) & (x < 1), up, np.float32(0)).astype(np.float32)
 
 
-def _trainer(arch, B, F, l1, l2, act, seed, fs=LS_FS.with_factorize(False)):
+def _trainer(arch, B, F, l1, l2, act, seed, fs=LS_FS.with_factorize(False), capacity=None):
     rng = np.random.default_rng(seed)
+    cap = capacity or B
     if arch == "layerstack":
         init = _perturb(tb.layerstack_default_init(fs, F, l1, l2, 9), rng, ["ft_b", "l1_b", "l1_shared_bias", "l2_w", "l2_b", "l3_w", "l3_b"])
-        tr = tb.GpuTrainer(B, F, l1, l2, 9, fs, optimizer="adamw", init=dict(init, ft_w=init["ft_w"] * 30))
+        tr = tb.GpuTrainer(cap, F, l1, l2, 9, fs, optimizer="adamw", init=dict(init, ft_w=init["ft_w"] * 30))
     else:
         init = _perturb(tb.simple_default_init(fs, F, l1, l2, pairwise=act == "pairwise"), rng, ["ft_b", "l1_b", "l2_w", "l2_b", "l3_w", "l3_b"])
-        tr = tb.SimpleGpuTrainer(B, F, l1, l2, fs, activation=act, optimizer="adamw", init=dict(init, ft_w=init["ft_w"] * 30))
+        tr = tb.SimpleGpuTrainer(cap, F, l1, l2, fs, activation=act, optimizer="adamw", init=dict(init, ft_w=init["ft_w"] * 30))
     batch = tb.synthetic_batch(tb.SYNTH_SEED + seed, B, fs, with_bucket=arch == "layerstack")
     if arch == "layerstack":
         batch.bucket_idx[:] = np.where(rng.random(B) < 0.4, 3, rng.choice([0, 1, 8, 9, -1], B)).astype(np.int32)  # some empty, some out of range
@@ -184,3 +185,62 @@ def test_l1_forward_is_one_chain_over_the_inputs(arch, F, l1, B):
         at = order[beg:end][:: max(1, (end - beg) // 300)]  # some of every bucket
         want[at] = _chain(x[at].T[:, :, None], weff[g][:, None, :]) + beff[g]
         _same_bits(tr.read_buffer("l1_total", B * l1).reshape(B, l1)[at], want[at], "bucket %d" % g)
+
+
+@pytest.mark.parametrize("arch,F,l1,B", [
+    ("layerstack", 256, 8, 16), ("layerstack", 640, 8, 9488), ("layerstack", 256, 16, 1040), ("layerstack", 256, 16, 19008),
+    ("layerstack", 256, 32, 1040), ("simple", 256, 32, 1040), ("simple", 128, 8, 512), ("simple", 128, 16, 40016)])
+def test_l1_weight_gradient_is_chains_of_256_positions(arch, F, l1, B):
+    """Whatever the batch size: units of 256 positions of a bucket, the bucket's units in order, the buckets in order."""
+    tr, w, batch, _ = _trainer(arch, B, F, l1, 16, "crelu", B + l1)
+    ls = arch == "layerstack"
+    K = F if ls else 2 * F
+    cols = np.unique(np.linspace(0, K - 1, 37).astype(int))
+    x = tr.read_buffer("combined", B * K).reshape(B, K)[:, cols]
+    d = tr.read_buffer("dl1_total", B * l1).reshape(B, l1)
+    order, seg = _segments(batch, B, 9 if ls else 0)
+    total = np.zeros((len(cols), l1), np.float32)
+    got = tr.download_grad("l1_w").reshape(9, l1, K) if ls else None
+    for g, (beg, end) in enumerate(zip(seg[:-1], seg[1:])):
+        bucket = np.zeros_like(total)
+        for u in range(beg, end, 256):
+            at = order[u: min(u + 256, end)]
+            bucket += _chain(x[at][:, :, None], d[at][:, None, :])
+        if ls and g < 9:
+            _same_bits(got[g][:, cols].T, bucket, "bucket %d" % g)
+        total += bucket
+    shared = tr.download_grad("l1_shared_weight" if ls else "l1_w").reshape(K, l1)
+    _same_bits(shared[cols], total, "all positions")
+
+
+@pytest.mark.parametrize("arch,F,l1,B,capacity,act", [
+    ("layerstack", 256, 8, 16, 16, ""), ("layerstack", 256, 16, 1040, 1040, ""), ("layerstack", 384, 32, 9488, 9488, ""),
+    ("layerstack", 256, 16, 18960, 18960, ""), ("layerstack", 256, 16, 1040, 20000, ""),
+    ("simple", 128, 32, 1040, 1040, "crelu"), ("simple", 128, 16, 9488, 9488, "screlu"), ("simple", 128, 32, 18960, 30000, "screlu"),
+    ("layerstack", 256, 12, 1040, 1040, "")])
+def test_ft_bias_gradient_is_chains_of_128_positions(arch, F, l1, B, capacity, act):
+    """Whatever the batch size: half units of 128 positions, then a warp's lanes.  The general kernel (l1 = 12): tiles dealt to as
+    many chains as the trainer's capacity gives."""
+    tr, w, batch, _ = _trainer(arch, B, F, l1, 16, act, B + l1, capacity=capacity)
+    ls = arch == "layerstack"
+    dft = [tr.read_buffer(k, B * F).reshape(B, F) for k in ("dft_stm", "dft_nstm")]
+    order, seg = _segments(batch, B, 9 if ls else 0)
+    lane_rows = 2 * ((capacity // 32 + 11) // 8 + 11)
+    lanes = np.zeros((32, F), np.float32)
+    if l1 == 12:
+        lane_rows = max(296, lane_rows)
+        tiles = [order[b: min(b + 32, end)] for beg, end in zip(seg[:-1], seg[1:]) for b in range(beg, end, 32)]
+        chains = [np.concatenate([t for t in tiles[r::lane_rows]] or [[]]).astype(int) for r in range(lane_rows)]
+    else:
+        chains = []
+        for beg, end in zip(seg[:-1], seg[1:]):
+            for u in range(beg, end, 256):
+                unit = order[u: min(u + 256, end)]
+                chains += [unit[:128], unit[128:]]
+    for p in range(2):
+        for r, at in enumerate(chains):
+            row = np.zeros(F, np.float32)
+            for b in at:
+                row += dft[p][b]
+            lanes[(p * lane_rows + r) % 32] += row
+    _same_bits(tr.download_grad("ft_b"), _halves(lanes), "ft_b")
