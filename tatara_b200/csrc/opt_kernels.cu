@@ -11,11 +11,11 @@ template <bool HS>
 __global__ void __launch_bounds__(256) k_radam(float4* __restrict__ w, void* __restrict__ m, void* __restrict__ v,
                                                 const float4* __restrict__ g, float4* __restrict__ slow, uint2* __restrict__ mirror,
                                                 long long n4, OptScalars sc) {
-    const float rate = sc.lr * sc.step_size;
-    const float decay_mul = 1.0f - sc.decay * rate;
+    const float rate = radam_rate(sc);
+    const float decay_mul = radam_decay(sc, rate);
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
         float4 mi = load_moment<HS>(m, i, 1.0f / TB_FT_OPT_M_SCALE, false), vi = load_moment<HS>(v, i, 1.0f / TB_FT_OPT_V_SCALE, false);
-        float4 p = radam_four(w[i], mi, vi, scale4(g[i], sc.grad_scale), sc, rate, decay_mul);
+        float4 p = radam_four<RADAM_TABLE>(w[i], mi, vi, scale4(g[i], sc.grad_scale), sc, rate, decay_mul);
         store_moment<HS>(m, i, mi, TB_FT_OPT_M_SCALE, true, false);
         store_moment<HS>(v, i, vi, TB_FT_OPT_V_SCALE, false, false);
         if (sc.lerp) {
@@ -49,11 +49,11 @@ __global__ void __launch_bounds__(256) k_radam_small(const __grid_constant__ Sma
     sc.decay = gr.decay;
     sc.min_w = gr.min_w;
     sc.max_w = gr.max_w;
-    const float rate = sc.lr * sc.step_size;
-    const float decay_mul = 1.0f - sc.decay * rate;
+    const float rate = radam_rate(sc);
+    const float decay_mul = radam_decay(sc, rate);
     for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < gr.n; i += gridDim.y * blockDim.x) {
         float mi = gr.m[i], vi = gr.v[i];
-        float p = radam_one(gr.w[i], mi, vi, gr.grad[i], sc, rate, decay_mul);
+        float p = radam_one<RADAM_SMALL>(gr.w[i], mi, vi, gr.grad[i], sc, rate, decay_mul);
         gr.m[i] = mi;
         gr.v[i] = vi;
         if (sc.lerp) {
@@ -72,6 +72,14 @@ int launch_radam_small(cudaStream_t s, const SmallGroups& groups, int max_n, Opt
     return 1;
 }
 
+// asynchronous copy of 8 or 16 bytes global -> shared (both aligned to that)
+template <int BYTES>
+static __device__ __forceinline__ void ok_cp(void* dst_shared, const void* src) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst_shared);
+    if (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+}
+
 // ------------------------------------------------------------------------------------------------
 // Factorised FT table (N = KB * pi real rows + pi virtual rows).  A block owns 32 adjacent float4 columns of one virtual row
 // vr, its warps share that row's KB real rows kb*pi + vr, up to FACT_ROWS neighbours each:
@@ -87,14 +95,6 @@ int launch_radam_small(cudaStream_t s, const SmallGroups& groups, int max_n, Opt
 // the measured HBM rate at 1536); fp16 moments and table at 1536: 566, now 499.  (Rows in registers: 667.  No folded table,
 // the forward adding the two rows as it loads a strip: 566 here, but 190 more there.  Every warp adding up its own rows and
 // the warps' sums after that: 637 / 325 / 122 and 492, another order.  The chain by a warp that reads the rows itself: 970.)
-// asynchronous copy of 8 or 16 bytes global -> shared (both aligned to that)
-template <int BYTES>
-static __device__ __forceinline__ void ok_cp(void* dst_shared, const void* src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst_shared);
-    if (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-    else asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
-}
-
 #define FACT_ROWS 9   // rows of a warp: 45 and 81 king buckets are 5 and 9 full warps
 #define FACT_BATCH 3  // of these, loaded together
 // HS: fp16 moments; HC: fp16 folded table.  The real rows' gradients are multiplied by sc.grad_scale on load; the virtual
@@ -112,8 +112,8 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, MIN_BLOCKS) k_radam_factorized
     const size_t cell = (size_t)blockIdx.x * 32 + lane;  // a row is a multiple of 32 float4 long
     const int KB = N / pi;
     const int kb0 = warp * FACT_ROWS;
-    const float rate = sc.lr * sc.step_size;
-    const float decay_mul = 1.0f - sc.decay * rate;
+    const float rate = radam_rate(sc);
+    const float decay_mul = radam_decay(sc, rate);
 #pragma unroll
     for (int u = 0; u < FACT_ROWS; ++u)
         if (kb0 + u < KB) ok_cp<16>(&s_row[u][threadIdx.x], g + (size_t)(kb0 + u) * plane + cell);
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, MIN_BLOCKS) k_radam_factorized
         const float4 gsum = s_virt[lane];
         g[iv] = gsum;
         float4 mv = load_moment<HS>(s_vm, lane, inv_ms, false), vv = load_moment<HS>(s_vv, lane, inv_vs, false);
-        float4 pv = radam_four(s_vw[lane], mv, vv, gsum, sc, rate, decay_mul);
+        float4 pv = radam_four<RADAM_FACT, RADAM_FACT_LAST>(s_vw[lane], mv, vv, gsum, sc, rate, decay_mul);
         store_moment<HS>(m, iv, mv, TB_FT_OPT_M_SCALE, true, false);
         store_moment<HS>(v, iv, vv, TB_FT_OPT_V_SCALE, false, false);
         if (sc.lerp) {
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, MIN_BLOCKS) k_radam_factorized
             const size_t i = (size_t)(kb0 + b + u) * plane + cell;
             float4 gi = s_row[b + u][threadIdx.x];
             if (HC) gi = scale4(gi, sc.grad_scale);
-            float4 q = radam_four(p[u], mi[u], vi[u], gi, sc, rate, decay_mul);
+            float4 q = radam_four<RADAM_FACT>(p[u], mi[u], vi[u], gi, sc, rate, decay_mul);
             store_moment<HS>(m, i, mi[u], TB_FT_OPT_M_SCALE, true, true);
             store_moment<HS>(v, i, vi[u], TB_FT_OPT_V_SCALE, false, true);
             if (sc.lerp) {
@@ -211,8 +211,8 @@ __global__ void __launch_bounds__(1024) k_radam_factorized_rows(float4* __restri
                                                                  int row4, int kb0, int kb1, OptScalars sc) {
     const int vr = blockIdx.x;
     const int c = threadIdx.x;
-    const float rate = sc.lr * sc.step_size;
-    const float decay_mul = 1.0f - sc.decay * rate;
+    const float rate = radam_rate(sc);
+    const float decay_mul = radam_decay(sc, rate);
     const float inv_ms = 1.0f / TB_FT_OPT_M_SCALE, inv_vs = 1.0f / TB_FT_OPT_V_SCALE;
     const size_t iv = (size_t)(N + vr) * row4 + c;
     float4 gsum = kb0 == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : g[iv];
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(1024) k_radam_factorized_rows(float4* __restri
         float4 gi = __ldcs(g + i);
         if (GS) gi = scale4(gi, sc.grad_scale);
         float4 mi = load_moment<HS>(m, i, inv_ms, true), vi = load_moment<HS>(v, i, inv_vs, true);
-        float4 p = radam_four(w[i], mi, vi, gi, sc, rate, decay_mul);
+        float4 p = radam_four<RADAM_FACT>(w[i], mi, vi, gi, sc, rate, decay_mul);
         store_moment<HS>(m, i, mi, TB_FT_OPT_M_SCALE, true, true);
         store_moment<HS>(v, i, vi, TB_FT_OPT_V_SCALE, false, true);
         if (sc.lerp) {
@@ -241,12 +241,12 @@ __global__ void __launch_bounds__(1024) k_radam_factorized_fold(float4* __restri
                                                                  void* __restrict__ comb, int N, int pi, int row4, OptScalars sc) {
     const int vr = blockIdx.x;
     const int c = threadIdx.x;
-    const float rate = sc.lr * sc.step_size;
-    const float decay_mul = 1.0f - sc.decay * rate;
+    const float rate = radam_rate(sc);
+    const float decay_mul = radam_decay(sc, rate);
     const int KB = N / pi;
     const size_t iv = (size_t)(N + vr) * row4 + c;
     float4 mv = load_moment<HS>(m, iv, 1.0f / TB_FT_OPT_M_SCALE, false), vv = load_moment<HS>(v, iv, 1.0f / TB_FT_OPT_V_SCALE, false);
-    float4 pv = radam_four(w[iv], mv, vv, g[iv], sc, rate, decay_mul);
+    float4 pv = radam_four<RADAM_FACT, RADAM_FACT_LAST>(w[iv], mv, vv, g[iv], sc, rate, decay_mul);
     store_moment<HS>(m, iv, mv, TB_FT_OPT_M_SCALE, true, false);
     store_moment<HS>(v, iv, vv, TB_FT_OPT_V_SCALE, false, false);
     if (sc.lerp) {

@@ -45,28 +45,49 @@ static __device__ __forceinline__ void store_moment(void* base, size_t i4, float
 }
 static __device__ __forceinline__ float4 scale4(float4 g, float k) { return make_float4(g.x * k, g.y * k, g.z * k, g.w * k); }
 
+// Of a sum of two products one is rounded before it is added.  Which one is part of the results (AdamW's first steps turn a last bit
+// into a visible difference after a few steps), so it is written out for every kernel and not left to the compiler, which chose
+// by what stood around the call.  The forms are those of the first kernels as they were compiled.
+//   moments, RADAM_OLD_FUSED: fma(beta, old, rounded new term), else fma(new factor, gradient, rounded beta * old)
+//   weights, RADAM_STEP_FUSED: p * decay rounded, then fma(-rate, value, .), else fma(p, decay, -rounded rate * value);
+//   RADAM_STEP_DENOM: the former where the value is divided by the root of the second moment, RADAM_STEP_LERP: on look-ahead steps
+enum { RADAM_OLD_FUSED = 1, RADAM_STEP_FUSED = 2, RADAM_STEP_DENOM = 4, RADAM_STEP_LERP = 8 };
+enum {
+    RADAM_SMALL = RADAM_OLD_FUSED | RADAM_STEP_DENOM,  // the small groups
+    RADAM_TABLE = RADAM_OLD_FUSED | RADAM_STEP_LERP,   // the FT table without a factorizer
+    RADAM_FACT = 0,                                    // with one
+    RADAM_FACT_LAST = RADAM_STEP_FUSED                 // with one: of a virtual row every fourth column
+};
+
+static __device__ __forceinline__ float radam_rate(const OptScalars& sc) { return __fmul_rn(sc.lr, sc.step_size); }
+static __device__ __forceinline__ float radam_decay(const OptScalars& sc, float rate) { return __fmaf_rn(-sc.decay, rate, 1.0f); }
+
+template <int FORM>
 static __device__ __forceinline__ float radam_one(float p, float& m, float& v, float g, const OptScalars& sc, float rate,
                                                    float decay_mul) {
-    p *= decay_mul;
-    const float mi = sc.beta1 * m + (1.0f - sc.beta1) * g;
-    const float vi = sc.beta2 * v + (1.0f - sc.beta2) * g * g;
+    const float gm = 1.0f - sc.beta1, gv = __fmul_rn(1.0f - sc.beta2, g);
+    const float mi = (FORM & RADAM_OLD_FUSED) ? __fmaf_rn(sc.beta1, m, __fmul_rn(gm, g)) : __fmaf_rn(gm, g, __fmul_rn(sc.beta1, m));
+    const float vi = (FORM & RADAM_OLD_FUSED) ? __fmaf_rn(sc.beta2, v, __fmul_rn(gv, g)) : __fmaf_rn(gv, g, __fmul_rn(sc.beta2, v));
     m = mi;
     v = vi;
     float val = mi;
-    if (sc.denom != 0) val /= sqrtf(vi) + sc.eps;
-    p -= rate * val;
+    if (sc.denom != 0) val = __fdiv_rn(val, __fadd_rn(__fsqrt_rn(vi), sc.eps));
+    const bool step_fused = (FORM & RADAM_STEP_FUSED) || ((FORM & RADAM_STEP_DENOM) && sc.denom != 0) || ((FORM & RADAM_STEP_LERP) && sc.lerp != 0);
+    p = step_fused ? __fmaf_rn(-rate, val, __fmul_rn(p, decay_mul)) : __fmaf_rn(p, decay_mul, -__fmul_rn(rate, val));
     p = p < sc.min_w ? sc.min_w : p;
     p = p > sc.max_w ? sc.max_w : p;
     return p;
 }
 
+// FORM of the first three, LAST of the fourth
+template <int FORM, int LAST = FORM>
 static __device__ __forceinline__ float4 radam_four(float4 p, float4& m, float4& v, float4 g, const OptScalars& sc,
                                                      float rate, float decay_mul) {
     float4 r;
-    r.x = radam_one(p.x, m.x, v.x, g.x, sc, rate, decay_mul);
-    r.y = radam_one(p.y, m.y, v.y, g.y, sc, rate, decay_mul);
-    r.z = radam_one(p.z, m.z, v.z, g.z, sc, rate, decay_mul);
-    r.w = radam_one(p.w, m.w, v.w, g.w, sc, rate, decay_mul);
+    r.x = radam_one<FORM>(p.x, m.x, v.x, g.x, sc, rate, decay_mul);
+    r.y = radam_one<FORM>(p.y, m.y, v.y, g.y, sc, rate, decay_mul);
+    r.z = radam_one<FORM>(p.z, m.z, v.z, g.z, sc, rate, decay_mul);
+    r.w = radam_one<LAST>(p.w, m.w, v.w, g.w, sc, rate, decay_mul);
     return r;
 }
 

@@ -209,7 +209,9 @@ __global__ void __launch_bounds__(T) k_tail(const float* __restrict__ l1_rows, c
                 if (ARCH != 0) dv[e] = tail_act_grad<ARCH>(in[i], dp[i]);
                 else if (i < L1E) {
                     const float ds = tail_act_grad<0>(in[i], dp[i]), dm = tail_act_grad<0>(in[L1E + i], dp[L1E + i]);
-                    dv[e] = dm + 2.0f * xv[e] * L1_SQR_SCALE * ds;
+                    // which of the two products is rounded first: as in L3, l1 = 32 has its own form
+                    const float k = __fmul_rn(__fmul_rn(2.0f, xv[e]), L1_SQR_SCALE);
+                    dv[e] = L1 <= 16 ? __fadd_rn(dm, __fmul_rn(k, ds)) : __fmaf_rn(k, ds, dm);
                 } else dv[e] = dy;
             }
             const float4 v = make_float4(dv[0], dv[1], dv[2], dv[3]);

@@ -1,6 +1,8 @@
 """The order in which fp32 sums are added up.  It is part of what a step returns: AdamW's first steps are normalised and not
 bias-corrected, so two correct orders can leave states that differ in the first digits after a few steps.  Every sum is added
 up again here, term by term in the stated order, and has to come out bit for bit."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -144,6 +146,16 @@ def test_small_layers(arch, l1, l2, B, act):
     _same_bits(tr.read_buffer("net_output", B), out, "net output")
     up = dy[:, None] * w3
     u = _masked(a2, up) if act != "screlu" else up * _masked(a2, 2 * a2)
+    d2 = np.where(live[:, None], u, np.float32(0))
+    dv = _chain(d2.T[:, :, None], np.moveaxis(w2, 1, 0))
+    if ls:  # the squared and the plain half of L2's inputs meet again
+        ds, dm = _masked(v[:, : l1 - 1], dv[:, : l1 - 1]), _masked(v[:, l1 - 1:], dv[:, l1 - 1:])
+        k = (np.float32(2) * m) * np.float32(127.0 / 128.0)
+        dm = _fma(k, ds, dm) if l1 == 32 else dm + k * ds
+        _same_bits(dl1, np.concatenate([dm, dy[:, None]], 1), "dl1")
+    else:
+        a = _crelu(x)
+        _same_bits(dl1, _masked(a, dv) if act != "screlu" else dv * _masked(a, 2 * a), "dl1")
     u, act2 = np.where(live[:, None], u, np.float32(0)), np.where(live[:, None], act2, np.float32(0))
     real = slice(0, 9 if ls else 1)
     split = 64 if ls else 128
@@ -244,3 +256,62 @@ def test_ft_bias_gradient_is_chains_of_128_positions(arch, F, l1, B, capacity, a
                 row += dft[p][b]
             lanes[(p * lane_rows + r) % 32] += row
     _same_bits(tr.download_grad("ft_b"), _halves(lanes), "ft_b")
+
+
+def _scalars(optimizer, step):
+    """Step size, whether the value is divided by the root of the second moment, beta1 (pointwise/radam_step.rs:63-86)."""
+    libm = C.CDLL("libm.so.6")
+    libm.powf.restype, libm.powf.argtypes = C.c_float, [C.c_float, C.c_float]
+    f = np.float32
+    b1, b2, t = f(0.99 if optimizer == "ranger" else 0.9), f(0.999), f(step)
+    if optimizer == "adamw":
+        return f(1), True, b1
+    b2t, top = f(libm.powf(b2, t)), f(2) / (f(1) - b2) - f(1)
+    n, bc = top - f(2) * t * b2t / (f(1) - b2t), f(1) - f(libm.powf(b1, t))
+    if not n > 5:
+        return f(1) / bc, False, b1
+    return np.sqrt((f(1) - b2t) * ((n - f(4)) / (top - f(4))) * ((n - f(2)) / n) * (top / (top - f(2)))) / bc, True, b1
+
+
+@pytest.mark.parametrize("factorize", [False, True])
+@pytest.mark.parametrize("optimizer", ["adamw", "radam", "ranger"])
+def test_update_rounds_the_same_products(optimizer, factorize):
+    """Which of two products is rounded before they are added, for every kernel and step: small groups, a plain table, a factorized
+    one with its virtual rows; before and after the second moment counts (step 6), on the look-ahead (6) and beside it."""
+    f = np.float32
+    fs = tb.FeatureSetSpec("test", 4, 10, 40, 8, factorize)
+    F, l1, l2, B, lr = 256, 8, 16, 256, 1e-3
+    rng = np.random.default_rng(7)
+    init = _perturb(tb.layerstack_default_init(fs, F, l1, l2, 9), rng, ["ft_w", "ft_b", "l1_b", "l1_shared_bias", "l2_b", "l3_b"])
+    d = random_index_batch(rng, B, fs.max_active, fs.piece_inputs, 1, fs.max_active)
+    for key in ("stm", "nstm"):
+        d[key] = np.where(d[key] >= 0, d[key] + rng.integers(0, 10, B)[:, None] * fs.piece_inputs, d[key]).astype(np.int32)
+    tr = tb.GpuTrainer(B, F, l1, l2, 9, fs, optimizer=optimizer, init=init)
+    batch = tb.BatchData(d["stm"], d["nstm"], d["nnz"], d["score"], d["wdl"], d["bucket"])
+    for step in range(1, 9):
+        before = {g: tr.download_group(g, ("w", "m", "v", "slow")) for g in tr.group_names}
+        tr.train_step(batch, lr, 0.0, tb.LossKind.sigmoid())
+        size, denom, b1 = _scalars(optimizer, step)
+        lerp = optimizer == "ranger" and step % 6 == 0
+        rate, b2 = f(lr) * size, f(0.999)
+        decay = _fma(-f(0.01), rate, f(1))
+        for name in tr.group_names:
+            old, new, g = before[name], tr.download_group(name, ("w", "m", "v", "slow")), tr.download_grad(name)
+            gm, gv = f(1) - b1, (f(1) - b2) * g
+            table = name == "ft_w"
+            if table and factorize:
+                m, v = _fma(gm, g, b1 * old["m"]), _fma(gv, g, b2 * old["v"])
+            else:
+                m, v = _fma(b1, old["m"], gm * g), _fma(b2, old["v"], gv * g)
+            _same_bits(new["m"], m, "%s m, step %d" % (name, step))
+            _same_bits(new["v"], v, "%s v, step %d" % (name, step))
+            val = m / (np.sqrt(v) + f(1e-8)) if denom else m
+            fused = np.full(g.size, lerp if table and not factorize else denom and not table)
+            if table and factorize:
+                fused[fs.ft_in * F + 3:: 4] = True
+            w = np.where(fused, _fma(-rate, val, old["w"] * decay), _fma(old["w"], decay, -(rate * val)))
+            if not table:
+                w = np.clip(w, -f(127.0 / 64.0), f(127.0 / 64.0)) if name in ("l1_w", "l1_shared_weight", "l2_w", "l3_w") else w
+            if lerp:
+                w = f(0.5) * w + f(0.5) * old["slow"]
+            _same_bits(new["w"], w, "%s w, step %d" % (name, step))
