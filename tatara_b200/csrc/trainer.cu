@@ -259,7 +259,7 @@ int nccl_host_allgather(void* ctx, const void* send, void* recv, size_t bytes) {
     unsigned char *ds = nullptr, *dr = nullptr;
     int rc = -1;
     if (cudaMalloc((void**)&ds, bytes) == cudaSuccess && cudaMalloc((void**)&dr, bytes * t->cfg.world_size) == cudaSuccess &&
-        cudaMemcpy(ds, send, bytes, cudaMemcpyHostToDevice) == cudaSuccess &&
+        cudaMemcpy(ds, send, bytes, cudaMemcpyHostToDevice) == cudaSuccess && cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess &&
         g_nccl.AllGather(ds, dr, bytes, /*ncclUint8*/ 1, t->comm, t->stream) == 0 && cudaStreamSynchronize(t->stream) == cudaSuccess &&
         cudaMemcpy(recv, dr, bytes * t->cfg.world_size, cudaMemcpyDeviceToHost) == cudaSuccess)
         rc = 0;
@@ -1343,6 +1343,9 @@ int tb_upload_group(tb_trainer* t, const char* name, const float* w, const float
         if (v) CU(t, cudaMemcpy(g->v, v, bytes, cudaMemcpyHostToDevice));
     }
     if (slow && t->cfg.optimizer == TB_OPT_RANGER) CU(t, cudaMemcpy(g->slow, slow, bytes, cudaMemcpyHostToDevice));
+    // cudaMemcpy from pageable memory may return before the last piece is on the device, and the trainer's streams do not wait for
+    // the default one
+    CU(t, cudaStreamSynchronize(cudaStreamLegacy));
     if (w && ft && (t->cfg.ft_factorize || t->p_ft16)) {
         // sync_ft_forward_weights: the table the forward reads follows the master weights (fold, and / or fp16 cast)
         if (t->cfg.ft_factorize)
