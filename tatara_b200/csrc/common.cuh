@@ -195,7 +195,7 @@ int launch_tail_simple(cudaStream_t s, const float* l1_pre, const float* score, 
 // gradients; arch 0 LayerStack, 1 Simple CReLU, 2 Simple SCReLU.  A block per run: partials [tail_blocks][cells],
 // loss_partials [tail_blocks], summed by launch_reduce_double.
 bool tail_tiled(int l1, int l2);
-int tail_blocks(int arch, int nb);
+int tail_blocks(int arch, int nb, int n_pos, int backward);
 int launch_tail(cudaStream_t s, int arch, int n_pos, const float* l1_rows, const int* order, const int* seg_start, const float* score,
                 const float* wdl, const float* l2_w, const float* l2_b, const float* l3_w, const float* l3_b, LossParams lp, int l1, int l2,
                 int nb, float* net_output, float* dy, float* dl1, float* partials, double* loss_partials, int backward);

@@ -309,12 +309,17 @@ __global__ void __launch_bounds__(256) k_tail_wgrad_final(const float* __restric
 }
 
 bool tail_tiled(int l1, int l2) { return (l1 == 8 || l1 == 16 || l1 == 32) && (l2 == 16 || l2 == 32); }
-int tail_blocks(int arch, int nb) { return arch == 0 ? (nb + 1) * TB_RUNS_LS : TB_RUNS_SIMPLE; }
+// Without the weight gradients the runs are no more than blocks of a launch: a batch of a few positions gets fewer.
+static int tail_runs(int arch, int n_pos, int backward) {
+    const int runs = arch == 0 ? TB_RUNS_LS : TB_RUNS_SIMPLE;
+    return backward || n_pos >= 64 * runs ? runs : n_pos < 64 ? 1 : n_pos / 64;
+}
+int tail_blocks(int arch, int nb, int n_pos, int backward) { return (arch == 0 ? nb + 1 : 1) * tail_runs(arch, n_pos, backward); }
 
 int launch_tail(cudaStream_t s, int arch, int n_pos, const float* l1_rows, const int* order, const int* seg_start, const float* score,
                 const float* wdl, const float* l2_w, const float* l2_b, const float* l3_w, const float* l3_b, LossParams lp, int l1, int l2,
                 int nb, float* net_output, float* dy, float* dl1, float* partials, double* loss_partials, int backward) {
-    const int blocks = tail_blocks(arch, nb), split = arch == 0 ? TB_RUNS_LS : TB_RUNS_SIMPLE;
+    const int blocks = tail_blocks(arch, nb, n_pos, backward), split = tail_runs(arch, n_pos, backward);
 #define TAIL_LAUNCH(A, L1, L2, T)                                                                                                 \
     do {                                                                                                                          \
         typedef TailShape<A, L1, L2, T> S;                                                                                        \

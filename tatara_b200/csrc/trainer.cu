@@ -551,7 +551,7 @@ int run_forward(tb_trainer* t, const DevBatch& d, const tb_loss* loss, float lam
         // in a training step nothing but the loss read-back waits for the sum
         const cudaStream_t sl = backward ? side_stream(t, 1) : t->stream;
         AFTER(t->ev_tail, t->stream, sl);
-        n += launch_reduce_double(sl, t->loss_partials, tail_blocks(tail_arch(c), ls ? c.num_buckets : 0), t->loss_acc);
+        n += launch_reduce_double(sl, t->loss_partials, tail_blocks(tail_arch(c), ls ? c.num_buckets : 0, B, backward), t->loss_acc);
         p.done(n);
     }
     return TB_OK;
