@@ -1652,15 +1652,22 @@ int launch_l1_dgrad_ftgrad(cudaStream_t s, int mode, const float* dl1, const int
         int n_chunks = 1;
         while (work_cols / n_chunks > 1024 || (work_cols / n_chunks) % 128 != 0 && (work_cols / n_chunks) > 256) n_chunks *= 2;
         const int CW = work_cols / n_chunks;
-        own_rows = half_act || unit_tiles(B) == TB_UNIT_TILES;
-        bias_rows = 2 * (own_rows ? max_units : sort_weight_units(B));
+        // Blocks of DG_POS positions, whose partial rows are the chains, for full batches; for smaller ones where the dft rows are
+        // more than stays in L2, so that reading them again costs more than the shorter blocks save (step, us, short / long
+        // blocks: 12 000 positions F = 1536 1580 / 1504; 10 000 F = 768 810 / 818; 4096 F = 512 495 / 512; 1024 F = 256 243 / 268).
+        const bool wide = unit_tiles(B) == TB_UNIT_TILES || (!half_act && 8ll * B * F > 96ll << 20);
+        own_rows = half_act || wide;
+        const int grid_rows = 2 * (wide ? sort_weight_units(B) : max_units);
+        const TileDesc* u = wide ? weight_units(tiles, max_tiles) : tiles + max_tiles;
+        const int *n_u = n_tiles + (wide ? 2 : 1), half_tiles = (wide ? TB_UNIT_TILES : unit_tiles(B)) / 2;
+        bias_rows = own_rows ? grid_rows : 2 * sort_weight_units(B);
         lane_rows = 2 * (max_tiles / TB_UNIT_TILES + TB_MAX_BUCKETS + 2);
-        dim3 grid(2 * max_units, 2, n_chunks), block(CW / 4);
+        dim3 grid(grid_rows, 2, n_chunks), block(CW / 4);
         const size_t smem = (size_t)DG_STAGES * 4 * (mode == 1 ? 2 : 1) * (CW / 4) * (half_act ? 8 : 16);
 #define DGRAD_REG(M, L, H)                                                                                               \
     do {                                                                                                                 \
         cudaFuncSetAttribute(k_l1_dgrad_ftgrad_stream<M, L, H>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024); \
-        k_l1_dgrad_ftgrad_stream<M, L, H><<<grid, block, smem, s>>>(dl1, order, tiles, tiles + max_tiles, n_tiles + 1, unit_tiles(B) / 2, wb, ws, pre_stm, \
+        k_l1_dgrad_ftgrad_stream<M, L, H><<<grid, block, smem, s>>>(dl1, order, tiles, u, n_u, half_tiles, wb, ws, pre_stm, \
                                                                     pre_nstm, ft_bias, scale, F, nb, CW, dft_stm, dft_nstm, \
                                                                     own_rows ? bias_partials : nullptr, grad_scale, clamp_counter); \
     } while (0)

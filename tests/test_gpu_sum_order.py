@@ -229,6 +229,7 @@ def test_l1_weight_gradient_is_chains_of_256_positions(arch, F, l1, B):
     ("layerstack", 256, 8, 16, 16, ""), ("layerstack", 256, 16, 1040, 1040, ""), ("layerstack", 384, 32, 9488, 9488, ""),
     ("layerstack", 256, 16, 18960, 18960, ""), ("layerstack", 256, 16, 1040, 20000, ""),
     ("simple", 128, 32, 1040, 1040, "crelu"), ("simple", 128, 16, 9488, 9488, "screlu"), ("simple", 128, 32, 18960, 30000, "screlu"),
+    ("layerstack", 1408, 8, 9488, 9488, ""),  # more dft rows than stay in L2
     ("layerstack", 256, 12, 1040, 1040, "")])
 def test_ft_bias_gradient_is_chains_of_128_positions(arch, F, l1, B, capacity, act):
     """Whatever the batch size: half units of 128 positions, then a warp's lanes.  The general kernel (l1 = 12): tiles dealt to as
