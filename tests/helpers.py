@@ -54,3 +54,15 @@ def random_index_batch(rng, B, A, N, nnz_lo, nnz_hi, with_bucket=9, pad=-1):
     if with_bucket:
         out["bucket"] = rng.integers(0, with_bucket, B).astype(np.int32)
     return out
+
+
+def ft_path(tr, batch, loss):
+    """Which FT weight gradient kernels a batch takes: "slices", "gather", or "both" (a large batch with a row outside its slice).
+    Told by the launches of the two phases; the forward and backward pass is run once more for it."""
+    tr.profile_enable(True)
+    tr.profile_reset()
+    tr.forward_backward(batch, 0.0, loss)
+    phases = tr.profile_read()
+    tr.profile_enable(False)
+    launches = (phases["ft_forward"][1], phases["inverse_index"][1], phases["ft_backward"][1])
+    return {(1, 4, 1): "gather", (2, 1, 2): "slices", (2, 5, 3): "both"}[launches]

@@ -21,7 +21,7 @@ import pytest
 import oracle_lib as O
 import ref_kernels as R
 import tatara_b200 as tb
-from helpers import assert_close, assert_close_scaled
+from helpers import assert_close, assert_close_scaled, ft_path
 from ref_kernels import F32, I32, U32, U64, Slice
 
 pytestmark = pytest.mark.gpu
@@ -123,7 +123,10 @@ def _check_step(tr, ot, batch, B, F, l1, mask, fs):
 @pytest.mark.parametrize("mask,factorize,F,l1,B", [
     (FT16, True, 256, 16, 512), (FT16 | OUT16, True, 256, 16, 512), (STATE16, True, 256, 16, 256),
     (FT16 | OUT16 | STATE16, True, 768, 8, 256), (FT16 | OUT16 | STATE16, False, 512, 32, 496), (FT16, False, 256, 16, 256),
-    (ALL_OPTIM, True, 256, 16, 512)])
+    (ALL_OPTIM, True, 256, 16, 512),
+    # large enough for the slice-resident FT kernels
+    (FT16, True, 256, 16, 3680), (FT16 | OUT16, False, 256, 8, 3680), (STATE16, True, 256, 16, 3680), (FT16 | OUT16 | STATE16, True, 384, 32, 3680),
+    (ALL_OPTIM, False, 256, 16, 3680)])
 def test_reduced_precision_step_matches_oracle(mask, factorize, F, l1, B):
     fs = LS_FS.with_factorize(factorize)
     rng = np.random.default_rng(F + B + mask)
@@ -132,13 +135,15 @@ def test_reduced_precision_step_matches_oracle(mask, factorize, F, l1, B):
     batch = tb.synthetic_batch(tb.SYNTH_SEED + 3, B, fs)
     batch.bucket_idx[::19] = 9       # rows with an out-of-range bucket
     _check_step(tr, ot, batch, B, F, l1, mask, fs)
+    assert ft_path(tr, batch, tb.LossKind.sigmoid()) == ("slices" if B > 3665 else "gather")
     tr.close()
 
 
-def test_reduced_precision_with_index_lists_outside_the_king_slices():
+@pytest.mark.parametrize("B", [128, 3680])
+def test_reduced_precision_with_index_lists_outside_the_king_slices(B):
     """Arbitrary index lists break the king-slice property: the generic fp16 kernels take over (same results)."""
     from helpers import random_index_batch
-    F, l1, B = 256, 16, 128
+    F, l1 = 256, 16
     fs = LS_FS.with_factorize(False)
     rng = np.random.default_rng(3)
     init = _init(fs, F, l1, 32, 9, rng)
@@ -149,6 +154,7 @@ def test_reduced_precision_with_index_lists_outside_the_king_slices():
     d["nstm"][::4, 1] = -1
     batch = tb.BatchData(d["stm"], d["nstm"], d["nnz"], d["score"], d["wdl"], d["bucket"])
     _check_step(tr, ot, batch, B, F, l1, mask, fs)
+    assert ft_path(tr, batch, tb.LossKind.sigmoid()) == ("both" if B > 3665 else "gather")
     tr.close()
 
 

@@ -15,7 +15,7 @@ import pytest
 
 import oracle_lib as O
 import tatara_b200 as tb
-from helpers import GOLDEN, assert_close, assert_close_scaled, random_index_batch
+from helpers import assert_close, assert_close_scaled, ft_path, GOLDEN, random_index_batch
 
 pytestmark = pytest.mark.gpu
 
@@ -479,10 +479,10 @@ def _sequential_ft_grad(stm, nstm, nnz, dft_stm, dft_nstm, N, F):
 
 @pytest.mark.parametrize("outside", [False, True])
 def test_ft_slice_backward_many_chunks_bit_exact(outside):
-    """King-sliced index lists with thousands of items in two slices: the slice-resident weight gradient walks several
-    chunks per slice and must reproduce the sequential sum bit for bit (lists of 256 entries or more: to rounding);
+    """King-sliced index lists with a thousand items and more in a few slices, one of them of both perspectives: the slice-resident
+    weight gradient walks several chunks per slice (up to the four of one group) and must reproduce the sequential sum bit for bit (lists of 256 entries or more: to rounding);
     with one row outside its item's slice the generic kernels take over and must do the same."""
-    F, l1, l2, B, A = 256, 8, 16, 2048, 40
+    F, l1, l2, B, A = 256, 8, 16, 3680, 40  # batches below 3680 positions take the gather kernels
     fs = LS_FS.with_factorize(False)
     pi, N = fs.piece_inputs, fs.ft_in
     rng = np.random.default_rng(11)
@@ -490,8 +490,8 @@ def test_ft_slice_backward_many_chunks_bit_exact(outside):
     init["ft_w"] *= 30.0
     d = random_index_batch(rng, B, A, pi, 25, A)
     hot = rng.integers(0, pi, 3)
-    for key, slices in (("stm", (3, 44)), ("nstm", (3, 17))):
-        k = np.asarray(slices)[rng.integers(0, 2, B)]
+    for key, slices in (("stm", (3, 44, 10, 30)), ("nstm", (3, 17, 25, 40))):
+        k = np.asarray(slices)[rng.integers(0, 4, B)]
         idx = d[key]
         idx[:, 1] = np.where(rng.random(B) < 0.9, hot[0], idx[:, 1])     # a row that nearly every item holds
         idx[:, 2] = np.where(rng.random(B) < 0.5, hot[1], idx[:, 2])
@@ -513,6 +513,7 @@ def test_ft_slice_backward_many_chunks_bit_exact(outside):
     assert short.sum() > 1000 and (~short).sum() >= 4
     assert np.array_equal(got[short].view(np.uint32), want[short].view(np.uint32))
     assert_close_scaled(got[~short], want[~short], 1e-6, "long lists")
+    assert ft_path(tr, batch, tb.LossKind.sigmoid()) == ("both" if outside else "slices")
 
 
 def test_config3_full_size_step_matches_oracle():
