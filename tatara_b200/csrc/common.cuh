@@ -9,10 +9,19 @@
 #define TB_MAX_L2 64
 #define TB_TILE_M 32      // positions per dense tile; a tile never mixes LayerStack buckets
 #define TB_UNIT_TILES 8   // most tiles of a work unit (consecutive tiles of one bucket)
+// SMs of the current device
+static inline int sm_count() {
+    int dev = 0, n = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n;
+}
 // Tiles per work unit for a batch: the dense kernels' blocks own half a unit and walk its positions one after the other, so a
 // batch that does not fill the chip with blocks of 128 positions gets smaller ones (B = 1024: the L1 input gradient took
 // 43 us on 16 of 148 SMs, 22 now).
-static inline int unit_tiles(int n_pos) { return n_pos >= 148 * 128 ? TB_UNIT_TILES : n_pos >= 148 * 64 ? 4 : 2; }
+static inline int unit_tiles(int n_pos) {
+    const int sms = sm_count();
+    return n_pos >= sms * 128 ? TB_UNIT_TILES : n_pos >= sms * 64 ? 4 : 2;
+}
 // The L1 weight gradient's work units have TB_UNIT_TILES tiles whatever the batch: a unit is one chain of its fp32 sums, whose order
 // is part of a step's results.
 // counts beside the tiles: {tiles, units, weight units, first weight unit of every bucket (and of the positions without one, and
@@ -72,12 +81,6 @@ struct SmallGroups {
 
 static __device__ __forceinline__ float crelu01(float x) { return x < 0.0f ? 0.0f : (x > 1.0f ? 1.0f : x); }
 
-// SMs of the current device
-static inline int sm_count() {
-    int dev = 0, n = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n;
-}
 static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 static inline int64_t ceil_div64(int64_t a, int64_t b) { return (a + b - 1) / b; }
 

@@ -691,7 +691,7 @@ int launch_tail_layerstack(cudaStream_t s, const float* l1_total, const int* buc
     if (l2 <= 32 && l2 % 4 == 0 && l2in <= 32 && wsmem <= 110 * 1024) {
         cudaFuncSetAttribute(k_tail_layerstack_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
         int blocks = ceil_div(B, 8);
-        if (blocks > 148 * 4) blocks = 148 * 4;
+        blocks = blocks < 4 * sm_count() ? blocks : 4 * sm_count();
         k_tail_layerstack_warp<<<blocks, 256, wsmem, s>>>(l1_total, bucket, score, wdl, l2_w, l2_b, l3_w, l3_b, lp, B, l1, l2, nb,
                                                         net_output, dy, dl1_total, l2_input, dl2_out, l2_acted, loss_partials,
                                                         backward);
@@ -839,7 +839,7 @@ int launch_tail_simple(cudaStream_t s, const float* l1_pre, const float* score, 
     const size_t smem = sizeof(float) * ((size_t)l1 * l2 + 2 * (size_t)l2);
     if (l1 <= 32 && l2 <= 32) {
         int blocks = ceil_div(B, 8);
-        if (blocks > 148 * 4) blocks = 148 * 4;
+        blocks = blocks < 4 * sm_count() ? blocks : 4 * sm_count();
         k_tail_simple_warp<<<blocks, 256, 0, s>>>(l1_pre, score, wdl, l2_w, l2_b, l3_w, l3_b, lp, act, B, l1, l2, net_output, dy,
                                                  dl1_pre, l1_acted, dl2_pre, l2_acted, loss_partials, backward);
         k_reduce_double<<<1, 256, 0, s>>>(loss_partials, blocks, loss_acc);
@@ -1250,7 +1250,7 @@ int launch_l1_wgrad(cudaStream_t s, const float* x, int K, const float* dl1, con
     } while (0)
         // 128-thread blocks at six per SM: with K = 1536 the 3 x 265 blocks of the benchmark then run as one wave
         // fewer units than SMs: more rounds in flight (1024 positions, K = 256, l1 = 16: 36 to 27 us; 16 384, K = 768, l1 = 8: 37 to 35)
-        const bool few = n_pos < WG_POS * 148;
+        const bool few = n_pos < WG_POS * sm_count();
         if (l1 == 8) { if (few) WGRAD(8, 128, 4, 6, true); else WGRAD(8, 128, 6, 2, true); }
         else if (l1 == 16) { if (few) WGRAD(16, 128, 3, 6, true); else WGRAD(16, 128, 6, 2, false); }
         else WGRAD(16, 256, 2, 4, true);

@@ -152,8 +152,7 @@ int launch_ft_forward(cudaStream_t s, int mode, const void* table, const int* id
     size_t smem = (size_t)ipc * (A + 1) * sizeof(int);
 #define FT_FWD_ARGS table, idx_stm, idx_nstm, nnz, bias, pre_stm, pre_nstm, combined, items, n_items, B, F, N, A, scale, ipc
     if (table_half) {
-        if (mode == 0 && !out_half) k_ft_forward<0, true, false><<<grid, block, smem, s>>>(FT_FWD_ARGS);
-        else if (mode == 1 && !out_half) k_ft_forward<1, true, false><<<grid, block, smem, s>>>(FT_FWD_ARGS);
+        if (mode == 1 && !out_half) k_ft_forward<1, true, false><<<grid, block, smem, s>>>(FT_FWD_ARGS);
         else if (mode == 1) k_ft_forward<1, true, true><<<grid, block, smem, s>>>(FT_FWD_ARGS);
         else return -1;
         return 1;
@@ -481,9 +480,8 @@ int launch_ft_forward_slice(cudaStream_t s, int mode, const void* table, const i
                                                                info, codes, wk, n_work, strips, B, F, N, A, A_pad, rps, \
                                                                scale);                                                   \
     } while (0)
-    if (table_half) {  // fp16 table: the raw gather (mode 0) and the LayerStack activation, with fp32 or fp16 pre-activations
-        if (mode == 0 && !out_half) FT_SLICE_LAUNCH(0, true, false);
-        else if (mode == 1 && !out_half) FT_SLICE_LAUNCH(1, true, false);
+    if (table_half) {  // fp16 table: the LayerStack activation, with fp32 or fp16 pre-activations
+        if (mode == 1 && !out_half) FT_SLICE_LAUNCH(1, true, false);
         else if (mode == 1) FT_SLICE_LAUNCH(1, true, true);
         else return -1;
     } else {
@@ -898,7 +896,7 @@ int launch_inverse_index(cudaStream_t s, const int* idx_stm, const int* idx_nstm
     int2* work = reinterpret_cast<int2*>(plan);
     int* split = plan + 2 * (size_t)ft_backward_max_work(B, A, n_persp);
     cudaMemsetAsync(counts, 0, sizeof(int) * ((size_t)2 * N + INV_COUNTERS), s);
-    const dim3 grid((unsigned)min(ceil_div(cells, 256), 148 * 16), n_persp);
+    const dim3 grid((unsigned)min(ceil_div(cells, 256), sm_count() * 16), n_persp);
     k_feat_count<<<grid, 256, 0, s>>>(idx_stm, idx_nstm, nnz, cells, A, N, counts, scratch);
     k_feat_scan<<<dim3(ceil_div(N, SCAN_CELLS), n_persp), 1024, 0, s>>>(counts, N, n_persp, BWD_SORT_CELLS / bwd_rows_per_warp(B, A, N),
                                                                         offsets, counters, long_queue, work, split);
@@ -907,7 +905,7 @@ int launch_inverse_index(cudaStream_t s, const int* idx_stm, const int* idx_nstm
     if ((size_t)words * 4 > 160 * 1024) words = 0;
     // per device and cheap: set before every launch (a process may drive several GPUs)
     cudaFuncSetAttribute(k_lists_sort_long, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-    k_lists_sort_long<<<148 * 4, 256, (size_t)words * 4, s>>>(counts, offsets, N, cells, lists, scratch, long_queue,
+    k_lists_sort_long<<<sm_count() * 4, 256, (size_t)words * 4, s>>>(counts, offsets, N, cells, lists, scratch, long_queue,
                                                               counters + INV_QUEUED, words);
     return 4;
 }
@@ -995,7 +993,7 @@ __global__ void k_cast_half(const float4* __restrict__ src, uint2* __restrict__ 
 int launch_cast_half(cudaStream_t s, const float* src, void* dst, int64_t n) {
     const long long n4 = n / 4;
     long long blocks = (n4 + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
+    blocks = blocks < 16 * sm_count() ? blocks : 16 * sm_count();
     if (blocks < 1) blocks = 1;
     k_cast_half<<<(int)blocks, 256, 0, s>>>(reinterpret_cast<const float4*>(src), static_cast<uint2*>(dst), n4);
     return 1;

@@ -497,7 +497,7 @@ int launch_ft_backward_slice(cudaStream_t s, const void* dft_stm, const void* df
     if (dft_half) FT_BWD_LAUNCH(true); else FT_BWD_LAUNCH(false);
 #undef FT_BWD_LAUNCH
     const int k0 = (int)((int64_t)n_slices * part / parts), k1 = (int)((int64_t)n_slices * (part + 1) / parts);
-    k_bwd_combine<<<dim3(148, k1 - k0), 256, 0, s>>>(P.groups, sb.outside_flag, reinterpret_cast<const float4*>(slabs),
+    k_bwd_combine<<<dim3(sm_count(), k1 - k0), 256, 0, s>>>(P.groups, sb.outside_flag, reinterpret_cast<const float4*>(slabs),
                                                      reinterpret_cast<float4*>(grad), rps, F, N, k0);
     return 2;
 }

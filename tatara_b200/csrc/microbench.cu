@@ -34,7 +34,7 @@ struct Timer {
     cudaError_t run(int iters, Fn fn) {
         total = 0.0;
         for (int i = -1; i < iters; ++i) {  // iteration -1 is the warm-up
-            if (flush) k_flush<<<148 * 8, 256>>>(reinterpret_cast<float4*>(flush), flush_floats / 4);
+            if (flush) k_flush<<<sm_count() * 8, 256>>>(reinterpret_cast<float4*>(flush), flush_floats / 4);
             cudaEventRecord(e0, 0);
             fn();
             cudaEventRecord(e1, 0);
@@ -82,8 +82,8 @@ extern "C" int tb_ft_microbench(int device, const int32_t* indices, const int32_
     MB(cudaMalloc(&d_lists, 4 * B * A * 4)); MB(cudaMalloc(&d_plan, (2 * max_work + 3 * N) * 4)); MB(cudaMalloc(&d_part, max_work * F * 4));
     MB(cudaMemcpy(d_idx, indices, B * A * 4, cudaMemcpyHostToDevice));
     MB(cudaMemcpy(d_nnz, nnz, B * 4, cudaMemcpyHostToDevice));
-    k_fill_pattern<<<148 * 8, 256>>>(d_table, N * F, 0.05f, 1u);
-    k_fill_pattern<<<148 * 8, 256>>>(d_m, N * F, 1e-4f, 2u);
+    k_fill_pattern<<<sm_count() * 8, 256>>>(d_table, N * F, 0.05f, 1u);
+    k_fill_pattern<<<sm_count() * 8, 256>>>(d_m, N * F, 1e-4f, 2u);
     MB(cudaMemset(d_v, 0, N * F * 4));
     if (flush_l2) {
         tm.flush_floats = (size_t)64 << 20;  // 256 MB, twice the L2
@@ -96,7 +96,7 @@ extern "C" int tb_ft_microbench(int device, const int32_t* indices, const int32_
     // generic path: L2-gather forward, global inverse index + per-row sums
     MB(tm.run(iters, [&] { launch_ft_forward(0, 0, d_table, d_idx, d_idx, d_nnz, nullptr, d_x, d_x, nullptr, nullptr, batch, ft_out, ft_in, max_active, 1.f, 1); }));
     out->fwd_ms = (float)(tm.total / iters);
-    k_fill_pattern<<<148 * 8, 256>>>(d_x, B * F, 1e-3f, 3u);  // the incoming gradient rows
+    k_fill_pattern<<<sm_count() * 8, 256>>>(d_x, B * F, 1e-3f, 3u);  // the incoming gradient rows
     MB(tm.run(iters, [&] {
         launch_inverse_index(0, d_idx, d_idx, d_nnz, batch, max_active, ft_in, 1, d_cnt, d_off, d_lists, d_plan);
         launch_ft_backward_split(0, d_x, d_x, d_cnt, d_off, d_lists, batch, max_active, ft_in, ft_out, 1, d_plan, d_part, d_grad);
@@ -116,7 +116,7 @@ extern "C" int tb_ft_microbench(int device, const int32_t* indices, const int32_
         MB(cudaMalloc(&d_fwd_work, ft_forward_slice_work_ints(batch, n_keys, max_active) * 4));
         MB(cudaMalloc(&d_bwd_work, ft_backward_slice_ints(batch, max_active, rps) * 4));
         MB(cudaMalloc(&d_slabs, ft_backward_slice_slab_floats(batch, max_active, rps, ft_out) * 4));
-        k_fill_pattern<<<148 * 8, 256>>>(d_table, N * F, 0.05f, 1u);
+        k_fill_pattern<<<sm_count() * 8, 256>>>(d_table, N * F, 0.05f, 1u);
         MB(tm.run(iters, [&] {
             launch_step_sorts(0, nullptr, batch, 0, d_order, d_tiles, d_ntiles, d_seg, max_tiles, d_idx, d_idx, d_nnz, max_active, ft_in, rps, 1,
                               d_items, d_itemseg, d_hist, d_fwd_work, d_bwd_work);
@@ -127,7 +127,7 @@ extern "C" int tb_ft_microbench(int device, const int32_t* indices, const int32_
         MB(cudaMemcpy(&outside, ft_slice_outside_flag(d_fwd_work, batch, ft_in, rps), 4, cudaMemcpyDeviceToHost));
         if (!outside) {
             out->fwd_slice_ms = (float)(tm.total / iters);
-            k_fill_pattern<<<148 * 8, 256>>>(d_x, B * F, 1e-3f, 3u);
+            k_fill_pattern<<<sm_count() * 8, 256>>>(d_x, B * F, 1e-3f, 3u);
             MB(tm.run(iters, [&] {
                 launch_inverse_slice(0, d_itemseg, d_fwd_work, d_bwd_work, batch, max_active, ft_in, rps, 1);
                 launch_ft_backward_slice(0, d_x, d_x, d_fwd_work, d_bwd_work, batch, max_active, ft_in, ft_out, rps, 1, 0, 1, d_grad, d_slabs);

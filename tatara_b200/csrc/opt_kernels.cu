@@ -31,7 +31,8 @@ int launch_radam(cudaStream_t s, float* w, void* m, void* v, const float* g, flo
                  void* mirror) {
     const long long n4 = n / 4;
     long long blocks = (n4 + 255) / 256;
-    if (blocks > 148 * 32) blocks = 148 * 32;
+    const long long most = 32 * sm_count();
+    if (blocks > most) blocks = most;
     if (blocks < 1) blocks = 1;
     if (half_state)
         k_radam<true><<<(int)blocks, 256, 0, s>>>(reinterpret_cast<float4*>(w), m, v, reinterpret_cast<const float4*>(g),

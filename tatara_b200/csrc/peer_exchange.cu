@@ -325,7 +325,7 @@ int px_exchange_part(PeerExchange* x, int part, int64_t e0, int64_t e1, bool wit
         SrcList src;
         for (int q = 0; q < G; ++q) src.p[q] = q == r ? x->arena + m0 : x->recv_window(x->block, q) + m0;
         const size_t n4 = (size_t)(m1 - m0) / 4;
-        const int blocks = (int)((n4 + 255) / 256 < 148 * 4 ? (n4 + 255) / 256 : 148 * 4);
+        const int blocks = (int)((n4 + 255) / 256 < 4 * sm_count() ? (n4 + 255) / 256 : 4 * sm_count());
         k_px_reduce<<<blocks, 256, 0, reduce_stream>>>(reinterpret_cast<float4*>(x->arena + m0), src, G, n4);
         *launches += 1;
     }

@@ -401,15 +401,15 @@ int launch_slice_check(cudaStream_t s, const int* idx_stm, const int* idx_nstm, 
                        int* outside) {
     if (B <= 0) return 0;
     const int blocks = ceil_div(B, 8);
-    k_slice_check<<<blocks < 148 * 8 ? blocks : 148 * 8, 256, 0, s>>>(idx_stm, idx_nstm, nnz, B, A, N, rows_per_slice, outside);
+    k_slice_check<<<blocks < 8 * sm_count() ? blocks : 8 * sm_count(), 256, 0, s>>>(idx_stm, idx_nstm, nnz, B, A, N, rows_per_slice, outside);
     return 1;
 }
 
 int sort_weight_units(int n_pos) { return n_pos / (TB_UNIT_TILES * TB_TILE_M) + TB_MAX_BUCKETS + 2; }
 int sort_units(int n_pos) { return n_pos / (unit_tiles(n_pos) * TB_TILE_M) + TB_MAX_BUCKETS + 2; }
-// at least the 148 units of the largest batches with smaller ones
+// at least a unit per SM: batches with smaller units have no more (unit_tiles)
 int sort_max_units(int max_tiles) {
-    const int n = max_tiles / TB_UNIT_TILES > 148 ? max_tiles / TB_UNIT_TILES : 148;
+    const int sms = sm_count(), n = max_tiles / TB_UNIT_TILES > sms ? max_tiles / TB_UNIT_TILES : sms;
     return n + TB_MAX_BUCKETS + 2;
 }
 

@@ -30,7 +30,7 @@
 #define RANGER_K 6
 #define N_SMA_THRESHOLD 5.0f
 #define FT_DFT_FP16_BASE_SCALE 16384.0f  // arch.rs:72-93: the fp16 dft rows carry gradient * 2^14 * batch
-#define DGRAD_CTAS (148 * 2)
+#define DGRAD_CTAS 296  // chains of the general L1 input gradient's FT bias sums, at least: part of their order, whatever the chip
 #define AR_PARTS_MAX 6
 #define PEER_DEADLINE_S 120  // peer exchange: longest wait for a step before the peers are given up
 // Number of launches the FT weight gradient is cut into in data-parallel runs (each part's all-reduce and row updates
@@ -1134,7 +1134,7 @@ int create_impl(tb_trainer* t) {
     CU(t, dalloc(&t->net_output, B)); CU(t, dalloc(&t->dy, B));
     CU(t, dalloc(&t->tail_a, B * (size_t)(ls ? t->l2in : l1)));
     CU(t, dalloc(&t->tail_b, B * l2)); CU(t, dalloc(&t->tail_c, B * l2));
-    CU(t, dalloc(&t->loss_partials, B / 128 + 1024)); CU(t, dalloc(&t->loss_acc, 1));  // one partial per tail block (<= 148 * 4 or B / 128)
+    CU(t, dalloc(&t->loss_partials, B / 128 + 1024)); CU(t, dalloc(&t->loss_acc, 1));  // one partial per tail block (<= 640 or 4 per SM or B / 128)
     CU(t, dalloc(&t->wrm_weight_sum, 1));
     t->max_tiles = (int)(B / TB_TILE_M) + TB_MAX_BUCKETS + 2;
     t->max_units = sort_max_units(t->max_tiles);
