@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(64) k_l1_forward_tiled(const float* __restrict
 // reads both operands as 128-bit rows along k; the row stride spreads the rows a quarter warp touches over the banks.
 // What bounds it is the shared-memory pipe, and a block's latency where the batch is small.  65 536 positions, K = 1536, l1 = 16:
 // 114 us (the x rows at HBM rate take 62), 128 with scalar multiply-adds and four positions a thread; K = 512, l1 = 32: 72;
-// 16 384, K = 768, l1 = 8: 21, from 60; 10 000, K = 1024, l1 = 32: 46.  (The columns of a chunk shared by a block's warps and packed
+// 16 384, K = 768, l1 = 8: 21, from 60; 10 000, K = 1024, l1 = 32: 40.  (The columns of a chunk shared by a block's warps and packed
 // pairs of columns, another order: 114, 83, 21, 38.)
 // ------------------------------------------------------------------------------------------------
 __global__ void k_l1_weff(const float* __restrict__ wb, const float* __restrict__ bb, const float* __restrict__ ws,
@@ -415,13 +415,13 @@ int launch_l1_forward(cudaStream_t s, const float* x, int K, const int* order, c
                                                                                           y, nbe);                          \
     } while (0)
         // Full batches: many outputs per thread, short chunks, many blocks (K = 1536, l1 = 16: 114 us, the small batches' shape 162;
-        // l1 = 32, K = 512: 70 against 97).  Batches that do not fill the chip: a chain's latency is what counts, so fewer
+        // l1 = 32, K = 512: 70).  Batches that do not fill the chip: a chain's latency is what counts, so fewer
         // outputs per thread and longer chunks (1024 positions, l1 = 16, K = 256: 10.5 us, the large batches' shape 14.4; 10 000, l1 = 32,
-        // K = 1024: 46 for either).
+        // K = 1024: 40.5, 45.7).
         const int ut = unit_tiles(n_pos);
         if (l1 == 8) { if (ut == TB_UNIT_TILES) L1F(8, 1, 8, 2, 16, 3); else L1F(8, 1, 4, 4, 64, 3); }
         else if (l1 == 16) { if (ut == TB_UNIT_TILES) L1F(16, 2, 8, 2, 16, 3); else L1F(16, 2, 2, 4, 32, 3); }
-        else { if (ut > 2) L1F(32, 4, 8, 2, 32, 3); else L1F(32, 2, 4, 4, 32, 3); }
+        else { if (ut == TB_UNIT_TILES) L1F(32, 4, 8, 2, 32, 3); else L1F(32, 4, 4, 2, 64, 3); }
 #undef L1F
         return 1;
     }
