@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, MIN_BLOCKS) k_radam_factorized
             for (int u = 0; u < FACT_ROWS; ++u, ++kb) {
                 if (kb >= KB) break;
                 float x = col[(u * 32 * MAX_WARPS + 32 * q) * 4];
-                if (HC) x *= sc.grad_scale;  // loss-scaled sums exist only next to an fp16 table
+                if (HC) x = __fmul_rn(x, sc.grad_scale);  // loss-scaled sums exist only next to an fp16 table
                 sum += x;
             }
         reinterpret_cast<float*>(s_virt)[c] = sum;

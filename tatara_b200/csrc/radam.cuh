@@ -1,5 +1,5 @@
 // The optimizer's arithmetic on four adjacent parameters (radam_step, native_kernels.cu:1291; pointwise/radam_step.rs:116-156),
-// shared by the optimizer kernels and the FT weight gradient that applies it to the rows it has just summed.
+// for the kernels of opt_kernels.cu.
 #pragma once
 #include "common.cuh"
 
@@ -43,7 +43,10 @@ static __device__ __forceinline__ void store_moment(void* base, size_t i4, float
         if (streaming) __stcs(p, val); else *p = val;
     }
 }
-static __device__ __forceinline__ float4 scale4(float4 g, float k) { return make_float4(g.x * k, g.y * k, g.z * k, g.w * k); }
+// rounded before it is added to anything (see radam_one)
+static __device__ __forceinline__ float4 scale4(float4 g, float k) {
+    return make_float4(__fmul_rn(g.x, k), __fmul_rn(g.y, k), __fmul_rn(g.z, k), __fmul_rn(g.w, k));
+}
 
 // Of a sum of two products one is rounded before it is added.  Which one is part of the results (AdamW's first steps turn a last bit
 // into a visible difference after a few steps), so it is written out for every kernel and not left to the compiler, which chose

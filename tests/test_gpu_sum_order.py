@@ -19,17 +19,20 @@ def _same_bits(got, want, what):
     assert bad.size == 0, "%s: %d of %d differ, first %d: %r, want %r" % (what, bad.size, got.size, bad[0], got[bad[0]], want[bad[0]])
 
 
-@pytest.mark.parametrize("kb", [1, 9, 10, 16, 45, 46, 81, 82])
-def test_virtual_row_gradient_is_one_chain_over_the_king_buckets(kb):
-    """The fused kernel up to 81 king buckets, the two data-parallel ones above."""
+@pytest.mark.parametrize("kb,half", [(1, False), (9, False), (10, False), (16, False), (45, False), (46, False), (81, False), (82, False),
+                                     (45, True), (82, True)])
+def test_virtual_row_gradient_is_one_chain_over_the_king_buckets(kb, half):
+    """The fused kernel up to 81 king buckets, the two data-parallel ones above.  half: gradient rows that carry a loss scale, here
+    no power of two, which is taken out of every term, rounded, before it is added."""
     fs = tb.FeatureSetSpec("test", 4, kb, 24, 8, True)
-    F, l1, l2, B = 256, 8, 16, 512
+    F, l1, l2, B = 256, 8, 16, 496
     rng = np.random.default_rng(kb)
     init = _perturb(tb.layerstack_default_init(fs, F, l1, l2, 9), rng, ["ft_w", "ft_b", "l1_b", "l1_shared_bias", "l2_b", "l3_b"])
     d = random_index_batch(rng, B, fs.max_active, fs.piece_inputs, 1, fs.max_active)
     for key in ("stm", "nstm"):
         d[key] = np.where(d[key] >= 0, d[key] + rng.integers(0, kb, B)[:, None] * fs.piece_inputs, d[key]).astype(np.int32)
-    tr = tb.GpuTrainer(B, F, l1, l2, 9, fs, optimizer="adamw", init=init)
+    precision = tb.PrecisionFlags(ft_fp16=half, ft_fp16_out=half)
+    tr = tb.GpuTrainer(B, F, l1, l2, 9, fs, optimizer="adamw", precision=precision, init=init)
     tr.forward_backward(tb.BatchData(d["stm"], d["nstm"], d["nnz"], d["score"], d["wdl"], d["bucket"]), 0.0, tb.LossKind.sigmoid())
     tr.apply_optimizer(1e-3)
     g = tr.download_grad("ft_w").reshape(kb + 1, -1)
@@ -37,6 +40,8 @@ def test_virtual_row_gradient_is_one_chain_over_the_king_buckets(kb):
     for k in range(kb):
         want += g[k]
     assert np.count_nonzero(want) > want.size // 2
+    if half:  # downloaded gradients have the loss scale taken out, of the virtual rows once more
+        want *= np.float32(1) / (np.float32(16384) * np.float32(B))
     _same_bits(g[kb], want, "virtual rows")
 
 
