@@ -58,8 +58,8 @@ SMEM_BYTES_PER_CLK_PER_SM = 128.0
 # cfg3 at B = 65 536, fp32, on one GPU (its summary is the launch-list file under profiles/).  Reported only for that
 # exact case; any other batch, precision or GPU count prints null.
 NCU_TRAFFIC_BYTES = {
-    ("cfg3", "ft_backward"): 1635.0e6, ("cfg3", "ft_forward"): 1750.2e6, ("cfg3", "opt_ft"): 4232.5e6,
-    ("cfg3", "l1_dgrad_ftgrad"): 1583.3e6, ("cfg3", "l1_forward"): 404.8e6, ("cfg3", "l1_wgrad"): 411.2e6,
+    ("cfg3", "ft_backward"): 1232.3e6, ("cfg3", "ft_forward"): 1615.3e6, ("cfg3", "opt_ft"): 3874.5e6,
+    ("cfg3", "l1_dgrad_ftgrad"): 1582.9e6, ("cfg3", "l1_forward"): 404.8e6, ("cfg3", "l1_wgrad"): 411.3e6,
 }
 MICRO_F = (256, 768, 1536, 3072)
 MICRO_B = (4096, 16384, 65536, 262144)
