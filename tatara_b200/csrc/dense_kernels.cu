@@ -415,13 +415,14 @@ int launch_l1_forward(cudaStream_t s, const float* x, int K, const int* order, c
                                                                                           y, nbe);                          \
     } while (0)
         // Full batches: many outputs per thread, short chunks, many blocks (K = 1536, l1 = 16: 114 us, the small batches' shape 162;
-        // l1 = 32, K = 512: 70).  Batches that do not fill the chip: a chain's latency is what counts, so fewer
-        // outputs per thread and longer chunks (1024 positions, l1 = 16, K = 256: 10.5 us, the large batches' shape 14.4; 10 000, l1 = 32,
-        // K = 1024: 40.5, 45.7).
+        // l1 = 32, K = 512: 70).  Batches that do not fill the chip: a chain's latency is what counts, so fewer outputs per thread
+        // and longer chunks (1024 positions, l1 = 16, K = 256: 10.5 us, the large batches' shape 14.4; 10 000, l1 = 32, K = 1024: 40,
+        // 46; 608, l1 = 32, K = 2816: 51, and 62 with the shape for 10 000; 4096, l1 = 8, K = 1536: 22, 29 with
+        // four outputs a thread).
         const int ut = unit_tiles(n_pos);
-        if (l1 == 8) { if (ut == TB_UNIT_TILES) L1F(8, 1, 8, 2, 16, 3); else L1F(8, 1, 4, 4, 64, 3); }
-        else if (l1 == 16) { if (ut == TB_UNIT_TILES) L1F(16, 2, 8, 2, 16, 3); else L1F(16, 2, 2, 4, 32, 3); }
-        else { if (ut == TB_UNIT_TILES) L1F(32, 4, 8, 2, 32, 3); else L1F(32, 4, 4, 2, 64, 3); }
+        if (l1 == 8) { if (ut == TB_UNIT_TILES) L1F(8, 1, 8, 2, 16, 3); else if (ut > 2) L1F(8, 1, 4, 4, 64, 3); else L1F(8, 1, 2, 4, 64, 4); }
+        else if (l1 == 16) { if (ut == TB_UNIT_TILES) L1F(16, 2, 8, 2, 16, 3); else L1F(16, 2, 2, 4, 64, 3); }
+        else { if (ut == TB_UNIT_TILES) L1F(32, 4, 8, 2, 32, 3); else if (ut > 2) L1F(32, 4, 4, 2, 64, 3); else L1F(32, 4, 2, 4, 64, 3); }
 #undef L1F
         return 1;
     }

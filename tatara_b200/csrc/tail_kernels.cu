@@ -330,12 +330,12 @@ int launch_tail(cudaStream_t s, int arch, int n_pos, const float* l1_rows, const
     } while (0)
     // Threads for the positions of an average run.  A warp for up to 32 (16 384 positions of a LayerStack net: 19.4 us, 21.5 with
     // two, 24 with four); for a few positions two, since what is left is the bucket's weights coming in (1024 positions: 25.4 to
-    // 23.0).  A Simple net's full batch, runs of 512, in rounds of 256: 46 us against 52 with 128.
+    // 23.0).  Up to 56 two: with four a LayerStack net's blocks take a second wave (23 312 positions: 30.6 to 22.8).  A Simple net's full batch, runs of 512, in rounds of 256: 46 us against 52 with 128.
     const int run = n_pos / blocks;
 #define TAIL_T(A, L1, L2)                                                                                                         \
     do {                                                                                                                          \
-        if (run <= 8 || (A == 0 && L1 == 32 && run <= 64)) TAIL_LAUNCH(A, L1, L2, 64);                                            \
-        else if (run <= 32) TAIL_LAUNCH(A, L1, L2, 32);                                                                           \
+        if (run > 8 && run <= 32 && !(A == 0 && L1 == 32)) TAIL_LAUNCH(A, L1, L2, (A == 0 && L1 == 32 ? 64 : 32));                \
+        else if (run <= 56) TAIL_LAUNCH(A, L1, L2, 64);                                                                           \
         else if (A == 0 || run <= 128) TAIL_LAUNCH(A, L1, L2, 128);                                                               \
         else TAIL_LAUNCH(A, L1, L2, (A == 0 ? 128 : 256));                                                                        \
     } while (0)

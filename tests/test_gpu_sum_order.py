@@ -113,8 +113,9 @@ def _segments(batch, B, nb):
 
 
 @pytest.mark.parametrize("arch,l1,l2,B,act", [
-    # blocks of 64, 32 and 128 threads; l1 = 32 also 64 for longer runs
+    # blocks of 64, 32, 64 and 128 threads; l1 = 32: 64 and 128
     ("layerstack", 8, 16, 16, ""), ("layerstack", 16, 32, 1040, ""), ("layerstack", 16, 32, 8208, ""), ("layerstack", 16, 16, 21136, ""),
+    ("layerstack", 8, 16, 36496, ""),
     ("layerstack", 32, 32, 400, ""), ("layerstack", 32, 16, 8208, ""), ("layerstack", 32, 32, 41616, ""),
     # blocks of 64, 32, 128 and 256 threads, the last one in one and in two rounds
     ("simple", 8, 32, 16, "crelu"), ("simple", 32, 32, 4112, "crelu"), ("simple", 16, 16, 16400, "screlu"),
